@@ -55,13 +55,18 @@ FLUSH_BYTES = 256 << 20
 
 
 
+HIST_VARIANT = 16  # the distance histogram: every pair once, whatever the number of q
+
+
 def _variant_name(v: int) -> str:
-    """Autotuner variant code Q*16 + jb; jb >= 8 is the q-packed kernel with (jb-8) % 4 chains,
+    """Autotuner variant code: 16 is the distance histogram, else Q*16 + jb; jb >= 8 is the q-packed kernel with (jb-8) % 4 chains,
     jb >= 12 its build for three CTAs per SM; jb 5, 6, 7, 3 the q-packed kernel with the weight
     folded into the recurrence (1 chain / 2 CTAs, 2 / 2, 1 / 3, 1 / 4); jb 11 the folded kernel with
     two chains per pair (q points 4n, 4n+1 and 4n+2, 4n+3); jb 14, 15 the folded
     recurrence with the set-up in its own warpgroup (1 or 2 chains per recurrence thread), jb 12
     the same with one recurrence warpgroup per q block, three blocks per work item."""
+    if int(v) == HIST_VARIANT:
+        return "distance-histogram"
     q, jb = int(v) // 16, int(v) % 16
     if jb in (14, 15):
         return f"Q{q}xJ{jb - 13}-split"
@@ -731,7 +736,11 @@ def run_ours(args, rank, world, local):
     ms_per_step = 1e3 * max_s / args.steps
     # roofline of this rank's kernel: its share of the kernel-evaluated pair·q (the
     # shards' items are near equal in cost) over its kernel time
-    achieved = 4.0 * kernel_pairq / world / (float(step_ms.mean()) * 1e-3) / 1e12
+    if chosen.value == HIST_VARIANT:  # per pair, not per pair·q: 23 FP32 operations and one MUFU root
+        units, flop_per_unit = kernel_pairq / len(Q), 23
+    else:
+        units, flop_per_unit = kernel_pairq, 4
+    achieved = flop_per_unit * units / world / (float(step_ms.mean()) * 1e-3) / 1e12
 
     # accuracy of this curve against the FP64 device reference (outside the timed region)
     import crabsaxs_b200.synth as synth
@@ -846,9 +855,9 @@ def run_ours(args, rank, world, local):
                        "l2": "flushed before every step (256 MiB memset, outside the step events)"},
             "roofline": {"bound": "fp32", "achieved": achieved, "peak": peak.value, "unit": "TFLOP/s",
                          "frac": achieved / peak.value, "traffic": traffic_per_launch(),
-                         "units_per_launch": kernel_pairq,
+                         "units_per_launch": units,
                          "peak_source": "FFMA microbenchmark measured in this run (MEASURED_PEAKS.json has no FP32)",
-                         "flop_per_unit": 4},
+                         "flop_per_unit": flop_per_unit},
             "kernel_evaluated": {"value": kernel_pairq * args.steps / max_s, "unit": UNIT,
                                  "note": "value without the site-site pair.q, which the exact lattice histogram "
                                          "sums instead of the pair kernel"},

@@ -1,4 +1,7 @@
-// Debye pair sums per atom-type pair on B200 (sm_100a).
+// Debye pair sums per atom-type pair on B200 (sm_100a): plans, and the kernels
+// that sum every pair at every q.  One-structure plans use the distance
+// histogram of debye_hist.cu where its bins fit; the recurrence kernels here
+// serve ensemble plans, wider ranges and the variants a caller selects.
 //
 // Replaces the O(N²·Nq) pair loops of crabSAXS src/scattering.rs:99-106 and
 // src/solvent.rs:533-577.  Instead of summing amplitude products per q, the
@@ -1353,6 +1356,9 @@ int2 default_variant(const std::vector<double>& q) {
 
 // (Re)build the q blocks and the work list of an FP32 plan for block length Q.
 void configure_fp32(crab_ctx* ctx, PairPlan& P, int Q, int jb) {
+  P.hist.active = false;
+  if (!P.d_atoms)
+    P.d_atoms = upload(ctx, P, P.owned, "atoms", (const float4*)P.L.atoms.data(), (size_t)P.L.n_pad, ctx->stream);
   P.jb = jb;
   for (void* p : P.qcfg) cudaFree(p);
   P.qcfg.clear();
@@ -1421,6 +1427,30 @@ void configure_fp32(crab_ctx* ctx, PairPlan& P, int Q, int jb) {
   P.d_qrange = upload(ctx, P, P.qcfg, "qrange", qrange.data(), qrange.size(), ctx->stream);
 }
 
+// Kernel variant `v` (Q*16 + jb, or kHistVariant) for a plan; false where the
+// histogram does not fit.
+bool pair_plan_use(crab_ctx* ctx, PairPlan& P, int v) {
+  if (v != kHistVariant) {
+    configure_fp32(ctx, P, v / 16, v % 16);
+    return true;
+  }
+  if (P.hist.d_pts) P.hist.active = true;
+  return P.hist.active || hist_plan_init(ctx, P);
+}
+
+// The FP32 form of a new plan: the context's variant if one is set, else the
+// distance histogram, else the recurrence, which has no bins to hold: where
+// q_max times the largest distance is over 168 the histogram of one class pair
+// would not fit an SM's shared memory (debye_hist.cu).  There is no size below
+// which the recurrence is the better one; kernels of one call, histogram
+// against the best recurrence variant: 20 atoms, 20 q 30 / 31 us; 300 atoms of
+// 14 classes, 101 q 33 / 60 us; 1,000 atoms, 100 q 37 / 72 us; 20,000 atoms of
+// four, 100 q 0.23 / 2.7 ms, 500 q 0.23 / 11.3 ms.
+void configure_auto(crab_ctx* ctx, PairPlan& P) {
+  const int2 v = default_variant(P.q);
+  if (!pair_plan_use(ctx, P, ctx->pair_variant ? ctx->pair_variant : kHistVariant)) configure_fp32(ctx, P, v.x, v.y);
+}
+
 std::unique_ptr<PairPlan> make_pair_plan(crab_ctx* ctx, Layout&& L, const double* q, int64_t nq, bool fp64,
                                          const LatticeSpec* lattice, bool pooled, int shard, int n_shards) {
   require(n_shards >= 1 && shard >= 0 && shard < n_shards, "shard index out of range");
@@ -1446,10 +1476,8 @@ std::unique_ptr<PairPlan> make_pair_plan(crab_ctx* ctx, Layout&& L, const double
     P->lattice_first_tile = first;
   }
   if (!fp64) {
-    P->d_atoms = upload(ctx, *P, P->owned, "atoms", (const float4*)P->L.atoms.data(), (size_t)P->L.n_pad, s);
-    const int2 v = ctx->pair_variant ? make_int2(ctx->pair_variant / 16, ctx->pair_variant % 16)
-                                      : default_variant(P->q);
-    configure_fp32(ctx, *P, v.x, v.y);
+    P->skip_last = lattice != nullptr;
+    configure_auto(ctx, *P);
   } else {
     P->n_qblocks = (int)((nq + kQD - 1) / kQD);
     const std::vector<int4> work = shard_work(make_work(P->L, P->n_qblocks, 8, P->L.n_tiles), shard, n_shards);
@@ -1490,6 +1518,7 @@ std::unique_ptr<PairPlan> make_batch_pair_plan(crab_ctx* ctx, std::vector<Layout
     L.tile_type.insert(L.tile_type.end(), part.tile_type.begin(), part.tile_type.end());
     L.extent = std::max(L.extent, part.extent);
     P->segments.push_back(L.n_tiles);
+    P->seg_extent.push_back(part.extent);
   }
   P->fp64 = false;
   P->nq = nq;
@@ -1498,10 +1527,12 @@ std::unique_ptr<PairPlan> make_batch_pair_plan(crab_ctx* ctx, std::vector<Layout
   P->lattice_first_tile = L.n_tiles;
   cudaStream_t s = ctx->stream;
   if (nq == 0 || L.n_tiles == 0) return P;
-  P->d_atoms = upload(ctx, *P, P->owned, "atoms", (const float4*)L.atoms.data(), (size_t)L.n_pad, s);
-  const int2 v = ctx->pair_variant ? make_int2(ctx->pair_variant / 16, ctx->pair_variant % 16)
-                                    : default_variant(P->q);
-  configure_fp32(ctx, *P, v.x, v.y);
+  // the recurrence unless the context or the autotuner says otherwise: the
+  // ensemble's weight fit takes fixed-length steps and ends on a cycle around
+  // its minimum, where the last bits of a curve decide which iterate is the
+  // last one, so a plan keeps the bits that it always had
+  const int2 v = default_variant(P->q);
+  if (!ctx->pair_variant || !pair_plan_use(ctx, *P, ctx->pair_variant)) configure_fp32(ctx, *P, v.x, v.y);
   P->d_tile_type = upload(ctx, *P, P->owned, "tile_type", L.tile_type.data(), L.tile_type.size(), s);
   P->d_out = upload<double>(ctx, *P, P->owned, "out", nullptr, (size_t)(P->segments.size() - 1) * P->n_pairs * nq, s);
   P->d_status = upload<int>(ctx, *P, P->owned, "status", nullptr, 2, s);
@@ -1523,6 +1554,8 @@ void pair_plan_launch(crab_ctx* ctx, PairPlan& P, cudaStream_t s, bool timed) {
     const int grid = std::max(1, std::min(P.n_work, ctx->sm_count * std::max(per_sm, 1)));
     k_pair_fp64<<<grid, kThreads, 0, s>>>(P.d_atoms64, P.d_tile_type, P.d_work, P.n_work, P.d_q, nq, T, P.d_out);
     CRAB_CUDA_CHECK(cudaGetLastError());
+  } else if (P.hist.active) {
+    hist_plan_launch(ctx, P, s);
   } else {
 #define CRAB_LAUNCH(QQ, JJ)                                                                                    \
   if (P.Q == QQ && P.jb == JJ) {                                                                                 \
@@ -1612,7 +1645,7 @@ void pair_plan_launch(crab_ctx* ctx, PairPlan& P, cudaStream_t s, bool timed) {
 #undef CRAB_LAUNCH_SPLIT3
     if (!launched) throw Error(CRAB_EINVAL, "unsupported q block");
   }
-  ctx->launches += 1;
+  if (!P.hist.active) ctx->launches += 1;
   if (P.lattice.active) lattice_plan_launch(ctx, P, s);
   if (timed) CRAB_CUDA_CHECK(cudaEventRecord(ctx->ev_stop, s));
 }
@@ -1757,24 +1790,23 @@ static const int kLaunchable[][2] = {{8, 2},   {16, 2}, {32, 2}, {48, 2}, {64, 2
 
 bool pair_variant_known(int variant) {
   const int Q = variant / 16, jb = variant % 16;
-  bool known = false;
+  bool known = variant == kHistVariant;
   for (const auto& v : kLaunchable) known = known || (v[0] == Q && v[1] == jb);
   return known;
 }
 
 void pair_plan_select(crab_ctx* ctx, PairPlan& P, int variant) {
   require(!P.fp64, "the FP64 plan has a single kernel");
-  const int Q = variant / 16, jb = variant % 16;
   require(pair_variant_known(variant), "unknown kernel variant " + std::to_string(variant));
   if (P.nq == 0 || P.L.n_tiles == 0) return;
-  configure_fp32(ctx, P, Q, jb);
+  require(pair_plan_use(ctx, P, variant), "the distance histogram of this plan exceeds the shared memory");
   CRAB_CUDA_CHECK(cudaStreamSynchronize(ctx->stream));
 }
 
 int pair_plan_autotune(crab_ctx* ctx, PairPlan& P, int* variants, double* ms_out, int capacity, int* n_out) {
   if (n_out) *n_out = 0;
   if (P.fp64 || P.nq == 0 || P.L.n_tiles == 0) return P.Q;
-  static const int kVariants[][2] = {{64, 2},  {96, 2},  {128, 2}, {64, 4}, {96, 4}, {64, 2 + kPackedQ},
+  static const int kVariants[][2] = {{kHistVariant / 16, kHistVariant % 16}, {64, 2},  {96, 2},  {128, 2}, {64, 4}, {96, 4}, {64, 2 + kPackedQ},
                                      {96, 2 + kPackedQ}, {128, 1 + kPackedQ}, {128, 2 + kPackedQ},
                                      {128, 1 + kPackedQ + kDenser}, {100, 1 + kPackedQ + kDenser},
                                      {126, 1 + kPackedQ + kDenser}, {150, 1 + kPackedQ}, {168, 1 + kPackedQ},
@@ -1782,13 +1814,13 @@ int pair_plan_autotune(crab_ctx* ctx, PairPlan& P, int* variants, double* ms_out
                                      {128, kFolded2}, {126, kFolded1x3}, {100, kFolded1x3}, {84, kFolded1x4}, {168, kFolded2c},
                                      {126, kSplit1}, {126, kSplit2}, {100, kSplit1}, {100, kSplit2},
                                      {84, kSplit3}, {100, kSplit3}};
-  int bestQ = P.Q, bestJ = P.jb, n = 0;
+  int bestQ = 0, bestJ = 0, n = 0;
   float best_ms = -1.0f;
   cudaEvent_t a, b;
   CRAB_CUDA_CHECK(cudaEventCreate(&a));
   CRAB_CUDA_CHECK(cudaEventCreate(&b));
   for (const auto& v : kVariants) {
-    configure_fp32(ctx, P, v[0], v[1]);
+    if (!pair_plan_use(ctx, P, v[0] * 16 + v[1])) continue;
     pair_plan_launch(ctx, P, ctx->stream, false);  // warm-up
     CRAB_CUDA_CHECK(cudaEventRecord(a, ctx->stream));
     pair_plan_launch(ctx, P, ctx->stream, false);
@@ -1809,7 +1841,7 @@ int pair_plan_autotune(crab_ctx* ctx, PairPlan& P, int* variants, double* ms_out
   }
   cudaEventDestroy(a);
   cudaEventDestroy(b);
-  configure_fp32(ctx, P, bestQ, bestJ);
+  pair_plan_use(ctx, P, bestQ * 16 + bestJ);
   CRAB_CUDA_CHECK(cudaStreamSynchronize(ctx->stream));
   if (n_out) *n_out = std::min(n, capacity);
   return bestQ * 16 + bestJ;

@@ -231,6 +231,44 @@ struct LatticePart {
   double* d_out = nullptr;  // [nq] Σ_{i<j} sinc(q r_ij) over sites
 };
 
+// Distance-histogram form of a pair plan (debye_hist.cu).
+struct HistRow {  // a class pair: i tiles and j tiles (the same ones when diag), bins, and its first bin's sums
+  int i0, ni, j0, nj, diag, bins;
+  // units of half a tile pair: 1 each, or igroups (groups of 32 i atoms) x 4 quarters of the j atoms
+  int split, igroups, quarters;
+  float inv_h;
+  int64_t acc;
+};
+struct HistOut {  // a type pair: its counted and its loose sums (-1: none), output row, weight product
+  int64_t uniform, loose;
+  int out, bins, seg;
+  double ww;
+};
+struct HistBlock {  // type pairs of one structure that the transform takes together
+  int out0, n, bins;
+  double h;
+};
+struct HistGroup {  // rows whose sums are resident together: one launch of every kernel
+  int row0 = 0, n_rows = 0, out0 = 0, n_out = 0, block0 = 0, n_blocks = 0, start0 = 0, grid = 0, slice = 0, slices = 0;
+};
+constexpr size_t kHistGroupBytes = (size_t)96 << 20;
+struct HistPart {
+  bool active = false;
+  double scale = 1.0;  // fixed-point scale of the loose sums
+  int loose_grid = 0, loose_start0 = 0, loose_row0 = 0, widest = 0;
+  int64_t acc_bins = 0, loose_bins = 0;
+  std::vector<HistGroup> groups;
+  unsigned char* d_pts = nullptr;
+  int* d_tile_cnt = nullptr;
+  double* d_weight = nullptr;
+  HistRow* d_rows = nullptr;
+  HistOut* d_outs = nullptr;
+  HistBlock* d_blocks = nullptr;
+  int2* d_start = nullptr;
+  unsigned long long* d_acc = nullptr;
+  double* d_part = nullptr;
+};
+
 // Device-resident pair-sum problem: layout, work list and q-block
 // parameters uploaded once; launched any number of times.
 struct PairPlan {
@@ -261,6 +299,9 @@ struct PairPlan {
   // the lattice block, so the shards' outputs add up to the whole
   int shard = 0, n_shards = 1;
   std::vector<int> segments;  // batch: tile start of every structure plus the end, else empty
+  std::vector<double> seg_extent;  // batch: every structure's largest-distance bound
+  bool skip_last = false;     // the last type's pairs with itself are summed by the lattice part
+  HistPart hist;              // active: the distance histogram runs instead of a recurrence kernel
   LatticePart lattice;
   ~PairPlan();
 };
@@ -284,6 +325,11 @@ struct LatticeSpec {
   int64_t m = 0;
   double spacing = 0.0;
 };
+constexpr int kHistVariant = 16;  // the distance histogram's variant code
+// Builds the histogram form of a plan and makes it active; false when its
+// bins do not fit an SM's shared memory or there is no pair to sum.
+bool hist_plan_init(crab_ctx* ctx, PairPlan& P);
+void hist_plan_launch(crab_ctx* ctx, PairPlan& P, cudaStream_t s);
 void lattice_plan_init(crab_ctx* ctx, PairPlan& P, const int32_t* cells, int64_t m, double spacing);
 void lattice_plan_launch(crab_ctx* ctx, PairPlan& P, cudaStream_t s);
 bool q_grid_uniform(const double* q, int64_t nq);
