@@ -11,8 +11,8 @@
 //   2. k_ens_curves recombines them into the curve of every (candidate,
 //      conformer) pair;
 //   3. k_ens_weights runs, one CTA per candidate, the projected-gradient
-//      simplex fit of ensemble.rs:317-381 (250 iterations, bitonic sort for
-//      the simplex projection of ensemble.rs:449-465);
+//      simplex fit of ensemble.rs:317-381 (250 iterations with the simplex
+//      projection of ensemble.rs:449-465);
 //   4. k_ens_reweight picks the best candidate, returns ∂χ²/∂(c1, c2) at its
 //      weights, and runs the maximum-entropy mirror descent of
 //      reweight.rs:84-154 from a uniform prior.
@@ -33,30 +33,9 @@
 namespace crab {
 namespace {
 
-constexpr int kEW = 256;  // threads of the weight kernels
+constexpr int kEW = 256;  // threads whose partial sums the weight fit adds
 constexpr int kMaxK = 1024;
-
-__device__ double block_sum(double v, double* red) {
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  __syncthreads();
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-  __syncthreads();
-  double t = 0.0;
-  for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += red[w];
-  __syncthreads();
-  return t;
-}
-
-__device__ double block_max(double v, double* red) {
-  for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-  __syncthreads();
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-  __syncthreads();
-  double t = -INFINITY;
-  for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t = fmax(t, red[w]);
-  __syncthreads();
-  return t;
-}
+constexpr size_t kEnsSmem = 225 * 1024;  // dynamic shared memory of the fit kernels at most
 
 // curves[cand][k][p] from raw partials [c][ab][p] (Σ w w sin(q r)/r) and the
 // per-candidate amplitude tables amp[cand][t][p] (Â_t = V - G E + c2 H).
@@ -97,43 +76,58 @@ struct EnsOpts {
   double regularization;
 };
 
-// ensemble.rs:383-434 on the mixture in smem.
-__device__ void solve_fixed(const double* mix, const double* y, const double* sg, int nq, const EnsOpts& o, double* red,
-                            double* s_out, double* b_out, double* chi_out) {
-  double num = 0.0, den = 0.0;
-  for (int p = threadIdx.x; p < nq; p += blockDim.x) {
-    const double w = 1.0 / (sg[p] * sg[p]);
-    num += mix[p] * y[p] * w;
-    den += mix[p] * mix[p] * w;
-  }
-  num = block_sum(num, red);
-  den = block_sum(den, red);
-  double scale = o.scale_mode == CRAB_SCALE_FIT ? (den > 0.0 ? num / den : 0.0) : o.scale_value;
-  scale = fmax(scale, 0.0);
-  double bg = 0.0;
-  if (o.bg_mode == CRAB_BG_FIT) {
-    double n2 = 0.0, d2 = 0.0;
-    for (int p = threadIdx.x; p < nq; p += blockDim.x) {
-      const double w = 1.0 / (sg[p] * sg[p]);
-      n2 += (y[p] - scale * mix[p]) * w;
-      d2 += w;
+// Sums over p < n of two terms, the terms of index t, t + kEW, ... in thread
+// t < kEW, its 32 lanes joined by halving and the warps in order: the same
+// additions in the same order whatever the block size.  `red` has two halves
+// that alternate, so one barrier is enough (a half is written again after the
+// barrier of the sum in between).
+struct BlockSums {
+  double* red;
+  int half = 0;
+  template <class F>
+  __device__ __forceinline__ double2 sum2(int n, F term) {
+    double* r = red + half * (2 * kEW / 32);
+    half ^= 1;
+    if (threadIdx.x < kEW) {
+      double2 v = make_double2(0.0, 0.0);
+      for (int p = threadIdx.x; p < n; p += kEW) term(p, v);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
+        v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
+      }
+      if ((threadIdx.x & 31) == 0) {
+        r[threadIdx.x >> 5] = v.x;
+        r[kEW / 32 + (threadIdx.x >> 5)] = v.y;
+      }
     }
-    n2 = block_sum(n2, red);
-    d2 = block_sum(d2, red);
-    bg = d2 > 0.0 ? n2 / d2 : 0.0;
-  } else if (o.bg_mode == CRAB_BG_FIXED) {
-    bg = o.bg_value;
+    __syncthreads();
+    double2 t = make_double2(0.0, 0.0);
+#pragma unroll
+    for (int w = 0; w < kEW / 32; ++w) {
+      t.x += r[w];
+      t.y += r[kEW / 32 + w];
+    }
+    return t;
   }
-  double chi = 0.0;
-  for (int p = threadIdx.x; p < nq; p += blockDim.x) {
-    const double r = (scale * mix[p] + bg - y[p]) / sg[p];
-    chi += r * r;
+  template <class F>
+  __device__ __forceinline__ double sum(int n, F term) {
+    double* r = red + half * (2 * kEW / 32);
+    half ^= 1;
+    if (threadIdx.x < kEW) {
+      double v = 0.0;
+      for (int p = threadIdx.x; p < n; p += kEW) term(p, v);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      if ((threadIdx.x & 31) == 0) r[threadIdx.x >> 5] = v;
+    }
+    __syncthreads();
+    double t = 0.0;
+#pragma unroll
+    for (int w = 0; w < kEW / 32; ++w) t += r[w];
+    return t;
   }
-  chi = block_sum(chi, red);
-  *s_out = scale;
-  *b_out = bg;
-  *chi_out = chi / (double)max(nq - 1, 1);
-}
+};
 
 // Descending bitonic sort of n (power of two) values in smem.
 __device__ void bitonic_desc(double* v, int n) {
@@ -154,98 +148,255 @@ __device__ void bitonic_desc(double* v, int n) {
     }
 }
 
-// ensemble.rs:449-465: out = max(v - θ, 0) with θ from the sorted prefix.
-__device__ void project_simplex_dev(const double* v, double* out, int K, double* sorted, int n2) {
-  for (int i = threadIdx.x; i < n2; i += blockDim.x) sorted[i] = i < K ? v[i] : -INFINITY;
-  __syncthreads();
-  bitonic_desc(sorted, n2);
-  __shared__ double theta;
-  if (threadIdx.x == 0) {
-    double cumulative = 0.0;
-    int rho = 0;
-    for (int i = 0; i < K; ++i) {
-      cumulative += sorted[i];
-      if (sorted[i] + (1.0 - cumulative) / (double)(i + 1) > 0.0) rho = i + 1;
+// ensemble.rs:449-465: v = max(v - θ, 0) with θ from the sorted prefix.  Up to
+// 128 values are sorted by counting, for each, the values before it (one pass;
+// the bitonic network's 28 barriers take three times as long); thread 0 forms
+// the running sums, and every thread tests its own index.
+__device__ void project_simplex_dev(double* v, int K, double* sorted, int n2, int* rho) {
+  const int tid = threadIdx.x;
+  if (K <= 128) {
+    for (int i = tid; i < n2; i += blockDim.x) sorted[i] = -INFINITY;
+    if (tid == 0) *rho = 0;
+    __syncthreads();
+    for (int i = tid; i < K; i += blockDim.x) {
+      const double x = v[i];
+      int at = 0;
+      for (int j = 0; j < K; ++j) {
+        const double u = v[j];
+        at += u > x || (!(u < x) && j < i);
+      }
+      sorted[at] = x;
     }
-    double top = 0.0;
-    for (int i = 0; i < rho; ++i) top += sorted[i];
-    theta = (top - 1.0) / (double)max(rho, 1);
+    __syncthreads();
+  } else {
+    for (int i = tid; i < n2; i += blockDim.x) sorted[i] = i < K ? v[i] : -INFINITY;
+    if (tid == 0) *rho = 0;
+    __syncthreads();
+    bitonic_desc(sorted, n2);
+  }
+  double* cum = sorted + n2;
+  if (tid == 0) {
+    double c = 0.0;
+#pragma unroll 8
+    for (int i = 0; i < K; ++i) {
+      c += sorted[i];
+      cum[i] = c;
+    }
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < K; i += blockDim.x) out[i] = fmax(v[i] - theta, 0.0);
+  for (int i = tid; i < K; i += blockDim.x)
+    if (sorted[i] + (1.0 - cum[i]) / (double)(i + 1) > 0.0) atomicMax(rho, i + 1);
+  __syncthreads();
+  const int r = *rho;
+  const double theta = ((r > 0 ? cum[r - 1] : 0.0) - 1.0) / (double)max(r, 1);
+  for (int i = tid; i < K; i += blockDim.x) v[i] = fmax(v[i] - theta, 0.0);
   __syncthreads();
 }
 
-// One CTA per candidate: ensemble.rs:317-381.
-__global__ void __launch_bounds__(kEW)
+// a / b with y = 1/b correctly rounded: Markstein's quotient (IBM J. Res. Dev.
+// 34, 1990), one step to bring q within an ulp and one that rounds it
+// correctly.  For a zero or in the range below, b within 1e-100 .. 1e100 (equal
+// to the division in 8.6e9 random quotients, half of them at mantissa ends).
+__device__ __forceinline__ double div_by(double a, double b, double y) {
+  // biased exponent within 2^-480 .. 2^480, or a zero
+  const unsigned ex = ((unsigned)__double2hiint(a) >> 20 & 0x7ffu) - 543u;
+  if (ex > 960u && a != 0.0) return a / b;
+  double q = a * y;
+  q = fma(fma(-q, b, a), y, q);
+  return fma(fma(-q, b, a), y, q);
+}
+
+// The weight kernel's shared memory, in doubles: weights, gradients and
+// proposals, the sorted values and their running sums; per q the mixture, the
+// weighted residual, y, sigma, 1/sigma and 1/sigma²; two chunks of gradient
+// terms; and the curves, where they fit.
+constexpr int kWT = 512;  // threads of k_ens_weights
+__host__ __device__ inline int ew_pow2(int K) {
+  int n2 = 1;
+  while (n2 < K) n2 <<= 1;
+  return n2;
+}
+// q per chunk of gradient terms (a power of two up to 32)
+__host__ __device__ inline int ew_chunk(int K) { return K <= 256 ? 32 : 8; }
+__host__ __device__ inline size_t ew_full(int K, int nq) {
+  return (size_t)4 * K + ew_pow2(K) + 6 * (size_t)nq + 2 * (size_t)ew_chunk(K) * (K | 1);
+}
+// Very long q grids keep only the mixture and the residual there, and one q
+// of gradient terms at a time.
+__host__ __device__ inline bool ew_lean(int K, int nq) { return ew_full(K, nq) * sizeof(double) > kEnsSmem; }
+__host__ __device__ inline size_t ew_doubles(int K, int nq) {
+  return ew_lean(K, nq) ? (size_t)4 * K + ew_pow2(K) + 2 * (size_t)nq + 2 * (size_t)(K | 1) : ew_full(K, nq);
+}
+__host__ __device__ inline bool ew_on_chip(int K, int nq) {
+  return (ew_doubles(K, nq) + (size_t)K * nq) * sizeof(double) <= kEnsSmem;
+}
+
+// Σ_p (rs[p] cv[k][p]) / sg[p] for every k into out[k], each in the order of p.
+// The terms of a chunk of P q are formed, one chunk ahead, by the warps beyond
+// the K threads that add them up (by all warps if those are too many), a lane
+// for each q of the chunk.
+__device__ __forceinline__ void ew_gradient(const double* cv, int K, int nq, const double* rs, const double* sg,
+                                            const double* isg, bool plain, int P, double* terms, double* out) {
+  const int tid = threadIdx.x, kp = (K + 31) & ~31, ks = K | 1;
+  const bool apart = kp <= kWT / 2;
+  const int t0 = apart ? tid - kp : tid, tn = apart ? kWT - kp : kWT;
+  const int lp = t0 & (P - 1), k_first = t0 / P, k_step = tn / P;
+  auto form = [&](int q0, double* to) {
+    const int p = q0 + lp;
+    if (t0 < 0 || p >= nq) return;
+    const double r = rs[p], b = sg[p], y = plain ? 0.0 : isg[p];
+    const double* c = cv + k_first * nq + p;
+    double* d = to + lp * ks + k_first;
+#pragma unroll 2
+    for (int k = k_first; k < K; k += k_step, c += k_step * nq, d += k_step) {
+      const double a = r * *c;
+      *d = plain ? a / b : div_by(a, b, y);
+    }
+  };
+  double acc[kMaxK / kWT] = {0.0, 0.0};
+  form(0, terms);
+  __syncthreads();
+  int buf = 0;
+  for (int q0 = 0; q0 < nq; q0 += P, buf ^= 1) {
+    const double* t = terms + buf * P * ks;
+    if (q0 + P < nq) form(q0 + P, terms + (buf ^ 1) * P * ks);
+    const int n = min(P, nq - q0);
+#pragma unroll
+    for (int j = 0; j < kMaxK / kWT; ++j) {
+      const int k = tid + j * kWT;
+      if (k >= K) break;
+      if (n == 32) {
+#pragma unroll
+        for (int p = 0; p < 32; ++p) acc[j] += t[p * ks + k];
+      } else {
+        for (int p = 0; p < n; ++p) acc[j] += t[p * ks + k];
+      }
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int j = 0; j < kMaxK / kWT; ++j)
+    if (tid + j * kWT < K) out[tid + j * kWT] = acc[j];
+  __syncthreads();
+}
+
+// One CTA per candidate: ensemble.rs:317-381.  Bound by latency: 250 steps, each
+// a chain of sums.  Every sum keeps its terms and their order (the final
+// iterate depends on the last bits), but the terms are formed in parallel: 41
+// us a step became 13 us for 48 curves of 300 q (one thread per curve ran the
+// gradient's 300 dependent divisions, and one thread the projection's).
+__global__ void __launch_bounds__(kWT)
     k_ens_weights(const double* __restrict__ curves, int K, int nq, const double* __restrict__ y,
                   const double* __restrict__ sg, EnsOpts o, double* __restrict__ weights, double* __restrict__ fit,
                   double* __restrict__ fitted, double* __restrict__ grad_w) {
   extern __shared__ double sm[];
-  double* w = sm;               // K
-  double* g = w + K;            // K
-  double* prop = g + K;         // K
-  double* mix = prop + K;       // nq
-  double* res = mix + nq;       // nq
-  int n2 = 1;
-  while (n2 < K) n2 <<= 1;
-  double* sorted = res + nq;    // n2
-  __shared__ double red[32];
+  const int n2 = ew_pow2(K), tid = threadIdx.x;
+  double* w = sm;                // K
+  double* g = w + K;             // K
+  double* prop = g + K;          // K
+  double* sorted = prop + K;     // n2, then K running sums
+  double* mix = sorted + n2 + K; // nq
+  double* rs = mix + nq;         // nq: residual / sigma x scale
+  const bool lean = ew_lean(K, nq);
+  const int P = lean ? 1 : ew_chunk(K);
+  double* terms = rs + nq;       // 2 x P x (K | 1)
+  double* perq = terms + 2 * (size_t)P * (K | 1);
+  double* isg = perq;            // nq: 1 / sigma
+  double* ww = perq + nq;        // nq: 1 / sigma²
+  const double* ys = lean ? y : perq + 2 * (size_t)nq;
+  const double* sgs = lean ? sg : perq + 3 * (size_t)nq;
+  double* cvs = perq + (lean ? 0 : 4 * (size_t)nq);
+  __shared__ double red[4 * kEW / 32];
+  __shared__ int rho, plain_s;
   const int cand = blockIdx.x;
   const double* cv = curves + (size_t)cand * K * nq;
-  for (int k = threadIdx.x; k < K; k += blockDim.x) w[k] = 1.0 / (double)K;
+  if (tid == 0) plain_s = lean ? 1 : 0;
   __syncthreads();
-  double s, b, chi;
-  const int iters = o.uniform ? 0 : 250;
-  for (int it = 0; it < iters; ++it) {
-    for (int p = threadIdx.x; p < nq; p += blockDim.x) {
+  for (int p = tid; p < nq && !lean; p += kWT) {
+    const double v = sg[p];
+    perq[2 * nq + p] = y[p];
+    perq[3 * nq + p] = v;
+    isg[p] = 1.0 / v;
+    ww[p] = 1.0 / (v * v);
+    if (!(v > 1e-100 && v < 1e100)) plain_s = 1;
+  }
+  BlockSums bs{red};
+  auto wgt = [&](int p) { return lean ? 1.0 / (sg[p] * sg[p]) : ww[p]; };
+  if (ew_on_chip(K, nq)) {
+    for (int i = tid; i < K * nq; i += kWT) cvs[i] = cv[i];
+    cv = cvs;
+  }
+  for (int k = tid; k < K; k += kWT) w[k] = 1.0 / (double)K;
+  __syncthreads();
+  const bool plain = plain_s != 0;
+  const double d2 =
+      o.bg_mode == CRAB_BG_FIT ? bs.sum(nq, [&](int p, double& v) { v += wgt(p); }) : 0.0;
+  // mixture, then scale and background (ensemble.rs:383-434)
+  double s, b;
+  auto mixture = [&]() {
+    for (int p = tid; p < nq; p += kWT) {
       double m = 0.0;
-      for (int k = 0; k < K; ++k) m += cv[(size_t)k * nq + p] * w[k];
+      const double* c = cv + p;
+#pragma unroll 8
+      for (int k = 0; k < K; ++k, c += nq) m += *c * w[k];
       mix[p] = m;
     }
     __syncthreads();
-    solve_fixed(mix, y, sg, nq, o, red, &s, &b, &chi);
-    for (int p = threadIdx.x; p < nq; p += blockDim.x) res[p] = (s * mix[p] + b - y[p]) / sg[p];
+    const double2 nd = bs.sum2(nq, [&](int p, double2& v) {
+      const double q = wgt(p);
+      v.x += mix[p] * ys[p] * q;
+      v.y += mix[p] * mix[p] * q;
+    });
+    s = o.scale_mode == CRAB_SCALE_FIT ? (nd.y > 0.0 ? nd.x / nd.y : 0.0) : o.scale_value;
+    s = fmax(s, 0.0);
+    b = 0.0;
+    if (o.bg_mode == CRAB_BG_FIT) {
+      const double n2s = bs.sum(nq, [&](int p, double& v) { v += (ys[p] - s * mix[p]) * wgt(p); });
+      b = d2 > 0.0 ? n2s / d2 : 0.0;
+    } else if (o.bg_mode == CRAB_BG_FIXED) {
+      b = o.bg_value;
+    }
+  };
+  const int iters = o.uniform ? 0 : 250;
+  for (int it = 0; it < iters; ++it) {
+    mixture();
+    for (int p = tid; p < nq; p += kWT) rs[p] = (s * mix[p] + b - ys[p]) / sgs[p] * s;
     __syncthreads();
-    for (int k = threadIdx.x; k < K; k += blockDim.x) {
-      double acc = 0.0;
-      for (int p = 0; p < nq; ++p) acc += res[p] * s * cv[(size_t)k * nq + p] / sg[p];
+    ew_gradient(cv, K, nq, rs, sgs, isg, plain, P, terms, g);
+    for (int k = tid; k < K; k += kWT) {
+      const double acc = g[k];
       g[k] = 2.0 * acc + 2.0 * o.regularization * (w[k] - 1.0 / (double)K);
     }
     __syncthreads();
-    double nrm = 0.0;
-    for (int k = threadIdx.x; k < K; k += blockDim.x) nrm += g[k] * g[k];
-    nrm = fmax(sqrt(block_sum(nrm, red)), 1.0);
-    for (int k = threadIdx.x; k < K; k += blockDim.x) prop[k] = w[k] - 0.05 * g[k] / nrm;
+    double nrm = bs.sum(K, [&](int k, double& v) { v += g[k] * g[k]; });
+    nrm = fmax(sqrt(nrm), 1.0);
+    for (int k = tid; k < K; k += kWT) prop[k] = w[k] - 0.05 * g[k] / nrm;
     __syncthreads();
-    project_simplex_dev(prop, prop, K, sorted, n2);
-    double delta = 0.0;
-    for (int k = threadIdx.x; k < K; k += blockDim.x) delta += fabs(prop[k] - w[k]);
-    delta = block_sum(delta, red);
-    for (int k = threadIdx.x; k < K; k += blockDim.x) w[k] = prop[k];
+    project_simplex_dev(prop, K, sorted, n2, &rho);
+    const double delta = bs.sum(K, [&](int k, double& v) { v += fabs(prop[k] - w[k]); });
+    for (int k = tid; k < K; k += kWT) w[k] = prop[k];
     __syncthreads();
     if (delta < 1e-8) break;
   }
-  for (int p = threadIdx.x; p < nq; p += blockDim.x) {
-    double m = 0.0;
-    for (int k = 0; k < K; ++k) m += cv[(size_t)k * nq + p] * w[k];
-    mix[p] = m;
-  }
-  __syncthreads();
-  solve_fixed(mix, y, sg, nq, o, red, &s, &b, &chi);
-  for (int p = threadIdx.x; p < nq; p += blockDim.x) {
+  mixture();
+  const double chi = bs.sum(nq, [&](int p, double& v) {
+                       const double r = (s * mix[p] + b - ys[p]) / sgs[p];
+                       v += r * r;
+                     }) /
+                     (double)max(nq - 1, 1);
+  for (int p = tid; p < nq; p += kWT) {
     fitted[(size_t)cand * nq + p] = s * mix[p] + b;
-    res[p] = (s * mix[p] + b - y[p]) / sg[p];
+    rs[p] = (s * mix[p] + b - ys[p]) / sgs[p] * s;
   }
   __syncthreads();
   // ∂χ²_red/∂w_k at the final weights (scale and background held)
-  for (int k = threadIdx.x; k < K; k += blockDim.x) {
-    double acc = 0.0;
-    for (int p = 0; p < nq; ++p) acc += res[p] * s * cv[(size_t)k * nq + p] / sg[p];
+  ew_gradient(cv, K, nq, rs, sgs, isg, plain, P, terms, g);
+  for (int k = tid; k < K; k += kWT) {
+    const double acc = g[k];
     grad_w[(size_t)cand * K + k] = 2.0 * acc / (double)max(nq - 1, 1);
     weights[(size_t)cand * K + k] = w[k];
   }
-  if (threadIdx.x == 0) {
+  if (tid == 0) {
     fit[4 * cand] = s;
     fit[4 * cand + 1] = b;
     fit[4 * cand + 2] = chi;
@@ -259,281 +410,337 @@ struct RwOpts {
   double scale_value, bg_value;
 };
 
-// reweight.rs:236-301 on the mixture mix[p] (scale, background, reduced χ²).
-__device__ void rw_solve(const double* mix, int nq, const double* y, const double* sg, const RwOpts& o, double* red,
-                         double* s_out, double* b_out, double* chi_out) {
-  double sw = 0, sx = 0, sy = 0, sxx = 0, sxy = 0;
-  for (int p = threadIdx.x; p < nq; p += blockDim.x) {
-    const double ww = 1.0 / (sg[p] * sg[p]);
-    sw += ww;
-    sx += ww * mix[p];
-    sy += ww * y[p];
-    sxx += ww * mix[p] * mix[p];
-    sxy += ww * mix[p] * y[p];
-  }
-  sw = block_sum(sw, red);
-  sx = block_sum(sx, red);
-  sy = block_sum(sy, red);
-  sxx = block_sum(sxx, red);
-  sxy = block_sum(sxy, red);
-  double s, b;
-  auto fscale = [&](double bb) { return sxx > 0.0 ? fmax((sxy - bb * sx) / sxx, 0.0) : 0.0; };
-  auto fbg = [&](double ss) { return sw > 0.0 ? (sy - ss * sx) / sw : 0.0; };
-  if (o.scale_mode == CRAB_SCALE_FIXED) {
-    s = fmax(o.scale_value, 0.0);
-    b = o.bg_mode == CRAB_BG_FIXED ? o.bg_value : (o.bg_mode == CRAB_BG_FIXED_ZERO ? 0.0 : fbg(s));
-  } else if (o.bg_mode == CRAB_BG_FIXED) {
-    s = fscale(o.bg_value);
-    b = o.bg_value;
-  } else if (o.bg_mode == CRAB_BG_FIXED_ZERO) {
-    s = fscale(0.0);
-    b = 0.0;
-  } else {
-    const double det = sxx * sw - sx * sx;
-    s = fabs(det) > 1e-20 ? fmax((sxy * sw - sx * sy) / det, 0.0) : 0.0;
-    b = fbg(s);
-  }
-  double chi = 0.0;
-  for (int p = threadIdx.x; p < nq; p += blockDim.x) {
-    const double r = (s * mix[p] + b - y[p]) / sg[p];
-    chi += r * r;
-  }
-  chi = block_sum(chi, red);
-  *s_out = s;
-  *b_out = b;
-  *chi_out = chi / (double)max(nq - 1, 1);
-}
-
-// ---- KL reweighting over a cluster of kRwCluster CTAs ----------------------
-// reweight.rs:84-154 on the best candidate's K curves.  CTA r of the cluster
-// keeps rows [r kr, (r+1) kr) of those curves (kr = ceil(K / kRwCluster)) in
-// its shared memory, with their weights, gradients and proposals; the
-// mixture and every sum or maximum over K are exchanged through distributed
-// shared memory: each CTA publishes its partial, one cluster barrier, and
-// every CTA adds the partials of all ranks in rank order, so every CTA holds
-// the same values and takes the same branches.  Exchange buffers alternate
-// between two halves, so the barrier of one exchange also releases the
-// buffer of the exchange before it.
+// ---- KL reweighting -------------------------------------------------------
+// reweight.rs:84-154 on the best candidate's K curves, bound by the latency of
+// its 500 steps, each with a line search of up to 14 evaluations.  Every CTA
+// holds all K weights, gradients and proposals and does all work on them, so
+// that an evaluation needs one exchange at most: with the curves split over a
+// cluster of CL CTAs (CTA r keeps the rows [r kr, (r+1) kr) in its shared
+// memory), the partial mixtures of all CTAs, added in rank order, and once per
+// step the gradients of their rows.  All CTAs therefore hold the same values and
+// take the same branches.  CL is one where the curves fit one CTA's shared
+// memory: a step of 48 curves of 300 q (five evaluations on average) then has
+// block barriers only, and takes 19 us (100 us on 8 CTAs that split the weights
+// too, with a cluster barrier for each of the six sums of an evaluation).
 constexpr int kRwCluster = 8;
 namespace cg = cooperative_groups;
 
-struct RwCluster {
-  cg::cluster_group cl;
-  double* xs;  // [2] scalar partial
-  double* pm;  // [2][3 nq] array partials
-  double* red;
-  int nq, par;
-  __device__ double sum(double v) {
-    v = block_sum(v, red);
-    if (threadIdx.x == 0) xs[par] = v;
-    cl.sync();
-    double t = 0.0;
-    for (int r = 0; r < kRwCluster; ++r) t += *cl.map_shared_rank(&xs[par], r);
-    par ^= 1;
-    return t;
-  }
-  __device__ double max(double v) {
-    v = block_max(v, red);
-    if (threadIdx.x == 0) xs[par] = v;
-    cl.sync();
-    double t = -INFINITY;
-    for (int r = 0; r < kRwCluster; ++r) t = fmax(t, *cl.map_shared_rank(&xs[par], r));
-    par ^= 1;
-    return t;
-  }
-  // out[i] = sum over ranks of the published part[i], i < n (n <= 3 nq); part
-  // is written by this CTA into pm[par] by the caller's loop before the call
-  __device__ double* slot() { return pm + (size_t)par * 3 * nq; }
-  __device__ void sum_array(double* out, int n) {
+// Threads of a CTA: about one per q, and a warp more for the K logarithms.
+inline int rw_threads(int nq) { return std::min(512, std::max(128, (nq + 31) / 32 * 32 + 64)); }
+
+// Sums over the block of N values per thread (a fixed tree, then the warps in
+// order); the two halves of `red` alternate, as in BlockSums.
+struct RwSums {
+  double* red;  // [2][4 x 16]
+  int half = 0;
+  template <int N>
+  __device__ __forceinline__ void operator()(double (&v)[N]) {
+    double* r = red + half * 64;
+    half ^= 1;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int i = 0; i < N; ++i) v[i] += __shfl_xor_sync(0xffffffffu, v[i], o);
+    if ((threadIdx.x & 31) == 0)
+#pragma unroll
+      for (int i = 0; i < N; ++i) r[i * 16 + (threadIdx.x >> 5)] = v[i];
     __syncthreads();
-    cl.sync();
-    double* mine = slot();
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-      double t = 0.0;
-      for (int r = 0; r < kRwCluster; ++r) t += cl.map_shared_rank(mine, r)[i];
-      out[i] = t;
-    }
-    par ^= 1;
+    const int warps = blockDim.x >> 5;
+#pragma unroll
+    for (int i = 0; i < N; ++i) v[i] = 0.0;
+#pragma unroll 4
+    for (int w = 0; w < warps; ++w)
+#pragma unroll
+      for (int i = 0; i < N; ++i) v[i] += r[i * 16 + w];
+  }
+  __device__ __forceinline__ double max(double v) {
+    double* r = red + half * 64;
+    half ^= 1;
+    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+    if ((threadIdx.x & 31) == 0) r[threadIdx.x >> 5] = v;
     __syncthreads();
+    v = r[0];
+    for (int w = 1; w < (int)(blockDim.x >> 5); ++w) v = fmax(v, r[w]);
+    return v;
   }
 };
 
-// The mixture Σ_k w_k I_k(q) over the cluster's rows, then reweight.rs:236-301.
-__device__ void rw_fit_cl(RwCluster& X, const double* cvr, const double* w, int nk, int nq, const double* y,
-                          const double* sg, const RwOpts& o, double* mix, double* s_out, double* b_out,
-                          double* chi_out) {
-  double* part = X.slot();
-  for (int p = threadIdx.x; p < nq; p += blockDim.x) {
-    double m = 0.0;
-    for (int k = 0; k < nk; ++k) m += cvr[(size_t)k * nq + p] * w[k];
-    part[p] = m;
-  }
-  X.sum_array(mix, nq);
-  rw_solve(mix, nq, y, sg, o, X.red, s_out, b_out, chi_out);
+__host__ __device__ inline int rw_rows(int K, int cl) { return (K + cl - 1) / cl; }
+// Shared memory in doubles without the curves: weights, gradients, proposals
+// and the logarithms of both; per q the mixture (then the gradient's factor), y
+// and 1/sigma²; in a cluster the partial mixtures (two halves) and the
+// gradients (two halves) that its CTAs exchange.
+__host__ __device__ inline size_t rw_doubles(int K, int nq, int cl) {
+  return 5 * (size_t)K + 3 * (size_t)nq + (cl > 1 ? 2 * (size_t)nq : 0) + 2 * (size_t)rw_rows(K, cl);
 }
-__device__ double kl_div_cl(RwCluster& X, const double* w, int nk, double prior) {
-  double s = 0.0;
-  for (int k = threadIdx.x; k < nk; k += blockDim.x) s += w[k] * log(w[k] / prior);
-  return X.sum(s);
+__host__ __device__ inline bool rw_on_chip(int K, int nq, int cl) {
+  return (rw_doubles(K, nq, cl) + (size_t)rw_rows(K, cl) * nq) * sizeof(double) <= kEnsSmem;
 }
-__device__ void apply_floor_cl(RwCluster& X, double* w, int nk, int K, double floor) {
-  double sum = 0.0;
-  for (int k = threadIdx.x; k < nk; k += blockDim.x) sum += w[k];
-  sum = fmax(X.sum(sum), 1e-300);
-  const double residual = 1.0 - floor * (double)K;
-  for (int k = threadIdx.x; k < nk; k += blockDim.x) w[k] = floor <= 0.0 ? w[k] / sum : floor + residual * w[k] / sum;
-  __syncthreads();
-}
-
-// Shared memory of one cluster CTA for K curves of nq points: weights,
-// gradients and proposals of its rows, the mixture, the exchange buffers and,
-// when they fit, its rows of the curves.
-__host__ __device__ inline int rw_rows(int K) { return (K + kRwCluster - 1) / kRwCluster; }
-__host__ __device__ inline bool rw_rows_on_chip(int K, int nq) {
-  return (size_t)rw_rows(K) * (size_t)nq * sizeof(double) <= 128 * 1024;
-}
-__host__ __device__ inline size_t rw_smem(int K, int nq) {
-  const size_t kr = (size_t)rw_rows(K);
-  return (3 * kr + (size_t)nq + 6 * (size_t)nq + 2 + (rw_rows_on_chip(K, nq) ? kr * (size_t)nq : 0)) * sizeof(double);
+__host__ __device__ inline size_t rw_smem(int K, int nq, int cl) {
+  return (rw_doubles(K, nq, cl) + (rw_on_chip(K, nq, cl) ? (size_t)rw_rows(K, cl) * nq : 0)) * sizeof(double);
 }
 
 // Best candidate, ∂χ²/∂(c1, c2) there, then reweight.rs:84-154.
 // out: [0] best candidate, [1] scale, [2] bg, [3] reduced chi2, [4] KL,
 // [5] iterations, [6] converged, [7] dchi/dc1, [8] dchi/dc2.
-__global__ void __cluster_dims__(kRwCluster, 1, 1) __launch_bounds__(kEW)
+template <int CL>
+__global__ void __launch_bounds__(512, 1)
     k_ens_reweight(const double* __restrict__ curves, const double* __restrict__ fitc, int n_cand, int K, int nq,
                    const double* __restrict__ y, const double* __restrict__ sg, const double* __restrict__ weights,
                    const double* __restrict__ dcurves, RwOpts o, double* __restrict__ w_out,
                    double* __restrict__ out) {
   extern __shared__ double sm[];
-  __shared__ double red[32];
+  __shared__ double red[2 * 64];
   __shared__ int best;
-  RwCluster X{cg::this_cluster(), nullptr, nullptr, red, nq, 0};
-  const int rank = (int)X.cl.block_rank();
-  const int kr = rw_rows(K), k0 = min(K, rank * kr), nk = min(K, k0 + kr) - k0;
-  double* w = sm;              // kr
-  double* g = w + kr;          // kr
-  double* pr = g + kr;         // kr
-  double* mix = pr + kr;       // nq
-  X.pm = mix + nq;             // 2 x 3 nq
-  X.xs = X.pm + 6 * (size_t)nq;  // 2
-  double* cvs = X.xs + 2;      // kr x nq, when the rows fit
-  if (threadIdx.x == 0) {
+  const int tid = threadIdx.x, nt = blockDim.x;
+  const int back = nt - 1 - tid;  // the K-wide work of an evaluation starts at the last warp
+  int rank = 0;
+  if constexpr (CL > 1) rank = (int)cg::this_cluster().block_rank();
+  const int kr = rw_rows(K, CL), k0 = min(K, rank * kr), nk = min(K, k0 + kr) - k0;
+  double* w = sm;              // K
+  double* g = w + K;           // K
+  double* pr = g + K;          // K
+  double* lw = pr + K;         // K: log(w / prior)
+  double* lp = lw + K;         // K: log(pr / prior)
+  double* mix = lp + K;        // nq
+  double* ys = mix + nq;       // nq
+  double* ww = ys + nq;        // nq
+  double* own = ww + nq;       // 2 x nq: this CTA's partial mixture (in a cluster)
+  double* gx = own + (CL > 1 ? 2 * (size_t)nq : 0);  // 2 x kr
+  double* cvs = gx + 2 * (size_t)kr;
+  RwSums sums{red};
+  if (tid == 0) {
     best = 0;
     for (int c = 1; c < n_cand; ++c)
       if (fitc[4 * c + 2] < fitc[4 * best + 2]) best = c;
   }
-  __syncthreads();
-  const double* cvg = curves + ((size_t)best * K + k0) * nq;  // this CTA's rows
-  const double* cvr = cvg;
-  if (rw_rows_on_chip(K, nq)) {
-    for (size_t i = threadIdx.x; i < (size_t)nk * nq; i += blockDim.x) cvs[i] = cvg[i];
-    cvr = cvs;
+  for (int p = tid; p < nq; p += nt) {
+    ys[p] = y[p];
+    ww[p] = 1.0 / (sg[p] * sg[p]);
   }
   __syncthreads();
+  const double* cvr = curves + ((size_t)best * K + k0) * nq;  // this CTA's rows
+  const double dof = (double)max(nq - 1, 1);
   // ∂χ²/∂c1 and ∂χ²/∂c2 at the best candidate's weights, scale and background
-  {
+  if (rank == 0) {
     const double s = fitc[4 * best], b = fitc[4 * best + 1];
-    const double* wb = weights + (size_t)best * K + k0;
-    const double* d1c = dcurves + ((size_t)(2 * best) * K + k0) * nq;
-    const double* d2c = dcurves + ((size_t)(2 * best + 1) * K + k0) * nq;
-    double* part = X.slot();
-    for (int p = threadIdx.x; p < nq; p += blockDim.x) {
+    const double* wb = weights + (size_t)best * K;
+    const double* cb = curves + (size_t)best * K * nq;
+    const double* d1c = dcurves + (size_t)(2 * best) * K * nq;
+    const double* d2c = dcurves + (size_t)(2 * best + 1) * K * nq;
+    double v[2] = {0.0, 0.0};
+    for (int p = tid; p < nq; p += nt) {
       double m = 0.0, d1 = 0.0, d2 = 0.0;
-      for (int k = 0; k < nk; ++k) {
-        m += cvr[(size_t)k * nq + p] * wb[k];
+#pragma unroll 4
+      for (int k = 0; k < K; ++k) {
+        m += cb[(size_t)k * nq + p] * wb[k];
         d1 += d1c[(size_t)k * nq + p] * wb[k];
         d2 += d2c[(size_t)k * nq + p] * wb[k];
       }
-      part[p] = m;
-      part[nq + p] = d1;
-      part[2 * nq + p] = d2;
+      const double wgt = 2.0 * (s * m + b - ys[p]) * ww[p] / dof * s;
+      v[0] += wgt * d1;
+      v[1] += wgt * d2;
     }
-    // the sums land in this CTA's other exchange half: no peer reads it
-    // before the next array exchange, which comes after their last use here
-    double* sums = X.pm + (size_t)(X.par ^ 1) * 3 * nq;
-    X.sum_array(sums, 3 * nq);
-    double g1 = 0.0, g2 = 0.0;
-    for (int p = threadIdx.x; p < nq; p += blockDim.x) {
-      const double wgt = 2.0 * (s * sums[p] + b - y[p]) / (sg[p] * sg[p]) / (double)max(nq - 1, 1) * s;
-      g1 += wgt * sums[nq + p];
-      g2 += wgt * sums[2 * nq + p];
+    sums(v);
+    if (tid == 0) {
+      out[7] = v[0];
+      out[8] = v[1];
     }
-    g1 = block_sum(g1, red);
-    g2 = block_sum(g2, red);
-    if (rank == 0 && threadIdx.x == 0) {
-      out[7] = g1;
-      out[8] = g2;
-    }
-    __syncthreads();
   }
-  const double prior = 1.0 / (double)K;
-  for (int k = threadIdx.x; k < nk; k += blockDim.x) w[k] = prior;
+  if (rw_on_chip(K, nq, CL)) {
+    for (int i = tid; i < nk * nq; i += nt) cvs[i] = cvr[i];
+    cvr = cvs;
+  }
+  const double prior = 1.0 / (double)K, residual = 1.0 - o.floor * (double)K;
+  double sw, sy;  // Σ 1/σ², Σ y/σ²
+  {
+    double v[3] = {0.0, 0.0, 0.0};
+    for (int p = tid; p < nq; p += nt) {
+      v[0] += ww[p];
+      v[1] += ww[p] * ys[p];
+    }
+    for (int k = tid; k < K; k += nt) v[2] += prior;
+    sums(v);
+    sw = v[0];
+    sy = v[1];
+    const double all = fmax(v[2], 1e-300);
+    for (int k = tid; k < K; k += nt) w[k] = o.floor <= 0.0 ? prior / all : o.floor + residual * prior / all;
+  }
   __syncthreads();
-  apply_floor_cl(X, w, nk, K, o.floor);
+  int par = 0, gpar = 0;
+  double s, b, chi, kl;
+  // log(wv / prior) into lv; the mixture of wv, then scale and background
+  // (reweight.rs:236-301), χ² and the KL term
+  auto evaluate = [&](const double* wv, double* lv) {
+    double v[4] = {0.0, 0.0, 0.0, 0.0};  // Σ m/σ², Σ m²/σ², Σ m y/σ², Σ w log(w/prior)
+    for (int k = back; k < K; k += nt) {
+      const double l = log(wv[k] / prior);
+      lv[k] = l;
+      v[3] += wv[k] * l;
+    }
+    double* mine = CL > 1 ? own + (size_t)par * nq : mix;
+    auto moments = [&](int p, double m) {
+      v[0] += ww[p] * m;
+      v[1] += ww[p] * m * m;
+      v[2] += ww[p] * m * ys[p];
+    };
+    for (int p = tid; p < nq; p += nt) {
+      double m = 0.0, m1 = 0.0;
+      const double* c = cvr + p;
+      int k = 0;
+#pragma unroll 4
+      for (; k + 1 < nk; k += 2, c += 2 * nq) {
+        m += c[0] * wv[k0 + k];
+        m1 += c[nq] * wv[k0 + k + 1];
+      }
+      if (k < nk) m += c[0] * wv[k0 + k];
+      m += m1;
+      mine[p] = m;
+      if (CL == 1) moments(p, m);
+    }
+    if constexpr (CL > 1) {
+      cg::this_cluster().sync();
+      for (int p = tid; p < nq; p += nt) {
+        double m = 0.0;
+#pragma unroll
+        for (int r = 0; r < CL; ++r) m += cg::this_cluster().map_shared_rank(mine, r)[p];
+        mix[p] = m;
+        moments(p, m);
+      }
+      par ^= 1;  // the barrier of the next exchange releases this half
+    }
+    sums(v);
+    const double sx = v[0], sxx = v[1], sxy = v[2];
+    kl = v[3];
+    auto fscale = [&](double bb) { return sxx > 0.0 ? fmax((sxy - bb * sx) / sxx, 0.0) : 0.0; };
+    auto fbg = [&](double ss) { return sw > 0.0 ? (sy - ss * sx) / sw : 0.0; };
+    if (o.scale_mode == CRAB_SCALE_FIXED) {
+      s = fmax(o.scale_value, 0.0);
+      b = o.bg_mode == CRAB_BG_FIXED ? o.bg_value : (o.bg_mode == CRAB_BG_FIXED_ZERO ? 0.0 : fbg(s));
+    } else if (o.bg_mode == CRAB_BG_FIXED) {
+      s = fscale(o.bg_value);
+      b = o.bg_value;
+    } else if (o.bg_mode == CRAB_BG_FIXED_ZERO) {
+      s = fscale(0.0);
+      b = 0.0;
+    } else {
+      const double det = sxx * sw - sx * sx;
+      s = fabs(det) > 1e-20 ? fmax((sxy * sw - sx * sy) / det, 0.0) : 0.0;
+      b = fbg(s);
+    }
+    double e[1] = {0.0};
+    for (int p = tid; p < nq; p += nt) {
+      const double r = s * mix[p] + b - ys[p];
+      e[0] += r * r * ww[p];
+    }
+    sums(e);
+    chi = e[0] / dof;
+  };
   int iterations = 0, converged = 0;
-  const double dof = (double)max(nq - 1, 1);
-  double s, b, chi;
+  evaluate(w, lw);
   for (int it = 0; it < o.max_iter; ++it) {
     iterations = it + 1;
-    rw_fit_cl(X, cvr, w, nk, nq, y, sg, o, mix, &s, &b, &chi);
-    for (int k = threadIdx.x; k < nk; k += blockDim.x) {
-      double dg = 0.0;
-      for (int p = 0; p < nq; ++p)
-        dg += 2.0 * ((s * mix[p] + b) - y[p]) * s * cvr[(size_t)k * nq + p] / (sg[p] * sg[p]) / dof;
-      g[k] = dg + o.kl * (log(w[k] / prior) + 1.0);
-    }
+    // gradient at w, whose mixture, scale and background the last evaluation left
+    for (int p = tid; p < nq; p += nt) mix[p] = 2.0 * ((s * mix[p] + b) - ys[p]) * s * ww[p] / dof;
     __syncthreads();
+    double* gown = gx + gpar * kr;
+    for (int k = tid >> 5; k < nk; k += nt >> 5) {  // a warp per curve
+      double dg = 0.0;
+      const double* c = cvr + k * nq;
+#pragma unroll 4
+      for (int p = tid & 31; p < nq; p += 32) dg += mix[p] * c[p];
+#pragma unroll
+      for (int q = 16; q > 0; q >>= 1) dg += __shfl_xor_sync(0xffffffffu, dg, q);
+      if ((tid & 31) == 0) gown[k] = dg;
+    }
+    if constexpr (CL > 1) cg::this_cluster().sync();
+    else __syncthreads();
     double gmax = 0.0;
-    for (int k = threadIdx.x; k < nk; k += blockDim.x) gmax = fmax(gmax, fabs(g[k]));
-    gmax = fmax(X.max(gmax), 1e-12);
+    for (int k = tid; k < K; k += nt) {
+      double v;
+      if constexpr (CL > 1) v = cg::this_cluster().map_shared_rank(gown, k / kr)[k % kr];
+      else v = gown[k];
+      v += o.kl * (lw[k] + 1.0);
+      g[k] = v;
+      gmax = fmax(gmax, fabs(v));
+    }
+    gpar ^= 1;
+    gmax = fmax(sums.max(gmax), 1e-12);
     double step = o.step / gmax;
-    const double objective = chi + o.kl * kl_div_cl(X, w, nk, prior);
+    const double objective = chi + o.kl * kl;
     bool accepted = false;
     for (int h = 0; h < 14 && !accepted; ++h) {
-      double mx = -INFINITY;
-      for (int k = threadIdx.x; k < nk; k += blockDim.x) {
-        pr[k] = log(fmax(w[k], 1e-300)) - step * g[k];
-        mx = fmax(mx, pr[k]);
+      // proposal exp(log w - step g), normalised and floored (w is at most one,
+      // and |step g| at most o.step: the largest exponent needs no search
+      // unless the step is very long)
+      double mx = o.step;
+      if (o.step > 100.0) {
+        mx = -INFINITY;
+        for (int k = tid; k < K; k += nt) mx = fmax(mx, lw[k] - step * g[k]);
+        mx = sums.max(mx);
       }
-      mx = X.max(mx);
-      for (int k = threadIdx.x; k < nk; k += blockDim.x) pr[k] = exp(pr[k] - mx);
+      double t[1] = {0.0};
+      for (int k = tid; k < K; k += nt) {
+        const double e = w[k] > 0.0 ? exp(lw[k] - step * g[k] - mx) : 0.0;
+        pr[k] = e;
+        t[0] += e;
+      }
+      sums(t);
+      const double all = fmax(t[0], 1e-300);
+      for (int k = tid; k < K; k += nt) pr[k] = fmax(o.floor, 0.0) + residual * (pr[k] / all);
       __syncthreads();
-      double sum = 0.0;
-      for (int k = threadIdx.x; k < nk; k += blockDim.x) sum += pr[k];
-      sum = fmax(X.sum(sum), 1e-300);
-      for (int k = threadIdx.x; k < nk; k += blockDim.x) pr[k] /= sum;
-      __syncthreads();
-      apply_floor_cl(X, pr, nk, K, o.floor);
-      double s2, b2, chi2;
-      rw_fit_cl(X, cvr, pr, nk, nq, y, sg, o, mix, &s2, &b2, &chi2);
-      if (chi2 + o.kl * kl_div_cl(X, pr, nk, prior) <= objective + 1e-12) accepted = true;
+      evaluate(pr, lp);
+      if (chi + o.kl * kl <= objective + 1e-12) accepted = true;
       else step *= 0.5;
     }
-    if (!accepted) break;
-    double delta = 0.0;
-    for (int k = threadIdx.x; k < nk; k += blockDim.x) delta += fabs(pr[k] - w[k]);
-    delta = X.sum(delta);
-    for (int k = threadIdx.x; k < nk; k += blockDim.x) w[k] = pr[k];
-    __syncthreads();
-    if (delta <= o.tol) {
+    if (!accepted) {
+      evaluate(w, lw);  // back at the last accepted weights
+      break;
+    }
+    double t[1] = {0.0};
+    for (int k = tid; k < K; k += nt) {
+      t[0] += fabs(pr[k] - w[k]);
+      w[k] = pr[k];
+      lw[k] = lp[k];
+    }
+    sums(t);
+    if (t[0] <= o.tol) {
       converged = 1;
       break;
     }
   }
-  rw_fit_cl(X, cvr, w, nk, nq, y, sg, o, mix, &s, &b, &chi);
-  const double kl = kl_div_cl(X, w, nk, prior);
-  for (int k = threadIdx.x; k < nk; k += blockDim.x) w_out[k0 + k] = w[k];
-  if (rank == 0 && threadIdx.x == 0) {
-    out[0] = best;
-    out[1] = s;
-    out[2] = b;
-    out[3] = chi;
-    out[4] = kl;
-    out[5] = iterations;
-    out[6] = converged;
+  if (rank == 0) {
+    for (int k = tid; k < K; k += nt) w_out[k] = w[k];
+    if (tid == 0) {
+      out[0] = best;
+      out[1] = s;
+      out[2] = b;
+      out[3] = chi;
+      out[4] = kl;
+      out[5] = iterations;
+      out[6] = converged;
+    }
   }
-  X.cl.sync();  // no CTA leaves while a peer may still read its shared memory
+  if constexpr (CL > 1) cg::this_cluster().sync();  // no CTA leaves while a peer may still read its shared memory
+}
+
+template <int CL>
+void launch_reweight(cudaStream_t s, size_t smem, const double* curves, const double* fitc, int n_cand, int K, int nq,
+                     const double* y, const double* sg, const double* weights, const double* dcurves, RwOpts o,
+                     double* w_out, double* out) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(CL);
+  cfg.blockDim = dim3(rw_threads(nq));
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = CL;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = CL > 1 ? 1 : 0;
+  CRAB_CUDA_CHECK(cudaLaunchKernelEx(&cfg, k_ens_reweight<CL>, curves, fitc, n_cand, K, nq, y, sg, weights, dcurves, o,
+                                     w_out, out));
 }
 
 // Derivative curves dI/dc1 and dI/dc2 of every conformer at every candidate:
@@ -737,18 +944,21 @@ static void ensemble_launch_curves(EnsemblePlan& E, int Ksel) {
 }
 
 static size_t weights_smem(int K, int64_t nq) {
-  int n2 = 1;
-  while (n2 < K) n2 <<= 1;
-  return (size_t)(3 * K + 2 * nq + n2) * sizeof(double);
+  return (ew_doubles(K, (int)nq) + (ew_on_chip(K, (int)nq) ? (size_t)K * nq : 0)) * sizeof(double);
 }
+
+// Cluster of the reweighting: one CTA while its shared memory holds the curves.
+static int rw_cluster(int K, int64_t nq) { return rw_on_chip(K, (int)nq, 1) ? 1 : kRwCluster; }
 
 static void ensemble_fit_buffers(EnsemblePlan& E, const double* y, const double* sg) {
   crab_ctx* ctx = E.ctx;
-  // shared-memory opt-in for the largest subset, done before any graph capture
-  const size_t shm = weights_smem(E.K, E.nq), shr = rw_smem(E.K, (int)E.nq);
-  require(shm <= 200 * 1024 && shr <= 200 * 1024, "ensemble too large for the on-chip weight fit");
-  CRAB_CUDA_CHECK(cudaFuncSetAttribute(k_ens_weights, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max<size_t>(shm, 48 * 1024)));
-  CRAB_CUDA_CHECK(cudaFuncSetAttribute(k_ens_reweight, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max<size_t>(shr, 48 * 1024)));
+  // shared-memory opt-in of both kernels, done before any graph capture
+  require(weights_smem(E.K, E.nq) <= kEnsSmem && rw_smem(E.K, (int)E.nq, rw_cluster(E.K, E.nq)) <= kEnsSmem,
+          "ensemble too large for the on-chip weight fit");
+  CRAB_CUDA_CHECK(cudaFuncSetAttribute(k_ens_weights, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kEnsSmem));
+  CRAB_CUDA_CHECK(cudaFuncSetAttribute(k_ens_reweight<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kEnsSmem));
+  CRAB_CUDA_CHECK(
+      cudaFuncSetAttribute(k_ens_reweight<kRwCluster>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kEnsSmem));
   if (!E.d_y) {
     E.d_y = E.alloc<double>(E.nq);
     E.d_sg = E.alloc<double>(E.nq);
@@ -769,7 +979,7 @@ static void ensemble_launch_fit(EnsemblePlan& E, int Ksel, const EnsOpts& eo, co
   cudaStream_t sm = ctx->stream;
   ensemble_launch_curves(E, Ksel);
   const size_t shm = weights_smem(Ksel, E.nq);
-  k_ens_weights<<<E.n_cand, kEW, shm, sm>>>(E.d_curves, Ksel, (int)E.nq, E.d_y, E.d_sg, eo, E.d_weights, E.d_fit,
+  k_ens_weights<<<E.n_cand, kWT, shm, sm>>>(E.d_curves, Ksel, (int)E.nq, E.d_y, E.d_sg, eo, E.d_weights, E.d_fit,
                                             E.d_fitted, E.d_gradw);
   CRAB_CUDA_CHECK(cudaGetLastError());
   ctx->launches += 1;
@@ -778,9 +988,11 @@ static void ensemble_launch_fit(EnsemblePlan& E, int Ksel, const EnsOpts& eo, co
                                                            E.d_damp, E.d_self, E.d_sumw, Ksel, E.d_curves,
                                                            E.d_dcurves);
     CRAB_CUDA_CHECK(cudaGetLastError());
-    const size_t shr = rw_smem(Ksel, (int)E.nq);
-    k_ens_reweight<<<kRwCluster, kEW, shr, sm>>>(E.d_curves, E.d_fit, E.n_cand, Ksel, (int)E.nq, E.d_y, E.d_sg,
-                                                 E.d_weights, E.d_dcurves, *ro, E.d_wkl, E.d_out);
+    const int cl = rw_cluster(Ksel, E.nq);
+    const size_t shr = rw_smem(Ksel, (int)E.nq, cl);
+    auto* go = cl == 1 ? launch_reweight<1> : launch_reweight<kRwCluster>;
+    go(sm, shr, E.d_curves, E.d_fit, E.n_cand, Ksel, (int)E.nq, E.d_y, E.d_sg, E.d_weights, E.d_dcurves, *ro, E.d_wkl,
+       E.d_out);
     CRAB_CUDA_CHECK(cudaGetLastError());
     ctx->launches += 2;
   }
