@@ -397,7 +397,8 @@ __device__ __forceinline__ void flush_split(unsigned long long (&acc2)[Q / 2], i
 
 template <int Q, int JB, int OCC = (Q <= 64 ? 4 : (Q <= 96 ? 3 : 2)), bool FOLD = false, int CH = 1>
 __global__ void __launch_bounds__(kThreads, OCC)
-    k_pair_fp32_pq(const float4* __restrict__ atoms, const int* __restrict__ tile_type, const int4* __restrict__ work,
+    k_pair_fp32_pq(const float4* __restrict__ atoms, const int* __restrict__ tile_type,
+                   const int* __restrict__ tile_fill, const int4* __restrict__ work,
                    int n_work, const float4* __restrict__ qpar, const int2* __restrict__ qrange, int nq, int T,
                    int wide, double* __restrict__ partials, int* __restrict__ status, int* __restrict__ next_work,
                    const int64_t* __restrict__ work_out,
@@ -434,7 +435,7 @@ __global__ void __launch_bounds__(kThreads, OCC)
     const float4 ai = atoms[(size_t)it * kTile + tid];
     const float4 qp = qpar[qb];
     const int2 qr = qrange[qb];
-    const int ti = tile_type[it];
+    const int ti = tile_type[it], fill_i = tile_fill[it];
     unsigned long long acc2[Q / 2];
 #pragma unroll
     for (int m = 0; m < Q / 2; ++m) acc2[m] = 0ull;
@@ -474,9 +475,13 @@ __global__ void __launch_bounds__(kThreads, OCC)
         break;
       }
       const bool diag = (jt == it);
+      // j atoms that add anything for this warp: no padding slots, none up to
+      // the warp's first i atom on the diagonal, none for a warp of padding
+      // (a zero weight adds zeros, so the sums keep their bits)
+      const int jlo = diag ? (tid & ~31) : 0, jhi = (tid & ~31) < fill_i ? (tile_fill[jt] + JB - 1) / JB * JB : 0;
       if constexpr (CH == 2) {
 #pragma unroll 1
-        for (int j = 0; j < kTile; ++j) {
+        for (int j = jlo; j < jhi; ++j) {
           const float4 aj = sj[buf][j];
           const float wj = (diag && j <= tid) ? 0.0f : aj.w;
           unsigned long long nl2, sx, dx, sy, dy;
@@ -493,7 +498,7 @@ __global__ void __launch_bounds__(kThreads, OCC)
         }
       } else
 #pragma unroll 1
-      for (int j = 0; j < kTile; j += JB) {
+      for (int j = jlo; j < jhi; j += JB) {
         unsigned long long u2[JB], nl2[JB], s2[JB], d2[JB];
 #pragma unroll
         for (int c = 0; c < JB; ++c) {
@@ -1069,7 +1074,7 @@ void launch_fp32(cudaStream_t stream, int sm_count, const float4* atoms, const i
 }
 
 template <int Q, int JB, int OCC, bool FOLD = false, int CH = 1>
-void launch_fp32_pq(cudaStream_t stream, int sm_count, const float4* atoms, const int* tt, const int4* work,
+void launch_fp32_pq(cudaStream_t stream, int sm_count, const float4* atoms, const int* tt, const int* fill, const int4* work,
                     int n_work, const float4* qpar, const int2* qrange, int nq, int T, int wide, double* partials,
                     int* status, int* next_work, const int64_t* work_out, const double* item_scale,
                     int budget) {
@@ -1077,7 +1082,7 @@ void launch_fp32_pq(cudaStream_t stream, int sm_count, const float4* atoms, cons
   CRAB_CUDA_CHECK(
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pair_fp32_pq<Q, JB, OCC, FOLD, CH>, kThreads, 0));
   int grid = std::max(1, std::min(n_work, sm_count * std::max(per_sm, 1)));
-  k_pair_fp32_pq<Q, JB, OCC, FOLD, CH><<<grid, kThreads, 0, stream>>>(atoms, tt, work, n_work, qpar, qrange, nq, T, wide, partials,
+  k_pair_fp32_pq<Q, JB, OCC, FOLD, CH><<<grid, kThreads, 0, stream>>>(atoms, tt, fill, work, n_work, qpar, qrange, nq, T, wide, partials,
                                                         status, next_work, work_out, item_scale, budget);
   CRAB_CUDA_CHECK(cudaGetLastError());
 }
@@ -1359,6 +1364,15 @@ void configure_fp32(crab_ctx* ctx, PairPlan& P, int Q, int jb) {
   P.hist.active = false;
   if (!P.d_atoms)
     P.d_atoms = upload(ctx, P, P.owned, "atoms", (const float4*)P.L.atoms.data(), (size_t)P.L.n_pad, ctx->stream);
+  if (!P.d_fill) {  // slots of each tile up to its last atom with a weight
+    std::vector<int> fill(P.L.n_tiles);
+    for (int t = 0; t < P.L.n_tiles; ++t) {
+      int n = kTile;
+      while (n > 0 && P.L.atoms[4 * ((size_t)t * kTile + n - 1) + 3] == 0.0f) --n;
+      fill[t] = n;
+    }
+    P.d_fill = upload(ctx, P, P.owned, "tile_fill", fill.data(), fill.size(), ctx->stream);
+  }
   P.jb = jb;
   for (void* p : P.qcfg) cudaFree(p);
   P.qcfg.clear();
@@ -1576,7 +1590,7 @@ void pair_plan_launch(crab_ctx* ctx, PairPlan& P, cudaStream_t s, bool timed) {
 #undef CRAB_LAUNCH
 #define CRAB_LAUNCH_PQ(QQ, JJ, OO, CODE)                                                                        \
   if (P.Q == QQ && P.jb == CODE) {                                                                               \
-    launch_fp32_pq<QQ, JJ, OO>(s, ctx->sm_count, P.d_atoms, P.d_tile_type, P.d_work, P.n_work, P.d_qpar,          \
+    launch_fp32_pq<QQ, JJ, OO>(s, ctx->sm_count, P.d_atoms, P.d_tile_type, P.d_fill, P.d_work, P.n_work, P.d_qpar,          \
                                P.d_qrange, nq, T, P.wide, P.d_out, P.d_status, P.d_next, P.d_work_out, P.d_scale,            \
                                ctx->wait_budget);                                                                 \
     launched = true;                                                                                             \
@@ -1593,7 +1607,7 @@ void pair_plan_launch(crab_ctx* ctx, PairPlan& P, cudaStream_t s, bool timed) {
 #undef CRAB_LAUNCH_PQ
 #define CRAB_LAUNCH_PQF(QQ, JJ, OO, CODE)                                                                       \
   if (P.Q == QQ && P.jb == CODE) {                                                                               \
-    launch_fp32_pq<QQ, JJ, OO, true>(s, ctx->sm_count, P.d_atoms, P.d_tile_type, P.d_work, P.n_work, P.d_qpar,    \
+    launch_fp32_pq<QQ, JJ, OO, true>(s, ctx->sm_count, P.d_atoms, P.d_tile_type, P.d_fill, P.d_work, P.n_work, P.d_qpar,    \
                                      P.d_qrange, nq, T, P.wide, P.d_out, P.d_status, P.d_next, P.d_work_out, P.d_scale,      \
                                      ctx->wait_budget);                                                           \
     launched = true;                                                                                             \
@@ -1612,11 +1626,11 @@ void pair_plan_launch(crab_ctx* ctx, PairPlan& P, cudaStream_t s, bool timed) {
 #define CRAB_LAUNCH_PQ2C(QQ)                                                                                    \
   if (P.Q == QQ && P.jb == kFolded2c) {                                                                          \
     if (P.hmax > kMax2cHalfAngle)                                                                                \
-      launch_fp32_pq<QQ, 1, 2, true>(s, ctx->sm_count, P.d_atoms, P.d_tile_type, P.d_work, P.n_work, P.d_qpar,    \
+      launch_fp32_pq<QQ, 1, 2, true>(s, ctx->sm_count, P.d_atoms, P.d_tile_type, P.d_fill, P.d_work, P.n_work, P.d_qpar,    \
                                      P.d_qrange, nq, T, P.wide, P.d_out, P.d_status, P.d_next, P.d_work_out, P.d_scale,      \
                                      ctx->wait_budget);                                                           \
     else                                                                                                         \
-      launch_fp32_pq<QQ, 1, 2, true, 2>(s, ctx->sm_count, P.d_atoms, P.d_tile_type, P.d_work, P.n_work,          \
+      launch_fp32_pq<QQ, 1, 2, true, 2>(s, ctx->sm_count, P.d_atoms, P.d_tile_type, P.d_fill, P.d_work, P.n_work,          \
                                         P.d_qpar, P.d_qrange, nq, T, P.wide, P.d_out, P.d_status, P.d_next,       \
                                         P.d_work_out, P.d_scale, ctx->wait_budget);                                          \
     launched = true;                                                                                             \

@@ -284,6 +284,7 @@ struct PairPlan {
   float4* d_atoms = nullptr;
   double4* d_atoms64 = nullptr;
   int* d_tile_type = nullptr;
+  int* d_fill = nullptr;  // recurrence plans: slots of each tile up to its last weighted atom
   int4* d_work = nullptr;
   float4* d_qpar = nullptr;
   int2* d_qrange = nullptr;
