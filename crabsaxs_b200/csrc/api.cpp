@@ -258,6 +258,7 @@ GridResult hydration_sites(crab_ctx* ctx, const crab_struct* st, const crab_solv
 void debye_basis(crab_ctx* ctx, const crab_struct* st, const double* q, int64_t nq, const crab_solvent& s,
                  bool implicit, double* out6, bool fp64, int shard, int n_shards) {
   TraceScope trace("debye_basis");
+  if (!fp64 && debye_terms_device(ctx, st, q, nq, &s, implicit, out6, shard, n_shards)) return;
   GridResult g;
   const bool grid = s.hydration_model != CRAB_HYD_ANALYTIC;
   if (grid) {
@@ -283,6 +284,10 @@ void debye_basis(crab_ctx* ctx, const crab_struct* st, const double* q, int64_t 
 
 void debye_vacuum(crab_ctx* ctx, const crab_struct* st, const double* q, int64_t nq, bool implicit, double* out,
                   bool fp64) {
+  if (!fp64 && debye_terms_device(ctx, st, q, nq, nullptr, implicit, out, 0, 1)) {
+    for (int64_t k = 0; k < nq; ++k) out[k] = std::fmax(out[k], 0.0);
+    return;
+  }
   TypedAtoms t = type_atoms(st, implicit, TermSet::Vacuum, nullptr);
   std::vector<double> V, E, H;
   amplitude_tables(t, q, nq, nullptr, implicit, 0.0, V, E, H);

@@ -60,8 +60,8 @@ using namespace dev;
 
 constexpr int kHT = 1024;                     // threads of a pair CTA
 constexpr int kHWarps = kHT / 32;
-constexpr int kChunkAtoms = 64;               // j atoms of a unit
-constexpr int kChunkBytes = kChunkAtoms * 12; // 32 x {x0,x1,y0,y1}, then 32 x {z0,z1}
+constexpr int kChunkAtoms = kHistChunkAtoms;  // j atoms of a unit
+constexpr int kChunkBytes = kHistChunkBytes;  // 32 x {x0,x1,y0,y1}, then 32 x {z0,z1}
 constexpr int kHistMaxBins = 22400;           // 2 words per bin beside the warps' double buffers in 227 KB
 constexpr int kHistMinBins = 4096;
 constexpr double kHistStep = 0.005;           // q_max h aimed at
@@ -549,38 +549,40 @@ int hist_bins(double reach, double qmax) {
   return ((int)std::max(want, (double)kHistMinBins - 8.0) + 8 + kHistW - 1) / kHistW * kHistW;
 }
 
+bool hist_structure_bins(double reach, double qmax, int* bins, float* inv_h) {
+  reach = std::max(reach, 1e-3) * 1.0001 + 1e-3;
+  *bins = std::min(hist_bins(reach, qmax), kHistMaxBins);
+  if (*bins == 0) return false;
+  *inv_h = (float)((double)(*bins - 4) / reach);  // every r/h stays below bins - 2 after its roundings
+  return true;
+}
+
 bool hist_plan_init(crab_ctx* ctx, PairPlan& P) {
-  HistPart& H = P.hist;
   double qmax = 0.0;
   for (double v : P.q) qmax = std::max(qmax, v);
   const Layout& L = P.L;
   const int T = L.T;
   const std::vector<int> seg = P.segments.empty() ? std::vector<int>{0, L.n_tiles} : P.segments;
   const int S = (int)seg.size() - 1;
-  struct Range {
-    int t0 = 0, n = 0;
-    int64_t atoms = 0;
-    double w = 0.0;
-  };
+  HistShape X;
+  X.S = S;
   // every structure's own bins: they span its largest distance, h being the
   // inverse of an FP32 number so that r/h carries no common error
-  std::vector<int> bins(S);
-  std::vector<float> inv_h(S);
-  for (int c = 0; c < S; ++c) {
-    const double reach = std::max(P.segments.empty() ? L.extent : P.seg_extent[c], 1e-3) * 1.0001 + 1e-3;
-    bins[c] = std::min(hist_bins(reach, qmax), kHistMaxBins);
-    if (bins[c] == 0) return false;
-    inv_h[c] = (float)((double)(bins[c] - 4) / reach);  // every r/h stays below bins - 2 after its roundings
-  }
-  std::vector<Range> uni((size_t)S * T), loose((size_t)S * T);
+  X.bins.resize(S);
+  X.inv_h.resize(S);
+  for (int c = 0; c < S; ++c)
+    if (!hist_structure_bins(P.segments.empty() ? L.extent : P.seg_extent[c], qmax, &X.bins[c], &X.inv_h[c]))
+      return false;
+  X.uni.resize((size_t)S * T);
+  X.loose.resize((size_t)S * T);
+  std::vector<HistRange>&uni = X.uni, &loose = X.loose;
   std::vector<unsigned char> pts;
   pts.reserve((size_t)(L.n_tiles + 2 * S) * 2 * kChunkBytes);
-  std::vector<int> tcnt;
   std::vector<double> weight;
-  bool any_loose = false;
-  double sumw = 0.0;
+  std::vector<int>& tcnt = X.tile_cnt;
+  double& sumw = X.sum_abs_w;
   std::vector<int64_t> other;
-  auto append = [&](Range& R, const float* a, double w, int64_t& fill) {
+  auto append = [&](HistRange& R, const float* a, double w, int64_t& fill) {
     if (fill % kTile == 0) {
       pts.resize(pts.size() + 2 * kChunkBytes, 0);
       tcnt.push_back(0);
@@ -616,8 +618,8 @@ bool hist_plan_init(crab_ctx* ctx, PairPlan& P) {
         if (votes == 0) major = w;
         votes += w == major ? 1 : -1;
       }
-      Range& U = uni[(size_t)c * T + ty];
-      Range& Lo = loose[(size_t)c * T + ty];
+      HistRange& U = uni[(size_t)c * T + ty];
+      HistRange& Lo = loose[(size_t)c * T + ty];
       U.w = (double)major;
       int64_t fill = 0;
       other.clear();
@@ -632,11 +634,25 @@ bool hist_plan_init(crab_ctx* ctx, PairPlan& P) {
       fill = 0;
       for (int64_t i = 0; i < m; ++i)
         if (a[4 * i + 3] != 0.0f && a[4 * i + 3] == major) append(U, a + 4 * i, (double)major, fill);
-      any_loose = any_loose || !other.empty();
+      X.any_loose = X.any_loose || !other.empty();
       t0 = t1;
     }
     sumw = std::max(sumw, s1);
   }
+  return hist_build(ctx, P, X, &pts, &weight);
+}
+
+bool hist_build(crab_ctx* ctx, PairPlan& P, HistShape& X, const std::vector<unsigned char>* pts,
+                const std::vector<double>* weight) {
+  typedef HistRange Range;
+  HistPart& H = P.hist;
+  const int T = P.L.T, S = X.S;
+  const std::vector<Range>&uni = X.uni, &loose = X.loose;
+  const std::vector<int>& bins = X.bins;
+  const std::vector<float>& inv_h = X.inv_h;
+  const std::vector<int>& tcnt = X.tile_cnt;
+  const bool any_loose = X.any_loose;
+  const double sumw = X.sum_abs_w;
   // rows: class pairs of uniform tiles, and the tile sets with a loose member
   std::vector<HistRow> rows, lrows;
   std::vector<double> pairs, lpairs;  // of every row
@@ -693,7 +709,8 @@ bool hist_plan_init(crab_ctx* ctx, PairPlan& P) {
         if (o.loose >= 0) loose_bins += bins[c];
         if (o.uniform >= 0 || o.loose >= 0) outs.push_back(o);
       }
-  if (outs.empty() || all_units > (int64_t)1 << 30) return false;  // unit numbers are 32-bit
+  // unit numbers are 32-bit, and rows with loose members are all resident
+  if (outs.empty() || all_units > (int64_t)1 << 30 || loose_bins > (int64_t)1 << 27) return false;
   // loose sums: the largest power of two that keeps Σ|w w| below 2^61 steps
   int ex = 0;
   std::frexp(std::max(sumw * sumw, 1e-300), &ex);
@@ -769,15 +786,18 @@ bool hist_plan_init(crab_ctx* ctx, PairPlan& P) {
     starts.insert(starts.end(), st.begin(), st.end());
   }
   HistBlob blob;
-  blob.bytes.reserve(pts.size() + weight.size() * 8 + drows.size() * 64 + outs.size() * 64 + 65536);
-  const size_t o_pts = blob.add(pts), o_cnt = blob.add(tcnt), o_rows = blob.add(drows), o_outs = blob.add(outs),
-               o_blocks = blob.add(blocks), o_start = blob.add(starts), o_q = blob.add(P.q),
-               o_w = any_loose ? blob.add(weight) : 0;
+  blob.bytes.reserve((pts ? pts->size() + weight->size() * 8 : 0) + drows.size() * 64 + outs.size() * 64 + 65536);
+  const size_t o_cnt = blob.add(tcnt), o_rows = blob.add(drows), o_outs = blob.add(outs), o_blocks = blob.add(blocks),
+               o_start = blob.add(starts), o_q = blob.add(P.q), o_pts = pts ? blob.add(*pts) : 0,
+               o_w = pts && any_loose ? blob.add(*weight) : 0, o_more = blob.add(X.more);
   auto* d = (unsigned char*)plan_alloc(ctx, P, P.owned, "hist_in", blob.bytes.size());
   copy_h2d(ctx, d, blob.bytes.data(), blob.bytes.size(), ctx->stream);
-  H.d_pts = d + o_pts;
+  H.d_pts = pts ? d + o_pts : (unsigned char*)plan_alloc(ctx, P, P.owned, "hist_pts", tcnt.size() * 2 * kChunkBytes);
+  H.d_weight = !any_loose ? nullptr
+               : pts      ? (double*)(d + o_w)
+                          : (double*)plan_alloc(ctx, P, P.owned, "hist_w", tcnt.size() * kTile * sizeof(double));
+  H.d_more = d + o_more;
   H.d_tile_cnt = (int*)(d + o_cnt);
-  H.d_weight = any_loose ? (double*)(d + o_w) : nullptr;
   H.d_rows = (HistRow*)(d + o_rows);
   H.d_outs = (HistOut*)(d + o_outs);
   H.d_blocks = (HistBlock*)(d + o_blocks);

@@ -171,6 +171,15 @@ double adaptive_site_volume(double spacing);
 int united_atom_group(const char* residue, const char* name);
 double sinc(double x);
 
+// One class's amplitudes as numbers: form factor sum_k a_k exp(-b_k (q/4 pi)²) + c (plus for water twice
+// its hydrogen's times sinc(0.9572 q)), displaced volume and analytic shell volume with their 2/3 powers.
+struct ClassAmp {
+  double a[5], b[5], c;
+  double volume, pv, shell, ps;
+  int water;
+};
+ClassAmp class_amp(const AtomClass& c, bool implicit_h, double thickness);
+
 // Per-class amplitudes without occupancy for the Debye solvent model
 // (solvent.rs:454-488): vacuum, excluded (times density), analytic shell.
 void debye_class_amplitudes(const AtomClass& c, bool implicit_h, double q, double density, double thickness,
@@ -244,6 +253,22 @@ struct HistOut {  // a type pair: its counted and its loose sums (-1: none), out
   int out, bins, seg;
   double ww;
 };
+constexpr int kHistChunkAtoms = 64, kHistChunkBytes = kHistChunkAtoms * 12;
+struct HistRange {  // the tiles of one type's counted or loose atoms
+  int t0 = 0, n = 0;
+  int64_t atoms = 0;
+  double w = 0.0;
+};
+struct HistShape {  // what a histogram plan is built from: per structure its bins, per (structure, type) its tiles
+  int S = 1;
+  std::vector<int> bins;
+  std::vector<float> inv_h;
+  std::vector<HistRange> uni, loose;  // a type's loose tiles come right before its counted ones
+  std::vector<int> tile_cnt;
+  double sum_abs_w = 0.0;
+  bool any_loose = false;
+  std::vector<unsigned char> more;  // uploaded with the plan's own tables (HistPart::d_more)
+};
 struct HistBlock {  // type pairs of one structure that the transform takes together
   int out0, n, bins;
   double h;
@@ -259,6 +284,7 @@ struct HistPart {
   int64_t acc_bins = 0, loose_bins = 0;
   std::vector<HistGroup> groups;
   unsigned char* d_pts = nullptr;
+  unsigned char* d_more = nullptr;
   int* d_tile_cnt = nullptr;
   double* d_weight = nullptr;
   HistRow* d_rows = nullptr;
@@ -330,8 +356,16 @@ constexpr int kHistVariant = 16;  // the distance histogram's variant code
 // Builds the histogram form of a plan and makes it active; false when its
 // bins do not fit an SM's shared memory or there is no pair to sum.
 bool hist_plan_init(crab_ctx* ctx, PairPlan& P);
+// Bins and 1/h of a structure of that largest distance (false: no fit).
+bool hist_structure_bins(double reach, double qmax, int* bins, float* inv_h);
+// Tables, work lists and buffers from the tiles; with pts null the points (and
+// loose weights) are left for the caller's kernels to write.
+bool hist_build(crab_ctx* ctx, PairPlan& P, HistShape& X, const std::vector<unsigned char>* pts,
+                const std::vector<double>* weight);
 void hist_plan_launch(crab_ctx* ctx, PairPlan& P, cudaStream_t s);
 void lattice_plan_init(crab_ctx* ctx, PairPlan& P, const int32_t* cells, int64_t m, double spacing);
+// The same with the cells (3 int32 each) on the device, every coordinate's span below `span` cells.
+void lattice_plan_init_device(crab_ctx* ctx, PairPlan& P, int64_t m, double spacing, const int64_t* span);
 void lattice_plan_launch(crab_ctx* ctx, PairPlan& P, cudaStream_t s);
 bool q_grid_uniform(const double* q, int64_t nq);
 std::unique_ptr<PairPlan> make_pair_plan(crab_ctx* ctx, Layout&& L, const double* q, int64_t nq, bool fp64,
@@ -379,6 +413,8 @@ struct GridResult {
   double spacing = 0.0;
   double voxel_volume = 0.0;
   int64_t m = 0;                   // number of sites
+  double outer = 0.0;               // no site is farther than this from some atom
+  const int32_t* d_cells = nullptr;
   const double* d_sites = nullptr;  // the sites on the device, valid until the context's next grid build
   uint64_t build = 0;               // crab_ctx::grid_builds of the build that made this result
 };

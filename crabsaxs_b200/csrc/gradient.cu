@@ -164,16 +164,9 @@ void chi2_grad_impl(crab_ctx* ctx, const crab_struct* st, const double* q, const
   require(std::isfinite(scale) && std::isfinite(background), "scale and background must be finite");
   TypedAtoms t = type_atoms(st, implicit, TermSet::SolventAnalytic, nullptr);
   const int T = t.T;
-  std::vector<double> V, E, H;
+  std::vector<double> V, E, H, b6(6 * nq), I(nq);
   amplitude_tables(t, q, nq, &s, implicit, 0.0, V, E, H);
-  Partials P = partials_for(ctx, t, q, nq, false, nullptr);
-  std::vector<double> b6(6 * nq), I(nq);
-  quadratic_terms(P, V.data(), V.data(), b6.data());
-  quadratic_terms(P, E.data(), E.data(), b6.data() + nq);
-  quadratic_terms(P, H.data(), H.data(), b6.data() + 2 * nq);
-  quadratic_terms(P, V.data(), E.data(), b6.data() + 3 * nq);
-  quadratic_terms(P, V.data(), H.data(), b6.data() + 4 * nq);
-  quadratic_terms(P, E.data(), H.data(), b6.data() + 5 * nq);
+  debye_basis(ctx, st, q, nq, s, implicit, b6.data(), false);
   combine_basis(q, nq, b6.data(), s.c1, s.c2, I.data());
   const double dof = (double)std::max<int64_t>(nq - 1, 1);
   std::vector<double> w(nq);
@@ -208,15 +201,19 @@ void chi2_grad_impl(crab_ctx* ctx, const crab_struct* st, const double* q, const
   std::vector<double> alpha((size_t)NP * nq, 0.0);
   double qmax = 0.0;
   for (int64_t k = 0; k < nq; ++k) qmax = std::max(qmax, q[k]);
+  for (int64_t k = 0; k < nq; ++k) {  // V becomes the combined amplitude
+    const double G = excluded_volume_scale(q[k], s.c1);
+    for (int a = 0; a < T; ++a) {
+      const size_t o = (size_t)a * nq + k;
+      V[o] = V[o] - G * E[o] + s.c2 * H[o];
+    }
+  }
   for (int a = 0; a < T; ++a)
     for (int bb = a; bb < T; ++bb)
-      for (int64_t k = 0; k < nq; ++k) {
-        if (!(q[k] > 0.0)) continue;
-        const double G = excluded_volume_scale(q[k], s.c1);
-        const double Aa = V[(size_t)a * nq + k] - G * E[(size_t)a * nq + k] + s.c2 * H[(size_t)a * nq + k];
-        const double Ab = V[(size_t)bb * nq + k] - G * E[(size_t)bb * nq + k] + s.c2 * H[(size_t)bb * nq + k];
-        alpha[(size_t)pair_index(a, bb, T) * nq + k] = 2.0 * w[k] * Aa * Ab;
-      }
+      for (int64_t k = 0; k < nq; ++k)
+        if (q[k] > 0.0)
+          alpha[(size_t)pair_index(a, bb, T) * nq + k] =
+              2.0 * w[k] * V[(size_t)a * nq + k] * V[(size_t)bb * nq + k];
   Layout L = build_layout(t.xyz.data(), t.w.data(), t.type.data(), (int64_t)t.w.size(), T, false);
   // radial grid: dr = 0.02 / q_max up to the largest pair distance (bounded by the layout's extent)
   const double dr = qmax > 0.0 ? 0.02 / qmax : 1.0;

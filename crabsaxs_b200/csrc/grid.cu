@@ -385,6 +385,7 @@ GridResult compact_sites(crab_ctx* ctx, const uint8_t* a, const uint8_t* b, uint
     k_emit<<<(unsigned)chunks, kScanThreads, 0, s>>>(a, b, count, kind, bx, d_off, d_sites, d_cells);
     CRAB_CUDA_CHECK(cudaGetLastError());
     r.d_sites = d_sites;
+    r.d_cells = d_cells;
     if (to_host) {
       r.sites.resize(3 * m);
       r.cells.resize(3 * m);
@@ -468,6 +469,7 @@ GridResult adaptive_grid_device(crab_ctx* ctx, const double* xyz, int64_t n, dou
   ctx->launches += 2;
   r = compact_sites(ctx, shell, mol, count, 0, b, to_host);
   r.voxel_volume = adaptive_site_volume(spacing);
+  r.outer = outer;
   return r;
 }
 
@@ -540,6 +542,7 @@ GridResult exterior_grid_device(crab_ctx* ctx, const double* xyz, const int8_t* 
   ctx->launches += 1;
   r = compact_sites(ctx, state, state, count, 1, b, to_host);
   r.voxel_volume = (spacing * spacing) * spacing;
+  r.outer = vmax + probe + thickness;
   return r;
 }
 

@@ -114,6 +114,22 @@ void lattice_plan_init(crab_ctx* ctx, PairPlan& P, const int32_t* cells, int64_t
   Lp.active = true;
 }
 
+void lattice_plan_init_device(crab_ctx* ctx, PairPlan& P, int64_t m, double spacing, const int64_t* span) {
+  LatticePart& Lp = P.lattice;
+  Lp.m = m;
+  Lp.spacing = spacing;
+  int64_t nmax = 0;
+  for (int d = 0; d < 3; ++d) nmax += span[d] * span[d];
+  require(nmax < (int64_t)1 << 30, "hydration lattice too large for the site histogram");
+  require((m + kLT - 1) / kLT <= 65535, "too many lattice sites for one histogram launch");
+  Lp.bins = (int)nmax + 1;
+  Lp.d_cells = (int4*)plan_alloc(ctx, P, P.owned, "lattice_cells", (size_t)std::max<int64_t>(m, 1) * sizeof(int4));
+  Lp.d_hist = (unsigned long long*)plan_alloc(ctx, P, P.owned, "lattice_hist",
+                                               (size_t)Lp.bins * sizeof(unsigned long long));
+  Lp.d_out = (double*)plan_alloc(ctx, P, P.owned, "lattice_out", (size_t)std::max<int64_t>(P.nq, 1) * sizeof(double));
+  Lp.active = true;
+}
+
 void lattice_plan_launch(crab_ctx* ctx, PairPlan& P, cudaStream_t s) {
   LatticePart& Lp = P.lattice;
   if (!Lp.active || P.nq == 0) return;

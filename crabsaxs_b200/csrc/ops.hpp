@@ -44,6 +44,8 @@ GridResult hydration_sites(crab_ctx* ctx, const crab_struct* st, const crab_solv
 // shard 0 only): the element-wise sum over all shards is the whole basis.
 void debye_basis(crab_ctx* ctx, const crab_struct* st, const double* q, int64_t nq, const crab_solvent& s,
                  bool implicit, double* out6, bool fp64, int shard = 0, int n_shards = 1);
+bool debye_terms_device(crab_ctx* ctx, const crab_struct* st, const double* q, int64_t nq, const crab_solvent* solvent,
+                        bool implicit, double* out, int shard, int n_shards);
 void debye_vacuum(crab_ctx* ctx, const crab_struct* st, const double* q, int64_t nq, bool implicit, double* out,
                   bool fp64);
 void combine_basis(const double* q, int64_t nq, const double* b, double c1, double c2, double* out);

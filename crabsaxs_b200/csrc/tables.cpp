@@ -170,6 +170,33 @@ void debye_class_amplitude_rows(const AtomClass& c, bool implicit_h, const doubl
   }
 }
 
+ClassAmp class_amp(const AtomClass& c, bool implicit_h, double thickness) {
+  ClassAmp r = {};
+  if (c.element < 0) {  // a hydration site: water, the hydrogen's terms below
+    r.water = 1;
+    for (int k = 0; k < 4; ++k) {
+      r.a[k] = kElement[CRAB_EL_O].a[k];
+      r.b[k] = kElement[CRAB_EL_O].b[k];
+    }
+    r.c = kElement[CRAB_EL_O].c;
+    return r;
+  }
+  if (!(implicit_h && c.element == CRAB_EL_H)) {
+    const Gauss& g = implicit_h && c.group >= 0 ? kGroup[c.group] : kElement[c.element];
+    for (int k = 0; k < g.terms; ++k) {
+      r.a[k] = g.a[k];
+      r.b[k] = g.b[k];
+    }
+    r.c = g.c;
+  }
+  r.volume = excluded_volume_for_atom(c.element, c.group, implicit_h);
+  const double rs = std::cbrt(3.0 * r.volume / (4.0 * kPi)) + thickness / 2.0;
+  r.shell = 4.0 * kPi * (rs * rs) * thickness;
+  r.pv = std::pow(r.volume, 2.0 / 3.0);
+  r.ps = std::pow(r.shell, 2.0 / 3.0);
+  return r;
+}
+
 void multipole_class_amplitudes(const AtomClass& c, bool implicit_h, double q, double density, double thickness,
                                 double* v, double* e, double* h) {
   const double volume = excluded_volume_for_atom(c.element, c.group, implicit_h);

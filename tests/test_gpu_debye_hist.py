@@ -84,3 +84,48 @@ def test_select_refuses_bins_that_do_not_fit(engine):
         engine.check(N.lib.crab_pair_plan_run(engine.handle, plan, 1, 0, None))
     finally:
         N.lib.crab_pair_plan_destroy(plan)
+
+
+def _occupancy(kind, n, rng):
+    occ = np.ones(n)
+    if kind == "altloc":
+        at = rng.random(n) < 0.1
+        occ[at] = np.round(rng.uniform(0.3, 0.7, size=int(at.sum())), 2)
+    elif kind == "odd first":  # every class's first atom has a weight of its own, some atoms none, some negative
+        occ[:] = 0.8
+        occ[:40] = rng.uniform(0.1, 0.5, size=min(40, n))
+        occ[rng.random(n) < 0.05] = 0.0
+        occ[rng.random(n) < 0.02] = -0.4
+    elif kind == "distinct":
+        occ = rng.uniform(0.2, 1.0, size=n)
+    return occ
+
+
+@pytest.mark.parametrize("hydration", [cs.HydrationModel.Analytic, cs.HydrationModel.AdaptiveGrid,
+                                       cs.HydrationModel.Grid])
+@pytest.mark.parametrize("kind", ["ones", "altloc", "odd first", "distinct"])
+@pytest.mark.parametrize("n,implicit", [(1, True), (129, True), (700, False)])
+def test_structure_calls_match_the_fp64_path(engine, n, implicit, kind, hydration):
+    """The one-structure calls type, place and recombine on the device; the FP64 option keeps the general path.  Terms
+    relative to their q = 0 value with all occupancies positive, which bounds every |X_i Y_j| sum."""
+    rng = np.random.default_rng(n)
+    xyz = rng.uniform(-11.0, 11.0, size=(n, 3)) - 40.0
+    el = rng.choice([0, 1, 2, 3, 4, 14], size=n, p=[0.1, 0.5, 0.15, 0.15, 0.05, 0.05]).astype(np.int8)
+    group = np.where(el == 1, rng.integers(-1, 4, size=n), np.where(el == 2, 7, -1)).astype(np.int8)
+    occ = _occupancy(kind, n, rng)
+    s = cs.Structure(xyz, el, occ, group)
+    p = cs.SolventParams(c1=1.02, c2=0.9, hydration_model=hydration)
+    q = np.concatenate([[0.0], np.linspace(0.004, 0.45, 45)])
+    got = cs.debye_solvent_basis(s, q, p, implicit, engine=engine)
+    ref = cs.debye_solvent_basis(s, q, p, implicit, engine=engine, fp64=True)
+    top = cs.debye_solvent_basis(cs.Structure(xyz, el, np.abs(occ), group), [0.0], p, implicit, engine=engine, fp64=True)
+    shell = np.concatenate([xyz - 14.0, xyz + 14.0])  # reach of the sites
+    tol = _bound(shell if hydration != cs.HydrationModel.Analytic else xyz, q)
+    assert (np.abs(got - ref) / np.maximum(np.abs(top), 1e-9)).max() <= tol
+    parts = [cs.debye_solvent_basis(s, q, p, implicit, engine=engine, shard=(k, 3)) for k in range(3)]
+    assert np.abs(sum(parts) - got).max() <= 1e-12 * np.abs(got).max()
+    assert np.array_equal(cs.debye_solvent_basis(s, q, p, implicit, engine=engine), got)
+    vac = cs.debye_intensity(s, q, implicit, engine=engine)
+    v = ref[0]
+    if hydration == cs.HydrationModel.Analytic:
+        assert (np.abs(vac - np.maximum(v, 0.0)) / max(abs(top[0, 0]), 1e-9)).max() <= tol
