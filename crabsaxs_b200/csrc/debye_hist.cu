@@ -52,6 +52,7 @@
 
 #include "device_math.cuh"
 #include "engine.hpp"
+#include "tile_rows.cuh"
 
 namespace crab {
 namespace {
@@ -213,20 +214,6 @@ __device__ __forceinline__ void hist_unit(const unsigned char* ch, int e0, int n
 #pragma unroll 2
   for (int e = 0; e < full; ++e) entry(e, true);
   if (nj & 1) entry(full, false);
-}
-
-__host__ __device__ __forceinline__ int hist_units(const HistRow& r) {
-  return 2 * r.split * (r.diag ? r.ni * (r.ni + 1) / 2 : r.ni * r.nj);
-}
-
-// Tile pair p of a row: i tile and j tile, j fastest; on the diagonal row the
-// pairs i <= j in the order of j(j+1)/2 + i.
-__device__ __forceinline__ int2 hist_tiles(const HistRow& r, int p) {
-  if (!r.diag) return make_int2(r.i0 + p / r.nj, r.j0 + p % r.nj);
-  int j = (int)((sqrtf(8.0f * (float)p + 1.0f) - 1.0f) * 0.5f);
-  while ((long long)j * (j + 1) / 2 > p) --j;
-  while ((long long)(j + 1) * (j + 2) / 2 <= p) ++j;
-  return make_int2(r.i0 + (p - j * (j + 1) / 2), r.j0 + j);
 }
 
 template <int MODE>
@@ -486,38 +473,8 @@ __global__ void __launch_bounds__(256) k_hist_reduce(const double* __restrict__ 
   }
 }
 
-// CTA starts over a row list: equal shares of the cost.  A row costs its pairs
-// in units of 8192, 0.1 per unit for empty tile space, and kRowCost for the
-// flush and the wait for its last units.  (The units of a row come first, so
-// that the first part of a split owns some.)
-constexpr double kRowCost = 8.0;
+constexpr double kRowCost = 8.0;  // of a row's flush, in units of 8192 pairs
 constexpr int kSplitUnits = 8 * kHWarps;
-std::vector<int2> cta_starts(const std::vector<HistRow>& rows, const std::vector<double>& pairs, size_t r0, size_t r1,
-                             int grid, int shard, int shards) {
-  auto work = [&](size_t r) { return pairs[r] / (128.0 * kChunkAtoms) + 0.1 * hist_units(rows[r]) / rows[r].split; };
-  double total = 0.0;
-  for (size_t r = r0; r < r1; ++r) total += kRowCost + work(r);
-  const int parts = grid * shards;
-  std::vector<int2> out;
-  size_t row = r0;
-  double before = 0.0;  // cost of the rows before `row`
-  for (int p = 0; p <= grid; ++p) {
-    const double at = total * (double)(shard * grid + p) / parts;
-    while (row + 1 < r1 && before + kRowCost + work(row) <= at) before += kRowCost + work(row++);
-    const int n = hist_units(rows[row]);
-    const double in = std::min(1.0, std::max(0.0, (at - before) / work(row)));
-    int u = (int)std::ceil(in * n);
-    // rows of less than a share are not cut: each cut costs another flush
-    if (work(row) + kRowCost < total / parts) u = in > 0.5 ? n : 0;
-    if (shards > 1) u -= u % (2 * rows[row].split);  // shards take whole tile pairs
-    if (shard * grid + p == parts) {
-      row = r1 - 1;
-      u = hist_units(rows[row]);
-    }
-    out.push_back(make_int2((int)(row - r0), u));
-  }
-  return out;
-}
 
 // The plan's host arrays as one block, uploaded in one copy.
 struct HistBlob {
@@ -659,16 +616,10 @@ bool hist_build(crab_ctx* ctx, PairPlan& P, HistShape& X, const std::vector<unsi
   std::vector<HistOut> outs;
   int64_t loose_bins = 0, all_units = 0;
   int widest = 0;
-  // rows of few units (32 warps share them) split each by its four groups of i atoms
+  bool fits = true;
   auto row_of = [&](const Range& x, const Range& y, int diag, int c, int64_t acc, bool split) {
     HistRow r{x.t0, x.n, y.t0, y.n, diag, bins[c], 1, 0, 0, inv_h[c], acc};
-    const int64_t units = 2 * (diag ? (int64_t)x.n * (x.n + 1) / 2 : (int64_t)x.n * y.n);
-    if (units < (split ? (int64_t)1 << 20 : kSplitUnits)) {
-      r.igroups = x.n == 1 ? (int)((x.atoms + 31) / 32) : 4;
-      r.quarters = split ? 1 : 0;
-      r.split = r.igroups * (split ? 4 : 1);
-    }
-    all_units += units * r.split;
+    fits = hist_row_units(r, x.atoms, split, split ? (int64_t)1 << 20 : kSplitUnits, &all_units) && fits;
     widest = std::max(widest, bins[c]);
     return r;
   };
@@ -710,7 +661,7 @@ bool hist_build(crab_ctx* ctx, PairPlan& P, HistShape& X, const std::vector<unsi
         if (o.uniform >= 0 || o.loose >= 0) outs.push_back(o);
       }
   // unit numbers are 32-bit, and rows with loose members are all resident
-  if (outs.empty() || all_units > (int64_t)1 << 30 || loose_bins > (int64_t)1 << 27) return false;
+  if (outs.empty() || !fits || loose_bins > (int64_t)1 << 27) return false;
   // loose sums: the largest power of two that keeps Σ|w w| below 2^61 steps
   int ex = 0;
   std::frexp(std::max(sumw * sumw, 1e-300), &ex);
@@ -764,7 +715,7 @@ bool hist_build(crab_ctx* ctx, PairPlan& P, HistShape& X, const std::vector<unsi
       g.grid = grid_of(drows, dpairs, g.row0, drows.size());
       g.start0 = (int)starts.size();
       const std::vector<int2> st =
-          cta_starts(drows, dpairs, g.row0, g.row0 + g.n_rows, g.grid, P.shard, P.n_shards);
+          hist_starts(drows, dpairs, g.row0, g.row0 + g.n_rows, g.grid, P.shard, P.n_shards, kRowCost);
       starts.insert(starts.end(), st.begin(), st.end());
     }
     // slices of the transform: about four CTAs per SM, whole steps of kHistB bins
@@ -782,7 +733,7 @@ bool hist_build(crab_ctx* ctx, PairPlan& P, HistShape& X, const std::vector<unsi
     dpairs.insert(dpairs.end(), lpairs.begin(), lpairs.end());
     H.loose_grid = grid_of(drows, dpairs, H.loose_row0, drows.size());
     const std::vector<int2> st =
-        cta_starts(drows, dpairs, H.loose_row0, drows.size(), H.loose_grid, P.shard, P.n_shards);
+        hist_starts(drows, dpairs, H.loose_row0, drows.size(), H.loose_grid, P.shard, P.n_shards, kRowCost);
     starts.insert(starts.end(), st.begin(), st.end());
   }
   HistBlob blob;

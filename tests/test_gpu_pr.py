@@ -188,3 +188,44 @@ def test_100k_atoms_size_properties(engine):
     assert dmax >= math.sqrt(np.max(np.sum(dd * dd, -1))) - 1e-9
     total_ms, hist_ms, pairs, mode = cs.pr_last_timing(engine)
     assert pairs == n * (n - 1) / 2 and 0.0 < hist_ms <= total_ms and mode == 1
+
+
+@pytest.mark.parametrize("n", [2, 31, 33, 63, 65, 127, 129, 257, 500])
+@pytest.mark.parametrize("classes", [1, 3, 60, 70])
+@pytest.mark.parametrize("bins", [1, 37, 1600])
+def test_tile_and_class_edges_are_exact(engine, n, classes, bins):
+    """Whole and ragged warps, half tiles and tiles, one class to more than can be counted (70), and bins on both
+    sides of 32 counters a bin: integer weights, so every bin is exact in any order and must equal the oracle's."""
+    rng = np.random.default_rng(n + 7 * classes + bins)
+    xyz = np.round(rng.uniform(-9.0, 9.0, size=(n, 3)), 1) + 55.0  # distances on a grid: many near or on edges
+    w = rng.integers(1, classes + 1, size=n).astype(float)
+    dmax, hist = cs.pair_distance_histogram(xyz, w, bins, engine=engine)
+    rd, rh = O.pair_distance_histogram(xyz, w, bins)
+    assert dmax == rd and np.array_equal(hist, rh)
+
+
+def test_longest_pair_is_found_in_shells_and_rods(engine):
+    """The atoms that can end the longest pair are found from one pair and its middle: a hollow sphere (all of them),
+    a bent rod (the middle lies off the atoms), two clusters, and equal atoms."""
+    rng = np.random.default_rng(8)
+    v = rng.normal(size=(3000, 3))
+    sphere = 40.0 * v / np.sqrt((v ** 2).sum(axis=1))[:, None]
+    t = rng.uniform(0.0, 2.2, size=2500)
+    rod = np.stack([60 * np.cos(t), 60 * np.sin(t), np.zeros_like(t)], axis=1) + rng.normal(size=(2500, 3))
+    two = np.concatenate([rng.normal(size=(400, 3)), rng.normal(size=(700, 3)) + [90.0, 3.0, -8.0]])
+    for xyz in (sphere, rod, two, np.repeat(two[:5], 40, axis=0)):
+        d, h = cs.pair_distance_histogram(xyz, np.ones(len(xyz)), 50, engine=engine)
+        rd, rh = O.pair_distance_histogram(xyz, np.ones(len(xyz)), 50)
+        assert d == rd and np.array_equal(h, rh)
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf, 1e101])
+def test_bad_coordinates_are_refused_in_every_mode(engine, bad):
+    rng = np.random.default_rng(1)
+    xyz = rng.normal(size=(300, 3))
+    xyz[211, 2] = bad
+    for w in (np.ones(300), rng.uniform(size=300)):
+        with pytest.raises(cs.InvalidInput):
+            cs.pair_distance_histogram(xyz, w, 20, engine=engine)
+    d, h = cs.pair_distance_histogram(xyz[:200], np.ones(200), 20, engine=engine)
+    assert d > 0 and h.sum() == 200 * 199 / 2
