@@ -137,6 +137,12 @@ static bool excluded_zero(const AtomClass& c, bool implicit) {
   return excluded_volume_for_atom(c.element, c.group, implicit) == 0.0;
 }
 
+bool class_dropped(const AtomClass& c, bool implicit, TermSet need) {
+  if (need == TermSet::Vacuum) return vacuum_zero(c, implicit);
+  if (need == TermSet::SolventGrid) return vacuum_zero(c, implicit) && excluded_zero(c, implicit);
+  return false;
+}
+
 TypedAtoms type_atoms(const crab_struct* st, bool implicit, TermSet need, const std::vector<double>* sites) {
   TypedAtoms t;
   type_atoms_into(st, implicit, need, sites, t);
@@ -159,11 +165,7 @@ void type_atoms_into(const crab_struct* st, bool implicit, TermSet need, const s
   bool drop[kE][kG];
   for (int e = 0; e < kE; ++e)
     for (int g = 0; g < kG; ++g) {
-      const AtomClass c{e, implicit ? g - 1 : -1};
-      bool d = false;
-      if (need == TermSet::Vacuum) d = vacuum_zero(c, implicit);
-      else if (need == TermSet::SolventGrid) d = vacuum_zero(c, implicit) && excluded_zero(c, implicit);
-      drop[e][g] = d;
+      drop[e][g] = class_dropped(AtomClass{e, implicit ? g - 1 : -1}, implicit, need);
     }
   int64_t present[kE][kG] = {};
   const int8_t* el = st->elem.data();
@@ -311,11 +313,12 @@ void centre_and_rmax(const crab_struct* st, double* c, double* rmax) {
     for (int d = 0; d < 3; ++d) c[d] = c[d] + st->xyz[3 * i + d];
   const double n = (double)std::max<int64_t>(st->n, 1);
   for (int d = 0; d < 3; ++d) c[d] = c[d] / n;
-  *rmax = 0.0;
+  double r2 = 0.0;  // the root of the largest square is the largest root
   for (int64_t i = 0; i < st->n; ++i) {
     const double dx = st->xyz[3 * i] - c[0], dy = st->xyz[3 * i + 1] - c[1], dz = st->xyz[3 * i + 2] - c[2];
-    *rmax = max_num(*rmax, std::sqrt(((0.0 + dx * dx) + dy * dy) + dz * dz));
+    r2 = max_num(r2, ((0.0 + dx * dx) + dy * dy) + dz * dz);
   }
+  *rmax = std::sqrt(r2);
 }
 
 }  // namespace crab
@@ -690,12 +693,11 @@ int crab_compute_curve(crab_ctx* ctx, crab_struct* st, const double* q, int64_t 
       else if (st->n < 500) method = CRAB_METHOD_DEBYE;
       else method = CRAB_METHOD_MULTIPOLE;
     }
-    double qmax = 0.0;
-    for (int64_t k = 0; k < nq; ++k) qmax = std::fmax(qmax, q[k]);
-    double c[3], rmax;
-    centre_and_rmax(st, c, &rmax);
     int l_max = opt->l_max;
-    if (l_max == 0) {
+    if (l_max == 0 && method == CRAB_METHOD_MULTIPOLE) {
+      double qmax = 0.0, c[3], rmax;
+      for (int64_t k = 0; k < nq; ++k) qmax = std::fmax(qmax, q[k]);
+      centre_and_rmax(st, c, &rmax);
       long v = (long)std::ceil(qmax * rmax) + 8;
       l_max = (int)std::min(64L, std::max(8L, v));
     }

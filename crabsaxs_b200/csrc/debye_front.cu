@@ -200,11 +200,9 @@ bool debye_terms_device(crab_ctx* ctx, const crab_struct* st, const double* q, i
   for (int code = 0; code < kCodes; ++code) {
     const int64_t m = part[0][code] + part[1][code] + part[2][code] + part[3][code];
     const AtomClass k{code / 16, code % 16 - 1};
-    bool drop = m == 0;
-    if (!drop && !(solvent && !grid)) {  // classes without any amplitude in the terms asked for
-      const bool vac = (implicit && k.element == CRAB_EL_H) || (k.element == CRAB_EL_OTHER && k.group < 0);
-      drop = vac && (!grid || excluded_volume_for_atom(k.element, k.group, implicit) == 0.0);
-    }
+    const bool drop = m == 0 || class_dropped(k, implicit, !solvent ? TermSet::Vacuum
+                                                          : grid   ? TermSet::SolventGrid
+                                                                   : TermSet::SolventAnalytic);
     cls_of[code] = drop ? -1 : (int)cls.size();
     if (!drop) {
       cls.push_back(k);

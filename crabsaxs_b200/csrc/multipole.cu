@@ -1508,10 +1508,72 @@ __global__ void __launch_bounds__(256) k_mp_gram_reduce(const double* __restrict
   }
 }
 
+// A point as the general path builds it: centred coordinates, weight, radius.
+__device__ __forceinline__ double mp_radius(double dx, double dy, double dz) {
+  return sqrt(__dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz)));
+}
+constexpr uint32_t kMpDropped = 0xFFFFFFFFu;
+__global__ void k_mp_place(const double* __restrict__ xyz, const double* __restrict__ occ,
+                           const uint32_t* __restrict__ word, int64_t n, const int64_t* __restrict__ begin, double cx,
+                           double cy, double cz, double* __restrict__ pts) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n || word[i] == kMpDropped) return;
+  double* p = pts + 5 * (begin[word[i] >> 24] + (word[i] & 0xffffffu));
+  const double dx = __dsub_rn(xyz[3 * i], cx), dy = __dsub_rn(xyz[3 * i + 1], cy), dz = __dsub_rn(xyz[3 * i + 2], cz);
+  p[0] = dx;
+  p[1] = dy;
+  p[2] = dz;
+  p[3] = occ[i];
+  p[4] = mp_radius(dx, dy, dz);
+}
+__global__ void k_mp_place_sites(const double* __restrict__ sites, int64_t m, int64_t begin, double cx, double cy,
+                                 double cz, double* __restrict__ pts) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= m) return;
+  double* p = pts + 5 * (begin + i);
+  const double dx = __dsub_rn(sites[3 * i], cx), dy = __dsub_rn(sites[3 * i + 1], cy),
+               dz = __dsub_rn(sites[3 * i + 2], cz);
+  p[0] = dx;
+  p[1] = dy;
+  p[2] = dz;
+  p[3] = 1.0;
+  p[4] = mp_radius(dx, dy, dz);
+}
+// The largest radius of the sites, as the bits of a non-negative double.
+__global__ void k_mp_site_rmax(const double* __restrict__ sites, int64_t m, double cx, double cy, double cz,
+                               unsigned long long* __restrict__ out) {
+  double r = 0.0;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m; i += (int64_t)gridDim.x * blockDim.x)
+    r = fmax(r, mp_radius(__dsub_rn(sites[3 * i], cx), __dsub_rn(sites[3 * i + 1], cy),
+                          __dsub_rn(sites[3 * i + 2], cz)));
+  for (int o = 16; o > 0; o >>= 1) r = fmax(r, __shfl_xor_sync(0xffffffffu, r, o));
+  if ((threadIdx.x & 31) == 0) atomicMax(out, (unsigned long long)__double_as_longlong(r));
+}
+
 // ------------------------------------------------------------------ host
+
+// The points of a call whose radial range needs one segment, on the device: the
+// host makes one word per atom (class << 24 | rank in the class, in input
+// order), and k_mp_place and k_mp_place_sites write the points where the general
+// path below would have put them, by the same f64 operations.  At 100,000
+// atoms the general path's passes (typing into three arrays, distances, groups,
+// 5 doubles per point into pinned memory) are 1.4 ms of host time, this one's
+// 0.5 ms.
+struct MpFront {
+  TypedAtoms t;                // classes only
+  std::vector<int64_t> count;  // points per class
+  int64_t n = 0;
+  double centre[3], rmax = 0.0, rmax_lq = 0.0;  // all atoms; atoms and sites
+  double R = 0.0;              // of the points kept
+  GridResult g;
+  double *d_xyz = nullptr, *d_occ = nullptr;
+  uint32_t* d_word = nullptr;
+  int64_t n_atoms = 0;
+};
 
 struct MpInput {
   const TypedAtoms* t;
+  const MpFront* front = nullptr;  // the points, when they are on the device
   double centre[3];
   double rmax_lq;                 // radius for the per-q order (atoms, or atoms and sites)
   std::vector<double> amp;        // K x T x nq amplitude combinations (no occupancy)
@@ -1589,7 +1651,8 @@ void multipole_run(crab_ctx* ctx, const MpInput& in, const double* q, int64_t nq
   TraceScope trace("multipole_run");
   const TypedAtoms& t = *in.t;
   const int T = t.T, K = in.K, P = K * (K + 1) / 2;
-  const int64_t n = (int64_t)t.w.size();
+  const MpFront* front = in.front;
+  const int64_t n = front ? front->n : (int64_t)t.w.size();
   std::fill(out, out + (size_t)P * nq, 0.0);
   if (n == 0 || nq == 0) return;
   require(in.n_shards >= 1 && in.shard >= 0 && in.shard < in.n_shards, "shard index out of range");
@@ -1598,9 +1661,9 @@ void multipole_run(crab_ctx* ctx, const MpInput& in, const double* q, int64_t nq
   const int64_t own0 = n * in.shard / in.n_shards, own1 = n * (in.shard + 1) / in.n_shards;
   // geometry relative to the structure centroid (spherical.rs:165-199)
   std::vector<double>& r = ctx->mp_r;  // the context's scratch: no fresh pages per call
-  r.resize((size_t)n);
-  double R = 0.0, qmax = 0.0;
-  for (int64_t i = 0; i < n; ++i) {
+  if (!front) r.resize((size_t)n);
+  double R = front ? front->R : 0.0, qmax = 0.0;
+  for (int64_t i = 0; i < n && !front; ++i) {
     const double dx = t.xyz[3 * i] - in.centre[0], dy = t.xyz[3 * i + 1] - in.centre[1],
                  dz = t.xyz[3 * i + 2] - in.centre[2];
     r[i] = std::sqrt(((0.0 + dx * dx) + dy * dy) + dz * dz);
@@ -1613,10 +1676,15 @@ void multipole_run(crab_ctx* ctx, const MpInput& in, const double* q, int64_t nq
   // group = type * S + segment; points sorted by group, padded per group
   std::vector<int32_t>& seg_of = ctx->mp_seg_of;  // written for the owned points before any read
   std::vector<int32_t>& group_of = ctx->mp_group_of;
-  seg_of.resize((size_t)n);
-  group_of.resize((size_t)n);
   std::vector<int64_t> count(G, 0);
-  for (int64_t i = own0; i < own1; ++i) {
+  if (front) {
+    require(S == 1, "one radial segment expected");
+    count = front->count;
+  } else {
+    seg_of.resize((size_t)n);
+    group_of.resize((size_t)n);
+  }
+  for (int64_t i = own0; i < own1 && !front; ++i) {
     seg_of[i] = std::min(S - 1, (int)(r[i] / R * S));
     group_of[i] = t.type[i] * S + seg_of[i];
     ++count[group_of[i]];
@@ -1628,24 +1696,28 @@ void multipole_run(crab_ctx* ctx, const MpInput& in, const double* q, int64_t nq
   const int64_t n_pad = std::max<int64_t>(begin[G], align);
   // points are built in the context's pinned staging buffers (reused across
   // calls, uploaded asynchronously); padding slots are zeroed explicitly
-  auto* pts = (double*)ctx->host("mp_pts", sizeof(double) * 5 * (size_t)n_pad);
-  auto* seg = (int32_t*)ctx->host("mp_seg", sizeof(int32_t) * (size_t)n_pad);
-  std::vector<int64_t> fill(begin.begin(), begin.end() - 1);
-  for (int g = 0; g < G; ++g) {
-    for (int64_t k = begin[g]; k < begin[g + 1]; ++k) seg[k] = g % S;
-    std::fill(pts + 5 * (begin[g] + count[g]), pts + 5 * begin[g + 1], 0.0);
-  }
-  if (begin[G] < n_pad) {  // no points at all: one zero tile
-    std::fill(pts + 5 * begin[G], pts + 5 * n_pad, 0.0);
-    std::fill(seg + begin[G], seg + n_pad, 0);
-  }
-  for (int64_t i = own0; i < own1; ++i) {
-    const int64_t k = fill[group_of[i]]++;
-    pts[5 * k] = t.xyz[3 * i] - in.centre[0];
-    pts[5 * k + 1] = t.xyz[3 * i + 1] - in.centre[1];
-    pts[5 * k + 2] = t.xyz[3 * i + 2] - in.centre[2];
-    pts[5 * k + 3] = t.w[i];
-    pts[5 * k + 4] = r[i];
+  double* pts = nullptr;
+  int32_t* seg = nullptr;
+  if (!front) {
+    pts = (double*)ctx->host("mp_pts", sizeof(double) * 5 * (size_t)n_pad);
+    seg = (int32_t*)ctx->host("mp_seg", sizeof(int32_t) * (size_t)n_pad);
+    std::vector<int64_t> fill(begin.begin(), begin.end() - 1);
+    for (int g = 0; g < G; ++g) {
+      for (int64_t k = begin[g]; k < begin[g + 1]; ++k) seg[k] = g % S;
+      std::fill(pts + 5 * (begin[g] + count[g]), pts + 5 * begin[g + 1], 0.0);
+    }
+    if (begin[G] < n_pad) {  // no points at all: one zero tile
+      std::fill(pts + 5 * begin[G], pts + 5 * n_pad, 0.0);
+      std::fill(seg + begin[G], seg + n_pad, 0);
+    }
+    for (int64_t i = own0; i < own1; ++i) {
+      const int64_t k = fill[group_of[i]]++;
+      pts[5 * k] = t.xyz[3 * i] - in.centre[0];
+      pts[5 * k + 1] = t.xyz[3 * i + 1] - in.centre[1];
+      pts[5 * k + 2] = t.xyz[3 * i + 2] - in.centre[2];
+      pts[5 * k + 3] = t.w[i];
+      pts[5 * k + 4] = r[i];
+    }
   }
   const int lm_count = (L + 1) * (L + 1);
   const int lm_pad = (lm_count + kGemmM - 1) / kGemmM * kGemmM;
@@ -1745,8 +1817,24 @@ void multipole_run(crab_ctx* ctx, const MpInput& in, const double* q, int64_t nq
     copy_h2d(ctx, d_tstart, tstart.data(), sizeof(int4) * tstart.size(), s);
     copy_h2d(ctx, d_snorm, snorm.data(), sizeof(double) * snorm.size(), s);
   }
-  copy_h2d(ctx, d_pts, pts, sizeof(double) * 5 * (size_t)n_pad, s);
-  copy_h2d(ctx, d_seg, seg, sizeof(int32_t) * n_pad, s);
+  if (front) {
+    CRAB_CUDA_CHECK(cudaMemsetAsync(d_pts, 0, sizeof(double) * 5 * (size_t)n_pad, s));
+    CRAB_CUDA_CHECK(cudaMemsetAsync(d_seg, 0, sizeof(int32_t) * n_pad, s));
+    auto* d_begin = (int64_t*)ctx->dev("mp_begin", sizeof(int64_t) * (G + 1));
+    copy_h2d(ctx, d_begin, begin.data(), sizeof(int64_t) * (G + 1), s);
+    const double* c = in.centre;
+    k_mp_place<<<(unsigned)((front->n_atoms + 255) / 256), 256, 0, s>>>(front->d_xyz, front->d_occ, front->d_word,
+                                                                       front->n_atoms, d_begin, c[0], c[1], c[2],
+                                                                       d_pts);
+    if (front->g.m)
+      k_mp_place_sites<<<(unsigned)((front->g.m + 255) / 256), 256, 0, s>>>(front->g.d_sites, front->g.m,
+                                                                           begin[T - 1], c[0], c[1], c[2], d_pts);
+    CRAB_CUDA_CHECK(cudaGetLastError());
+    ctx->launches += front->g.m ? 2 : 1;
+  } else {
+    copy_h2d(ctx, d_pts, pts, sizeof(double) * 5 * (size_t)n_pad, s);
+    copy_h2d(ctx, d_seg, seg, sizeof(int32_t) * n_pad, s);
+  }
   copy_h2d(ctx, d_norms, norms.data(), sizeof(double) * norms.size(), s);
   copy_h2d(ctx, d_inv, inv.data(), sizeof(double) * inv.size(), s);
   copy_h2d(ctx, d_nodes, B.nodes.data(), sizeof(double) * B.nodes.size(), s);
@@ -1913,6 +2001,93 @@ void validate_multipole(const crab_struct* st, const double* q, int64_t nq, int 
   require(l_max >= 0 && l_max <= kMaxL, "multipole l_max must be between 0 and 64");
 }
 
+// Classes, words and device copies of a structure's atoms, and its sites; false
+// where the general path has to serve (several radial segments, very many atoms
+// or classes).
+bool mp_front(crab_ctx* ctx, const crab_struct* st, const double* q, int64_t nq, const crab_solvent* solvent,
+              bool implicit, MpFront& F) {
+  const int64_t n = st->n;
+  if (n >= (1 << 24)) return false;
+  TraceScope trace("mp_front");
+  const bool grid = solvent && solvent->hydration_model != CRAB_HYD_ANALYTIC;
+  const int8_t *el = st->elem.data(), *gr = st->group.data();
+  constexpr int kCodes = 256;  // element * 16 + group + 1
+  const int gmask = implicit ? 0xff : 0;
+  int64_t part[4][kCodes] = {};
+  for (int64_t i = 0; i < n; ++i) ++part[i & 3][el[i] * 16 + ((gr[i] + 1) & gmask)];
+  int cls_of[kCodes];
+  bool dropped = false;
+  for (int code = 0; code < kCodes; ++code) {
+    const int64_t m = part[0][code] + part[1][code] + part[2][code] + part[3][code];
+    const AtomClass k{code / 16, code % 16 - 1};
+    const bool drop = m > 0 && class_dropped(k, implicit, !solvent ? TermSet::Vacuum
+                                                          : grid   ? TermSet::SolventGrid
+                                                                   : TermSet::SolventAnalytic);
+    dropped = dropped || drop;
+    cls_of[code] = m == 0 || drop ? -1 : F.t.T++;
+    if (cls_of[code] >= 0) {
+      F.t.cls.push_back(k);
+      F.count.push_back(m);
+      F.n += m;
+    }
+  }
+  if (F.t.T == 0 || F.t.T > 200) return false;
+  const double* x = st->xyz.data();
+  centre_and_rmax(st, F.centre, &F.rmax);
+  F.rmax_lq = F.R = F.rmax;
+  double qmax = 0.0;
+  for (int64_t k = 0; k < nq; ++k) qmax = std::max(qmax, q[k]);
+  // sites add at most a shell; a range that needs more segments is the general path's
+  if (nodes_needed(qmax * (F.rmax + (grid ? 16.0 : 0.0)) * (1.0 + 1e-9) / 2.0) > kMaxNodes) return false;
+  cudaStream_t s = ctx->stream;
+  auto* hx = (double*)ctx->host("front.xyz", (size_t)n * 4 * sizeof(double));
+  std::memcpy(hx, x, (size_t)n * 3 * sizeof(double));
+  std::memcpy(hx + 3 * n, st->occ.data(), (size_t)n * sizeof(double));
+  F.d_xyz = (double*)ctx->dev("front.xyz", (size_t)n * 4 * sizeof(double));
+  F.d_occ = F.d_xyz + 3 * n;
+  copy_h2d(ctx, F.d_xyz, hx, (size_t)n * 4 * sizeof(double), s);
+  auto* word = (uint32_t*)ctx->host("front.word", (size_t)n * sizeof(uint32_t));
+  std::vector<uint32_t> rank(F.t.T, 0);
+  double r2 = 0.0;
+  for (int64_t i = 0; i < n; ++i) {
+    const int k = cls_of[el[i] * 16 + ((gr[i] + 1) & gmask)];
+    word[i] = k < 0 ? kMpDropped : (uint32_t)k << 24 | rank[k]++;
+    if (dropped && k >= 0) {
+      const double dx = x[3 * i] - F.centre[0], dy = x[3 * i + 1] - F.centre[1], dz = x[3 * i + 2] - F.centre[2];
+      r2 = max_num(r2, ((0.0 + dx * dx) + dy * dy) + dz * dz);
+    }
+  }
+  if (dropped) F.R = std::sqrt(r2);
+  F.d_word = (uint32_t*)ctx->dev("front.word", (size_t)n * sizeof(uint32_t));
+  copy_h2d(ctx, F.d_word, word, (size_t)n * sizeof(uint32_t), s);
+  F.n_atoms = n;
+  trace_mark("words");
+  if (grid) {
+    F.g = solvent->hydration_model == CRAB_HYD_ADAPTIVE
+              ? adaptive_grid_device(ctx, x, n, solvent->grid_spacing, 3.0, 12.0, false)
+              : exterior_grid_device(ctx, x, el, n, 1.0, 1.4, solvent->shell_thickness, false);
+    F.t.cls.push_back(AtomClass{-1, -1});
+    ++F.t.T;
+    F.count.push_back(F.g.m);
+    F.n += F.g.m;
+    if (F.g.m) {  // spherical.rs:423-427, 489-493: the order also covers the sites
+      auto* d_r = (unsigned long long*)ctx->dev("mp_site_r", sizeof(unsigned long long));
+      auto* h_r = (double*)ctx->host("mp_site_r", sizeof(double));
+      CRAB_CUDA_CHECK(cudaMemsetAsync(d_r, 0, sizeof(unsigned long long), s));
+      k_mp_site_rmax<<<(unsigned)std::min<int64_t>(148, (F.g.m + 255) / 256), 256, 0, s>>>(
+          F.g.d_sites, F.g.m, F.centre[0], F.centre[1], F.centre[2], d_r);
+      CRAB_CUDA_CHECK(cudaGetLastError());
+      ctx->launches += 1;
+      copy_d2h(ctx, h_r, d_r, sizeof(double), s);
+      CRAB_CUDA_CHECK(cudaStreamSynchronize(s));
+      F.rmax_lq = std::max(F.rmax, *h_r);
+      F.R = std::max(F.R, *h_r);
+    }
+  }
+  const double R = F.R > 0.0 ? F.R * (1.0 + 1e-12) : 1.0;
+  return nodes_needed(qmax * R / 2.0) <= kMaxNodes;
+}
+
 // Per-type multipole amplitudes without occupancy (spherical.rs:205-231):
 // V, E, H [T][nq].  Hydration sites (element -1) carry the grid amplitude
 // rho/10 * V_voxel * f_water(q) in H.
@@ -1941,14 +2116,29 @@ void multipole_tables(const TypedAtoms& t, const double* q, int64_t nq, const cr
 struct MpSolventSetup {
   GridResult g;
   TypedAtoms t;
+  MpFront F;
+  bool front = false;  // the points are F's
   std::vector<double> V, E, H;
   double centre[3], rmax_lq;
+  void into(MpInput& in) const {
+    in.t = front ? &F.t : &t;
+    in.front = front ? &F : nullptr;
+    std::copy(centre, centre + 3, in.centre);
+    in.rmax_lq = rmax_lq;
+  }
 };
 
 void solvent_setup(crab_ctx* ctx, const crab_struct* st, const double* q, int64_t nq, const crab_solvent& s,
-                   bool implicit, MpSolventSetup& u) {
+                   bool implicit, bool whole, MpSolventSetup& u) {
   TraceScope trace("mp_solvent_setup");
   const bool grid = s.hydration_model != CRAB_HYD_ANALYTIC;
+  if (whole && mp_front(ctx, st, q, nq, &s, implicit, u.F)) {
+    u.front = true;
+    multipole_tables(u.F.t, q, nq, &s, implicit, u.F.g.voxel_volume, u.V, u.E, u.H);
+    std::copy(u.F.centre, u.F.centre + 3, u.centre);
+    u.rmax_lq = u.F.rmax_lq;
+    return;
+  }
   if (grid) u.g = hydration_sites(ctx, st, s);
   trace_mark("hydration sites");
   u.t = type_atoms(st, implicit, grid ? TermSet::SolventGrid : TermSet::SolventAnalytic, grid ? &u.g.sites : nullptr);
@@ -1981,10 +2171,17 @@ void multipole_intensity_impl(crab_ctx* ctx, const crab_struct* st, const double
     return;
   }
   TraceScope trace("multipole_intensity");
-  TypedAtoms& t = typed_scratch(ctx);
   MpInput in;
   std::vector<double> V, E, H;
-  {
+  MpFront F;
+  if (shard.n_shards == 1 && mp_front(ctx, st, q, nq, nullptr, implicit, F)) {
+    multipole_tables(F.t, q, nq, nullptr, implicit, 0.0, V, E, H);
+    in.t = &F.t;
+    in.front = &F;
+    std::copy(F.centre, F.centre + 3, in.centre);
+    in.rmax_lq = F.rmax_lq;
+  } else {
+    TypedAtoms& t = typed_scratch(ctx);
     TraceScope tt("mp_type_atoms+tables");
     type_atoms_into(st, implicit, TermSet::Vacuum, nullptr, t);
     in.t = &t;
@@ -2014,11 +2211,9 @@ void multipole_solvent_basis_impl(crab_ctx* ctx, const crab_struct* st, const do
     return;
   }
   MpSolventSetup u;
-  solvent_setup(ctx, st, q, nq, s, implicit, u);
+  solvent_setup(ctx, st, q, nq, s, implicit, shard.n_shards == 1, u);
   MpInput in;
-  in.t = &u.t;
-  std::copy(u.centre, u.centre + 3, in.centre);
-  in.rmax_lq = u.rmax_lq;
+  u.into(in);
   in.K = 3;
   in.amp.reserve(u.V.size() * 3);
   in.amp.insert(in.amp.end(), u.V.begin(), u.V.end());
@@ -2041,18 +2236,18 @@ void multipole_solvent_intensity_impl(crab_ctx* ctx, const crab_struct* st, cons
     return;
   }
   MpSolventSetup u;
-  solvent_setup(ctx, st, q, nq, s, implicit, u);
+  solvent_setup(ctx, st, q, nq, s, implicit, true, u);
   MpInput in;
-  in.t = &u.t;
-  std::copy(u.centre, u.centre + 3, in.centre);
-  in.rmax_lq = u.rmax_lq;
+  u.into(in);
   in.K = 1;
   // spherical.rs:438-444, 453-462: f = v - G(q) e + c2 h per atom, c2 * amplitude per site
   in.amp.resize(u.V.size());
-  for (int a = 0; a < u.t.T; ++a)
+  std::vector<double> scale(nq);
+  for (int64_t k = 0; k < nq; ++k) scale[k] = excluded_volume_scale(q[k], s.c1);
+  for (int a = 0; a < in.t->T; ++a)
     for (int64_t k = 0; k < nq; ++k) {
       const size_t o = (size_t)a * nq + k;
-      in.amp[o] = u.V[o] - excluded_volume_scale(q[k], s.c1) * u.E[o] + s.c2 * u.H[o];
+      in.amp[o] = u.V[o] - scale[k] * u.E[o] + s.c2 * u.H[o];
     }
   multipole_run(ctx, in, q, nq, l_max, mp.fp64, mp.tc_terms, mp.gemm, out);
   for (int64_t k = 0; k < nq; ++k) out[k] = std::fmax(out[k], 0.0);

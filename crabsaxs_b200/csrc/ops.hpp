@@ -17,6 +17,9 @@ void validate_solvent(const crab_solvent& s);
 // because all their amplitudes vanish.
 enum class TermSet { Vacuum, SolventAnalytic, SolventGrid };
 
+// Whether every amplitude of a class vanishes for those terms.
+bool class_dropped(const AtomClass& c, bool implicit, TermSet need);
+
 // Atoms (plus optional hydration sites as the last type, element -1) mapped
 // to dense scattering types.
 struct TypedAtoms {
