@@ -341,6 +341,8 @@ int crab_ctx_create(int device, crab_ctx** out) {
   int rc = guarded_impl(ctx, [&]() {
     CRAB_CUDA_CHECK(cudaDeviceGetAttribute(&ctx->sm_count, cudaDevAttrMultiProcessorCount, device));
     CRAB_CUDA_CHECK(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
+    CRAB_CUDA_CHECK(cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking));
+    CRAB_CUDA_CHECK(cudaEventCreateWithFlags(&ctx->ev_side, cudaEventDisableTiming));
     CRAB_CUDA_CHECK(cudaEventCreate(&ctx->ev_start));
     CRAB_CUDA_CHECK(cudaEventCreate(&ctx->ev_stop));
   });
@@ -356,10 +358,13 @@ int crab_ctx_destroy(crab_ctx* ctx) {
   if (!ctx) return CRAB_OK;
   cudaSetDevice(ctx->device);
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
+  if (ctx->side) cudaStreamSynchronize(ctx->side);
   for (auto& kv : ctx->bufs)
     if (kv.second.ptr) cudaFree(kv.second.ptr);
   for (auto& kv : ctx->hbufs)
     if (kv.second.ptr) cudaFreeHost(kv.second.ptr);
+  if (ctx->ev_side) cudaEventDestroy(ctx->ev_side);
+  if (ctx->side) cudaStreamDestroy(ctx->side);
   if (ctx->ev_start) cudaEventDestroy(ctx->ev_start);
   if (ctx->ev_stop) cudaEventDestroy(ctx->ev_stop);
   if (ctx->stream) cudaStreamDestroy(ctx->stream);

@@ -88,7 +88,9 @@ struct crab_ctx {
   int device = 0;
   int sm_count = 148;
   cudaStream_t stream = nullptr;
-  cudaEvent_t ev_start = nullptr, ev_stop = nullptr;
+  // work of a call that runs beside the main stream and joins it by ev_side before the call's results are read
+  cudaStream_t side = nullptr;
+  cudaEvent_t ev_start = nullptr, ev_stop = nullptr, ev_side = nullptr;
   std::mutex mu;
   std::string last_error;
   std::map<std::string, crab::DevBuf> bufs;

@@ -130,11 +130,20 @@ __host__ __device__ __forceinline__ int64_t mp_blocked(int row, int64_t k, int r
 // Lagrange basis of its radial segment.  pts: x, y, z (centred), w, r.
 // The recurrence divides by (l - m) as the reference does, here as a product
 // with the f64 reciprocal inv[l - m] (at most one ulp apart per step).
+// Rows in m-major order, cos before sin (fused_row_walk), snorm their norms:
+// a warp's stores then run through memory line by line, and a part of the
+// orders is a run of rows.  blockIdx.y takes the orders mstart[y] ..
+// mstart[y + 1) of its points, brought up to the first one by the same
+// operations; the last one also writes the radial basis.  Bound: the latency of
+// the recurrence at one thread a point (eight parts: 1,481 atoms with sites 47
+// to 23 us, 58,870 224 to 178 us), then the stores (100,000 atoms: 315 to 293
+// us for 1.07 GB).
 template <typename E>
-__global__ void k_mp_prep(const double* __restrict__ pts, const int32_t* __restrict__ seg, int64_t n_pad, int L,
-                          int lm_pad, int nb, const double* __restrict__ norms, const double* __restrict__ nodes,
-                          const double* __restrict__ bary, const double* __restrict__ inv, E* __restrict__ YT,
-                          E* __restrict__ WT) {
+__global__ void __launch_bounds__(128)
+    k_mp_prep(const double* __restrict__ pts, const int32_t* __restrict__ seg, int64_t n_pad, int L, int lm_pad, int nb,
+              const double* __restrict__ snorm, const int* __restrict__ mstart, const double* __restrict__ nodes,
+              const double* __restrict__ bary, const double* __restrict__ inv, E* __restrict__ YT,
+              E* __restrict__ WT) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n_pad) return;
   const double px = pts[5 * i], py = pts[5 * i + 1], pz = pts[5 * i + 2], w = pts[5 * i + 3], r = pts[5 * i + 4];
@@ -149,38 +158,47 @@ __global__ void k_mp_prep(const double* __restrict__ pts, const int32_t* __restr
   const double sin_theta = sqrt(fmax(__dadd_rn(1.0, -__dmul_rn(x, x)), 0.0));
   double sin_phi, cos_phi;
   sincos(phi, &sin_phi, &cos_phi);
-  const double sqrt2 = sqrt(2.0);
+  const int ma = mstart[blockIdx.y], mb = mstart[blockIdx.y + 1];
   double sin_m = 0.0, cos_m = 1.0, pmm = 1.0;
-  auto emit = [&](int l, int m, double p) {
-    const int pos = l * l + l + m;
-    if (m == 0) {
-      YT[mp_blocked(pos, i, lm_pad)] = (E)__dmul_rn(norms[pos], p);
-    } else {
-      const double v = __dmul_rn(__dmul_rn(sqrt2, norms[pos]), p);
-      YT[mp_blocked(pos, i, lm_pad)] = (E)__dmul_rn(v, cos_m);
-      YT[mp_blocked(l * l + l - m, i, lm_pad)] = (E)__dmul_rn(v, sin_m);
-    }
+  auto next_m = [&](int m) {
+    pmm = __dmul_rn(pmm, __dmul_rn(-(double)(2 * m - 1), sin_theta));
+    const double next_cos = __dadd_rn(__dmul_rn(cos_m, cos_phi), -__dmul_rn(sin_m, sin_phi));
+    sin_m = __dadd_rn(__dmul_rn(sin_m, cos_phi), __dmul_rn(cos_m, sin_phi));
+    cos_m = next_cos;
   };
-  for (int m = 0; m <= L; ++m) {
-    if (m > 0) {
-      pmm = __dmul_rn(pmm, __dmul_rn(-(double)(2 * m - 1), sin_theta));
-      const double next_cos = __dadd_rn(__dmul_rn(cos_m, cos_phi), -__dmul_rn(sin_m, sin_phi));
-      sin_m = __dadd_rn(__dmul_rn(sin_m, cos_phi), __dmul_rn(cos_m, sin_phi));
-      cos_m = next_cos;
-    }
-    emit(m, m, pmm);
-    if (m == L) continue;
-    const double pm1 = __dmul_rn(__dmul_rn(x, (double)(2 * m + 1)), pmm);
-    emit(m + 1, m, pm1);
-    double prev = pmm, cur = pm1;
-    for (int l = m + 2; l <= L; ++l) {
-      const double num = __dadd_rn(__dmul_rn(__dmul_rn((double)(2 * l - 1), x), cur), -__dmul_rn((double)(l + m - 1), prev));
-      const double next = __dmul_rn(num, inv[l - m]);
-      emit(l, m, next);
+  for (int m = 1; m < ma; ++m) next_m(m);
+  // first row of order ma: L + 1 rows of order 0, then 2 (L + 1 - m) of order m
+  int row = ma == 0 ? 0 : (L + 1) + (ma - 1) * (2 * L + 2 - ma);
+  E* out = YT + mp_blocked(row, i, lm_pad);
+  for (int m = ma; m < mb; ++m) {
+    if (m > 0) next_m(m);
+    double prev = 0.0, cur = pmm;
+    for (int l = m; l <= L; ++l) {
+      if (m == 0) {
+        *out = (E)__dmul_rn(snorm[row], cur);
+        out += 32;
+        ++row;
+      } else {
+        const double v = __dmul_rn(snorm[row], cur);
+        out[0] = (E)__dmul_rn(v, cos_m);
+        out[32] = (E)__dmul_rn(v, sin_m);
+        out += 64;
+        row += 2;
+      }
+      double next;
+      if (l == m) {
+        next = __dmul_rn(__dmul_rn(x, (double)(2 * m + 1)), pmm);
+      } else {
+        const int n = l + 1;  // the step from l to l + 1
+        const double num = __dadd_rn(__dmul_rn(__dmul_rn((double)(2 * n - 1), x), cur),
+                                     -__dmul_rn((double)(n + m - 1), prev));
+        next = __dmul_rn(num, inv[n - m]);
+      }
       prev = cur;
       cur = next;
     }
   }
+  if (blockIdx.y + 1 < gridDim.y) return;
   for (int pos = (L + 1) * (L + 1); pos < lm_pad; ++pos) YT[mp_blocked(pos, i, lm_pad)] = (E)0;
   // Barycentric Lagrange basis at the segment's first-kind Chebyshev nodes.
   const double* nd = nodes + (int64_t)seg[i] * nb;
@@ -1371,37 +1389,54 @@ __global__ void k_mp_node_bessel(const double* __restrict__ q, const int32_t* __
 //   A^c_lm(q) = sum_t amp[c][t][q] sum_s sum_b M[t*S+s][b][lm] j_l(q rho_{s,b})
 // and 4 pi sum_{l <= l_q, m} A^c A^d accumulates per q for c <= d (order
 // (0,0), (1,1), (2,2), (0,1), (0,2), (1,2) for three combinations).
-// k_mp_gram: one block per (l, chunk of 32 m, chunk of 128 q).  Each warp
-// owns 4 m and each lane 4 q (lane + 32 j), so one thread keeps a 4 x 4 tile
+// k_mp_gram: one block per (l, chunk of 32 m, chunk of 32 QL q).  Each warp
+// owns 4 m and each lane QL q (lane + 32 j), so one thread keeps a 4 x QL tile
 // of the contraction over the radial nodes in registers; the block's moments
 // (per group) and node values (per segment) are staged in shared memory,
 // where a warp's moment loads are broadcasts and its node-value loads are
 // contiguous.  Each block writes its partial sums per (combination, q);
 // k_mp_gram_reduce adds the rows in (l, m) order (deterministic).
-constexpr int kGramM = 32, kGramQ = 128, kGramThreads = 256;
+// With few q the blocks are too few for the chip and their latency is what the
+// pass takes: QL, the q of a lane, is then one (1,481 atoms of 14 classes with
+// sites, 101 q: 65 us with four, 50 with one, 32 with the moments of the next
+// group fetched while this one is used; 58,870 atoms 101, 94, 84 us).
+constexpr int kGramM = 32, kGramThreads = 256;
 
-template <int K>
+template <int K, int QL>
 __global__ void __launch_bounds__(kGramThreads)
     k_mp_gram(const double* __restrict__ M, const double* __restrict__ Jn, const int32_t* __restrict__ lq,
               const double* __restrict__ amp, const int2* __restrict__ rows, int T, int S, int nb, int n_nodes,
               int lm_pad, int64_t nq, double* __restrict__ part) {
   constexpr int P = K * (K + 1) / 2;
+  constexpr int kGramQ = 32 * QL;
   extern __shared__ double gram_smem[];
   double* Js = gram_smem;                               // [nb][kGramQ] node values of one segment
-  double* Ms = gram_smem + (size_t)kMaxNodes * kGramQ;  // [nb][kGramM] moments of one group
+  double* Ms = gram_smem + (size_t)kMaxNodes * kGramQ;  // [2][nb][kGramM] moments of a group and the next
   const int2 row = rows[blockIdx.x];
   const int l = row.x, m0 = row.y;
   const int nm = min(kGramM, 2 * l + 1 - m0);
   const int64_t q0 = (int64_t)blockIdx.y * kGramQ;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t jrow = (int64_t)l * n_nodes;
-  double A[K][4][4];
+  double A[K][4][QL];
 #pragma unroll
   for (int c = 0; c < K; ++c)
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) A[c][i][j] = 0.0;
+      for (int j = 0; j < QL; ++j) A[c][i][j] = 0.0;
+  // the moments of the next group are on their way while this one's are used
+  constexpr int kPre = kMaxNodes * kGramM / kGramThreads;
+  double pre[kPre];
+  auto load = [&](int g) {
+#pragma unroll
+    for (int u = 0; u < kPre; ++u) {
+      const int idx = threadIdx.x + u * kGramThreads, b = idx / kGramM, mi = idx % kGramM;
+      pre[u] = b < nb && mi < nm ? M[((int64_t)g * kMaxNodes + b) * lm_pad + l * l + m0 + mi] : 0.0;
+    }
+  };
+  load(0);
+  int buf = 0;
   for (int sg = 0; sg < S; ++sg) {
     __syncthreads();
     for (int idx = threadIdx.x; idx < nb * kGramQ; idx += kGramThreads) {
@@ -1409,35 +1444,34 @@ __global__ void __launch_bounds__(kGramThreads)
       const int64_t q = q0 + ql;
       Js[idx] = q < nq ? Jn[(jrow + sg * nb + b) * nq + q] : 0.0;
     }
-    for (int t = 0; t < T; ++t) {
-      const int g = t * S + sg;
+    for (int t = 0; t < T; ++t, buf ^= 1) {
+      double* Mb = Ms + buf * kMaxNodes * kGramM;
+#pragma unroll
+      for (int u = 0; u < kPre; ++u) Mb[threadIdx.x + u * kGramThreads] = pre[u];
       __syncthreads();
-      for (int idx = threadIdx.x; idx < nb * kGramM; idx += kGramThreads) {
-        const int b = idx / kGramM, mi = idx % kGramM;
-        Ms[idx] = mi < nm ? M[((int64_t)g * kMaxNodes + b) * lm_pad + l * l + m0 + mi] : 0.0;
-      }
-      __syncthreads();
-      double C[4][4];
+      const int tn = t + 1 < T ? t + 1 : 0, sn = t + 1 < T ? sg : sg + 1;
+      if (sn < S) load(tn * S + sn);
+      double C[4][QL];
 #pragma unroll
       for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) C[i][j] = 0.0;
-      const double* mrow = Ms + warp * 4;
+        for (int j = 0; j < QL; ++j) C[i][j] = 0.0;
+      const double* mrow = Mb + warp * 4;
       const double* jcol = Js + lane;
 #pragma unroll 2
       for (int b = 0; b < nb; ++b) {
-        double mv[4], jv[4];
+        double mv[4], jv[QL];
 #pragma unroll
         for (int i = 0; i < 4; ++i) mv[i] = mrow[b * kGramM + i];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) jv[j] = jcol[b * kGramQ + 32 * j];
+        for (int j = 0; j < QL; ++j) jv[j] = jcol[b * kGramQ + 32 * j];
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
-          for (int j = 0; j < 4; ++j) C[i][j] = fma(mv[i], jv[j], C[i][j]);
+          for (int j = 0; j < QL; ++j) C[i][j] = fma(mv[i], jv[j], C[i][j]);
       }
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
+      for (int j = 0; j < QL; ++j) {
         const int64_t q = q0 + lane + 32 * j;
 #pragma unroll
         for (int c = 0; c < K; ++c) {
@@ -1448,9 +1482,9 @@ __global__ void __launch_bounds__(kGramThreads)
       }
     }
   }
-  double acc[P][4];
+  double acc[P][QL];
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
+  for (int j = 0; j < QL; ++j) {
     const int64_t q = q0 + lane + 32 * j;
     const bool on = q < nq && l <= lq[q];
     int p = 0;
@@ -1476,7 +1510,7 @@ __global__ void __launch_bounds__(kGramThreads)
 #pragma unroll
   for (int p = 0; p < P; ++p)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) red[(warp * P + p) * kGramQ + lane + 32 * j] = acc[p][j];
+    for (int j = 0; j < QL; ++j) red[(warp * P + p) * kGramQ + lane + 32 * j] = acc[p][j];
   __syncthreads();
   for (int idx = threadIdx.x; idx < P * kGramQ; idx += kGramThreads) {
     const int p = idx / kGramQ, ql = idx % kGramQ;
@@ -1639,6 +1673,23 @@ void fused_row_walk(int L, int lm_pad, std::vector<int4>& tstart, std::vector<in
   }
 }
 
+// Splits of the staged prep's orders m over blockIdx.y, of about equal numbers of
+// rows: eight at every size (1, 2, 4, 8, 16 parts: 58, 37, 29, 23, 21 us at
+// 1,481 atoms with sites, 265, 174, 181, 179, 172 at 58,870, 352, 346, 326, 293,
+// 293 at 100,000).
+std::vector<int> prep_splits(int L) {
+  constexpr int parts = 8;
+  std::vector<int> start{0};
+  const double rows = (double)(L + 1) * (L + 1);
+  double done = 0.0;
+  for (int m = 0; m <= L; ++m) {
+    done += (m ? 2 : 1) * (L + 1 - m);
+    if ((int)start.size() < parts && done >= rows * (double)start.size() / parts && m < L) start.push_back(m + 1);
+  }
+  start.push_back(L + 1);
+  return start;
+}
+
 // GEMM kernel of a precision mode: gemm = 0 SIMT (FP32, or FP64 with fp64),
 // 1 the staged tensor-core kernel (Y_lm through device memory), 2 the fused
 // tensor-core kernel with TF32 operands, 3 the fused kernel with BF16
@@ -1759,17 +1810,18 @@ void multipole_run(crab_ctx* ctx, const MpInput& in, const double* q, int64_t nq
   const std::vector<double> norms = harmonic_norms(L);
   std::vector<double> inv(L + 2, 0.0);
   for (int k = 1; k <= L + 1; ++k) inv[k] = 1.0 / (double)k;
-  if (fused) {  // the walk's tile starts, and per row the norm as k_mp_prep applies it
-    fused_row_walk(L, lm_pad, tstart, perm);
-    snorm.assign((size_t)lm_pad, 0.0);  // row order; zero past the last harmonic
-    const double sqrt2 = std::sqrt(2.0);
-    for (int row = 0; row < lm_pad; ++row) {
-      if (perm[row] >= lm_count) continue;
-      const int l = (int)std::sqrt((double)perm[row]), m = std::abs(perm[row] - l * l - l);
-      const int pos = l * l + l + m;
-      snorm[row] = m == 0 ? norms[pos] : sqrt2 * norms[pos];
-    }
+  // rows in m-major order: the walk's tile starts, and per row the norm
+  fused_row_walk(L, lm_pad, tstart, perm);
+  snorm.assign((size_t)lm_pad, 0.0);  // row order; zero past the last harmonic
+  const double sqrt2 = std::sqrt(2.0);
+  for (int row = 0; row < lm_pad; ++row) {
+    if (perm[row] >= lm_count) continue;
+    const int l = (int)std::sqrt((double)perm[row]), m = std::abs(perm[row] - l * l - l);
+    const int pos = l * l + l + m;
+    snorm[row] = m == 0 ? norms[pos] : sqrt2 * norms[pos];
   }
+  const std::vector<int> mstart = prep_splits(L);
+  const unsigned prep_parts = (unsigned)mstart.size() - 1;
   const size_t n_items = fused ? fwork.size() * (size_t)n_lmt : work.size();
 
   trace_mark("mp_host_prep");
@@ -1778,7 +1830,9 @@ void multipole_run(crab_ctx* ctx, const MpInput& in, const double* q, int64_t nq
   const size_t esz = fp64 ? sizeof(double) : sizeof(float);
   double* d_pts = (double*)ctx->dev("mp_pts", sizeof(double) * 5 * (size_t)n_pad);
   int32_t* d_seg = (int32_t*)ctx->dev("mp_seg", sizeof(int32_t) * n_pad);
-  double* d_norms = (double*)ctx->dev("mp_norms", sizeof(double) * norms.size());
+  int* d_mstart = (int*)ctx->dev("mp_mstart", sizeof(int) * mstart.size());
+  double* d_snorm = (double*)ctx->dev("mp_snorm", sizeof(double) * snorm.size());
+  int32_t* d_perm = (int32_t*)ctx->dev("mp_perm", sizeof(int32_t) * perm.size());
   double* d_inv = (double*)ctx->dev("mp_inv", sizeof(double) * inv.size());
   double* d_nodes = (double*)ctx->dev("mp_nodes", sizeof(double) * B.nodes.size());
   double* d_bary = (double*)ctx->dev("mp_bary", sizeof(double) * B.bary.size());
@@ -1800,22 +1854,16 @@ void multipole_run(crab_ctx* ctx, const MpInput& in, const double* q, int64_t nq
   unsigned char* d_Bimg = nullptr;
   FuState fst{};
   int4* d_fwork = nullptr;
-  int32_t* d_perm = nullptr;
   int4* d_tstart = nullptr;
-  double* d_snorm = nullptr;
   if (fused) {
     d_cst = (double4*)ctx->dev("mp_cst", sizeof(double4) * (size_t)n_pad);
     d_Bimg = (unsigned char*)ctx->dev("mp_Bimg", (size_t)(n_pad / KS) * tc_terms * kTcBBytes);
     double* st = (double*)ctx->dev("mp_walk", sizeof(double) * 5 * (size_t)n_pad);
     fst = FuState{st, st + n_pad, st + 2 * n_pad, st + 3 * n_pad, st + 4 * n_pad};
     d_fwork = (int4*)ctx->dev("mp_fwork", sizeof(int4) * std::max<size_t>(fwork.size(), 1));
-    d_perm = (int32_t*)ctx->dev("mp_perm", sizeof(int32_t) * perm.size());
     d_tstart = (int4*)ctx->dev("mp_tstart", sizeof(int4) * tstart.size());
-    d_snorm = (double*)ctx->dev("mp_snorm", sizeof(double) * snorm.size());
     copy_h2d(ctx, d_fwork, fwork.data(), sizeof(int4) * fwork.size(), s);
-    copy_h2d(ctx, d_perm, perm.data(), sizeof(int32_t) * perm.size(), s);
     copy_h2d(ctx, d_tstart, tstart.data(), sizeof(int4) * tstart.size(), s);
-    copy_h2d(ctx, d_snorm, snorm.data(), sizeof(double) * snorm.size(), s);
   }
   if (front) {
     CRAB_CUDA_CHECK(cudaMemsetAsync(d_pts, 0, sizeof(double) * 5 * (size_t)n_pad, s));
@@ -1835,7 +1883,9 @@ void multipole_run(crab_ctx* ctx, const MpInput& in, const double* q, int64_t nq
     copy_h2d(ctx, d_pts, pts, sizeof(double) * 5 * (size_t)n_pad, s);
     copy_h2d(ctx, d_seg, seg, sizeof(int32_t) * n_pad, s);
   }
-  copy_h2d(ctx, d_norms, norms.data(), sizeof(double) * norms.size(), s);
+  copy_h2d(ctx, d_perm, perm.data(), sizeof(int32_t) * perm.size(), s);
+  copy_h2d(ctx, d_snorm, snorm.data(), sizeof(double) * snorm.size(), s);
+  copy_h2d(ctx, d_mstart, mstart.data(), sizeof(int) * mstart.size(), s);
   copy_h2d(ctx, d_inv, inv.data(), sizeof(double) * inv.size(), s);
   copy_h2d(ctx, d_nodes, B.nodes.data(), sizeof(double) * B.nodes.size(), s);
   copy_h2d(ctx, d_bary, B.bary.data(), sizeof(double) * B.bary.size(), s);
@@ -1857,6 +1907,20 @@ void multipole_run(crab_ctx* ctx, const MpInput& in, const double* q, int64_t nq
   } ev_guard{ev};
   for (int i = 0; i < 4; ++i) CRAB_CUDA_CHECK(cudaEventCreate(&ev[i]));
   CRAB_CUDA_CHECK(cudaEventRecord(ev[0], s));
+  // the node values need only q and the nodes: on the side stream, beside the
+  // harmonics and the GEMM, and joined before the q pass (on an error too)
+  struct SideJoin {
+    cudaStream_t side;
+    bool on = true;
+    ~SideJoin() {
+      if (on) cudaStreamSynchronize(side);
+    }
+  } side_join{ctx->side};
+  CRAB_CUDA_CHECK(cudaStreamWaitEvent(ctx->side, ev[0], 0));
+  k_mp_node_bessel<<<(unsigned)((nq * S * nb + 127) / 128), 128, 0, ctx->side>>>(d_q, d_lq, nq, d_nodes, S * nb, L,
+                                                                                 d_Jn);
+  CRAB_CUDA_CHECK(cudaGetLastError());
+  CRAB_CUDA_CHECK(cudaEventRecord(ctx->ev_side, ctx->side));
   const unsigned prep_blocks = (unsigned)((n_pad + 127) / 128);
   if (fused) {
 #define CRAB_FUSED(EE, SS)                                                                                        \
@@ -1876,15 +1940,16 @@ void multipole_run(crab_ctx* ctx, const MpInput& in, const double* q, int64_t nq
     CRAB_FUSED(1, 2)
 #undef CRAB_FUSED
   } else if (fp64) {
-    k_mp_prep<double><<<prep_blocks, 128, 0, s>>>(d_pts, d_seg, n_pad, L, lm_pad, nb, d_norms, d_nodes, d_bary,
-                                                   d_inv, (double*)d_YT, (double*)d_WT);
+    k_mp_prep<double><<<dim3(prep_blocks, prep_parts), 128, 0, s>>>(d_pts, d_seg, n_pad, L, lm_pad, nb, d_snorm, d_mstart,
+                                                                      d_nodes, d_bary, d_inv, (double*)d_YT,
+                                                                      (double*)d_WT);
     CRAB_CUDA_CHECK(cudaEventRecord(ev[1], s));
     if (!work.empty())  // empty only for a rank of a sharded call that owns no atoms
       k_mp_moments<double><<<(unsigned)work.size(), 256, 0, s>>>((const double*)d_YT, (const double*)d_WT, n_pad,
                                                                   lm_pad, d_work, d_part);
   } else {
-    k_mp_prep<float><<<prep_blocks, 128, 0, s>>>(d_pts, d_seg, n_pad, L, lm_pad, nb, d_norms, d_nodes, d_bary,
-                                                  d_inv, (float*)d_YT, (float*)d_WT);
+    k_mp_prep<float><<<dim3(prep_blocks, prep_parts), 128, 0, s>>>(d_pts, d_seg, n_pad, L, lm_pad, nb, d_snorm, d_mstart,
+                                                                     d_nodes, d_bary, d_inv, (float*)d_YT, (float*)d_WT);
     CRAB_CUDA_CHECK(cudaEventRecord(ev[1], s));
     if (work.empty()) {
       // a rank of a sharded call that owns no atoms: k_mp_reduce writes zero moments
@@ -1907,7 +1972,7 @@ void multipole_run(crab_ctx* ctx, const MpInput& in, const double* q, int64_t nq
     }
   }
   k_mp_reduce<<<dim3((unsigned)(G * n_lmt), kReduceSplit), 256, 0, s>>>(d_part, d_gfirst, d_gsplits, n_lmt, lm_pad,
-                                                                         fused ? d_perm : nullptr, d_M);
+                                                                         d_perm, d_M);
   CRAB_CUDA_CHECK(cudaEventRecord(ev[2], s));
   if (in.n_shards > 1) {
     // every rank's moments summed by the caller (an all-reduce over the GPUs),
@@ -1932,8 +1997,7 @@ void multipole_run(crab_ctx* ctx, const MpInput& in, const double* q, int64_t nq
     }
   }
   const int n_nodes = S * nb;
-  const int64_t nbess = nq * n_nodes;
-  k_mp_node_bessel<<<(unsigned)((nbess + 127) / 128), 128, 0, s>>>(d_q, d_lq, nq, d_nodes, n_nodes, L, d_Jn);
+  CRAB_CUDA_CHECK(cudaStreamWaitEvent(s, ctx->ev_side, 0));  // the node values
   {
     std::vector<int2> rows;
     for (int l = 0; l <= L; ++l)
@@ -1941,17 +2005,13 @@ void multipole_run(crab_ctx* ctx, const MpInput& in, const double* q, int64_t nq
     auto* d_rows = (int2*)ctx->dev("mp_gram_rows", sizeof(int2) * rows.size());
     copy_h2d(ctx, d_rows, rows.data(), sizeof(int2) * rows.size(), s);
     auto* d_gpart = (double*)ctx->dev("mp_gram_part", sizeof(double) * rows.size() * (size_t)P * nq);
-    const size_t gram_smem = sizeof(double) * (size_t)kMaxNodes * (kGramQ + kGramM);
-    const dim3 grid((unsigned)rows.size(), (unsigned)((nq + kGramQ - 1) / kGramQ));
-    if (K == 1) {
-      CRAB_CUDA_CHECK(cudaFuncSetAttribute(k_mp_gram<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gram_smem));
-      k_mp_gram<1><<<grid, kGramThreads, gram_smem, s>>>(d_M, d_Jn, d_lq, d_amp, d_rows, T, S, nb, n_nodes, lm_pad,
-                                                          nq, d_gpart);
-    } else {
-      CRAB_CUDA_CHECK(cudaFuncSetAttribute(k_mp_gram<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gram_smem));
-      k_mp_gram<3><<<grid, kGramThreads, gram_smem, s>>>(d_M, d_Jn, d_lq, d_amp, d_rows, T, S, nb, n_nodes, lm_pad,
-                                                          nq, d_gpart);
-    }
+    // four q a lane where that fills the chip twice over, else one
+    const int ql = rows.size() * (size_t)((nq + 127) / 128) >= 2 * (size_t)ctx->sm_count ? 4 : 1;
+    const size_t gram_smem = sizeof(double) * (size_t)kMaxNodes * (32 * ql + 2 * kGramM);
+    const dim3 grid((unsigned)rows.size(), (unsigned)((nq + 32 * ql - 1) / (32 * ql)));
+    auto* gram = K == 1 ? (ql == 4 ? k_mp_gram<1, 4> : k_mp_gram<1, 1>) : (ql == 4 ? k_mp_gram<3, 4> : k_mp_gram<3, 1>);
+    CRAB_CUDA_CHECK(cudaFuncSetAttribute(gram, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gram_smem));
+    gram<<<grid, kGramThreads, gram_smem, s>>>(d_M, d_Jn, d_lq, d_amp, d_rows, T, S, nb, n_nodes, lm_pad, nq, d_gpart);
     CRAB_CUDA_CHECK(cudaGetLastError());
     k_mp_gram_reduce<<<(unsigned)(((int64_t)P * nq + 31) / 32), dim3(32, 8), 0, s>>>(d_gpart, (int)rows.size(), P,
                                                                                        nq, d_out);
@@ -1964,6 +2024,7 @@ void multipole_run(crab_ctx* ctx, const MpInput& in, const double* q, int64_t nq
   int status = 0;
   if (gemm != kGemmSimt) copy_d2h(ctx, &status, d_status, sizeof(int), s);
   CRAB_CUDA_CHECK(cudaStreamSynchronize(s));
+  side_join.on = false;  // the main stream has waited for it
   if (status != 0) throw Error(status, "multipole tensor-core GEMM: an mbarrier wait ran out");
   float total_ms = 0.0f, gemm_ms = 0.0f;
   CRAB_CUDA_CHECK(cudaEventElapsedTime(&total_ms, ev[0], ev[3]));
