@@ -310,7 +310,7 @@ int crab_hydration_grid_adaptive(crab_ctx* ctx, crab_struct* st, double spacing,
  * are caller-owned DEVICE pointers: d_xyz (n*3 f64) and d_sites (capacity*3
  * f64); `stream` is a cudaStream_t (NULL = default stream) on the current
  * device.  Every temporary lives in one file-scope __device__ array sized for
- * CRAB_NOALLOC_MAX_VOXELS voxels (about 8 MiB, held by every GPU that loads
+ * CRAB_NOALLOC_MAX_VOXELS voxels (about 1 MiB, held by every GPU that loads
  * the library until the process exits); a larger box returns CRAB_EINVAL.
  * The function calls no cudaMalloc, cudaFree or allocating library routine.
  * Its first call on a device looks up the array's device address (once per
