@@ -48,7 +48,7 @@ constexpr int kMaxNodes = 64;       // Chebyshev nodes per radial segment (GEMM 
 constexpr int kMaxSegments = 16;
 constexpr int kGemmM = 128;         // lm rows per GEMM tile
 constexpr int kPointAlign = 32;     // group padding (GEMM K step for FP32)
-constexpr int64_t kSplitK = 4096;   // points per GEMM work item
+constexpr int64_t kSplitK = 4096;   // most points per GEMM work item
 constexpr int kTileElems = kGemmM * kMaxNodes;  // one partial tile
 
 // spherical.rs:201-203
@@ -113,7 +113,7 @@ RadialBasis radial_basis(double R, double qmax) {
 }
 
 struct MpWork {
-  int32_t group, lm0;
+  int32_t slot, lm0;  // partial tile written, first lm row
   int64_t k0, k1;
 };
 
@@ -136,8 +136,9 @@ __host__ __device__ __forceinline__ int64_t mp_blocked(int row, int64_t k, int r
 // mstart[y + 1) of its points, brought up to the first one by the same
 // operations; the last one also writes the radial basis.  Bound: the latency of
 // the recurrence at one thread a point (eight parts: 1,481 atoms with sites 47
-// to 23 us, 58,870 224 to 178 us), then the stores (100,000 atoms: 315 to 293
-// us for 1.07 GB).
+// to 23 us, 58,870 224 to 178 us), then issue and the narrow conversion
+// unit (100,000 atoms, 1.07 GB of stores: 315 to 293 us; 278 us, and 159 at
+// 58,870, with the step's integer factors kept as doubles).
 template <typename E>
 __global__ void __launch_bounds__(128)
     k_mp_prep(const double* __restrict__ pts, const int32_t* __restrict__ seg, int64_t n_pad, int L, int lm_pad, int nb,
@@ -173,7 +174,10 @@ __global__ void __launch_bounds__(128)
   for (int m = ma; m < mb; ++m) {
     if (m > 0) next_m(m);
     double prev = 0.0, cur = pmm;
-    for (int l = m; l <= L; ++l) {
+    // 2 n - 1 and n + m - 1 of the step from l = m + 1 on, kept as doubles
+    // (integer conversions run on the narrow unit that rounds the stores)
+    double c1 = (double)(2 * m + 1), c0 = (double)(2 * m);
+    for (int l = m; l <= L; ++l, c1 += 2.0, c0 += 1.0) {
       if (m == 0) {
         *out = (E)__dmul_rn(snorm[row], cur);
         out += 32;
@@ -187,12 +191,10 @@ __global__ void __launch_bounds__(128)
       }
       double next;
       if (l == m) {
-        next = __dmul_rn(__dmul_rn(x, (double)(2 * m + 1)), pmm);
-      } else {
-        const int n = l + 1;  // the step from l to l + 1
-        const double num = __dadd_rn(__dmul_rn(__dmul_rn((double)(2 * n - 1), x), cur),
-                                     -__dmul_rn((double)(n + m - 1), prev));
-        next = __dmul_rn(num, inv[n - m]);
+        next = __dmul_rn(__dmul_rn(x, c1), pmm);
+      } else {  // the step from l to n = l + 1: 2 n - 1 = c1, n + m - 1 = c0
+        const double num = __dadd_rn(__dmul_rn(__dmul_rn(c1, x), cur), -__dmul_rn(c0, prev));
+        next = __dmul_rn(num, inv[l + 1 - m]);
       }
       prev = cur;
       cur = next;
@@ -219,7 +221,7 @@ __global__ void __launch_bounds__(128)
   }
 }
 
-// Partial tile of work item w: part[w][b][r] = sum_{k in [k0, k1)} YT[lm0 + r][k] WT[b][k]
+// Partial tile of a work item: part[slot][b][r] = sum_{k in [k0, k1)} YT[lm0 + r][k] WT[b][k]
 // (128 lm rows x 64 nodes, plain stores; k_mp_reduce sums the point splits).
 // 256 threads, 8 x 4 outputs each; operands staged through shared memory in
 // 128-byte rows (32 floats or 16 doubles of K per step).
@@ -271,7 +273,7 @@ __global__ void __launch_bounds__(256) k_mp_moments(const E* __restrict__ YT, co
     }
     __syncthreads();
   }
-  double* tile = part + (int64_t)blockIdx.x * kTileElems;
+  double* tile = part + (int64_t)wk.slot * kTileElems;
 #pragma unroll
   for (int x = 0; x < 8; ++x)
 #pragma unroll
@@ -581,7 +583,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       mbar_arrive(&accfree[a]);
     }
     if (ok) {
-      double* tile = part + (int64_t)blockIdx.x * kTileElems + quarter * 32 + lane;
+      double* tile = part + (int64_t)wk.slot * kTileElems + quarter * 32 + lane;
 #pragma unroll
       for (int i = 0; i < 32; ++i) tile[(half * 32 + i) * kGemmM] = acc[i];
     }
@@ -1777,8 +1779,8 @@ void multipole_run(crab_ctx* ctx, const MpInput& in, const double* q, int64_t nq
   const int n_lmt = lm_pad / kGemmM;
   const bool fused = gemm == kGemmFusedTf32 || gemm == kGemmFusedBf16;
   std::vector<int32_t> gfirst(G), gsplits(G);
-  // staged and SIMT GEMMs: items (group, point split, lm tile), lm tile fastest
-  // (k_mp_reduce relies on this order)
+  // staged and SIMT GEMMs: items (group, point split, lm tile), partial tiles
+  // in this order, lm tile fastest (k_mp_reduce relies on it)
   std::vector<MpWork> work;
   // fused GEMM: items (group, first stage, stage count), each over every lm
   // tile; partial tiles item-major, lm tile fastest (the same order for
@@ -1788,13 +1790,26 @@ void multipole_run(crab_ctx* ctx, const MpInput& in, const double* q, int64_t nq
   std::vector<double> snorm;
   const int KS = gemm == kGemmFusedBf16 ? 64 : 32;
   if (!fused) {
+    // Points per item: kSplitK, or, where the items take several rounds of the
+    // SMs, as many as fill the last round too.  The longest run first, so that
+    // the short ones at the groups' ends level the SMs (58,870 atoms with
+    // grid: 285 to 230 us; 100,000 atoms, L = 50: 453 to 412 us).
+    int64_t stages = 0;
+    for (int g = 0; g < G; ++g) stages += (begin[g + 1] - begin[g]) / KS * n_lmt;
+    const int64_t sms = ctx->sm_count, rounds = (stages * KS + sms * kSplitK - 1) / (sms * kSplitK);
+    const int64_t split = rounds < 2 ? kSplitK : (stages + sms * rounds - 1) / (sms * rounds) * KS;
+    std::vector<MpWork> runs;
+    int32_t slot = 0;
     for (int g = 0; g < G; ++g) {
-      gfirst[g] = (int32_t)work.size();
+      gfirst[g] = slot;
       gsplits[g] = 0;
-      for (int64_t k0 = begin[g]; k0 < begin[g + 1]; k0 += kSplitK, ++gsplits[g])
-        for (int lm0 = 0; lm0 < lm_pad; lm0 += kGemmM)
-          work.push_back(MpWork{g, lm0, k0, std::min(begin[g + 1], k0 + kSplitK)});
+      for (int64_t k0 = begin[g]; k0 < begin[g + 1]; k0 += split, ++gsplits[g], slot += n_lmt)
+        runs.push_back(MpWork{slot, 0, k0, std::min(begin[g + 1], k0 + split)});
     }
+    std::stable_sort(runs.begin(), runs.end(),
+                     [](const MpWork& a, const MpWork& b) { return a.k1 - a.k0 > b.k1 - b.k0; });
+    for (const MpWork& r : runs)
+      for (int t = 0; t < n_lmt; ++t) work.push_back(MpWork{r.slot + t, t * kGemmM, r.k0, r.k1});
   } else {
     std::vector<int64_t> gst(G);
     for (int g = 0; g < G; ++g) gst[g] = (begin[g + 1] - begin[g]) / KS;
