@@ -307,18 +307,45 @@ void combine_basis(const double* q, int64_t nq, const double* b, double c1, doub
   }
 }
 
-void centre_and_rmax(const crab_struct* st, double* c, double* rmax) {
-  c[0] = c[1] = c[2] = 0.0;
-  for (int64_t i = 0; i < st->n; ++i)
-    for (int d = 0; d < 3; ++d) c[d] = c[d] + st->xyz[3 * i + d];
-  const double n = (double)std::max<int64_t>(st->n, 1);
-  for (int d = 0; d < 3; ++d) c[d] = c[d] / n;
-  double r2 = 0.0;  // the root of the largest square is the largest root
-  for (int64_t i = 0; i < st->n; ++i) {
-    const double dx = st->xyz[3 * i] - c[0], dy = st->xyz[3 * i + 1] - c[1], dz = st->xyz[3 * i + 2] - c[2];
-    r2 = max_num(r2, ((0.0 + dx * dx) + dy * dy) + dz * dz);
+void sweep_box(const double* xyz, int64_t n, AtomSweep& w) {
+  double c[3] = {0.0, 0.0, 0.0};
+  for (int d = 0; d < 3; ++d) w.mn[d] = w.mx[d] = xyz[d];
+  for (int64_t i = 0; i < n; ++i)
+    for (int d = 0; d < 3; ++d) {
+      const double v = xyz[3 * i + d];
+      c[d] = c[d] + v;
+      w.mn[d] = min_num(w.mn[d], v);
+      w.mx[d] = max_num(w.mx[d], v);
+    }
+  for (int d = 0; d < 3; ++d) w.centre[d] = c[d] / (double)n;
+}
+
+void sweep_radii(const double* xyz, int64_t n, AtomSweep& w, double* copy) {
+  double acc = 0.0, r2 = 0.0;  // the root of the largest square is the largest root
+  for (int64_t i = 0; i < n; ++i) {
+    const double x = xyz[3 * i], y = xyz[3 * i + 1], z = xyz[3 * i + 2];
+    const double dx = x - w.centre[0], dy = y - w.centre[1], dz = z - w.centre[2];
+    const double d2 = ((0.0 + dx * dx) + dy * dy) + dz * dz;
+    acc += d2;
+    r2 = max_num(r2, d2);
+    if (copy) {
+      copy[3 * i] = x;
+      copy[3 * i + 1] = y;
+      copy[3 * i + 2] = z;
+    }
   }
-  *rmax = std::sqrt(r2);
+  w.rg = std::sqrt(acc / (double)n);
+  w.rmax = std::sqrt(r2);
+}
+
+void centre_and_rmax(const crab_struct* st, double* c, double* rmax) {
+  AtomSweep w = {};
+  if (st->n) {
+    sweep_box(st->xyz.data(), st->n, w);
+    sweep_radii(st->xyz.data(), st->n, w);
+  }
+  std::copy(w.centre, w.centre + 3, c);
+  *rmax = w.rmax;
 }
 
 }  // namespace crab

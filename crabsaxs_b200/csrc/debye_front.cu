@@ -211,21 +211,21 @@ bool debye_terms_device(crab_ctx* ctx, const crab_struct* st, const double* q, i
   }
   const int TA = (int)cls.size(), T = TA + (grid ? 1 : 0);
   if (TA == 0 || T > 200) return false;
+  auto* hx = (double*)ctx->host("front.xyz", (size_t)n * 3 * sizeof(double));
+  std::memcpy(hx, x, (size_t)n * 3 * sizeof(double));
+  auto* d_xyz = (double*)ctx->dev("front.xyz", (size_t)n * 3 * sizeof(double));
+  copy_h2d(ctx, d_xyz, hx, (size_t)n * 3 * sizeof(double), ctx->stream);
   GridResult g;
   if (grid) {
     TraceScope tg("hydration_sites");
     g = solvent->hydration_model == CRAB_HYD_ADAPTIVE
-            ? adaptive_grid_device(ctx, x, n, solvent->grid_spacing, 3.0, 12.0, false)
-            : exterior_grid_device(ctx, x, el, n, 1.0, 1.4, solvent->shell_thickness, false);
+            ? adaptive_grid_device(ctx, x, n, solvent->grid_spacing, 3.0, 12.0, false, GridAtoms{d_xyz, nullptr})
+            : exterior_grid_device(ctx, x, el, n, 1.0, 1.4, solvent->shell_thickness, false, GridAtoms{d_xyz, nullptr});
     if (!hist_structure_bins(2.0 * (rmax + g.outer), qmax, &X.bins[0], &X.inv_h[0])) return false;
   }
   // words: a class's candidate for its counted weight is the weight of its
   // first atom; should that turn out rarer than half, the majority vote's
   auto* word = (uint32_t*)ctx->host("front.word", (size_t)n * sizeof(uint32_t));
-  auto* hx = (double*)ctx->host("front.xyz", (size_t)n * 3 * sizeof(double));
-  std::memcpy(hx, x, (size_t)n * 3 * sizeof(double));
-  auto* d_xyz = (double*)ctx->dev("front.xyz", (size_t)n * 3 * sizeof(double));
-  copy_h2d(ctx, d_xyz, hx, (size_t)n * 3 * sizeof(double), ctx->stream);
   const double* occ = st->occ.data();
   std::vector<double> w0(TA, 0.0);
   std::vector<int64_t> nu(TA), nl(TA);

@@ -650,17 +650,18 @@ GridResult compact_sites(crab_ctx* ctx, const uint32_t* a, const uint32_t* b, ui
   return r;
 }
 
+const double* upload_xyz(crab_ctx* ctx, const double* xyz, int64_t n) {
+  double* d = pool<double>(ctx, "grid.xyz", 3 * n);
+  copy_h2d(ctx, d, xyz, 3 * n * sizeof(double), ctx->stream);
+  return d;
+}
+
 // Box set-up shared by both grids (solvent.rs:160-176 / 290-306).
-bool make_box(const double* xyz, int64_t n, double pad, double spacing, Box* b, uint64_t* count) {
-  double mn[3] = {xyz[0], xyz[1], xyz[2]}, mx[3] = {xyz[0], xyz[1], xyz[2]};
-  for (int64_t i = 1; i < n; ++i)
-    for (int d = 0; d < 3; ++d) {
-      mn[d] = min_num(mn[d], xyz[3 * i + d]);
-      mx[d] = max_num(mx[d], xyz[3 * i + d]);
-    }
+bool make_box(const AtomSweep& w, double pad, double spacing, Box* b, uint64_t* count) {
+  double mx[3];
   for (int d = 0; d < 3; ++d) {
-    b->mn[d] = mn[d] - pad;
-    mx[d] = mx[d] + pad;
+    b->mn[d] = w.mn[d] - pad;
+    mx[d] = w.mx[d] + pad;
   }
   b->spacing = spacing;
   unsigned __int128 total = 1;
@@ -678,7 +679,7 @@ bool make_box(const double* xyz, int64_t n, double pad, double spacing, Box* b, 
 }  // namespace
 
 GridResult adaptive_grid_device(crab_ctx* ctx, const double* xyz, int64_t n, double spacing, double clearance,
-                                double padding, bool to_host) {
+                                double padding, bool to_host, const GridAtoms& have) {
   GridResult r;
   if (n == 0) {
     r.voxel_volume = adaptive_site_volume(spacing);
@@ -687,21 +688,16 @@ GridResult adaptive_grid_device(crab_ctx* ctx, const double* xyz, int64_t n, dou
   require(std::isfinite(spacing) && spacing > 0.0 && std::isfinite(clearance) && clearance > 0.0 &&
               std::isfinite(padding) && padding >= 0.0,
           "adaptive hydration-grid dimensions must be finite and positive");
-  // centroid and radius of gyration in the reference's order (solvent.rs:144-155)
-  double c[3] = {0, 0, 0};
-  for (int64_t i = 0; i < n; ++i)
-    for (int d = 0; d < 3; ++d) c[d] = c[d] + xyz[3 * i + d];
-  for (int d = 0; d < 3; ++d) c[d] = c[d] / (double)n;
-  double acc = 0.0;
-  for (int64_t i = 0; i < n; ++i) {
-    const double dx = xyz[3 * i] - c[0], dy = xyz[3 * i + 1] - c[1], dz = xyz[3 * i + 2] - c[2];
-    acc += ((0.0 + dx * dx) + dy * dy) + dz * dz;
+  AtomSweep own;
+  if (!have.sweep) {
+    sweep_box(xyz, n, own);
+    sweep_radii(xyz, n, own);
   }
-  const double rg = std::sqrt(acc / (double)n);
-  const double inner = clearance, outer = clearance + adaptive_shell_width(rg);
+  const AtomSweep& w = have.sweep ? *have.sweep : own;
+  const double inner = clearance, outer = clearance + adaptive_shell_width(w.rg);
   Box b;
   uint64_t count = 0;
-  require(make_box(xyz, n, padding, spacing, &b, &count), "adaptive hydration grid is too large");
+  require(make_box(w, padding, spacing, &b, &count), "adaptive hydration grid is too large");
   require(count <= (uint64_t)4000000000ull, "adaptive hydration grid exceeds 4e9 voxels");
   TraceScope trace("adaptive_grid");
   ++ctx->grid_builds;
@@ -710,9 +706,8 @@ GridResult adaptive_grid_device(crab_ctx* ctx, const double* xyz, int64_t n, dou
   const uint64_t words = mask_words(count);
   uint32_t* shell = pool<uint32_t>(ctx, "grid.masks", 2 * words);
   uint32_t* mol = shell + words;
-  double* d_xyz = pool<double>(ctx, "grid.xyz", 3 * n);
+  const double* d_xyz = have.d_xyz ? have.d_xyz : upload_xyz(ctx, xyz, n);
   CRAB_CUDA_CHECK(cudaMemsetAsync(shell, 0, 2 * words * sizeof(uint32_t), s));
-  copy_h2d(ctx, d_xyz, xyz, 3 * n * sizeof(double), s);
   const unsigned blocks = (unsigned)((n * 32 + 255) / 256);
   k_rasterize<<<blocks, 256, 0, s>>>(d_xyz, nullptr, outer, inner, n, b, 1.0 / spacing, shell, mol);
   CRAB_CUDA_CHECK(cudaGetLastError());
@@ -724,7 +719,7 @@ GridResult adaptive_grid_device(crab_ctx* ctx, const double* xyz, int64_t n, dou
 }
 
 GridResult exterior_grid_device(crab_ctx* ctx, const double* xyz, const int8_t* elem, int64_t n, double spacing,
-                                double probe, double thickness, bool to_host) {
+                                double probe, double thickness, bool to_host, const GridAtoms& have) {
   GridResult r;
   if (n == 0) {
     r.voxel_volume = (spacing * spacing) * spacing;
@@ -740,9 +735,11 @@ GridResult exterior_grid_device(crab_ctx* ctx, const double* xyz, const int8_t* 
     vmax = max_num(vmax, radius[i]);
   }
   const double margin = vmax + probe + thickness + spacing;
+  AtomSweep own;
+  if (!have.sweep) sweep_box(xyz, n, own);
   Box b;
   uint64_t count = 0;
-  require(make_box(xyz, n, margin, spacing, &b, &count), "solvent grid is too large");
+  require(make_box(have.sweep ? *have.sweep : own, margin, spacing, &b, &count), "solvent grid is too large");
   if (count > 250000000ull)
     throw Error(CRAB_EINVAL, "solvent grid requires " + std::to_string(count) + " voxels; limit is 250000000");
   TraceScope trace("exterior_grid");
@@ -754,10 +751,9 @@ GridResult exterior_grid_device(crab_ctx* ctx, const double* xyz, const int8_t* 
   uint32_t* near = pool<uint32_t>(ctx, "grid.masks", 3 * words);
   uint32_t* mol = near + words;
   uint32_t* exterior = mol + words;
-  double* d_xyz = pool<double>(ctx, "grid.xyz", 3 * n);
+  const double* d_xyz = have.d_xyz ? have.d_xyz : upload_xyz(ctx, xyz, n);
   double* d_rad = pool<double>(ctx, "grid.radius", n);
   CRAB_CUDA_CHECK(cudaMemsetAsync(near, 0, 3 * words * sizeof(uint32_t), s));
-  copy_h2d(ctx, d_xyz, xyz, 3 * n * sizeof(double), s);
   copy_h2d(ctx, d_rad, radius.data(), n * sizeof(double), s);
   const unsigned blocks = (unsigned)((n * 32 + 255) / 256);
   k_rasterize<<<blocks, 256, 0, s>>>(d_xyz, d_rad, probe + thickness, probe, n, b, 1.0 / spacing, near, mol);

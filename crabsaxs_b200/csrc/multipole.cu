@@ -32,6 +32,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <functional>
 #include <type_traits>
 #include <vector>
 
@@ -60,16 +61,20 @@ int adaptive_l(double q, double max_radius, int maximum) {
   return (int)v;
 }
 
-// spherical.rs:33-51
-std::vector<double> harmonic_norms(int L) {
-  std::vector<double> norms((size_t)(L + 1) * (L + 1), 0.0);
-  for (int l = 0; l <= L; ++l)
-    for (int m = 0; m <= l; ++m) {
-      double ratio = 1.0;
-      for (int k = l - m + 1; k <= l + m; ++k) ratio /= (double)k;
-      norms[(size_t)l * l + l + m] = std::sqrt(((double)(2 * l + 1) / (4.0 * kPiD)) * ratio);
-    }
-  return norms;
+// Norms of the real harmonics (spherical.rs:33-51) at l^2 + l + m for every l
+// a call may ask for: constants, formed once (90,000 divisions).
+const std::vector<double>& harmonic_norms() {
+  static const std::vector<double> table = [] {
+    std::vector<double> norms((size_t)(kMaxL + 1) * (kMaxL + 1), 0.0);
+    for (int l = 0; l <= kMaxL; ++l)
+      for (int m = 0; m <= l; ++m) {
+        double ratio = 1.0;
+        for (int k = l - m + 1; k <= l + m; ++k) ratio /= (double)k;
+        norms[(size_t)l * l + l + m] = std::sqrt(((double)(2 * l + 1) / (4.0 * kPiD)) * ratio);
+      }
+    return norms;
+  }();
+  return table;
 }
 
 // Smallest node count whose Chebyshev interpolation of exp(i w s) on [-1, 1]
@@ -1612,7 +1617,9 @@ struct MpInput {
   const MpFront* front = nullptr;  // the points, when they are on the device
   double centre[3];
   double rmax_lq;                 // radius for the per-q order (atoms, or atoms and sites)
-  std::vector<double> amp;        // K x T x nq amplitude combinations (no occupancy)
+  // writes the K x T x nq amplitude combinations (no occupancy); called once,
+  // while the device forms the moments
+  std::function<void(double*)> amp;
   int K = 1;
   // multi-GPU: this rank takes the atoms [n*shard/n_shards, n*(shard+1)/n_shards)
   // into its moments, and `sum` replaces them by the sum over all ranks
@@ -1697,6 +1704,29 @@ std::vector<int> prep_splits(int L) {
 // tensor-core kernel with TF32 operands, 3 the fused kernel with BF16
 // operands; tc_terms = operand terms (1, or 2 for hi + lo).
 enum { kGemmSimt = 0, kGemmStaged = 1, kGemmFusedTf32 = 2, kGemmFusedBf16 = 3 };
+
+// Tables of a few hundred bytes that go to the device as one block.
+struct SmallTables {
+  struct Item {
+    const void* src;
+    size_t bytes, at;
+  };
+  std::vector<Item> items;
+  size_t size = 0;
+  size_t add(const void* src, size_t bytes) {
+    items.push_back(Item{src, bytes, size});
+    size += (bytes + 255) / 256 * 256;
+    return items.back().at;
+  }
+  unsigned char* upload(crab_ctx* ctx, cudaStream_t s) const {
+    auto* h = (unsigned char*)ctx->host("mp_tables", size);
+    auto* d = (unsigned char*)ctx->dev("mp_tables", size);
+    for (const Item& i : items)
+      if (i.bytes) std::memcpy(h + i.at, i.src, i.bytes);
+    copy_h2d(ctx, d, h, size, s);
+    return d;
+  }
+};
 
 // Sums 4 pi sum A^c A^d for the requested combinations; out is [K(K+1)/2][nq].
 void multipole_run(crab_ctx* ctx, const MpInput& in, const double* q, int64_t nq, int L, bool fp64, int tc_terms,
@@ -1822,7 +1852,7 @@ void multipole_run(crab_ctx* ctx, const MpInput& in, const double* q, int64_t nq
         fwork.push_back(make_int4(g, (int)s0, (int)std::min<int64_t>(cs, begin[g + 1] / KS - s0), 0));
     }
   }
-  const std::vector<double> norms = harmonic_norms(L);
+  const std::vector<double>& norms = harmonic_norms();
   std::vector<double> inv(L + 2, 0.0);
   for (int k = 1; k <= L + 1; ++k) inv[k] = 1.0 / (double)k;
   // rows in m-major order: the walk's tile starts, and per row the norm
@@ -1842,52 +1872,66 @@ void multipole_run(crab_ctx* ctx, const MpInput& in, const double* q, int64_t nq
   trace_mark("mp_host_prep");
   TraceScope tdev("multipole_device");
   cudaStream_t s = ctx->stream;
+  // the tables of the call in one copy (twelve of a few hundred bytes took 5 us each)
+  SmallTables tab;
+  const size_t o_perm = tab.add(perm.data(), sizeof(int32_t) * perm.size());
+  const size_t o_snorm = tab.add(snorm.data(), sizeof(double) * snorm.size());
+  const size_t o_mstart = tab.add(mstart.data(), sizeof(int) * mstart.size());
+  const size_t o_inv = tab.add(inv.data(), sizeof(double) * inv.size());
+  const size_t o_nodes = tab.add(B.nodes.data(), sizeof(double) * B.nodes.size());
+  const size_t o_bary = tab.add(B.bary.data(), sizeof(double) * B.bary.size());
+  const size_t o_work = tab.add(work.data(), sizeof(MpWork) * work.size());
+  const size_t o_fwork = tab.add(fwork.data(), sizeof(int4) * fwork.size());
+  const size_t o_tstart = tab.add(tstart.data(), sizeof(int4) * tstart.size());
+  const size_t o_q = tab.add(q, sizeof(double) * nq);
+  const size_t o_lq = tab.add(lq.data(), sizeof(int32_t) * nq);
+  const size_t o_gfirst = tab.add(gfirst.data(), sizeof(int32_t) * G);
+  const size_t o_gsplits = tab.add(gsplits.data(), sizeof(int32_t) * G);
+  const size_t o_begin = tab.add(begin.data(), sizeof(int64_t) * (G + 1));
+  const int no_status = 0;
+  const size_t o_status = tab.add(&no_status, sizeof(int));
+  unsigned char* d_tab = tab.upload(ctx, s);
+  const auto* d_perm = (const int32_t*)(d_tab + o_perm);
+  const auto* d_snorm = (const double*)(d_tab + o_snorm);
+  const auto* d_mstart = (const int*)(d_tab + o_mstart);
+  const auto* d_inv = (const double*)(d_tab + o_inv);
+  const auto* d_nodes = (const double*)(d_tab + o_nodes);
+  const auto* d_bary = (const double*)(d_tab + o_bary);
+  const auto* d_work = (const MpWork*)(d_tab + o_work);
+  const auto* d_fwork = (const int4*)(d_tab + o_fwork);
+  const auto* d_tstart = (const int4*)(d_tab + o_tstart);
+  const auto* d_q = (const double*)(d_tab + o_q);
+  const auto* d_lq = (const int32_t*)(d_tab + o_lq);
+  const auto* d_gfirst = (const int32_t*)(d_tab + o_gfirst);
+  const auto* d_gsplits = (const int32_t*)(d_tab + o_gsplits);
+  int* d_status = (int*)(d_tab + o_status);
   const size_t esz = fp64 ? sizeof(double) : sizeof(float);
   double* d_pts = (double*)ctx->dev("mp_pts", sizeof(double) * 5 * (size_t)n_pad);
   int32_t* d_seg = (int32_t*)ctx->dev("mp_seg", sizeof(int32_t) * n_pad);
-  int* d_mstart = (int*)ctx->dev("mp_mstart", sizeof(int) * mstart.size());
-  double* d_snorm = (double*)ctx->dev("mp_snorm", sizeof(double) * snorm.size());
-  int32_t* d_perm = (int32_t*)ctx->dev("mp_perm", sizeof(int32_t) * perm.size());
-  double* d_inv = (double*)ctx->dev("mp_inv", sizeof(double) * inv.size());
-  double* d_nodes = (double*)ctx->dev("mp_nodes", sizeof(double) * B.nodes.size());
-  double* d_bary = (double*)ctx->dev("mp_bary", sizeof(double) * B.bary.size());
   void* d_YT = fused ? nullptr : ctx->dev("mp_Y", esz * (size_t)lm_pad * n_pad);
   void* d_WT = fused ? nullptr : ctx->dev("mp_W", esz * (size_t)kMaxNodes * n_pad);
-  MpWork* d_work = fused ? nullptr : (MpWork*)ctx->dev("mp_work", sizeof(MpWork) * std::max<size_t>(work.size(), 1));
   double* d_M = (double*)ctx->dev("mp_M", sizeof(double) * (size_t)G * kMaxNodes * lm_pad);
   double* d_part = (double*)ctx->dev("mp_part", sizeof(double) * (size_t)kTileElems * std::max<size_t>(n_items, 1));
-  int32_t* d_gfirst = (int32_t*)ctx->dev("mp_gfirst", sizeof(int32_t) * G);
-  int32_t* d_gsplits = (int32_t*)ctx->dev("mp_gsplits", sizeof(int32_t) * G);
-  double* d_q = (double*)ctx->dev("mp_q", sizeof(double) * nq);
-  int32_t* d_lq = (int32_t*)ctx->dev("mp_lq", sizeof(int32_t) * nq);
   double* d_Jn = (double*)ctx->dev("mp_Jn", sizeof(double) * (size_t)nq * S * nb * (L + 1));
-  double* d_amp = (double*)ctx->dev("mp_amp", sizeof(double) * in.amp.size());
+  const size_t amp_bytes = sizeof(double) * (size_t)K * T * nq;
+  double* d_amp = (double*)ctx->dev("mp_amp", amp_bytes);
   double* d_out = (double*)ctx->dev("mp_out", sizeof(double) * (size_t)P * nq);
-  int* d_status = (int*)ctx->dev("mp_status", sizeof(int));
   // fused GEMM: recurrence constants, W blocks, walk state, row tables
   double4* d_cst = nullptr;
   unsigned char* d_Bimg = nullptr;
   FuState fst{};
-  int4* d_fwork = nullptr;
-  int4* d_tstart = nullptr;
   if (fused) {
     d_cst = (double4*)ctx->dev("mp_cst", sizeof(double4) * (size_t)n_pad);
     d_Bimg = (unsigned char*)ctx->dev("mp_Bimg", (size_t)(n_pad / KS) * tc_terms * kTcBBytes);
     double* st = (double*)ctx->dev("mp_walk", sizeof(double) * 5 * (size_t)n_pad);
     fst = FuState{st, st + n_pad, st + 2 * n_pad, st + 3 * n_pad, st + 4 * n_pad};
-    d_fwork = (int4*)ctx->dev("mp_fwork", sizeof(int4) * std::max<size_t>(fwork.size(), 1));
-    d_tstart = (int4*)ctx->dev("mp_tstart", sizeof(int4) * tstart.size());
-    copy_h2d(ctx, d_fwork, fwork.data(), sizeof(int4) * fwork.size(), s);
-    copy_h2d(ctx, d_tstart, tstart.data(), sizeof(int4) * tstart.size(), s);
   }
   if (front) {
     CRAB_CUDA_CHECK(cudaMemsetAsync(d_pts, 0, sizeof(double) * 5 * (size_t)n_pad, s));
     CRAB_CUDA_CHECK(cudaMemsetAsync(d_seg, 0, sizeof(int32_t) * n_pad, s));
-    auto* d_begin = (int64_t*)ctx->dev("mp_begin", sizeof(int64_t) * (G + 1));
-    copy_h2d(ctx, d_begin, begin.data(), sizeof(int64_t) * (G + 1), s);
     const double* c = in.centre;
     k_mp_place<<<(unsigned)((front->n_atoms + 255) / 256), 256, 0, s>>>(front->d_xyz, front->d_occ, front->d_word,
-                                                                       front->n_atoms, d_begin, c[0], c[1], c[2],
+                                                                       front->n_atoms, (const int64_t*)(d_tab + o_begin), c[0], c[1], c[2],
                                                                        d_pts);
     if (front->g.m)
       k_mp_place_sites<<<(unsigned)((front->g.m + 255) / 256), 256, 0, s>>>(front->g.d_sites, front->g.m,
@@ -1898,19 +1942,6 @@ void multipole_run(crab_ctx* ctx, const MpInput& in, const double* q, int64_t nq
     copy_h2d(ctx, d_pts, pts, sizeof(double) * 5 * (size_t)n_pad, s);
     copy_h2d(ctx, d_seg, seg, sizeof(int32_t) * n_pad, s);
   }
-  copy_h2d(ctx, d_perm, perm.data(), sizeof(int32_t) * perm.size(), s);
-  copy_h2d(ctx, d_snorm, snorm.data(), sizeof(double) * snorm.size(), s);
-  copy_h2d(ctx, d_mstart, mstart.data(), sizeof(int) * mstart.size(), s);
-  copy_h2d(ctx, d_inv, inv.data(), sizeof(double) * inv.size(), s);
-  copy_h2d(ctx, d_nodes, B.nodes.data(), sizeof(double) * B.nodes.size(), s);
-  copy_h2d(ctx, d_bary, B.bary.data(), sizeof(double) * B.bary.size(), s);
-  if (!fused) copy_h2d(ctx, d_work, work.data(), sizeof(MpWork) * work.size(), s);
-  copy_h2d(ctx, d_q, q, sizeof(double) * nq, s);
-  copy_h2d(ctx, d_lq, lq.data(), sizeof(int32_t) * nq, s);
-  copy_h2d(ctx, d_amp, in.amp.data(), sizeof(double) * in.amp.size(), s);
-  CRAB_CUDA_CHECK(cudaMemsetAsync(d_status, 0, sizeof(int), s));
-  copy_h2d(ctx, d_gfirst, gfirst.data(), sizeof(int32_t) * G, s);
-  copy_h2d(ctx, d_gsplits, gsplits.data(), sizeof(int32_t) * G, s);
 
   cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
   struct EvGuard {
@@ -1935,7 +1966,6 @@ void multipole_run(crab_ctx* ctx, const MpInput& in, const double* q, int64_t nq
   k_mp_node_bessel<<<(unsigned)((nq * S * nb + 127) / 128), 128, 0, ctx->side>>>(d_q, d_lq, nq, d_nodes, S * nb, L,
                                                                                  d_Jn);
   CRAB_CUDA_CHECK(cudaGetLastError());
-  CRAB_CUDA_CHECK(cudaEventRecord(ctx->ev_side, ctx->side));
   const unsigned prep_blocks = (unsigned)((n_pad + 127) / 128);
   if (fused) {
 #define CRAB_FUSED(EE, SS)                                                                                        \
@@ -2012,7 +2042,12 @@ void multipole_run(crab_ctx* ctx, const MpInput& in, const double* q, int64_t nq
     }
   }
   const int n_nodes = S * nb;
-  CRAB_CUDA_CHECK(cudaStreamWaitEvent(s, ctx->ev_side, 0));  // the node values
+  // the amplitudes, while the device forms the moments
+  auto* h_amp = (double*)ctx->host("mp_amp", amp_bytes);
+  in.amp(h_amp);
+  copy_h2d(ctx, d_amp, h_amp, amp_bytes, ctx->side);
+  CRAB_CUDA_CHECK(cudaEventRecord(ctx->ev_side, ctx->side));
+  CRAB_CUDA_CHECK(cudaStreamWaitEvent(s, ctx->ev_side, 0));  // the node values and the amplitudes
   {
     std::vector<int2> rows;
     for (int l = 0; l <= L; ++l)
@@ -2109,15 +2144,21 @@ bool mp_front(crab_ctx* ctx, const crab_struct* st, const double* q, int64_t nq,
   }
   if (F.t.T == 0 || F.t.T > 200) return false;
   const double* x = st->xyz.data();
-  centre_and_rmax(st, F.centre, &F.rmax);
-  F.rmax_lq = F.R = F.rmax;
   double qmax = 0.0;
   for (int64_t k = 0; k < nq; ++k) qmax = std::max(qmax, q[k]);
+  AtomSweep w;
+  sweep_box(x, n, w);
+  // a range that is too wide by the box alone is refused before anything is copied
+  double reach = 0.0;
+  for (int d = 0; d < 3; ++d) reach = std::max(reach, std::max(w.mx[d] - w.centre[d], w.centre[d] - w.mn[d]));
+  if (nodes_needed(qmax * reach * (1.0 - 1e-9) / 2.0) > kMaxNodes) return false;
+  auto* hx = (double*)ctx->host("front.xyz", (size_t)n * 4 * sizeof(double));
+  sweep_radii(x, n, w, hx);
+  std::copy(w.centre, w.centre + 3, F.centre);
+  F.rmax = F.rmax_lq = F.R = w.rmax;
   // sites add at most a shell; a range that needs more segments is the general path's
   if (nodes_needed(qmax * (F.rmax + (grid ? 16.0 : 0.0)) * (1.0 + 1e-9) / 2.0) > kMaxNodes) return false;
   cudaStream_t s = ctx->stream;
-  auto* hx = (double*)ctx->host("front.xyz", (size_t)n * 4 * sizeof(double));
-  std::memcpy(hx, x, (size_t)n * 3 * sizeof(double));
   std::memcpy(hx + 3 * n, st->occ.data(), (size_t)n * sizeof(double));
   F.d_xyz = (double*)ctx->dev("front.xyz", (size_t)n * 4 * sizeof(double));
   F.d_occ = F.d_xyz + 3 * n;
@@ -2140,8 +2181,8 @@ bool mp_front(crab_ctx* ctx, const crab_struct* st, const double* q, int64_t nq,
   trace_mark("words");
   if (grid) {
     F.g = solvent->hydration_model == CRAB_HYD_ADAPTIVE
-              ? adaptive_grid_device(ctx, x, n, solvent->grid_spacing, 3.0, 12.0, false)
-              : exterior_grid_device(ctx, x, el, n, 1.0, 1.4, solvent->shell_thickness, false);
+              ? adaptive_grid_device(ctx, x, n, solvent->grid_spacing, 3.0, 12.0, false, GridAtoms{F.d_xyz, &w})
+              : exterior_grid_device(ctx, x, el, n, 1.0, 1.4, solvent->shell_thickness, false, GridAtoms{F.d_xyz, &w});
     F.t.cls.push_back(AtomClass{-1, -1});
     ++F.t.T;
     F.count.push_back(F.g.m);
@@ -2187,15 +2228,18 @@ void multipole_tables(const TypedAtoms& t, const double* q, int64_t nq, const cr
   }
 }
 
-// Atoms (and grid sites) with their amplitude tables, the centroid and the
-// radius that sets l_q.
+// Atoms (and grid sites), the centroid and the radius that sets l_q.
 struct MpSolventSetup {
   GridResult g;
   TypedAtoms t;
   MpFront F;
   bool front = false;  // the points are F's
-  std::vector<double> V, E, H;
   double centre[3], rmax_lq;
+  // V, E, H tables of the classes
+  void tables(const double* q, int64_t nq, const crab_solvent& s, bool implicit, std::vector<double>& V,
+              std::vector<double>& E, std::vector<double>& H) const {
+    multipole_tables(front ? F.t : t, q, nq, &s, implicit, front ? F.g.voxel_volume : g.voxel_volume, V, E, H);
+  }
   void into(MpInput& in) const {
     in.t = front ? &F.t : &t;
     in.front = front ? &F : nullptr;
@@ -2210,7 +2254,6 @@ void solvent_setup(crab_ctx* ctx, const crab_struct* st, const double* q, int64_
   const bool grid = s.hydration_model != CRAB_HYD_ANALYTIC;
   if (whole && mp_front(ctx, st, q, nq, &s, implicit, u.F)) {
     u.front = true;
-    multipole_tables(u.F.t, q, nq, &s, implicit, u.F.g.voxel_volume, u.V, u.E, u.H);
     std::copy(u.F.centre, u.F.centre + 3, u.centre);
     u.rmax_lq = u.F.rmax_lq;
     return;
@@ -2219,8 +2262,6 @@ void solvent_setup(crab_ctx* ctx, const crab_struct* st, const double* q, int64_
   trace_mark("hydration sites");
   u.t = type_atoms(st, implicit, grid ? TermSet::SolventGrid : TermSet::SolventAnalytic, grid ? &u.g.sites : nullptr);
   trace_mark("type_atoms");
-  multipole_tables(u.t, q, nq, &s, implicit, u.g.voxel_volume, u.V, u.E, u.H);
-  trace_mark("tables");
   double rmax;
   centre_and_rmax(st, u.centre, &rmax);
   u.rmax_lq = rmax;
@@ -2248,25 +2289,26 @@ void multipole_intensity_impl(crab_ctx* ctx, const crab_struct* st, const double
   }
   TraceScope trace("multipole_intensity");
   MpInput in;
-  std::vector<double> V, E, H;
   MpFront F;
   if (shard.n_shards == 1 && mp_front(ctx, st, q, nq, nullptr, implicit, F)) {
-    multipole_tables(F.t, q, nq, nullptr, implicit, 0.0, V, E, H);
     in.t = &F.t;
     in.front = &F;
     std::copy(F.centre, F.centre + 3, in.centre);
     in.rmax_lq = F.rmax_lq;
   } else {
     TypedAtoms& t = typed_scratch(ctx);
-    TraceScope tt("mp_type_atoms+tables");
+    TraceScope tt("mp_type_atoms");
     type_atoms_into(st, implicit, TermSet::Vacuum, nullptr, t);
     in.t = &t;
     double rmax;
     centre_and_rmax(st, in.centre, &rmax);
     in.rmax_lq = rmax;
-    multipole_tables(t, q, nq, nullptr, implicit, 0.0, V, E, H);
   }
-  in.amp = V;
+  in.amp = [&](double* amp) {
+    std::vector<double> V, E, H;
+    multipole_tables(*in.t, q, nq, nullptr, implicit, 0.0, V, E, H);
+    std::copy(V.begin(), V.end(), amp);
+  };
   in.K = 1;
   in.shard = shard.shard;
   in.n_shards = shard.n_shards;
@@ -2291,10 +2333,11 @@ void multipole_solvent_basis_impl(crab_ctx* ctx, const crab_struct* st, const do
   MpInput in;
   u.into(in);
   in.K = 3;
-  in.amp.reserve(u.V.size() * 3);
-  in.amp.insert(in.amp.end(), u.V.begin(), u.V.end());
-  in.amp.insert(in.amp.end(), u.E.begin(), u.E.end());
-  in.amp.insert(in.amp.end(), u.H.begin(), u.H.end());
+  in.amp = [&](double* amp) {
+    std::vector<double> V, E, H;
+    u.tables(q, nq, s, implicit, V, E, H);
+    std::copy(H.begin(), H.end(), std::copy(E.begin(), E.end(), std::copy(V.begin(), V.end(), amp)));
+  };
   in.shard = shard.shard;
   in.n_shards = shard.n_shards;
   in.sum = shard.sum;
@@ -2317,14 +2360,16 @@ void multipole_solvent_intensity_impl(crab_ctx* ctx, const crab_struct* st, cons
   u.into(in);
   in.K = 1;
   // spherical.rs:438-444, 453-462: f = v - G(q) e + c2 h per atom, c2 * amplitude per site
-  in.amp.resize(u.V.size());
-  std::vector<double> scale(nq);
-  for (int64_t k = 0; k < nq; ++k) scale[k] = excluded_volume_scale(q[k], s.c1);
-  for (int a = 0; a < in.t->T; ++a)
-    for (int64_t k = 0; k < nq; ++k) {
-      const size_t o = (size_t)a * nq + k;
-      in.amp[o] = u.V[o] - scale[k] * u.E[o] + s.c2 * u.H[o];
-    }
+  in.amp = [&](double* amp) {
+    std::vector<double> V, E, H, scale(nq);
+    u.tables(q, nq, s, implicit, V, E, H);
+    for (int64_t k = 0; k < nq; ++k) scale[k] = excluded_volume_scale(q[k], s.c1);
+    for (int a = 0; a < in.t->T; ++a)
+      for (int64_t k = 0; k < nq; ++k) {
+        const size_t o = (size_t)a * nq + k;
+        amp[o] = V[o] - scale[k] * E[o] + s.c2 * H[o];
+      }
+  };
   multipole_run(ctx, in, q, nq, l_max, mp.fp64, mp.tc_terms, mp.gemm, out);
   for (int64_t k = 0; k < nq; ++k) out[k] = std::fmax(out[k], 0.0);
 }
