@@ -422,7 +422,13 @@ struct RwOpts {
 // memory: a step of 48 curves of 300 q (five evaluations on average) then has
 // block barriers only, and takes 19 us (100 us on 8 CTAs that split the weights
 // too, with a cluster barrier for each of the six sums of an evaluation).
+// Where the buffers fit too, SP = kRwCluster such CTAs, each with all curves,
+// evaluate the next SP step lengths of the line search at once; the first one
+// that decreases the objective is taken from the CTA that has it, so that the
+// steps and their values are those of the search one by one (500 steps: 9.5 to
+// 4.1 ms).
 constexpr int kRwCluster = 8;
+constexpr int kRwHalvings = 14;  // step lengths of a line search
 namespace cg = cooperative_groups;
 
 // Threads of a CTA: about one per q, and a warp more for the K logarithms.
@@ -480,10 +486,16 @@ __host__ __device__ inline size_t rw_smem(int K, int nq, int cl) {
   return (rw_doubles(K, nq, cl) + (rw_on_chip(K, nq, cl) ? (size_t)rw_rows(K, cl) * nq : 0)) * sizeof(double);
 }
 
+// Doubles more of a CTA that searches step lengths in a cluster: two halves of
+// proposal, logarithms, mixture, and of the cluster's (χ², KL, scale, background).
+__host__ __device__ inline size_t rw_search_doubles(int K, int nq) {
+  return 2 * (2 * (size_t)K + (size_t)nq + 4 * kRwCluster);
+}
+
 // Best candidate, ∂χ²/∂(c1, c2) there, then reweight.rs:84-154.
 // out: [0] best candidate, [1] scale, [2] bg, [3] reduced chi2, [4] KL,
 // [5] iterations, [6] converged, [7] dchi/dc1, [8] dchi/dc2.
-template <int CL>
+template <int CL, int SP>
 __global__ void __launch_bounds__(512, 1)
     k_ens_reweight(const double* __restrict__ curves, const double* __restrict__ fitc, int n_cand, int K, int nq,
                    const double* __restrict__ y, const double* __restrict__ sg, const double* __restrict__ weights,
@@ -495,7 +507,10 @@ __global__ void __launch_bounds__(512, 1)
   const int tid = threadIdx.x, nt = blockDim.x;
   const int back = nt - 1 - tid;  // the K-wide work of an evaluation starts at the last warp
   int rank = 0;
+  static_assert(CL == 1 || SP == 1, "the cluster splits the curves or the step lengths");
   if constexpr (CL > 1) rank = (int)cg::this_cluster().block_rank();
+  int srank = 0;
+  if constexpr (SP > 1) srank = (int)cg::this_cluster().block_rank();
   const int kr = rw_rows(K, CL), k0 = min(K, rank * kr), nk = min(K, k0 + kr) - k0;
   double* w = sm;              // K
   double* g = w + K;           // K
@@ -507,7 +522,9 @@ __global__ void __launch_bounds__(512, 1)
   double* ww = ys + nq;        // nq
   double* own = ww + nq;       // 2 x nq: this CTA's partial mixture (in a cluster)
   double* gx = own + (CL > 1 ? 2 * (size_t)nq : 0);  // 2 x kr
-  double* cvs = gx + 2 * (size_t)kr;
+  double* found = gx + 2 * (size_t)kr;  // the search's two halves
+  const size_t half_doubles = SP > 1 ? rw_search_doubles(K, nq) / 2 : 0;
+  double* cvs = found + 2 * half_doubles;
   RwSums sums{red};
   if (tid == 0) {
     best = 0;
@@ -522,7 +539,7 @@ __global__ void __launch_bounds__(512, 1)
   const double* cvr = curves + ((size_t)best * K + k0) * nq;  // this CTA's rows
   const double dof = (double)max(nq - 1, 1);
   // ∂χ²/∂c1 and ∂χ²/∂c2 at the best candidate's weights, scale and background
-  if (rank == 0) {
+  if (rank == 0 && srank == 0) {
     const double s = fitc[4 * best], b = fitc[4 * best + 1];
     const double* wb = weights + (size_t)best * K;
     const double* cb = curves + (size_t)best * K * nq;
@@ -571,7 +588,7 @@ __global__ void __launch_bounds__(512, 1)
   double s, b, chi, kl;
   // log(wv / prior) into lv; the mixture of wv, then scale and background
   // (reweight.rs:236-301), χ² and the KL term
-  auto evaluate = [&](const double* wv, double* lv) {
+  auto evaluate = [&](const double* wv, double* lv, double* mix) {
     double v[4] = {0.0, 0.0, 0.0, 0.0};  // Σ m/σ², Σ m²/σ², Σ m y/σ², Σ w log(w/prior)
     for (int k = back; k < K; k += nt) {
       const double l = log(wv[k] / prior);
@@ -637,7 +654,8 @@ __global__ void __launch_bounds__(512, 1)
     chi = e[0] / dof;
   };
   int iterations = 0, converged = 0;
-  evaluate(w, lw);
+  if constexpr (SP > 1) cg::this_cluster().sync();  // every CTA runs before one writes into another
+  evaluate(w, lw, mix);
   for (int it = 0; it < o.max_iter; ++it) {
     iterations = it + 1;
     // gradient at w, whose mixture, scale and background the last evaluation left
@@ -668,11 +686,10 @@ __global__ void __launch_bounds__(512, 1)
     gmax = fmax(sums.max(gmax), 1e-12);
     double step = o.step / gmax;
     const double objective = chi + o.kl * kl;
-    bool accepted = false;
-    for (int h = 0; h < 14 && !accepted; ++h) {
-      // proposal exp(log w - step g), normalised and floored (w is at most one,
-      // and |step g| at most o.step: the largest exponent needs no search
-      // unless the step is very long)
+    // proposal exp(log w - step g), normalised and floored (w is at most one,
+    // and |step g| at most o.step: the largest exponent needs no search
+    // unless the step is very long)
+    auto propose = [&](double step, double* pr) {
       double mx = o.step;
       if (o.step > 100.0) {
         mx = -INFINITY;
@@ -689,19 +706,58 @@ __global__ void __launch_bounds__(512, 1)
       const double all = fmax(t[0], 1e-300);
       for (int k = tid; k < K; k += nt) pr[k] = fmax(o.floor, 0.0) + residual * (pr[k] / all);
       __syncthreads();
-      evaluate(pr, lp);
-      if (chi + o.kl * kl <= objective + 1e-12) accepted = true;
-      else step *= 0.5;
+    };
+    bool accepted = false;
+    const double *np = pr, *nl = lp;  // the accepted weights and their logarithms
+    if constexpr (SP > 1) {
+      for (int h0 = 0; h0 < kRwHalvings && !accepted; h0 += SP) {
+        double* mine = found + par * half_doubles;  // proposal, logarithms, mixture, table
+        double* table = mine + 2 * K + nq;
+        par ^= 1;  // a half is written again only after the barrier that follows its readers
+        double length = step;
+        for (int h = 0; h < h0 + srank; ++h) length *= 0.5;
+        if (h0 + srank < kRwHalvings) {
+          propose(length, mine);
+          evaluate(mine, mine + K, mine + 2 * K);
+          if (tid < SP) {
+            double* t = cg::this_cluster().map_shared_rank(table, tid) + 4 * srank;
+            t[0] = chi;
+            t[1] = kl;
+            t[2] = s;
+            t[3] = b;
+          }
+        }
+        cg::this_cluster().sync();
+        for (int r = 0; r < SP && h0 + r < kRwHalvings && !accepted; ++r)
+          if (table[4 * r] + o.kl * table[4 * r + 1] <= objective + 1e-12) {
+            accepted = true;
+            chi = table[4 * r];
+            kl = table[4 * r + 1];
+            s = table[4 * r + 2];
+            b = table[4 * r + 3];
+            np = cg::this_cluster().map_shared_rank(mine, r);
+            nl = np + K;
+            for (int p = tid; p < nq; p += nt) mix[p] = np[2 * K + p];
+          }
+      }
+    } else {
+      for (int h = 0; h < kRwHalvings && !accepted; ++h) {
+        propose(step, pr);
+        evaluate(pr, lp, mix);
+        if (chi + o.kl * kl <= objective + 1e-12) accepted = true;
+        else step *= 0.5;
+      }
     }
     if (!accepted) {
-      evaluate(w, lw);  // back at the last accepted weights
+      evaluate(w, lw, mix);  // back at the last accepted weights
       break;
     }
     double t[1] = {0.0};
     for (int k = tid; k < K; k += nt) {
-      t[0] += fabs(pr[k] - w[k]);
-      w[k] = pr[k];
-      lw[k] = lp[k];
+      const double v = np[k];
+      t[0] += fabs(v - w[k]);
+      w[k] = v;
+      lw[k] = nl[k];
     }
     sums(t);
     if (t[0] <= o.tol) {
@@ -709,7 +765,7 @@ __global__ void __launch_bounds__(512, 1)
       break;
     }
   }
-  if (rank == 0) {
+  if (rank == 0 && srank == 0) {
     for (int k = tid; k < K; k += nt) w_out[k] = w[k];
     if (tid == 0) {
       out[0] = best;
@@ -721,25 +777,25 @@ __global__ void __launch_bounds__(512, 1)
       out[6] = converged;
     }
   }
-  if constexpr (CL > 1) cg::this_cluster().sync();  // no CTA leaves while a peer may still read its shared memory
+  if constexpr (CL * SP > 1) cg::this_cluster().sync();  // no CTA leaves while a peer may still read its shared memory
 }
 
-template <int CL>
+template <int CL, int SP>
 void launch_reweight(cudaStream_t s, size_t smem, const double* curves, const double* fitc, int n_cand, int K, int nq,
                      const double* y, const double* sg, const double* weights, const double* dcurves, RwOpts o,
                      double* w_out, double* out) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(CL);
+  cfg.gridDim = dim3(CL * SP);
   cfg.blockDim = dim3(rw_threads(nq));
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = CL;
+  at[0].val.clusterDim.x = CL * SP;
   at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
-  cfg.numAttrs = CL > 1 ? 1 : 0;
-  CRAB_CUDA_CHECK(cudaLaunchKernelEx(&cfg, k_ens_reweight<CL>, curves, fitc, n_cand, K, nq, y, sg, weights, dcurves, o,
+  cfg.numAttrs = CL * SP > 1 ? 1 : 0;
+  CRAB_CUDA_CHECK(cudaLaunchKernelEx(&cfg, k_ens_reweight<CL, SP>, curves, fitc, n_cand, K, nq, y, sg, weights, dcurves, o,
                                      w_out, out));
 }
 
@@ -956,9 +1012,10 @@ static void ensemble_fit_buffers(EnsemblePlan& E, const double* y, const double*
   require(weights_smem(E.K, E.nq) <= kEnsSmem && rw_smem(E.K, (int)E.nq, rw_cluster(E.K, E.nq)) <= kEnsSmem,
           "ensemble too large for the on-chip weight fit");
   CRAB_CUDA_CHECK(cudaFuncSetAttribute(k_ens_weights, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kEnsSmem));
-  CRAB_CUDA_CHECK(cudaFuncSetAttribute(k_ens_reweight<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kEnsSmem));
-  CRAB_CUDA_CHECK(
-      cudaFuncSetAttribute(k_ens_reweight<kRwCluster>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kEnsSmem));
+  constexpr auto smem_max = cudaFuncAttributeMaxDynamicSharedMemorySize;
+  CRAB_CUDA_CHECK(cudaFuncSetAttribute(k_ens_reweight<1, 1>, smem_max, (int)kEnsSmem));
+  CRAB_CUDA_CHECK(cudaFuncSetAttribute(k_ens_reweight<1, kRwCluster>, smem_max, (int)kEnsSmem));
+  CRAB_CUDA_CHECK(cudaFuncSetAttribute(k_ens_reweight<kRwCluster, 1>, smem_max, (int)kEnsSmem));
   if (!E.d_y) {
     E.d_y = E.alloc<double>(E.nq);
     E.d_sg = E.alloc<double>(E.nq);
@@ -989,8 +1046,11 @@ static void ensemble_launch_fit(EnsemblePlan& E, int Ksel, const EnsOpts& eo, co
                                                            E.d_dcurves);
     CRAB_CUDA_CHECK(cudaGetLastError());
     const int cl = rw_cluster(Ksel, E.nq);
-    const size_t shr = rw_smem(Ksel, (int)E.nq, cl);
-    auto* go = cl == 1 ? launch_reweight<1> : launch_reweight<kRwCluster>;
+    size_t shr = rw_smem(Ksel, (int)E.nq, cl);
+    const size_t more = rw_search_doubles(Ksel, (int)E.nq) * sizeof(double);
+    const bool search = cl == 1 && shr + more <= kEnsSmem;
+    if (search) shr += more;
+    auto* go = cl > 1 ? launch_reweight<kRwCluster, 1> : search ? launch_reweight<1, kRwCluster> : launch_reweight<1, 1>;
     go(sm, shr, E.d_curves, E.d_fit, E.n_cand, Ksel, (int)E.nq, E.d_y, E.d_sg, E.d_weights, E.d_dcurves, *ro, E.d_wkl,
        E.d_out);
     CRAB_CUDA_CHECK(cudaGetLastError());

@@ -23,7 +23,7 @@ def _conformers(k, rng):
     return out
 
 
-@pytest.mark.parametrize("k,nq", [(1, 20), (2, 33), (31, 64), (33, 300), (128, 40), (129, 40), (200, 300), (300, 500),
+@pytest.mark.parametrize("k,nq", [(1, 20), (2, 33), (31, 64), (33, 300), (88, 300), (90, 300), (128, 40), (129, 40), (200, 300), (300, 500),
                                   (1024, 40), (40, 3300), (1024, 3300)])
 def test_fit_and_reweighting_are_consistent(engine, k, nq):
     rng = np.random.default_rng(1000 * k + nq)
