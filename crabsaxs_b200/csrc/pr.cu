@@ -7,9 +7,10 @@
 //
 //   k_pr_far     farthest atom from the first one, then from that one: a pair,
 //                whose distance bounds dmax from below; then the largest
-//                distance R of an atom from the pair's middle
+//                distance R of an atom from the pair's middle, and from where
+//                Ritter's sphere moves it to
 //   k_pr_rim     the atoms that can belong to a longer pair: an atom at distance
-//                d from the middle is in no pair longer than d + R
+//                d from the centre is in no pair longer than d + R
 //   k_pr_dmax    the exact f64 maximum of d2 over the pairs of those (a few per
 //                cent of a globule's atoms)
 //   k_pr_edges   per bin k the smallest f64 d2 that the reference's
@@ -41,7 +42,7 @@
 // 100,000 atoms, 160 bins: 5.0e9 pairs in 3.3 ms (1.5e12 a second, issue slots
 // 82 % busy, 17 instructions a pair), where one i atom a thread, a copy of the
 // counters per warp and a branch around each near-edge pair took 5.4 ms (23
-// instructions a pair).  The call went from 10.3 to 4.1 ms: dmax takes 60 us
+// instructions a pair).  The call went from 10.3 to 3.6 ms: dmax takes 0.1 ms
 // (0.9 ms over spatially ordered tiles), the order itself and the packing of the
 // tiles, 3.6 ms of host work, are gone.
 
@@ -92,6 +93,7 @@ __device__ __forceinline__ void pr_tri_decode(int64_t w, int& a, int& b) {
 }
 
 constexpr int kPrFarBlocks = 148;
+constexpr int kPrMaxSteps = 5;
 struct PrFar {  // of a block: largest squared distance and its atom
   double d2;
   long long at;
@@ -121,30 +123,49 @@ __device__ __forceinline__ PrFar pr_block_far(PrFar v, PrFar* red) {
   return v;
 }
 
+// The farthest atom that step k found; `steps` holds the steps' results, one
+// run of kPrFarBlocks after the other.
+__device__ __forceinline__ PrFar pr_step_far(const PrFar* __restrict__ steps, int k, PrFar* red) {
+  PrFar v{-1.0, 0};
+  for (int i = threadIdx.x; i < kPrFarBlocks; i += blockDim.x) v = pr_farther(v, steps[k * kPrFarBlocks + i]);
+  return pr_block_far(v, red);
+}
+
+// Centre of step `step` (2 or more): the middle of the pair of steps 0 and 1,
+// moved towards the farthest atom of each step between as far as a ball needs
+// that covers the pair, or the last ball, and that atom (Ritter's sphere).
+__device__ __forceinline__ void pr_centre(const double* __restrict__ xyz, const PrFar* __restrict__ steps, int step,
+                                          PrFar* red, double (&c)[3]) {
+  const PrFar e0 = pr_step_far(steps, 0, red), e1 = pr_step_far(steps, 1, red);
+  for (int d = 0; d < 3; ++d) c[d] = 0.5 * (xyz[3 * e0.at + d] + xyz[3 * e1.at + d]);
+  double r = 0.5 * sqrt(e1.d2);
+  for (int k = 2; k < step; ++k) {
+    const PrFar f = pr_step_far(steps, k, red);
+    const double R = sqrt(f.d2);
+    if (R > r) {
+      const double move = 0.5 * (R - r) / R;
+      for (int d = 0; d < 3; ++d) c[d] += move * (xyz[3 * f.at + d] - c[d]);
+      r = 0.5 * (R + r);
+    }
+  }
+}
+
 // far[block]: the farthest atom from atom 0 (step 0), from the farthest of
-// step 0 (step 1), or from the centre (step 2: the middle of the pair that
-// steps 0 and 1 found, unless given).  `prev` holds the steps' results, one
-// run of kPrFarBlocks after the other.  Step 0 also flags a coordinate that is
-// not finite or 1e100 and over.
+// step 0 (step 1), or from the step's centre (the given one, if it is given).
+// Step 0 also flags a coordinate that is not finite or 1e100 and over.
 __global__ void __launch_bounds__(256) k_pr_far(const double* __restrict__ xyz, int64_t n, int step, int given,
-                                                double* __restrict__ centre, PrFar* __restrict__ prev,
+                                                const double* __restrict__ centre, PrFar* __restrict__ steps,
                                                 unsigned* __restrict__ invalid) {
   __shared__ PrFar red[8];
   double base[3] = {xyz[0], xyz[1], xyz[2]};
-  double ends[2][3];
-  for (int k = 0; k < 2 && k < step; ++k) {
-    PrFar v{-1.0, 0};
-    for (int i = threadIdx.x; i < kPrFarBlocks; i += blockDim.x) v = pr_farther(v, prev[k * kPrFarBlocks + i]);
-    const int64_t at = pr_block_far(v, red).at;
-    for (int d = 0; d < 3; ++d) ends[k][d] = xyz[3 * at + d];
+  if (step == 1) {
+    const int64_t at = pr_step_far(steps, 0, red).at;
+    for (int d = 0; d < 3; ++d) base[d] = xyz[3 * at + d];
+  } else if (step > 1 && given) {
+    for (int d = 0; d < 3; ++d) base[d] = centre[d];
+  } else if (step > 1) {
+    pr_centre(xyz, steps, step, red, base);
   }
-  if (step == 1)
-    for (int d = 0; d < 3; ++d) base[d] = ends[0][d];
-  if (step == 2)
-    for (int d = 0; d < 3; ++d) {
-      base[d] = given ? centre[d] : 0.5 * (ends[0][d] + ends[1][d]);
-      if (!given && blockIdx.x == 0 && threadIdx.x == 0) centre[d] = base[d];
-    }
   PrFar v{-1.0, 0};
   bool fine = true;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
@@ -154,43 +175,63 @@ __global__ void __launch_bounds__(256) k_pr_far(const double* __restrict__ xyz, 
   }
   if (!fine) *invalid = 1u;
   v = pr_block_far(v, red);
-  if (threadIdx.x == 0) prev[step * kPrFarBlocks + blockIdx.x] = v;
+  if (threadIdx.x == 0) steps[step * kPrFarBlocks + blockIdx.x] = v;
 }
 
 // count, then list: the atoms that may belong to a pair at least as long as
-// the known one; radius[0]: the largest distance R from the centre.  Distances
-// are f64 with relative errors below 1e-14; 1e-9 of R covers them.
-__global__ void __launch_bounds__(256) k_pr_rim(const double* __restrict__ xyz, int64_t n,
-                                                const PrFar* __restrict__ steps, const double* __restrict__ centre,
+// the known one, from the step (2 .. n_steps - 1) whose centre has the atoms
+// nearest; radius[0]: the largest distance R from it.  Distances are f64 with
+// relative errors below 1e-14; 1e-9 of R covers them.
+__global__ void __launch_bounds__(256) k_pr_rim(const double* __restrict__ xyz, int64_t n, int n_steps, int given,
+                                                const PrFar* __restrict__ steps, double* __restrict__ centre,
                                                 int* __restrict__ list,
                                                 unsigned* __restrict__ count, unsigned long long* __restrict__ dmax2,
                                                 double* __restrict__ radius) {
   __shared__ PrFar red[8];
-  PrFar v{-1.0, 0}, c{-1.0, 0};
-  for (int k = threadIdx.x; k < kPrFarBlocks; k += blockDim.x) {
-    v = pr_farther(v, steps[kPrFarBlocks + k]);
-    c = pr_farther(c, steps[2 * kPrFarBlocks + k]);
+  const PrFar v = pr_step_far(steps, 1, red);
+  int use = 2;
+  double r2 = pr_step_far(steps, 2, red).d2;
+  for (int k = 3; k < n_steps; ++k) {
+    const double k2 = pr_step_far(steps, k, red).d2;
+    if (k2 < r2) {
+      r2 = k2;
+      use = k;
+    }
   }
-  v = pr_block_far(v, red);
-  c = pr_block_far(c, red);
-  const double R = sqrt(c.d2);
+  double c[3];
+  if (given)
+    for (int d = 0; d < 3; ++d) c[d] = centre[d];
+  else
+    pr_centre(xyz, steps, use, red, c);
+  const double R = sqrt(r2);
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     *radius = R;
+    if (!given)
+      for (int d = 0; d < 3; ++d) centre[d] = c[d];
     atomicMax(dmax2, (unsigned long long)__double_as_longlong(v.d2));
   }
   const double least = sqrt(v.d2) - R * (1.0 + 1e-9);
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    if (sqrt(pr_sqdist3(centre, xyz + 3 * i)) >= least) list[atomicAdd(count, 1u)] = (int)i;
+    if (sqrt(pr_sqdist3(c, xyz + 3 * i)) >= least) list[atomicAdd(count, 1u)] = (int)i;
 }
 
 // The f64 maximum of d2 over the listed atoms' pairs, tile pairs taken in turn.
+// FP32 first: with coordinates from the centre, each within R, a squared
+// distance (at most 4 R²) is off by less than 2^-20 R² x 4, and pairs that are
+// below the longest known one by 1e-5 R² are left out; eight at a time, so that
+// an f64 pair (a few in a million) costs no branch per pair.  With eleven f64
+// instructions a pair and the first pair's middle as the centre, 100,000 atoms
+// of a ball took 60 to 470 us, depending on the first pair; so 66 where they
+// took 470.
 __global__ void __launch_bounds__(kPrThreads)
     k_pr_dmax(const double* __restrict__ xyz, const int* __restrict__ list, const unsigned* __restrict__ count,
-              unsigned long long* __restrict__ out) {
+              const double* __restrict__ centre, const double* __restrict__ radius, unsigned long long* out) {
   __shared__ double sj[3][kPrThreads];
-  __shared__ double red[kPrThreads / 32];
+  __shared__ float4 fj[kPrThreads];
   const int m = (int)*count, tid = threadIdx.x;
   const int64_t nt = (m + kPrThreads - 1) / kPrThreads, n_work = nt * (nt + 1) / 2;
+  const double c[3] = {centre[0], centre[1], centre[2]}, R = *radius;
+  const bool narrow = R > 1e-15 && R < 1e15;  // squares well inside FP32's range
   double best = 0.0;
   for (int64_t w = blockIdx.x; w < n_work; w += gridDim.x) {
     int a, b;
@@ -201,23 +242,36 @@ __global__ void __launch_bounds__(kPrThreads)
       const double* p = xyz + 3 * (int64_t)list[b * kPrThreads + tid];
       for (int d = 0; d < 3; ++d) sj[d][tid] = p[d];
     }
+    // past the end: the last atom again
+    {
+      const double* p = xyz + 3 * (int64_t)list[b * kPrThreads + min(tid, nb - 1)];
+      fj[tid] = make_float4((float)(p[0] - c[0]), (float)(p[1] - c[1]), (float)(p[2] - c[2]), 0.0f);
+    }
     __syncthreads();
     if (i < m) {
       const double* p = xyz + 3 * (int64_t)list[i];
       const double pi[3] = {p[0], p[1], p[2]};
-      for (int j = 0; j < nb; ++j) {
-        const double pj[3] = {sj[0][j], sj[1][j], sj[2][j]};
-        best = fmax(best, pr_sqdist3(pi, pj));
+      const float fx = (float)(pi[0] - c[0]), fy = (float)(pi[1] - c[1]), fz = (float)(pi[2] - c[2]);
+      const double known = fmax(best, __longlong_as_double((long long)__ldcg(out)));
+      const float least = narrow ? (float)(known - 1e-5 * R * R) * (1.0f - 1e-6f) : -1.0f;
+      for (int j0 = 0; j0 < nb; j0 += 8) {
+        float far = 0.0f;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const float4 f = fj[j0 + j];
+          const float dx = fx - f.x, dy = fy - f.y, dz = fz - f.z;
+          far = fmaxf(far, fmaf(dx, dx, fmaf(dy, dy, dz * dz)));
+        }
+        if (far >= least)
+          for (int j = j0; j < min(j0 + 8, nb); ++j) {
+            const double pj[3] = {sj[0][j], sj[1][j], sj[2][j]};
+            best = fmax(best, pr_sqdist3(pi, pj));
+          }
       }
     }
-  }
-  for (int o = 16; o > 0; o >>= 1) best = fmax(best, __shfl_xor_sync(0xffffffffu, best, o));
-  if ((tid & 31) == 0) red[tid >> 5] = best;
-  __syncthreads();
-  if (tid == 0) {
-    for (int k = 1; k < kPrThreads / 32; ++k) best = fmax(best, red[k]);
-    // non-negative doubles order as their bit patterns
-    atomicMax(out, (unsigned long long)__double_as_longlong(best));
+    // the next tiles know what this one found
+    const double top = __longlong_as_double((long long)__ldcg(out));
+    if (best > top) atomicMax(out, (unsigned long long)__double_as_longlong(best));  // non-negative doubles order as their bits
   }
 }
 
@@ -871,7 +925,7 @@ double histogram_of(crab_ctx* ctx, const double* xyz, PrClasses& C, const std::f
     for (int d = 0; d < 3; ++d) h_misc->centre[d] = 0.5 * (lo[d] + hi[d]);
   }
   auto* d_misc = (Misc*)ctx->dev("pr.misc", sizeof(Misc));
-  auto* d_far = (PrFar*)ctx->dev("pr.far", 3 * kPrFarBlocks * sizeof(PrFar));
+  auto* d_far = (PrFar*)ctx->dev("pr.far", kPrMaxSteps * kPrFarBlocks * sizeof(PrFar));
   auto* d_rim = (int*)ctx->dev("pr.rim", (size_t)n * sizeof(int));
   auto* d_edges = (double*)ctx->dev("pr.edges", edge_bytes);
   auto* d_out = (double*)ctx->dev("pr.out", (size_t)bins * sizeof(double));
@@ -888,15 +942,17 @@ double histogram_of(crab_ctx* ctx, const double* xyz, PrClasses& C, const std::f
   CRAB_CUDA_CHECK(cudaEventRecord(ev[0], s));
   double* d_centre = d_misc->centre;
   PrParams* d_par = &d_misc->par;
-  for (int step = 0; step < 3; ++step)
-    k_pr_far<<<kPrFarBlocks, 256, 0, s>>>(d_xyz, n, step, mode != kPrCounts, d_centre, d_far, &d_misc->invalid);
-  k_pr_rim<<<kPrFarBlocks, 256, 0, s>>>(d_xyz, n, d_far, d_centre, d_rim, &d_misc->rim, &d_misc->dmax2,
+  // two moves of the centre (7 us each) where the rim's pairs can take more than that
+  const int given = mode != kPrCounts, steps = !given && n >= 8192 ? kPrMaxSteps : 3;
+  for (int step = 0; step < steps; ++step)
+    k_pr_far<<<kPrFarBlocks, 256, 0, s>>>(d_xyz, n, step, given, d_centre, d_far, &d_misc->invalid);
+  k_pr_rim<<<kPrFarBlocks, 256, 0, s>>>(d_xyz, n, steps, given, d_far, d_centre, d_rim, &d_misc->rim, &d_misc->dmax2,
                                         &d_misc->radius);
-  k_pr_dmax<<<8 * ctx->sm_count, kPrThreads, 0, s>>>(d_xyz, d_rim, &d_misc->rim, &d_misc->dmax2);
+  k_pr_dmax<<<8 * ctx->sm_count, kPrThreads, 0, s>>>(d_xyz, d_rim, &d_misc->rim, d_centre, &d_misc->radius, &d_misc->dmax2);
   k_pr_edges<<<(unsigned)((bins + 1 + 127) / 128), 128, 0, s>>>(&d_misc->dmax2, bins, &d_misc->radius, &d_misc->invalid,
                                                                 d_edges, d_par);
   CRAB_CUDA_CHECK(cudaGetLastError());
-  ctx->launches += 6;
+  ctx->launches += steps + 3;
   const int ibins = (int)bins;
   if (mode == kPrCounts) {
     // tables in one copy: weight products, words, tile starts and counts, rows, CTA starts

@@ -229,3 +229,30 @@ def test_bad_coordinates_are_refused_in_every_mode(engine, bad):
             cs.pair_distance_histogram(xyz, w, 20, engine=engine)
     d, h = cs.pair_distance_histogram(xyz[:200], np.ones(200), 20, engine=engine)
     assert d > 0 and h.sum() == 200 * 199 / 2
+
+
+def _longest(xyz):
+    """Largest squared pair distance in the reference's order of operations."""
+    best = 0.0
+    for i in range(0, len(xyz), 256):
+        d = xyz[i:i + 256, None, :] - xyz[None, :, :]
+        best = max(best, np.max(d[..., 0] * d[..., 0] + d[..., 1] * d[..., 1] + d[..., 2] * d[..., 2]))
+    return best
+
+
+@pytest.mark.parametrize("shape", ["ball", "rod", "outlier", "shell", "far", "huge", "tiny", "equal"])
+@pytest.mark.parametrize("n", [130, 8191, 8192])
+def test_dmax_is_the_longest_pair(engine, n, shape):
+    """The longest pair from the rim atoms, with and without moves of the
+    centre, where FP32 squares apply and where they would overflow or vanish,
+    and with many equally long pairs: dmax equals the f64 maximum exactly."""
+    rng = np.random.default_rng(n)
+    u = rng.normal(size=(n, 3))
+    u /= np.linalg.norm(u, axis=1, keepdims=True)
+    ball = u * rng.uniform(size=(n, 1)) ** (1.0 / 3.0) * 30.0
+    xyz = {"ball": ball, "rod": ball * [4.0, 0.2, 0.2], "outlier": np.vstack([ball[1:], [[200.0, 3.0, -7.0]]]),
+           "shell": 30.0 * u, "far": ball + 1.0e6, "huge": ball * 1.0e20, "tiny": ball * 1.0e-20,
+           "equal": np.sign(ball) * 10.0}[shape]
+    s = cs.Structure(xyz, np.ones(n, np.int8))
+    got = cs.coordinate_features(s, cs.PrOptions(bins=40), engine=engine).dmax
+    assert got == np.sqrt(_longest(xyz))
