@@ -78,7 +78,7 @@ struct TermsArg {
   int T, nq, terms, shard;  // terms: 6, or 1 for the vacuum
   double density, site_volume;
 };
-constexpr int kTQ = 32, kTR = 8;  // q and row groups of a CTA
+constexpr int kTQ = 8, kTR = 32;  // q and row groups of a CTA
 
 __device__ __forceinline__ double gauss_sum(const ClassAmp& c, double q) {
   const double s = q / (4.0 * kPi), s2 = s * s;
@@ -88,10 +88,11 @@ __device__ __forceinline__ double gauss_sum(const ClassAmp& c, double q) {
   return v + c.c;
 }
 
-// Σ_ab of the quadratic forms X_a Y_b at 32 q per CTA: the amplitudes of all
-// classes go to shared memory, eight threads per q take every eighth type
-// pair each (partials read as they lie, a warp along q), and their sums are
-// added in order.
+// Σ_ab of the quadratic forms X_a Y_b at 8 q per CTA: the amplitudes of all
+// classes go to shared memory, 32 threads per q take every 32nd type pair each
+// (partials read in runs of 8 q), and their sums are added in order.  A chain
+// of exponentials and pairs per thread, so few q a CTA
+// (14 classes, 100 q: 8.7 us; 15 at 32 q a CTA and 8 threads per q).
 __global__ void __launch_bounds__(kTQ * kTR) k_debye_terms(TermsArg A, double* __restrict__ out) {
   extern __shared__ double amp[];  // [3][T][kTQ]
   __shared__ double red[kTR][6][kTQ];
