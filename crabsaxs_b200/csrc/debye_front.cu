@@ -164,7 +164,7 @@ __global__ void __launch_bounds__(kTQ * kTR) k_debye_terms(TermsArg A, double* _
 // unclamped sum (out [nq]); false where the histogram does not apply (nothing
 // done, the caller takes the general path).
 bool debye_terms_device(crab_ctx* ctx, const crab_struct* st, const double* q, int64_t nq, const crab_solvent* solvent,
-                        bool implicit, double* out, int shard, int n_shards) {
+                        bool implicit, double* out, int shard, int n_shards, FrontKeep* keep) {
   const int64_t n = st->n;
   if (ctx->pair_variant || n == 0 || nq == 0 || n >= (int64_t)kRankMask) return false;
   const bool grid = solvent && solvent->hydration_model != CRAB_HYD_ANALYTIC;
@@ -333,7 +333,7 @@ bool debye_terms_device(crab_ctx* ctx, const crab_struct* st, const double* q, i
   auto* d_word = (uint32_t*)ctx->dev("front.word", (size_t)n * sizeof(uint32_t));
   copy_h2d(ctx, d_word, word, (size_t)n * sizeof(uint32_t), s);
   double* d_occ = nullptr;
-  if (X.any_loose) {
+  if (X.any_loose || keep) {
     d_occ = (double*)ctx->dev("front.occ", (size_t)n * sizeof(double));
     copy_h2d(ctx, d_occ, occ, (size_t)n * sizeof(double), s);
   }
@@ -374,6 +374,19 @@ bool debye_terms_device(crab_ctx* ctx, const crab_struct* st, const double* q, i
   ctx->launches += 2;
   auto* h_res = (unsigned char*)ctx->host("front.result", out_bytes + 2 * sizeof(int));
   copy_d2h(ctx, h_res, d_res, out_bytes + sizeof(int), s);
+  if (keep) {
+    keep->d_xyz = d_xyz;
+    keep->d_occ = d_occ;
+    keep->d_word = d_word;
+    keep->tile0 = tile0;
+    keep->tile_type.assign(X.tile_cnt.size(), 0);
+    for (int k = 0; k < T; ++k)
+      for (const HistRange* R : {&X.loose[k], &X.uni[k]})
+        std::fill_n(keep->tile_type.begin() + R->t0, R->n, k);
+    std::copy(c, c + 3, keep->centre);
+    keep->rmax = rmax;
+    keep->meanwhile(cls);
+  }
   CRAB_CUDA_CHECK(cudaStreamSynchronize(s));
   float ms = 0.0f;
   CRAB_CUDA_CHECK(cudaEventElapsedTime(&ms, ctx->ev_start, ctx->ev_stop));

@@ -3,6 +3,8 @@
 
 #include <cuda_runtime.h>
 
+#include <cstring>
+
 #include <chrono>
 #include <cstdint>
 #include <cstdio>
@@ -150,6 +152,29 @@ inline void copy_d2h(crab_ctx* ctx, void* dst, const void* src, size_t bytes, cu
   CRAB_CUDA_CHECK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s));
   ctx->d2h_bytes += (int64_t)bytes;
 }
+
+// Tables of a few hundred bytes that go to the device as one block.
+struct SmallTables {
+  struct Item {
+    const void* src;
+    size_t bytes, at;
+  };
+  std::vector<Item> items;
+  size_t size = 0;
+  size_t add(const void* src, size_t bytes) {
+    items.push_back(Item{src, bytes, size});
+    size += (bytes + 255) / 256 * 256;
+    return items.back().at;
+  }
+  unsigned char* upload(crab_ctx* ctx, const char* slot, cudaStream_t s) const {
+    auto* h = (unsigned char*)ctx->host(slot, size);
+    auto* d = (unsigned char*)ctx->dev(slot, size);
+    for (const Item& i : items)
+      if (i.bytes) std::memcpy(h + i.at, i.src, i.bytes);
+    copy_h2d(ctx, d, h, size, s);
+    return d;
+  }
+};
 
 // ---------------------------------------------------------------- tables
 // Scattering class of an atom: element plus the united-atom group that is in

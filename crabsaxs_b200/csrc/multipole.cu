@@ -1705,29 +1705,6 @@ std::vector<int> prep_splits(int L) {
 // operands; tc_terms = operand terms (1, or 2 for hi + lo).
 enum { kGemmSimt = 0, kGemmStaged = 1, kGemmFusedTf32 = 2, kGemmFusedBf16 = 3 };
 
-// Tables of a few hundred bytes that go to the device as one block.
-struct SmallTables {
-  struct Item {
-    const void* src;
-    size_t bytes, at;
-  };
-  std::vector<Item> items;
-  size_t size = 0;
-  size_t add(const void* src, size_t bytes) {
-    items.push_back(Item{src, bytes, size});
-    size += (bytes + 255) / 256 * 256;
-    return items.back().at;
-  }
-  unsigned char* upload(crab_ctx* ctx, cudaStream_t s) const {
-    auto* h = (unsigned char*)ctx->host("mp_tables", size);
-    auto* d = (unsigned char*)ctx->dev("mp_tables", size);
-    for (const Item& i : items)
-      if (i.bytes) std::memcpy(h + i.at, i.src, i.bytes);
-    copy_h2d(ctx, d, h, size, s);
-    return d;
-  }
-};
-
 // Sums 4 pi sum A^c A^d for the requested combinations; out is [K(K+1)/2][nq].
 void multipole_run(crab_ctx* ctx, const MpInput& in, const double* q, int64_t nq, int L, bool fp64, int tc_terms,
                    int gemm, double* out) {
@@ -1890,7 +1867,7 @@ void multipole_run(crab_ctx* ctx, const MpInput& in, const double* q, int64_t nq
   const size_t o_begin = tab.add(begin.data(), sizeof(int64_t) * (G + 1));
   const int no_status = 0;
   const size_t o_status = tab.add(&no_status, sizeof(int));
-  unsigned char* d_tab = tab.upload(ctx, s);
+  unsigned char* d_tab = tab.upload(ctx, "mp_tables", s);
   const auto* d_perm = (const int32_t*)(d_tab + o_perm);
   const auto* d_snorm = (const double*)(d_tab + o_snorm);
   const auto* d_mstart = (const int*)(d_tab + o_mstart);

@@ -47,8 +47,20 @@ GridResult hydration_sites(crab_ctx* ctx, const crab_struct* st, const crab_solv
 // shard 0 only): the element-wise sum over all shards is the whole basis.
 void debye_basis(crab_ctx* ctx, const crab_struct* st, const double* q, int64_t nq, const crab_solvent& s,
                  bool implicit, double* out6, bool fp64, int shard = 0, int n_shards = 1);
+// What a caller of debye_terms_device goes on with: the atoms as they lie on the
+// device (valid until the context's next call) and where each one's slot is.
+struct FrontKeep {
+  std::function<void(const std::vector<AtomClass>&)> meanwhile;  // called once, while the device works
+  double* d_xyz = nullptr;      // [n][3]
+  double* d_occ = nullptr;      // [n]
+  uint32_t* d_word = nullptr;   // class << 24 | loose << 23 | rank, all ones: no slot (no weight, or a class without terms)
+  std::vector<int> tile0;       // per class its first counted and first loose tile
+  std::vector<int> tile_type;   // per tile of kTile slots its class
+  double centre[3], rmax;       // largest distance from the centre
+};
 bool debye_terms_device(crab_ctx* ctx, const crab_struct* st, const double* q, int64_t nq, const crab_solvent* solvent,
-                        bool implicit, double* out, int shard, int n_shards);
+                        bool implicit, double* out, int shard, int n_shards,
+                        FrontKeep* keep = nullptr);
 void debye_vacuum(crab_ctx* ctx, const crab_struct* st, const double* q, int64_t nq, bool implicit, double* out,
                   bool fp64);
 void combine_basis(const double* q, int64_t nq, const double* b, double c1, double c2, double* out);
