@@ -1406,7 +1406,8 @@ __global__ void k_mp_node_bessel(const double* __restrict__ q, const int32_t* __
 // With few q the blocks are too few for the chip and their latency is what the
 // pass takes: QL, the q of a lane, is then one (1,481 atoms of 14 classes with
 // sites, 101 q: 65 us with four, 50 with one, 32 with the moments of the next
-// group fetched while this one is used; 58,870 atoms 101, 94, 84 us).
+// group fetched while this one is used, TODO_GRAM with its amplitudes too;
+// 58,870 atoms 101, 94, 84, 83 us).
 constexpr int kGramM = 32, kGramThreads = 256;
 
 template <int K, int QL>
@@ -1458,6 +1459,14 @@ __global__ void __launch_bounds__(kGramThreads)
       __syncthreads();
       const int tn = t + 1 < T ? t + 1 : 0, sn = t + 1 < T ? sg : sg + 1;
       if (sn < S) load(tn * S + sn);
+      double a[K][QL];  // on their way during the contraction
+#pragma unroll
+      for (int c = 0; c < K; ++c)
+#pragma unroll
+        for (int j = 0; j < QL; ++j) {
+          const int64_t q = q0 + lane + 32 * j;
+          a[c][j] = q < nq ? amp[((int64_t)c * T + t) * nq + q] : 0.0;
+        }
       double C[4][QL];
 #pragma unroll
       for (int i = 0; i < 4; ++i)
@@ -1465,11 +1474,12 @@ __global__ void __launch_bounds__(kGramThreads)
         for (int j = 0; j < QL; ++j) C[i][j] = 0.0;
       const double* mrow = Mb + warp * 4;
       const double* jcol = Js + lane;
-#pragma unroll 2
+#pragma unroll(QL == 1 ? 4 : 2)
       for (int b = 0; b < nb; ++b) {
-        double mv[4], jv[QL];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) mv[i] = mrow[b * kGramM + i];
+        const double2 m01 = *reinterpret_cast<const double2*>(mrow + b * kGramM);
+        const double2 m23 = *reinterpret_cast<const double2*>(mrow + b * kGramM + 2);
+        const double mv[4] = {m01.x, m01.y, m23.x, m23.y};
+        double jv[QL];
 #pragma unroll
         for (int j = 0; j < QL; ++j) jv[j] = jcol[b * kGramQ + 32 * j];
 #pragma unroll
@@ -1478,15 +1488,11 @@ __global__ void __launch_bounds__(kGramThreads)
           for (int j = 0; j < QL; ++j) C[i][j] = fma(mv[i], jv[j], C[i][j]);
       }
 #pragma unroll
-      for (int j = 0; j < QL; ++j) {
-        const int64_t q = q0 + lane + 32 * j;
+      for (int j = 0; j < QL; ++j)
 #pragma unroll
-        for (int c = 0; c < K; ++c) {
-          const double a = q < nq ? amp[((int64_t)c * T + t) * nq + q] : 0.0;
+        for (int c = 0; c < K; ++c)
 #pragma unroll
-          for (int i = 0; i < 4; ++i) A[c][i][j] = fma(a, C[i][j], A[c][i][j]);
-        }
-      }
+          for (int i = 0; i < 4; ++i) A[c][i][j] = fma(a[c][j], C[i][j], A[c][i][j]);
     }
   }
   double acc[P][QL];
@@ -1531,8 +1537,10 @@ __global__ void __launch_bounds__(kGramThreads)
 // 32 (combination, q) outputs per CTA; thread row y sums the rows r = y, y + 8,
 // ... in order, then row 0 adds the eight partial sums in order.
 __global__ void __launch_bounds__(256) k_mp_gram_reduce(const double* __restrict__ part, int n_rows, int P,
-                                                        int64_t nq, double* __restrict__ out) {
+                                                        int64_t nq, const int* __restrict__ status,
+                                                        double* __restrict__ out) {
   __shared__ double red[8][32];
+  if (blockIdx.x == 0 && threadIdx.x + threadIdx.y == 0) *(int*)(out + (int64_t)P * nq) = *status;
   const int64_t idx = (int64_t)blockIdx.x * 32 + threadIdx.x;
   const bool on = idx < (int64_t)P * nq;
   const int p = on ? (int)(idx / nq) : 0;
@@ -1865,6 +1873,10 @@ void multipole_run(crab_ctx* ctx, const MpInput& in, const double* q, int64_t nq
   const size_t o_gfirst = tab.add(gfirst.data(), sizeof(int32_t) * G);
   const size_t o_gsplits = tab.add(gsplits.data(), sizeof(int32_t) * G);
   const size_t o_begin = tab.add(begin.data(), sizeof(int64_t) * (G + 1));
+  std::vector<int2> rows;  // (l, first m) of the q pass
+  for (int l = 0; l <= L; ++l)
+    for (int m0 = 0; m0 < 2 * l + 1; m0 += kGramM) rows.push_back(make_int2(l, m0));
+  const size_t o_rows = tab.add(rows.data(), sizeof(int2) * rows.size());
   const int no_status = 0;
   const size_t o_status = tab.add(&no_status, sizeof(int));
   unsigned char* d_tab = tab.upload(ctx, "mp_tables", s);
@@ -1881,6 +1893,7 @@ void multipole_run(crab_ctx* ctx, const MpInput& in, const double* q, int64_t nq
   const auto* d_lq = (const int32_t*)(d_tab + o_lq);
   const auto* d_gfirst = (const int32_t*)(d_tab + o_gfirst);
   const auto* d_gsplits = (const int32_t*)(d_tab + o_gsplits);
+  const auto* d_rows = (const int2*)(d_tab + o_rows);
   int* d_status = (int*)(d_tab + o_status);
   const size_t esz = fp64 ? sizeof(double) : sizeof(float);
   double* d_pts = (double*)ctx->dev("mp_pts", sizeof(double) * 5 * (size_t)n_pad);
@@ -1892,7 +1905,8 @@ void multipole_run(crab_ctx* ctx, const MpInput& in, const double* q, int64_t nq
   double* d_Jn = (double*)ctx->dev("mp_Jn", sizeof(double) * (size_t)nq * S * nb * (L + 1));
   const size_t amp_bytes = sizeof(double) * (size_t)K * T * nq;
   double* d_amp = (double*)ctx->dev("mp_amp", amp_bytes);
-  double* d_out = (double*)ctx->dev("mp_out", sizeof(double) * (size_t)P * nq);
+  const size_t out_bytes = sizeof(double) * (size_t)P * nq;  // the status after them
+  double* d_out = (double*)ctx->dev("mp_out", out_bytes + sizeof(int));
   // fused GEMM: recurrence constants, W blocks, walk state, row tables
   double4* d_cst = nullptr;
   unsigned char* d_Bimg = nullptr;
@@ -2026,11 +2040,6 @@ void multipole_run(crab_ctx* ctx, const MpInput& in, const double* q, int64_t nq
   CRAB_CUDA_CHECK(cudaEventRecord(ctx->ev_side, ctx->side));
   CRAB_CUDA_CHECK(cudaStreamWaitEvent(s, ctx->ev_side, 0));  // the node values and the amplitudes
   {
-    std::vector<int2> rows;
-    for (int l = 0; l <= L; ++l)
-      for (int m0 = 0; m0 < 2 * l + 1; m0 += kGramM) rows.push_back(make_int2(l, m0));
-    auto* d_rows = (int2*)ctx->dev("mp_gram_rows", sizeof(int2) * rows.size());
-    copy_h2d(ctx, d_rows, rows.data(), sizeof(int2) * rows.size(), s);
     auto* d_gpart = (double*)ctx->dev("mp_gram_part", sizeof(double) * rows.size() * (size_t)P * nq);
     // four q a lane where that fills the chip twice over, else one
     const int ql = rows.size() * (size_t)((nq + 127) / 128) >= 2 * (size_t)ctx->sm_count ? 4 : 1;
@@ -2041,18 +2050,20 @@ void multipole_run(crab_ctx* ctx, const MpInput& in, const double* q, int64_t nq
     gram<<<grid, kGramThreads, gram_smem, s>>>(d_M, d_Jn, d_lq, d_amp, d_rows, T, S, nb, n_nodes, lm_pad, nq, d_gpart);
     CRAB_CUDA_CHECK(cudaGetLastError());
     k_mp_gram_reduce<<<(unsigned)(((int64_t)P * nq + 31) / 32), dim3(32, 8), 0, s>>>(d_gpart, (int)rows.size(), P,
-                                                                                       nq, d_out);
+                                                                                       nq, d_status, d_out);
     ctx->launches += 1;
   }
   CRAB_CUDA_CHECK(cudaGetLastError());
   CRAB_CUDA_CHECK(cudaEventRecord(ev[3], s));
   ctx->launches += 5;
-  copy_d2h(ctx, out, d_out, sizeof(double) * (size_t)P * nq, s);
-  int status = 0;
-  if (gemm != kGemmSimt) copy_d2h(ctx, &status, d_status, sizeof(int), s);
+  auto* h_out = (unsigned char*)ctx->host("mp_out", out_bytes + sizeof(int));
+  copy_d2h(ctx, h_out, d_out, out_bytes + sizeof(int), s);
   CRAB_CUDA_CHECK(cudaStreamSynchronize(s));
+  int status;
+  std::memcpy(&status, h_out + out_bytes, sizeof(int));
   side_join.on = false;  // the main stream has waited for it
   if (status != 0) throw Error(status, "multipole tensor-core GEMM: an mbarrier wait ran out");
+  std::memcpy(out, h_out, out_bytes);
   float total_ms = 0.0f, gemm_ms = 0.0f;
   CRAB_CUDA_CHECK(cudaEventElapsedTime(&total_ms, ev[0], ev[3]));
   CRAB_CUDA_CHECK(cudaEventElapsedTime(&gemm_ms, ev[1], ev[2]));
