@@ -1406,7 +1406,7 @@ __global__ void k_mp_node_bessel(const double* __restrict__ q, const int32_t* __
 // With few q the blocks are too few for the chip and their latency is what the
 // pass takes: QL, the q of a lane, is then one (1,481 atoms of 14 classes with
 // sites, 101 q: 65 us with four, 50 with one, 32 with the moments of the next
-// group fetched while this one is used, TODO_GRAM with its amplitudes too;
+// group fetched while this one is used, 26 with its amplitudes too;
 // 58,870 atoms 101, 94, 84, 83 us).
 constexpr int kGramM = 32, kGramThreads = 256;
 
@@ -1564,15 +1564,17 @@ __device__ __forceinline__ double mp_radius(double dx, double dy, double dz) {
 constexpr uint32_t kMpDropped = 0xFFFFFFFFu;
 __global__ void k_mp_place(const double* __restrict__ xyz, const double* __restrict__ occ,
                            const uint32_t* __restrict__ word, int64_t n, const int64_t* __restrict__ begin, double cx,
-                           double cy, double cz, double* __restrict__ pts) {
+                           double cy, double cz, int S, double* __restrict__ pts, int32_t* __restrict__ seg) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n || word[i] == kMpDropped) return;
-  double* p = pts + 5 * (begin[word[i] >> 24] + (word[i] & 0xffffffu));
+  const int64_t at = begin[word[i] >> 24] + (word[i] & 0xffffffu);
+  if (S > 1) seg[at] = (int32_t)((word[i] >> 24) % (uint32_t)S);
+  double* p = pts + 5 * at;
   const double dx = __dsub_rn(xyz[3 * i], cx), dy = __dsub_rn(xyz[3 * i + 1], cy), dz = __dsub_rn(xyz[3 * i + 2], cz);
   p[0] = dx;
   p[1] = dy;
   p[2] = dz;
-  p[3] = occ[i];
+  p[3] = occ ? occ[i] : 1.0;
   p[4] = mp_radius(dx, dy, dz);
 }
 __global__ void k_mp_place_sites(const double* __restrict__ sites, int64_t m, int64_t begin, double cx, double cy,
@@ -1599,24 +1601,63 @@ __global__ void k_mp_site_rmax(const double* __restrict__ sites, int64_t m, doub
   if ((threadIdx.x & 31) == 0) atomicMax(out, (unsigned long long)__double_as_longlong(r));
 }
 
+// Words of the sites where the radial range has S > 1 segments: group group0 +
+// segment << 24 | rank in the segment, in order; count[S]: the sites of each.
+// One CTA, a thread per site and round, ranks by ballots and the warps' counts.
+__global__ void __launch_bounds__(1024)
+    k_mp_site_words(const double* __restrict__ sites, int64_t m, double cx, double cy, double cz, double R, int S,
+                    uint32_t group0, uint32_t* __restrict__ word, uint32_t* __restrict__ count) {
+  __shared__ uint32_t in_warp[kMaxSegments][32], before[kMaxSegments];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (threadIdx.x < S) before[threadIdx.x] = 0u;
+  for (int64_t base = 0; base < m; base += 1024) {
+    const int64_t i = base + threadIdx.x;
+    int g = -1;
+    if (i < m) {
+      const double r = mp_radius(__dsub_rn(sites[3 * i], cx), __dsub_rn(sites[3 * i + 1], cy),
+                                 __dsub_rn(sites[3 * i + 2], cz));
+      g = min(S - 1, (int)__dmul_rn(__ddiv_rn(r, R), (double)S));
+    }
+    uint32_t rank = 0u;
+    for (int v = 0; v < S; ++v) {
+      const uint32_t b = __ballot_sync(0xffffffffu, g == v);
+      if (g == v) rank = __popc(b & ((1u << lane) - 1u));
+      if (lane == 0) in_warp[v][warp] = __popc(b);
+    }
+    __syncthreads();
+    if (g >= 0) {
+      rank += before[g];
+      for (int w = 0; w < warp; ++w) rank += in_warp[g][w];
+      word[i] = (group0 + (uint32_t)g) << 24 | rank;
+    }
+    __syncthreads();
+    if (threadIdx.x < S)
+      for (int w = 0; w < 32; ++w) before[threadIdx.x] += in_warp[threadIdx.x][w];
+    __syncthreads();
+  }
+  if (threadIdx.x < S) count[threadIdx.x] = before[threadIdx.x];
+}
+
 // ------------------------------------------------------------------ host
 
-// The points of a call whose radial range needs one segment, on the device: the
-// host makes one word per atom (class << 24 | rank in the class, in input
-// order), and k_mp_place and k_mp_place_sites write the points where the general
-// path below would have put them, by the same f64 operations.  At 100,000
+// The points of a call on the device: the host makes one word per atom (group
+// << 24 | rank in the group, in input order; a group is a class's atoms of one
+// radial segment), and k_mp_place and k_mp_place_sites write the points where
+// the general path below would have put them, by the same f64 operations.  At 100,000
 // atoms the general path's passes (typing into three arrays, distances, groups,
 // 5 doubles per point into pinned memory) are 1.4 ms of host time, this one's
 // 0.5 ms.
 struct MpFront {
   TypedAtoms t;                // classes only
-  std::vector<int64_t> count;  // points per class
+  int S = 1;                   // radial segments
+  std::vector<int64_t> count;  // points per group
   int64_t n = 0;
   double centre[3], rmax = 0.0, rmax_lq = 0.0;  // all atoms; atoms and sites
   double R = 0.0;              // of the points kept
   GridResult g;
   double *d_xyz = nullptr, *d_occ = nullptr;
   uint32_t* d_word = nullptr;
+  uint32_t* d_site_word = nullptr;  // with several segments
   int64_t n_atoms = 0;
 };
 
@@ -1746,7 +1787,7 @@ void multipole_run(crab_ctx* ctx, const MpInput& in, const double* q, int64_t nq
   std::vector<int32_t>& group_of = ctx->mp_group_of;
   std::vector<int64_t> count(G, 0);
   if (front) {
-    require(S == 1, "one radial segment expected");
+    require(S == front->S, "radial segments of the points");
     count = front->count;
   } else {
     seg_of.resize((size_t)n);
@@ -1923,8 +1964,12 @@ void multipole_run(crab_ctx* ctx, const MpInput& in, const double* q, int64_t nq
     const double* c = in.centre;
     k_mp_place<<<(unsigned)((front->n_atoms + 255) / 256), 256, 0, s>>>(front->d_xyz, front->d_occ, front->d_word,
                                                                        front->n_atoms, (const int64_t*)(d_tab + o_begin), c[0], c[1], c[2],
-                                                                       d_pts);
-    if (front->g.m)
+                                                                       S, d_pts, d_seg);
+    if (front->g.m && S > 1)
+      k_mp_place<<<(unsigned)((front->g.m + 255) / 256), 256, 0, s>>>(front->g.d_sites, nullptr, front->d_site_word,
+                                                                     front->g.m, (const int64_t*)(d_tab + o_begin),
+                                                                     c[0], c[1], c[2], S, d_pts, d_seg);
+    else if (front->g.m)
       k_mp_place_sites<<<(unsigned)((front->g.m + 255) / 256), 256, 0, s>>>(front->g.d_sites, front->g.m,
                                                                            begin[T - 1], c[0], c[1], c[2], d_pts);
     CRAB_CUDA_CHECK(cudaGetLastError());
@@ -2101,8 +2146,8 @@ void validate_multipole(const crab_struct* st, const double* q, int64_t nq, int 
 }
 
 // Classes, words and device copies of a structure's atoms, and its sites; false
-// where the general path has to serve (several radial segments, very many atoms
-// or classes).
+// where the general path has to serve (very many atoms, or classes times
+// segments).
 bool mp_front(crab_ctx* ctx, const crab_struct* st, const double* q, int64_t nq, const crab_solvent* solvent,
               bool implicit, MpFront& F) {
   const int64_t n = st->n;
@@ -2136,36 +2181,63 @@ bool mp_front(crab_ctx* ctx, const crab_struct* st, const double* q, int64_t nq,
   for (int64_t k = 0; k < nq; ++k) qmax = std::max(qmax, q[k]);
   AtomSweep w;
   sweep_box(x, n, w);
-  // a range that is too wide by the box alone is refused before anything is copied
-  double reach = 0.0;
-  for (int d = 0; d < 3; ++d) reach = std::max(reach, std::max(w.mx[d] - w.centre[d], w.centre[d] - w.mn[d]));
-  if (nodes_needed(qmax * reach * (1.0 - 1e-9) / 2.0) > kMaxNodes) return false;
   auto* hx = (double*)ctx->host("front.xyz", (size_t)n * 4 * sizeof(double));
   sweep_radii(x, n, w, hx);
   std::copy(w.centre, w.centre + 3, F.centre);
   F.rmax = F.rmax_lq = F.R = w.rmax;
-  // sites add at most a shell; a range that needs more segments is the general path's
-  if (nodes_needed(qmax * (F.rmax + (grid ? 16.0 : 0.0)) * (1.0 + 1e-9) / 2.0) > kMaxNodes) return false;
   cudaStream_t s = ctx->stream;
   std::memcpy(hx + 3 * n, st->occ.data(), (size_t)n * sizeof(double));
   F.d_xyz = (double*)ctx->dev("front.xyz", (size_t)n * 4 * sizeof(double));
   F.d_occ = F.d_xyz + 3 * n;
   copy_h2d(ctx, F.d_xyz, hx, (size_t)n * 4 * sizeof(double), s);
-  auto* word = (uint32_t*)ctx->host("front.word", (size_t)n * sizeof(uint32_t));
-  std::vector<uint32_t> rank(F.t.T, 0);
-  double r2 = 0.0;
-  for (int64_t i = 0; i < n; ++i) {
-    const int k = cls_of[el[i] * 16 + ((gr[i] + 1) & gmask)];
-    word[i] = k < 0 ? kMpDropped : (uint32_t)k << 24 | rank[k]++;
-    if (dropped && k >= 0) {
-      const double dx = x[3 * i] - F.centre[0], dy = x[3 * i + 1] - F.centre[1], dz = x[3 * i + 2] - F.centre[2];
-      r2 = max_num(r2, ((0.0 + dx * dx) + dy * dy) + dz * dz);
-    }
-  }
-  if (dropped) F.R = std::sqrt(r2);
-  F.d_word = (uint32_t*)ctx->dev("front.word", (size_t)n * sizeof(uint32_t));
-  copy_h2d(ctx, F.d_word, word, (size_t)n * sizeof(uint32_t), s);
   F.n_atoms = n;
+  auto square = [&](int64_t i) {
+    const double dx = x[3 * i] - F.centre[0], dy = x[3 * i + 1] - F.centre[1], dz = x[3 * i + 2] - F.centre[2];
+    return ((0.0 + dx * dx) + dy * dy) + dz * dz;
+  };
+  auto class_at = [&](int64_t i) { return cls_of[el[i] * 16 + ((gr[i] + 1) & gmask)]; };
+  if (dropped) {
+    double r2 = 0.0;
+    for (int64_t i = 0; i < n; ++i)
+      if (class_at(i) >= 0) r2 = max_num(r2, square(i));
+    F.R = std::sqrt(r2);
+  }
+  const int TA = F.t.T;
+  auto* word = (uint32_t*)ctx->host("front.word", (size_t)n * sizeof(uint32_t));
+  F.d_word = (uint32_t*)ctx->dev("front.word", (size_t)n * sizeof(uint32_t));
+  // words for S segments up to R; the segment is min(S - 1, floor(r / R * S)),
+  // formed itself only where r² lies within 1e-12 of a border's square
+  auto make_words = [&](int S, double R) {
+    std::vector<uint32_t> rank((size_t)TA * S, 0);
+    double border[kMaxSegments] = {};
+    for (int k = 1; k < S; ++k) border[k] = (R * k / S) * (R * k / S);
+    for (int64_t i = 0; i < n; ++i) {
+      const int k = class_at(i);
+      if (k < 0) {
+        word[i] = kMpDropped;
+        continue;
+      }
+      int g = k * S;
+      if (S > 1) {
+        const double d2 = square(i);
+        int seg = 0;
+        bool near = false;
+        for (int v = 1; v < S; ++v) {
+          seg += d2 >= border[v];
+          near = near || std::fabs(d2 - border[v]) <= 1e-12 * border[v];
+        }
+        if (near) seg = std::min(S - 1, (int)(std::sqrt(d2) / R * S));
+        g += seg;
+      }
+      word[i] = (uint32_t)g << 24 | rank[g]++;
+    }
+    copy_h2d(ctx, F.d_word, word, (size_t)n * sizeof(uint32_t), s);
+    if (S > 1) F.count.assign(rank.begin(), rank.end());
+  };
+  // sites add at most a shell: where that leaves one segment, the words go up
+  // before the grid is built
+  const bool narrow = nodes_needed(qmax * (F.R + (grid ? 16.0 : 0.0)) * (1.0 + 1e-9) / 2.0) <= kMaxNodes;
+  if (narrow) make_words(1, 1.0);
   trace_mark("words");
   if (grid) {
     F.g = solvent->hydration_model == CRAB_HYD_ADAPTIVE
@@ -2190,7 +2262,26 @@ bool mp_front(crab_ctx* ctx, const crab_struct* st, const double* q, int64_t nq,
     }
   }
   const double R = F.R > 0.0 ? F.R * (1.0 + 1e-12) : 1.0;
-  return nodes_needed(qmax * R / 2.0) <= kMaxNodes;
+  if (narrow) return nodes_needed(qmax * R / 2.0) <= kMaxNodes;
+  F.S = radial_basis(R, qmax).S;
+  if (F.t.T * F.S > 200 || F.g.m >= (1 << 24)) return false;
+  make_words(F.S, R);
+  if (F.S == 1 || !grid) return true;
+  const int S = F.S;
+  F.count.resize((size_t)F.t.T * S, 0);
+  if (F.g.m) {
+    F.d_site_word = (uint32_t*)ctx->dev("mp_site_word", (size_t)F.g.m * sizeof(uint32_t));
+    auto* d_count = (uint32_t*)ctx->dev("mp_site_count", kMaxSegments * sizeof(uint32_t));
+    auto* h_count = (uint32_t*)ctx->host("mp_site_count", kMaxSegments * sizeof(uint32_t));
+    k_mp_site_words<<<1, 1024, 0, s>>>(F.g.d_sites, F.g.m, F.centre[0], F.centre[1], F.centre[2], R, S,
+                                       (uint32_t)(TA * S), F.d_site_word, d_count);
+    CRAB_CUDA_CHECK(cudaGetLastError());
+    ctx->launches += 1;
+    copy_d2h(ctx, h_count, d_count, S * sizeof(uint32_t), s);
+    CRAB_CUDA_CHECK(cudaStreamSynchronize(s));
+    std::copy(h_count, h_count + S, F.count.end() - S);
+  }
+  return true;
 }
 
 // Per-type multipole amplitudes without occupancy (spherical.rs:205-231):
