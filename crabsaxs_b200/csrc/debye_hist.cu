@@ -39,7 +39,7 @@
 // pairs and 13,000 bins (B200, 1965 MHz), the inner loop takes 0.41 ms, 0.28 ms
 // without its atomics, and 1.05 ms with one 64-bit atomic per pair instead of
 // two 32-bit ones; four i atoms a lane take 0.41 ms, two 0.44, one 0.50.
-// 20,000 atoms with 9,369 sites at 500 q: k_hist_pairs 0.33 ms (1.0e12 pairs/s),
+// 20,000 atoms with 9,369 sites at 500 q: k_hist_pairs 0.36 to 0.41 ms (1e12 pairs/s),
 // transform and reduction 0.02 ms, against 18 ms for the recurrence kernel.
 // The error against the FP64 kernel falls from 1.2e-9 to 9e-11 of the basis
 // (2-norm), as counts do not round.
