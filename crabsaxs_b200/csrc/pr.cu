@@ -94,6 +94,7 @@ __device__ __forceinline__ void pr_tri_decode(int64_t w, int& a, int& b) {
 
 constexpr int kPrFarBlocks = 148;
 constexpr int kPrMaxSteps = 5;
+constexpr int64_t kPrEvery = 4096;  // atoms up to which every pair is looked at for the longest
 struct PrFar {  // of a block: largest squared distance and its atom
   double d2;
   long long at;
@@ -231,6 +232,7 @@ __global__ void __launch_bounds__(kPrThreads)
   const int m = (int)*count, tid = threadIdx.x;
   const int64_t nt = (m + kPrThreads - 1) / kPrThreads, n_work = nt * (nt + 1) / 2;
   const double c[3] = {centre[0], centre[1], centre[2]}, R = *radius;
+  auto atom = [&](int k) { return list ? (int64_t)list[k] : (int64_t)k; };  // no list: every atom
   const bool narrow = R > 1e-15 && R < 1e15;  // squares well inside FP32's range
   double best = 0.0;
   for (int64_t w = blockIdx.x; w < n_work; w += gridDim.x) {
@@ -239,17 +241,17 @@ __global__ void __launch_bounds__(kPrThreads)
     const int nb = min(kPrThreads, m - b * kPrThreads), i = a * kPrThreads + tid;
     __syncthreads();
     if (tid < nb) {
-      const double* p = xyz + 3 * (int64_t)list[b * kPrThreads + tid];
+      const double* p = xyz + 3 * atom(b * kPrThreads + tid);
       for (int d = 0; d < 3; ++d) sj[d][tid] = p[d];
     }
     // past the end: the last atom again
     {
-      const double* p = xyz + 3 * (int64_t)list[b * kPrThreads + min(tid, nb - 1)];
+      const double* p = xyz + 3 * atom(b * kPrThreads + min(tid, nb - 1));
       fj[tid] = make_float4((float)(p[0] - c[0]), (float)(p[1] - c[1]), (float)(p[2] - c[2]), 0.0f);
     }
     __syncthreads();
     if (i < m) {
-      const double* p = xyz + 3 * (int64_t)list[i];
+      const double* p = xyz + 3 * atom(i);
       const double pi[3] = {p[0], p[1], p[2]};
       const float fx = (float)(pi[0] - c[0]), fy = (float)(pi[1] - c[1]), fz = (float)(pi[2] - c[2]);
       const double known = fmax(best, __longlong_as_double((long long)__ldcg(out)));
@@ -913,7 +915,11 @@ double histogram_of(crab_ctx* ctx, const double* xyz, PrClasses& C, const std::f
   };
   auto* h_misc = (Misc*)ctx->host("pr.misc", sizeof(Misc));
   std::memset(h_misc, 0, sizeof(Misc));
-  if (mode != kPrCounts) {  // the weighted kernels' tiles are centred on the host
+  // few atoms: looking at all their pairs takes less than the four passes that
+  // leave some out (354 atoms, 444 bins: 146 us a call with the passes, 128
+  // without; 4,000 atoms, 160 bins: 168 and 155)
+  const bool every = n <= kPrEvery;
+  if (mode != kPrCounts || every) {  // the weighted kernels' tiles are centred on the host
     double lo[3] = {xyz[0], xyz[1], xyz[2]}, hi[3] = {xyz[0], xyz[1], xyz[2]};
     for (int64_t i = 0; i < n; ++i)
       for (int d = 0; d < 3; ++d) {
@@ -923,6 +929,16 @@ double histogram_of(crab_ctx* ctx, const double* xyz, PrClasses& C, const std::f
         hi[d] = max_num(hi[d], v);
       }
     for (int d = 0; d < 3; ++d) h_misc->centre[d] = 0.5 * (lo[d] + hi[d]);
+  }
+  if (every) {
+    const double* c = h_misc->centre;
+    double r2 = 0.0;
+    for (int64_t i = 0; i < n; ++i) {
+      const double dx = xyz[3 * i] - c[0], dy = xyz[3 * i + 1] - c[1], dz = xyz[3 * i + 2] - c[2];
+      r2 = max_num(r2, dx * dx + dy * dy + dz * dz);
+    }
+    h_misc->radius = std::sqrt(r2) * (1.0 + 1e-12);
+    h_misc->rim = (unsigned)n;
   }
   auto* d_misc = (Misc*)ctx->dev("pr.misc", sizeof(Misc));
   auto* d_far = (PrFar*)ctx->dev("pr.far", kPrMaxSteps * kPrFarBlocks * sizeof(PrFar));
@@ -942,17 +958,21 @@ double histogram_of(crab_ctx* ctx, const double* xyz, PrClasses& C, const std::f
   CRAB_CUDA_CHECK(cudaEventRecord(ev[0], s));
   double* d_centre = d_misc->centre;
   PrParams* d_par = &d_misc->par;
-  // two moves of the centre (7 us each) where the rim's pairs can take more than that
-  const int given = mode != kPrCounts, steps = !given && n >= 8192 ? kPrMaxSteps : 3;
-  for (int step = 0; step < steps; ++step)
-    k_pr_far<<<kPrFarBlocks, 256, 0, s>>>(d_xyz, n, step, given, d_centre, d_far, &d_misc->invalid);
-  k_pr_rim<<<kPrFarBlocks, 256, 0, s>>>(d_xyz, n, steps, given, d_far, d_centre, d_rim, &d_misc->rim, &d_misc->dmax2,
-                                        &d_misc->radius);
-  k_pr_dmax<<<8 * ctx->sm_count, kPrThreads, 0, s>>>(d_xyz, d_rim, &d_misc->rim, d_centre, &d_misc->radius, &d_misc->dmax2);
+  if (!every) {
+    // two moves of the centre (7 us each) where the rim's pairs can take more than that
+    const int given = mode != kPrCounts, steps = !given && n >= 8192 ? kPrMaxSteps : 3;
+    for (int step = 0; step < steps; ++step)
+      k_pr_far<<<kPrFarBlocks, 256, 0, s>>>(d_xyz, n, step, given, d_centre, d_far, &d_misc->invalid);
+    k_pr_rim<<<kPrFarBlocks, 256, 0, s>>>(d_xyz, n, steps, given, d_far, d_centre, d_rim, &d_misc->rim, &d_misc->dmax2,
+                                          &d_misc->radius);
+    ctx->launches += steps + 1;
+  }
+  k_pr_dmax<<<8 * ctx->sm_count, kPrThreads, 0, s>>>(d_xyz, every ? nullptr : d_rim, &d_misc->rim, d_centre,
+                                                     &d_misc->radius, &d_misc->dmax2);
   k_pr_edges<<<(unsigned)((bins + 1 + 127) / 128), 128, 0, s>>>(&d_misc->dmax2, bins, &d_misc->radius, &d_misc->invalid,
                                                                 d_edges, d_par);
   CRAB_CUDA_CHECK(cudaGetLastError());
-  ctx->launches += steps + 3;
+  ctx->launches += 2;
   const int ibins = (int)bins;
   if (mode == kPrCounts) {
     // tables in one copy: weight products, words, tile starts and counts, rows, CTA starts

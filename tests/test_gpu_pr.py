@@ -241,7 +241,7 @@ def _longest(xyz):
 
 
 @pytest.mark.parametrize("shape", ["ball", "rod", "outlier", "shell", "far", "huge", "tiny", "equal"])
-@pytest.mark.parametrize("n", [130, 8191, 8192])
+@pytest.mark.parametrize("n", [130, 4096, 4097, 8191, 8192])
 def test_dmax_is_the_longest_pair(engine, n, shape):
     """The longest pair from the rim atoms, with and without moves of the
     centre, where FP32 squares apply and where they would overflow or vanish,
