@@ -206,9 +206,9 @@ def typed_arrays(s, sites):
     return xyz, w, t, len(classes) + 1
 
 
-def traffic_per_launch():
-    """DRAM bytes per pair-kernel launch from the committed ncu summary, if present."""
-    p = ROOT / "profiles" / "debye_pair_fp32_20k_500q.txt"
+def traffic_per_launch(variant):
+    """DRAM bytes per pair-kernel launch from the kernel's committed ncu summary, if present."""
+    p = ROOT / "profiles" / ("debye_hist_20k_500q.txt" if variant == HIST_VARIANT else "debye_pair_fp32_20k_500q.txt")
     if not p.exists():
         return None
     m = re.search(r"dram_bytes_per_launch:\s*([0-9.eE+]+)", p.read_text())
@@ -854,7 +854,7 @@ def run_ours(args, rank, world, local):
                        "allreduce_ms_per_step": float(np.mean(reduce_ms)) if world > 1 else 0.0,
                        "l2": "flushed before every step (256 MiB memset, outside the step events)"},
             "roofline": {"bound": "fp32", "achieved": achieved, "peak": peak.value, "unit": "TFLOP/s",
-                         "frac": achieved / peak.value, "traffic": traffic_per_launch(),
+                         "frac": achieved / peak.value, "traffic": traffic_per_launch(chosen.value),
                          "units_per_launch": units,
                          "peak_source": "FFMA microbenchmark measured in this run (MEASURED_PEAKS.json has no FP32)",
                          "flop_per_unit": flop_per_unit},

@@ -259,9 +259,10 @@ __device__ __forceinline__ uint32_t fill_row(const uint32_t* __restrict__ bits, 
 // point is.  Every round but the last labels a voxel, so there are no more
 // rounds than voxels.  Rows are an odd number of words apart and so are the
 // lanes' parts along y: a warp's words lie in different banks.  One launch
-// instead of three per round of sweeps over bytes (20,000 atoms, 1.28 million
-// voxels: 250 us in the sweeps' launches, 138 us with a thread per line of
-// words along y and rows a multiple of four words apart, 26 us so).
+// instead of three per round of sweeps over bytes: 20,000 atoms, 1.17 million
+// voxels, few rounds: 250 us in the sweeps' launches, 138 us with a thread per
+// line of words along y and rows a multiple of four words apart, 26 us so; a box
+// of 1.28 million whose pockets take eleven rounds 97 us (450 with the sweeps).
 constexpr int kFillCtas = 8, kFillThreads = 1024;
 constexpr size_t kFillSmem = 220 * 1024;
 __host__ __device__ inline uint64_t fill_row_words(const Box& b) { return ((b.n[0] + 31) / 32) | 1; }
