@@ -366,7 +366,7 @@ __global__ void __cluster_dims__(kFillCtas, 1, 1) __launch_bounds__(kFillThreads
       }
     }
     // the neighbours' boundary planes are read as they stand: a label that is
-    // missed now was set in this round, which is then not the last
+    // missed now was set since the last agreement, which then is not the last one
     cl.sync();
     const uint32_t* below = rank > 0 ? cl.map_shared_rank(ext, rank - 1) + (size_t)(slab - 1) * plane : nullptr;
     const uint32_t* above = rank + 1 < kFillCtas && z0 + zs < nz ? cl.map_shared_rank(ext, rank + 1) : nullptr;

@@ -2,7 +2,7 @@
 ragged warps, the counting sort (up to 128) against the network, curves in and out of shared memory, one CTA against a
 cluster, and q grids too long for the per-q tables.
 
-The checker restates one step's outcome from the returned weights in f64: χ², its gradient in the weights, and the KL
+The test restates one step's outcome from the returned weights in f64: χ², its gradient in the weights, and the KL
 objective's stationarity.  Sums of m f64 terms in another order differ by at most m 2^-53 of their absolute sum, and
 the fit of scale and background passes that on with the conditioning of a 2 x 2 system: 1e-9 leaves a factor 1e4.
 """
