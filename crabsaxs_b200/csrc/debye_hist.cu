@@ -71,8 +71,6 @@ constexpr int kHistFlush = 256;               // units between flushes: 2^21 pai
 constexpr int kHistStagingBytes = kHWarps * 2 * kChunkBytes;
 constexpr int kHistBarBytes = kHWarps * 2 * 8;
 constexpr int kHistSumOffset = kHistMaxBins * 4;  // Σu words after the counts
-constexpr int kHistSmem = kHistStagingBytes + kHistBarBytes + 2 * kHistSumOffset;
-static_assert(kHistSmem <= 232448, "histogram and staging exceed the shared memory of an SM");
 static_assert((long long)kHistFlush * 128 * kChunkAtoms <= (1ll << 21), "Σu of one bin must stay below 2^31");
 constexpr float kMagicBin = 12582912.0f;      // 1.5 x 2^23: adding it rounds to an integer in the low bits
 constexpr unsigned kMagicBinBits = 0x4B400000u;
@@ -80,8 +78,16 @@ constexpr float kMagicU = 6144.0f;            // 1.5 x 2^12: low bits in units o
 constexpr unsigned kMagicUBits = 0x45C00000u;
 constexpr int kLooseMaxBins = 11424;          // 64-bit sums in shared memory; wider rows add into device memory
 constexpr int kLooseSumOffset = kLooseMaxBins * 8;
-static_assert(kHistStagingBytes + kHistBarBytes + 2 * kLooseSumOffset <= 232448, "loose sums exceed the shared memory");
 enum { kCounts = 0, kLooseShared = 1, kLooseGlobal = 2 };  // where the pairs of a launch go
+// Dynamic shared memory of a launch: staging, barriers and the sums that its
+// mode keeps there.
+template <int MODE>
+constexpr int hist_smem() {
+  return kHistStagingBytes + kHistBarBytes +
+         2 * (MODE == kCounts ? kHistSumOffset : MODE == kLooseShared ? kLooseSumOffset : 0);
+}
+static_assert(hist_smem<kCounts>() <= 232448, "histogram and staging exceed the shared memory of an SM");
+static_assert(hist_smem<kLooseShared>() <= 232448, "loose sums and staging exceed the shared memory of an SM");
 constexpr int kHistQ = 128, kHistR = 16;      // q and type pairs of a transform CTA
 constexpr int kHistW = 16, kHistM = 5;        // bins of a wide bin, and its moments
 constexpr int kHistB = 16;                    // wide bins per step of the transform
@@ -759,11 +765,10 @@ bool hist_build(crab_ctx* ctx, PairPlan& P, HistShape& X, const std::vector<unsi
   H.loose_bins = loose_bins;
   H.d_acc = (unsigned long long*)plan_alloc(ctx, P, P.owned, "hist_acc", (size_t)(acc_bins + loose_bins) * 16);
   H.d_part = (double*)plan_alloc(ctx, P, P.owned, "hist_part", part_rows * (size_t)P.nq * sizeof(double));
-  CRAB_CUDA_CHECK(cudaFuncSetAttribute(k_hist_pairs<kCounts>, cudaFuncAttributeMaxDynamicSharedMemorySize, kHistSmem));
-  CRAB_CUDA_CHECK(
-      cudaFuncSetAttribute(k_hist_pairs<kLooseShared>, cudaFuncAttributeMaxDynamicSharedMemorySize, kHistSmem));
-  CRAB_CUDA_CHECK(
-      cudaFuncSetAttribute(k_hist_pairs<kLooseGlobal>, cudaFuncAttributeMaxDynamicSharedMemorySize, kHistSmem));
+  constexpr auto smem_max = cudaFuncAttributeMaxDynamicSharedMemorySize;
+  CRAB_CUDA_CHECK(cudaFuncSetAttribute(k_hist_pairs<kCounts>, smem_max, hist_smem<kCounts>()));
+  CRAB_CUDA_CHECK(cudaFuncSetAttribute(k_hist_pairs<kLooseShared>, smem_max, hist_smem<kLooseShared>()));
+  CRAB_CUDA_CHECK(cudaFuncSetAttribute(k_hist_pairs<kLooseGlobal>, smem_max, hist_smem<kLooseGlobal>()));
   H.active = true;
   return true;
 }
@@ -779,19 +784,19 @@ void hist_plan_launch(crab_ctx* ctx, PairPlan& P, cudaStream_t s) {
     const HistGroup& g = H.groups[i];
     CRAB_CUDA_CHECK(cudaMemsetAsync(H.d_acc, 0, (size_t)(H.acc_bins + H.loose_bins) * 16, s));
     if (g.n_rows) {
-      k_hist_pairs<kCounts><<<g.grid, kHT, kHistSmem, s>>>(H.d_pts, H.d_tile_cnt, nullptr, H.d_rows + g.row0,
-                                                           H.d_start + g.start0, cnt, sum, H.widest, 1.0, P.d_status,
-                                                           ctx->wait_budget);
+      k_hist_pairs<kCounts><<<g.grid, kHT, hist_smem<kCounts>(), s>>>(
+          H.d_pts, H.d_tile_cnt, nullptr, H.d_rows + g.row0, H.d_start + g.start0, cnt, sum, H.widest, 1.0, P.d_status,
+          ctx->wait_budget);
       CRAB_CUDA_CHECK(cudaGetLastError());
       ctx->launches += 1;
     }
     if (H.loose_grid) {  // with loose rows there is one group
       if (H.widest <= kLooseMaxBins)
-        k_hist_pairs<kLooseShared><<<H.loose_grid, kHT, kHistSmem, s>>>(
+        k_hist_pairs<kLooseShared><<<H.loose_grid, kHT, hist_smem<kLooseShared>(), s>>>(
             H.d_pts, H.d_tile_cnt, H.d_weight, H.d_rows + H.loose_row0, H.d_start + H.loose_start0, lcnt, lsum,
             H.widest, H.scale, P.d_status, ctx->wait_budget);
       else
-        k_hist_pairs<kLooseGlobal><<<H.loose_grid, kHT, kHistSmem, s>>>(
+        k_hist_pairs<kLooseGlobal><<<H.loose_grid, kHT, hist_smem<kLooseGlobal>(), s>>>(
             H.d_pts, H.d_tile_cnt, H.d_weight, H.d_rows + H.loose_row0, H.d_start + H.loose_start0, lcnt, lsum, 0,
             H.scale, P.d_status, ctx->wait_budget);
       CRAB_CUDA_CHECK(cudaGetLastError());
