@@ -67,6 +67,7 @@ constexpr int kHistMaxBins = 22400;           // 2 words per bin beside the warp
 constexpr int kHistMinBins = 4096;
 constexpr double kHistStep = 0.005;           // q_max h aimed at
 constexpr double kHistMaxStep = 0.0075;       // beyond it (q_max x extent > 168) the recurrence kernels run
+constexpr double kHistMaxReach = 1e18;        // squares of distances below FP32's largest number
 constexpr int kHistFlush = 256;               // units between flushes: 2^21 pairs, |Σu| 2^11 < 2^31 in one bin
 constexpr int kHistStagingBytes = kHWarps * 2 * kChunkBytes;
 constexpr int kHistBarBytes = kHWarps * 2 * 8;
@@ -512,7 +513,12 @@ int hist_bins(double reach, double qmax) {
   return ((int)std::max(want, (double)kHistMinBins - 8.0) + 8 + kHistW - 1) / kHistW * kHistW;
 }
 
+// A pair's bin is an address as it stands, so nothing may come here whose FP32
+// distance is not a number: beyond kHistMaxReach the squares overflow, and
+// coordinates or weights that are not finite go to the recurrence kernels,
+// whose addresses do not depend on them.
 bool hist_structure_bins(double reach, double qmax, int* bins, float* inv_h) {
+  if (!(reach < kHistMaxReach)) return false;
   reach = std::max(reach, 1e-3) * 1.0001 + 1e-3;
   *bins = std::min(hist_bins(reach, qmax), kHistMaxBins);
   if (*bins == 0) return false;
@@ -577,6 +583,9 @@ bool hist_plan_init(crab_ctx* ctx, PairPlan& P) {
       int64_t votes = 0;
       for (int64_t i = 0; i < m; ++i) {
         const float w = a[4 * i + 3];
+        if (!std::isfinite(a[4 * i]) || !std::isfinite(a[4 * i + 1]) || !std::isfinite(a[4 * i + 2]) ||
+            !std::isfinite(w))
+          return false;
         if (w == 0.0f) continue;
         if (votes == 0) major = w;
         votes += w == major ? 1 : -1;
@@ -666,6 +675,7 @@ bool hist_build(crab_ctx* ctx, PairPlan& P, HistShape& X, const std::vector<unsi
         if (o.loose >= 0) loose_bins += bins[c];
         if (o.uniform >= 0 || o.loose >= 0) outs.push_back(o);
       }
+  if (any_loose && !std::isfinite(sumw * sumw)) return false;  // no fixed-point scale
   // unit numbers are 32-bit, and rows with loose members are all resident
   if (outs.empty() || !fits || loose_bins > (int64_t)1 << 27) return false;
   // loose sums: the largest power of two that keeps Σ|w w| below 2^61 steps

@@ -1,9 +1,12 @@
 """The distance histogram at the limits of its shared memory, its inputs and its tables."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
 import crabsaxs_b200 as cs
 import oracle as O
+from crabsaxs_b200 import _native as N
 
 pytestmark = pytest.mark.gpu
 
@@ -41,3 +44,58 @@ def test_loose_weights_over_the_range_of_bins(engine, bins, weights):
     s = np.array([w[t == a].sum() for a in range(3)])
     scale = np.array([s[a] * s[b] for a in range(3) for b in range(a, 3)])[:, None]
     assert (np.abs(got - ref) / scale).max() <= _tol(q, reach)
+
+
+def _plan(engine, xyz, w, t, n_types, q):
+    plan = C.c_void_p()
+    xyz, w, q = (np.ascontiguousarray(v, dtype=np.float64) for v in (xyz, w, q))
+    t = np.ascontiguousarray(t, dtype=np.int32)
+    engine.check(N.lib.crab_pair_plan_create(engine.handle, xyz.ctypes.data_as(N.D), w.ctypes.data_as(N.D),
+                                             t.ctypes.data_as(N.I32P), len(w), n_types, q.ctypes.data_as(N.D), len(q),
+                                             C.byref(plan)))
+    return plan
+
+
+@pytest.mark.parametrize("where", ["x", "z", "w"])
+@pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf, 1e39])
+def test_what_is_not_finite_takes_the_recurrence(engine, where, bad):
+    """A pair's bin is an address: a plan with values that have none (1e39: in FP32) is refused the histogram and made
+    of the recurrence, which takes them as it always did; q = 0 is the product of the weights."""
+    rng = np.random.default_rng(7)
+    xyz, w, t = rng.uniform(-9.0, 9.0, size=(200, 3)), np.ones(200), np.zeros(200, dtype=int)
+    if where == "w":
+        w[150] = bad
+    else:
+        xyz[150, "xyz".index(where)] = bad
+    q = np.array([0.0, 0.01, 0.2, 0.4])
+    plan = _plan(engine, xyz, w, t, 1, q)
+    try:
+        assert N.lib.crab_pair_plan_select(engine.handle, plan, 16) == N.EINVAL
+    finally:
+        N.lib.crab_pair_plan_destroy(plan)
+    got, _ = cs.debye_partials(xyz, w, t, 1, q, engine=engine)
+    assert got.shape == (1, 4)
+    if where != "w":
+        assert got[0, 0] == 200 * 199 / 2
+
+
+@pytest.mark.parametrize("scale", [1e15, 1e17, 1e19, 1e21, 1e30])
+def test_reach_whose_squares_leave_fp32(engine, scale):
+    """Distances of 1e15 and more, with q_max x reach small: the histogram while the squares are FP32 numbers, refused
+    beyond."""
+    rng = np.random.default_rng(11)
+    xyz = _mirrored(64, 2.0 * scale, rng)
+    w, t = np.ones(64), np.zeros(64, dtype=int)
+    q = np.linspace(0.5, 6.0, 12) / scale
+    plan = _plan(engine, xyz, w, t, 1, q)
+    try:
+        fits = N.lib.crab_pair_plan_select(engine.handle, plan, 16) == N.OK
+    finally:
+        N.lib.crab_pair_plan_destroy(plan)
+    assert fits == (scale < 1e18)
+    got, _ = cs.debye_partials(xyz, w, t, 1, q, engine=engine)
+    if fits:
+        ref, _ = O.debye_partials(xyz, w, t, 1, q)
+        assert np.abs(got - ref).max() / 64.0 ** 2 <= _tol(q * scale, 2.0)
+    one = cs.debye_intensity(cs.Structure(xyz, np.full(64, 1, dtype=np.int8)), q, engine=engine)
+    assert one.shape == q.shape
