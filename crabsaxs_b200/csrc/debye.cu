@@ -1377,6 +1377,7 @@ void configure_fp32(crab_ctx* ctx, PairPlan& P, int Q, int jb) {
   for (void* p : P.qcfg) cudaFree(p);
   P.qcfg.clear();
   P.d_work_out = nullptr;
+  P.d_work = nullptr;  // set again at the end: what fails on the way leaves no list to launch on
   const std::vector<int2> qrange = q_blocks(P.q, Q);
   P.Q = Q;
   P.n_qblocks = (int)qrange.size();
@@ -1436,9 +1437,9 @@ void configure_fp32(crab_ctx* ctx, PairPlan& P, int Q, int jb) {
   }
   P.d_scale = upload(ctx, P, P.qcfg, "scale", scale.data(), scale.size(), ctx->stream);
   P.n_work = (int)work.size();
-  P.d_work = upload(ctx, P, P.qcfg, "work", work.data(), work.size(), ctx->stream);
   P.d_qpar = upload(ctx, P, P.qcfg, "qpar", qpar.data(), qpar.size(), ctx->stream);
   P.d_qrange = upload(ctx, P, P.qcfg, "qrange", qrange.data(), qrange.size(), ctx->stream);
+  P.d_work = upload(ctx, P, P.qcfg, "work", work.data(), work.size(), ctx->stream);
 }
 
 // Kernel variant `v` (Q*16 + jb, or kHistVariant) for a plan; false where the
@@ -1557,6 +1558,7 @@ std::unique_ptr<PairPlan> make_batch_pair_plan(crab_ctx* ctx, std::vector<Layout
 
 void pair_plan_launch(crab_ctx* ctx, PairPlan& P, cudaStream_t s, bool timed) {
   if (P.nq == 0 || P.L.n_tiles == 0) return;
+  require(P.hist.active || P.d_work, "the plan's last change of kernel failed: select one");
   const size_t n_out = (size_t)P.n_pairs * P.nq * (P.segments.empty() ? 1 : P.segments.size() - 1);
   CRAB_CUDA_CHECK(cudaMemsetAsync(P.d_out, 0, n_out * sizeof(double), s));
   CRAB_CUDA_CHECK(cudaMemsetAsync(P.d_status, 0, 2 * sizeof(int), s));  // status and work counter

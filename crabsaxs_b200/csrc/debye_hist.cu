@@ -49,6 +49,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <utility>
 
 #include "device_math.cuh"
 #include "engine.hpp"
@@ -617,7 +618,17 @@ bool hist_plan_init(crab_ctx* ctx, PairPlan& P) {
 bool hist_build(crab_ctx* ctx, PairPlan& P, HistShape& X, const std::vector<unsigned char>* pts,
                 const std::vector<double>* weight) {
   typedef HistRange Range;
-  HistPart& H = P.hist;
+  // all of the plan's part or nothing: an allocation that fails leaves no half
+  // of it to be taken as built
+  HistPart H;
+  struct Undo {
+    PairPlan& P;
+    size_t kept;
+    bool on = true;
+    ~Undo() {
+      for (; on && P.owned.size() > kept; P.owned.pop_back()) cudaFree(P.owned.back());
+    }
+  } undo{P, P.owned.size()};
   const int T = P.L.T, S = X.S;
   const std::vector<Range>&uni = X.uni, &loose = X.loose;
   const std::vector<int>& bins = X.bins;
@@ -769,7 +780,6 @@ bool hist_build(crab_ctx* ctx, PairPlan& P, HistShape& X, const std::vector<unsi
   H.d_outs = (HistOut*)(d + o_outs);
   H.d_blocks = (HistBlock*)(d + o_blocks);
   H.d_start = (int2*)(d + o_start);
-  if (!P.d_q) P.d_q = (double*)(d + o_q);
   H.acc_bins = acc_bins;
   H.widest = widest;
   H.loose_bins = loose_bins;
@@ -780,6 +790,9 @@ bool hist_build(crab_ctx* ctx, PairPlan& P, HistShape& X, const std::vector<unsi
   CRAB_CUDA_CHECK(cudaFuncSetAttribute(k_hist_pairs<kLooseShared>, smem_max, hist_smem<kLooseShared>()));
   CRAB_CUDA_CHECK(cudaFuncSetAttribute(k_hist_pairs<kLooseGlobal>, smem_max, hist_smem<kLooseGlobal>()));
   H.active = true;
+  P.hist = std::move(H);
+  if (!P.d_q) P.d_q = (double*)(d + o_q);
+  undo.on = false;
   return true;
 }
 

@@ -99,3 +99,46 @@ def test_reach_whose_squares_leave_fp32(engine, scale):
         assert np.abs(got - ref).max() / 64.0 ** 2 <= _tol(q * scale, 2.0)
     one = cs.debye_intensity(cs.Structure(xyz, np.full(64, 1, dtype=np.int8)), q, engine=engine)
     assert one.shape == q.shape
+
+
+@pytest.mark.parametrize("weights", ["ones", "distinct"])
+def test_allocation_failure_inside_a_change_of_kernel(weights):
+    """Every allocation of a change to the histogram (and back) fails once; the plan is then as it was, refuses to run,
+    or has the new kernel, and the next change works."""
+    from crabsaxs_b200.api import Engine
+
+    rng = np.random.default_rng(3)
+    n, q = 400, np.linspace(0.01, 0.4, 30)
+    xyz, t = rng.uniform(-10.0, 10.0, size=(n, 3)), rng.integers(0, 2, size=n)
+    w = np.ones(n) if weights == "ones" else rng.uniform(0.2, 1.0, size=n)
+    ref, _ = O.debye_partials(xyz, w, t, 2, q)
+    s = np.array([w[t == a].sum() for a in range(2)])
+    scale = np.array([s[a] * s[b] for a in range(2) for b in range(a, 2)])[:, None]
+
+    def check(engine, plan):
+        out = np.empty((3, len(q)))
+        engine.check(N.lib.crab_pair_plan_run(engine.handle, plan, 1, 0, None))
+        engine.check(N.lib.crab_pair_plan_read(engine.handle, plan, out.ctypes.data_as(N.D), None))
+        assert (np.abs(out - ref) / scale).max() <= 96 * 2.0 ** -23  # at most 96 recurrence steps, two roundings each
+
+    engine = Engine(0)
+    engine.check(N.lib.crab_ctx_set_pair_variant(engine.handle, 64 * 16 + 2))
+    for variant in (16, 96 * 16 + 2):
+        for after in range(12):
+            plan = _plan(engine, xyz, w, t, 2, q)
+            if variant != 16:
+                engine.check(N.lib.crab_pair_plan_select(engine.handle, plan, 16))
+            engine.fail_allocations(after)
+            status = N.lib.crab_pair_plan_select(engine.handle, plan, variant)
+            engine.fail_allocations(None)
+            if status == N.OK:
+                break
+            if N.lib.crab_pair_plan_run(engine.handle, plan, 1, 0, None) == N.OK:
+                check(engine, plan)
+            engine.check(N.lib.crab_pair_plan_select(engine.handle, plan, variant))
+            check(engine, plan)
+            N.lib.crab_pair_plan_destroy(plan)
+        assert after > 0 and status == N.OK
+        check(engine, plan)
+        N.lib.crab_pair_plan_destroy(plan)
+    engine.close()
