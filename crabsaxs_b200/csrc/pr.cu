@@ -295,7 +295,9 @@ __device__ __forceinline__ int64_t pr_bin_of(double d2, double step, int64_t bin
 // side of the difference; the difference, the sum of squares, a 4-ulp
 // sqrt.approx and the rounded reciprocal step relative to d).  delta is four
 // times that with d <= bins + 1; when delta would exceed a quarter bin, or
-// above 2^20 bins, every pair takes the exact path.
+// above 2^20 bins, every pair takes the exact path.  So it does where 1/step is
+// not a normal FP32 number (steps above 8e37 or below 3e-39): x is then off by
+// any factor, and the bin of a counted pair is an address.
 __global__ void k_pr_edges(const unsigned long long* __restrict__ dmax2_bits, int64_t bins,
                            const double* __restrict__ rim_radius, const unsigned* __restrict__ invalid,
                            double* __restrict__ edges, PrParams* __restrict__ par) {
@@ -312,7 +314,7 @@ __global__ void k_pr_edges(const unsigned long long* __restrict__ dmax2_bits, in
     par->inv_step = (float)fmin(1.0 / step, (double)FLT_MAX);
     const double bound = (1.7320508075688772 * 0x1p-22 * radius / step + 11.5 * 0x1p-24 * (double)(bins + 1));
     par->delta = bins > (1 << 20) ? FLT_MAX : (float)fmin(4.0 * bound, 0.25);
-    if (4.0 * bound > 0.25) par->delta = FLT_MAX;
+    if (4.0 * bound > 0.25 || !(1.0 / step >= (double)FLT_MIN && 1.0 / step <= (double)FLT_MAX)) par->delta = FLT_MAX;
     par->degenerate = 0;
   }
   if (k > bins) return;

@@ -256,3 +256,17 @@ def test_dmax_is_the_longest_pair(engine, n, shape):
     s = cs.Structure(xyz, np.ones(n, np.int8))
     got = cs.coordinate_features(s, cs.PrOptions(bins=40), engine=engine).dmax
     assert got == np.sqrt(_longest(xyz))
+
+
+@pytest.mark.parametrize("scale", [1e-150, 1e-60, 1e-42, 1e-39, 1e-36, 1e30, 1e36, 3e37, 1e38, 3e39, 2e44, 7e45, 3e46, 1e60, 1e98])
+@pytest.mark.parametrize("n", [200, 4500])
+def test_steps_whose_inverse_is_not_an_fp32_number(engine, scale, n):
+    """The counting kernel's bins are addresses: where 1/step is subnormal, zero or past FP32's largest number, every
+    pair is placed by its f64 distance.  Whole numbers, equal to the oracle's."""
+    rng = np.random.default_rng(n)
+    xyz = rng.uniform(-0.5, 0.5, size=(n, 3)) * scale
+    for bins in (1, 16, 160):
+        d, h = cs.pair_distance_histogram(xyz, np.ones(n), bins, engine=engine)
+        assert _mode(engine) == 0
+        rd, rh = O.pair_distance_histogram(xyz, np.ones(n), bins)
+        assert d == rd and np.array_equal(h, rh), bins
