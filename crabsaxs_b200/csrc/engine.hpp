@@ -441,8 +441,8 @@ struct GridResult {
   double voxel_volume = 0.0;
   int64_t m = 0;                   // number of sites
   double outer = 0.0;               // no site is farther than this from some atom
-  const int32_t* d_cells = nullptr;
-  const double* d_sites = nullptr;  // the sites on the device, valid until the context's next grid build
+  const int32_t* d_cells = nullptr;  // the sites' voxels and the sites on the device, valid until the context's next
+  const double* d_sites = nullptr;   // grid build or trim_grid_pool
   uint64_t build = 0;               // crab_ctx::grid_builds of the build that made this result
 };
 // Key of a grid build: structure serial, grid kind (0 adaptive, 1 exterior)
@@ -476,9 +476,13 @@ GridResult adaptive_grid_device(crab_ctx* ctx, const double* xyz, int64_t n, dou
                                 double padding, bool to_host = true, const GridAtoms& have = {});
 GridResult exterior_grid_device(crab_ctx* ctx, const double* xyz, const int8_t* elem, int64_t n, double spacing,
                                 double probe, double thickness, bool to_host = true, const GridAtoms& have = {});
-// Releases "grid." device slots above the keep size (after a caller copied
-// out the sites of a build made without to_host).
+// Releases "grid." device slots above the keep size (after a caller has read
+// the sites and cells of a build made without to_host).
 void trim_grid_pool(crab_ctx* ctx);
+struct GridPoolRelease {  // the same at the end of a scope, also on an error
+  crab_ctx* ctx;
+  ~GridPoolRelease() { trim_grid_pool(ctx); }
+};
 
 }  // namespace crab
 

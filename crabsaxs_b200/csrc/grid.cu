@@ -586,8 +586,8 @@ __global__ void k_sweep_warp(uint8_t* __restrict__ s, Box b, int axis, const int
 // Grid buffers live in the context's pool ("grid." slots), so repeated calls
 // allocate nothing.  A slot above kGridKeepBytes (a box of more than 2^28
 // voxels) is released when the build ends, so a one-off large box does not
-// keep its memory; a build that leaves its sites on the device keeps the
-// sites slot, which trim_grid_pool releases once they are copied out.
+// keep its memory; a build that leaves its sites and their cells on the device
+// keeps those slots, which trim_grid_pool releases once they are read.
 constexpr size_t kGridKeepBytes = 256ull << 20;
 
 template <class T>
@@ -598,7 +598,7 @@ T* pool(crab_ctx* ctx, const char* name, size_t count) {
 void trim_slots(crab_ctx* ctx, bool keep_sites) {
   for (auto it = ctx->bufs.begin(); it != ctx->bufs.end();) {
     if (it->first.compare(0, 5, "grid.") == 0 && it->second.bytes > kGridKeepBytes &&
-        !(keep_sites && it->first == "grid.sites")) {
+        !(keep_sites && (it->first == "grid.sites" || it->first == "grid.cells"))) {
       cudaFree(it->second.ptr);
       it = ctx->bufs.erase(it);
     } else {

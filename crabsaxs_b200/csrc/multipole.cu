@@ -2408,6 +2408,7 @@ void multipole_solvent_basis_impl(crab_ctx* ctx, const crab_struct* st, const do
     return;
   }
   MpSolventSetup u;
+  GridPoolRelease grid_release{ctx};
   solvent_setup(ctx, st, q, nq, s, implicit, shard.n_shards == 1, u);
   MpInput in;
   u.into(in);
@@ -2434,6 +2435,7 @@ void multipole_solvent_intensity_impl(crab_ctx* ctx, const crab_struct* st, cons
     return;
   }
   MpSolventSetup u;
+  GridPoolRelease grid_release{ctx};
   solvent_setup(ctx, st, q, nq, s, implicit, true, u);
   MpInput in;
   u.into(in);

@@ -142,3 +142,32 @@ def test_allocation_failure_inside_a_change_of_kernel(weights):
         check(engine, plan)
         N.lib.crab_pair_plan_destroy(plan)
     engine.close()
+
+
+def test_sites_and_cells_past_the_kept_slots(engine):
+    """23 million sites (552 MB, their cells 276 MB): the grid's slots are above the size that a context keeps, and the
+    call still reads them.  A shard without the site-site sums, against the sites themselves: the share is their last
+    tiles, as many sites as the sum says near q = 0.  The call leaves no such slot behind."""
+    s = cs.Structure(np.array([[3.0, -2.0, 1.0]]), np.array([1], dtype=np.int8))
+    p = cs.SolventParams(shell_thickness_angstrom=176.0, hydration_model=cs.HydrationModel.Grid)
+    q = np.array([1e-9, 0.004, 0.05, 0.3])
+    got = cs.debye_solvent_basis(s, q, p, engine=engine, shard=(1, 2))
+    held = C.c_int64()
+    engine.check(N.lib.crab_ctx_workspace_bytes(engine.handle, C.byref(held)))
+    few, _ = cs.hydration_grid_exterior(s, 1.0, 1.4, 3.0, engine=engine)  # releases what a call may have left
+    left = C.c_int64()
+    engine.check(N.lib.crab_ctx_workspace_bytes(engine.handle, C.byref(left)))
+    assert held.value - left.value < 1 << 28
+    sites, _ = cs.hydration_grid_exterior(s, 1.0, 1.4, 176.0, engine=engine)
+    assert len(sites) > 22_400_000
+    # v h sinc: the whole sum at q ~ 0 from the FP64 path's definition of both amplitudes
+    site = cs.debye_solvent_basis(s, q, cs.SolventParams(hydration_model=cs.HydrationModel.Grid), engine=engine,
+                                  fp64=True)
+    v = np.sqrt(site[0])  # one atom: vv = v²
+    r = np.sqrt(((few - s.xyz) ** 2).sum(axis=1))
+    h = site[4] / (v * np.sinc(q[:, None] * r / np.pi).sum(axis=1))  # the site's amplitude
+    count = got[4, 0] / (v[0] * h[0])
+    assert abs(count - round(count)) <= 1e-3 and 0 < round(count) < len(sites)
+    r = np.sqrt(((sites[len(sites) - round(count):] - s.xyz) ** 2).sum(axis=1))
+    ref = np.array([np.sinc(k * r / np.pi).sum() for k in q])
+    assert np.abs(got[4] / (v * h) - ref).max() / count <= _tol(q, 2.0 * r.max())
