@@ -103,6 +103,10 @@ struct EnsOpts {
   double scale_value, bg_value;
   int uniform;
   double regularization;
+  bool operator==(const EnsOpts& o) const {
+    return scale_mode == o.scale_mode && bg_mode == o.bg_mode && scale_value == o.scale_value &&
+           bg_value == o.bg_value && uniform == o.uniform && regularization == o.regularization;
+  }
 };
 
 // Sums over p < n of two terms, the terms of index t, t + kEW, ... in thread
@@ -437,6 +441,11 @@ struct RwOpts {
   double kl, step, tol, floor;
   int max_iter, scale_mode, bg_mode;
   double scale_value, bg_value;
+  bool operator==(const RwOpts& o) const {
+    return kl == o.kl && step == o.step && tol == o.tol && floor == o.floor && max_iter == o.max_iter &&
+           scale_mode == o.scale_mode && bg_mode == o.bg_mode && scale_value == o.scale_value &&
+           bg_value == o.bg_value;
+  }
 };
 
 // ---- KL reweighting -------------------------------------------------------
@@ -880,7 +889,10 @@ struct EnsemblePlan {
   double *d_y = nullptr, *d_sg = nullptr, *d_weights = nullptr, *d_fit = nullptr, *d_fitted = nullptr,
          *d_gradw = nullptr, *d_wkl = nullptr, *d_out = nullptr;
   cudaGraphExec_t graph = nullptr;
-  int graph_k = -1;
+  // what the graph's nodes hold by value
+  int graph_k = -1, graph_budget = 0;
+  EnsOpts graph_fit{};
+  RwOpts graph_reweight{};
   int64_t graph_kernels = 0;
   ~EnsemblePlan() {
     if (graph) cudaGraphExecDestroy(graph);
@@ -1081,10 +1093,12 @@ static void ensemble_launch_fit(EnsemblePlan& E, int Ksel, const EnsOpts& eo, co
 
 // The full scoring pass of a plan as one CUDA graph: pair sums of every
 // conformer, curves at every candidate, weight fits, ∂χ²/∂(c1,c2), KL
-// reweighting.  Captured on first use and replayed.
+// reweighting.  Captured on first use and replayed while the options and the
+// wait budget, which its nodes hold, stay the same.
 static void ensemble_graph_launch(EnsemblePlan& E, const EnsOpts& eo, const RwOpts& ro) {
   crab_ctx* ctx = E.ctx;
-  if (!E.graph || E.graph_k != E.K) {
+  if (!E.graph || E.graph_k != E.K || E.graph_budget != ctx->wait_budget || !(E.graph_fit == eo) ||
+      !(E.graph_reweight == ro)) {
     if (E.graph) {
       cudaGraphExecDestroy(E.graph);
       E.graph = nullptr;
@@ -1104,6 +1118,9 @@ static void ensemble_graph_launch(EnsemblePlan& E, const EnsOpts& eo, const RwOp
     CRAB_CUDA_CHECK(cudaGraphInstantiate(&E.graph, g, 0));
     cudaGraphDestroy(g);
     E.graph_k = E.K;
+    E.graph_budget = ctx->wait_budget;
+    E.graph_fit = eo;
+    E.graph_reweight = ro;
     E.graph_kernels = ctx->launches - before;  // kernels recorded into the graph
     ctx->launches = before;
   }
