@@ -1128,6 +1128,15 @@ static void ensemble_graph_launch(EnsemblePlan& E, const EnsOpts& eo, const RwOp
   ctx->launches += E.graph_kernels;
 }
 
+// Throws when a wait of the plan's pair kernel ran out; waits for the pair sums.
+static void check_pair_status(EnsemblePlan& E) {
+  if (!E.pair) return;
+  int status = 0;
+  copy_d2h(E.ctx, &status, E.pair->d_status, sizeof(int), E.ctx->stream);
+  CRAB_CUDA_CHECK(cudaStreamSynchronize(E.ctx->stream));
+  if (status) throw Error(status, "pair kernel: a bounded wait on a j-tile copy ran out");
+}
+
 static EnsOpts ens_opts(const crab_fit_options* fo, bool uniform, double reg) {
   EnsOpts o;
   o.scale_mode = fo ? fo->scale_mode : CRAB_SCALE_FIT;
@@ -1160,6 +1169,7 @@ int crab_ensemble_curves(crab_ctx* ctx, crab_struct* const* structures, int32_t 
     auto E = make_ensemble_plan(ctx, structures, k, q, nq, *solvent, implicit_hydrogen != 0, cand, n_cand);
     pair_plan_launch(ctx, *E->pair, ctx->stream, false);
     ensemble_launch_curves(*E, k);
+    check_pair_status(*E);
     copy_d2h(ctx, curves, E->d_curves, (size_t)n_cand * k * nq * sizeof(double), ctx->stream);
     CRAB_CUDA_CHECK(cudaStreamSynchronize(ctx->stream));
   });
@@ -1219,6 +1229,7 @@ int crab_ensemble_plan_score(crab_ctx* ctx, crab_ensemble_plan* plan, const doub
     CRAB_CUDA_CHECK(cudaStreamSynchronize(ctx->stream));
     float ms = 0.0f;
     CRAB_CUDA_CHECK(cudaEventElapsedTime(&ms, ctx->ev_start, ctx->ev_stop));
+    check_pair_status(E);
     if (elapsed_ms) *elapsed_ms = ms;
     const int best = (int)out[0];
     if (best_fit) {
@@ -1394,6 +1405,7 @@ int crab_ensemble_fit(crab_ctx* ctx, crab_struct* const* structures, int32_t k, 
     const std::vector<double> cand = fit_candidates(fopt);
     auto E = make_ensemble_plan(ctx, structures, k, q, nq, fopt->solvent, fopt->implicit_hydrogen != 0, cand.data(), 25);
     pair_plan_launch(ctx, *E->pair, ctx->stream, false);
+    check_pair_status(*E);
     ensemble_fit_rounds(ctx, E, cand, y, sigma, nq, *eopt, fopt, result, selected_out, weights_out, fitted_out,
                         intervals_out, bootstrap_chi2_out);
   });

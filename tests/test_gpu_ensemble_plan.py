@@ -65,3 +65,33 @@ def test_every_call_has_its_own_options(engine, other):
         plan.close()
     for g, want in zip(got, [base, changed, changed, base]):
         assert _equal(g, want)
+
+
+@pytest.mark.parametrize("variant", [0, 16])
+def test_wait_that_runs_out_is_reported_by_every_ensemble_call(engine, variant):
+    """The pair kernel's bounded wait shortened to nothing, for the plan's own kernel and the distance histogram: the
+    calls report it instead of returning what incomplete sums give, and the context goes on."""
+    from crabsaxs_b200 import _native as N
+    from crabsaxs_b200.api import Engine, Other
+
+    rng = np.random.default_rng(5)
+    structures, q, cand = _ensemble(5, 50, rng)
+    y, sigma = _observed(structures, q, cand, rng, engine)
+    exp = cs.ExperimentalCurve(q, y, sigma)
+    fresh = Engine(0)
+    fresh.check(N.lib.crab_ctx_set_pair_variant(fresh.handle, variant))
+    plan = cs.EnsemblePlan(structures, q, candidates=cand, engine=fresh)
+    fitter = cs.EnsembleFitter(structures, [str(k) for k in range(5)], exp, engine=fresh)
+    calls = [lambda: plan.score(y, sigma), fitter.fit,
+             lambda: cs.ensemble_curves(structures, q, cs.SolventParams(), cand, engine=fresh)]
+    before = [calls[0](), calls[1]().weights, calls[2]()]
+    fresh.set_wait_budget(0)
+    for call in calls:
+        for _ in range(2):
+            with pytest.raises(Other, match="ETIMEOUT"):
+                call()
+    fresh.set_wait_budget(None)
+    assert _equal(calls[0](), before[0])
+    assert np.array_equal(calls[1]().weights, before[1]) and np.array_equal(calls[2](), before[2])
+    plan.close()
+    fresh.close()
