@@ -34,6 +34,7 @@ namespace {
 constexpr double kPi = 3.14159265358979323846264338327950288;
 constexpr uint32_t kDropped = 0xFFFFFFFFu, kLooseBit = 1u << 23, kRankMask = kLooseBit - 1;
 constexpr int kCodes = 256;  // element * 16 + group + 1
+constexpr int kFrontClasses = 200;  // scattering classes at most, sites among them
 
 // Word of an atom: class << 24 | loose << 23 | rank among its class's counted
 // or loose atoms.  tile0[2 c], tile0[2 c + 1]: first counted and loose tile.
@@ -211,7 +212,7 @@ bool debye_terms_device(crab_ctx* ctx, const crab_struct* st, const double* q, i
     }
   }
   const int TA = (int)cls.size(), T = TA + (grid ? 1 : 0);
-  if (TA == 0 || T > 200) return false;
+  if (TA == 0 || T > kFrontClasses) return false;
   auto* hx = (double*)ctx->host("front.xyz", (size_t)n * 3 * sizeof(double));
   std::memcpy(hx, x, (size_t)n * 3 * sizeof(double));
   auto* d_xyz = (double*)ctx->dev("front.xyz", (size_t)n * 3 * sizeof(double));
@@ -368,8 +369,10 @@ bool debye_terms_device(crab_ctx* ctx, const crab_struct* st, const double* q, i
   A.shard = shard;
   A.density = solvent ? solvent->bulk_density : 0.0;
   A.site_volume = g.voxel_volume;
+  // the attribute belongs to the function, whatever context sets it: always the same value
+  constexpr size_t kTermsSmem = 3 * (size_t)kFrontClasses * kTQ * sizeof(double);
+  CRAB_CUDA_CHECK(cudaFuncSetAttribute(k_debye_terms, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTermsSmem));
   const size_t smem = 3 * (size_t)T * kTQ * sizeof(double);
-  CRAB_CUDA_CHECK(cudaFuncSetAttribute(k_debye_terms, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   k_debye_terms<<<(unsigned)((nq + kTQ - 1) / kTQ), dim3(kTQ, kTR), smem, s>>>(A, (double*)d_res);
   CRAB_CUDA_CHECK(cudaGetLastError());
   ctx->launches += 2;
