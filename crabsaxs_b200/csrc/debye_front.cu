@@ -342,7 +342,7 @@ bool debye_terms_device(crab_ctx* ctx, const crab_struct* st, const double* q, i
   if (grid && shard == 0) {
     int64_t span[3];
     for (int d = 0; d < 3; ++d) span[d] = (int64_t)std::ceil((hi[d] - lo[d] + 2.0 * g.outer) / g.spacing) + 1;
-    lattice_plan_init_device(ctx, P, g.m, g.spacing, span);
+    lattice_plan_init_device(ctx, P, g.d_cells, g.m, g.spacing, span);
   }
   const int* d_tile0 = (const int*)(H.d_more + o_tile);
   k_front_points<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(d_xyz, d_word, d_occ, d_tile0, n, c[0], c[1], c[2], H.d_pts,

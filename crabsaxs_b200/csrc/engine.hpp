@@ -391,8 +391,9 @@ bool hist_build(crab_ctx* ctx, PairPlan& P, HistShape& X, const std::vector<unsi
                 const std::vector<double>* weight);
 void hist_plan_launch(crab_ctx* ctx, PairPlan& P, cudaStream_t s);
 void lattice_plan_init(crab_ctx* ctx, PairPlan& P, const int32_t* cells, int64_t m, double spacing);
-// The same with the cells (3 int32 each) on the device, every coordinate's span below `span` cells.
-void lattice_plan_init_device(crab_ctx* ctx, PairPlan& P, int64_t m, double spacing, const int64_t* span);
+// The same with the cells (3 int32 each) on the device, every coordinate's span at most `span` cells.
+void lattice_plan_init_device(crab_ctx* ctx, PairPlan& P, const int32_t* d_cells, int64_t m, double spacing,
+                              const int64_t* span);
 void lattice_plan_launch(crab_ctx* ctx, PairPlan& P, cudaStream_t s);
 bool q_grid_uniform(const double* q, int64_t nq);
 std::unique_ptr<PairPlan> make_pair_plan(crab_ctx* ctx, Layout&& L, const double* q, int64_t nq, bool fp64,

@@ -14,6 +14,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 
 #include "engine.hpp"
@@ -83,6 +84,27 @@ __global__ void __launch_bounds__(kLThreads)
   if (shared_hist) flush();
 }
 
+// out[d], out[3 + d]: least and largest cell along d (set to INT_MAX and INT_MIN before).
+__global__ void __launch_bounds__(256)
+    k_lattice_span(const int32_t* __restrict__ cells, int64_t m, int* __restrict__ out) {
+  int lo[3] = {INT_MAX, INT_MAX, INT_MAX}, hi[3] = {INT_MIN, INT_MIN, INT_MIN};
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m; i += (int64_t)gridDim.x * blockDim.x)
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const int c = cells[3 * i + d];
+      lo[d] = min(lo[d], c);
+      hi[d] = max(hi[d], c);
+    }
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    const int l = __reduce_min_sync(0xffffffffu, lo[d]), h = __reduce_max_sync(0xffffffffu, hi[d]);
+    if ((threadIdx.x & 31) == 0) {
+      atomicMin(out + d, l);
+      atomicMax(out + 3 + d, h);
+    }
+  }
+}
+
 // out[k] = Σ_n count[n] sinc(q_k spacing √n) with the reference sinc
 // (|x| < 1e-8 -> 1), one CTA per q.
 __global__ void k_lattice_transform(const unsigned long long* __restrict__ hist, int bins, double spacing,
@@ -141,15 +163,36 @@ void lattice_plan_init(crab_ctx* ctx, PairPlan& P, const int32_t* cells, int64_t
   Lp.active = true;
 }
 
-void lattice_plan_init_device(crab_ctx* ctx, PairPlan& P, int64_t m, double spacing, const int64_t* span) {
+void lattice_plan_init_device(crab_ctx* ctx, PairPlan& P, const int32_t* d_cells, int64_t m, double spacing,
+                              const int64_t* span) {
   LatticePart& Lp = P.lattice;
   Lp.m = m;
   Lp.spacing = spacing;
-  int64_t nmax = 0;
-  for (int d = 0; d < 3; ++d) nmax += span[d] * span[d];
-  require(nmax < (int64_t)1 << 30, "hydration lattice too large for the site histogram");
-  require((m + kLT - 1) / kLT <= 65535, "too many lattice sites for one histogram launch");
-  Lp.bins = (int)nmax + 1;
+  Lp.bins = 1;
+  if (m >= 2) {
+    int64_t nmax = 0;
+    for (int d = 0; d < 3; ++d) nmax += span[d] * span[d];
+    if (nmax >= kSharedBins) {
+      // The bound is a cell or two an axis above the cells' own span, which
+      // decides between counters in shared and in device memory (294 atoms with
+      // 53,353 sites on a 1 Å grid just under the line: 39.4 ms a call by the
+      // bound, 1.8 so) and whether the lattice is refused.
+      int ext[6] = {INT_MAX, INT_MAX, INT_MAX, INT_MIN, INT_MIN, INT_MIN};
+      auto* d_ext = (int*)ctx->dev("lattice.span", sizeof(ext));
+      copy_h2d(ctx, d_ext, ext, sizeof(ext), ctx->stream);
+      k_lattice_span<<<(unsigned)std::min<int64_t>((m + 255) / 256, ctx->sm_count), 256, 0, ctx->stream>>>(d_cells, m,
+                                                                                                         d_ext);
+      CRAB_CUDA_CHECK(cudaGetLastError());
+      ctx->launches += 1;
+      copy_d2h(ctx, ext, d_ext, sizeof(ext), ctx->stream);
+      CRAB_CUDA_CHECK(cudaStreamSynchronize(ctx->stream));
+      nmax = 0;
+      for (int d = 0; d < 3; ++d) nmax += (int64_t)(ext[3 + d] - ext[d]) * (ext[3 + d] - ext[d]);
+    }
+    require(nmax < (int64_t)1 << 30, "hydration lattice too large for the site histogram");
+    require((m + kLT - 1) / kLT <= 65535, "too many lattice sites for one histogram launch");
+    Lp.bins = (int)nmax + 1;
+  }
   Lp.d_cells = (int4*)plan_alloc(ctx, P, P.owned, "lattice_cells", (size_t)std::max<int64_t>(m, 1) * sizeof(int4));
   Lp.d_hist = (unsigned long long*)plan_alloc(ctx, P, P.owned, "lattice_hist",
                                                (size_t)Lp.bins * sizeof(unsigned long long));

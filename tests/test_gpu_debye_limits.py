@@ -171,3 +171,58 @@ def test_sites_and_cells_past_the_kept_slots(engine):
     r = np.sqrt(((sites[len(sites) - round(count):] - s.xyz) ** 2).sum(axis=1))
     ref = np.array([np.sinc(k * r / np.pi).sum() for k in q])
     assert np.abs(got[4] / (v * h) - ref).max() / count <= _tol(q, 2.0 * r.max())
+
+
+def _site_row(engine, s, q, p, grid):
+    got = cs.debye_solvent_basis(s, q, p, engine=engine)
+    ref = O.debye_solvent_basis(O.Atoms(s.xyz, s.element, s.group, s.occupancy), q, 1.0, 0.0,
+                                spacing=p.hydration_grid_spacing_angstrom, model=grid)
+    return np.abs(got[2] - ref[2]).max() / np.abs(ref[2]).max()
+
+
+def test_lattice_refused_by_a_bound_only():
+    """Two atoms 131,053 Å apart with a 4 Å shell: the cells' own squared span is 131,050 below 2^30, the span of the
+    atoms' box with its shell above."""
+    from crabsaxs_b200.api import Engine
+
+    s = cs.Structure(np.array([[0.0, 0.0, 0.0], [131053.0, 0.3, -0.2]]), np.array([1, 3], dtype=np.int8))
+    engine = Engine(0)
+    p = cs.SolventParams(hydration_model=cs.HydrationModel.AdaptiveGrid)
+    assert _site_row(engine, s, np.array([4e-4, 1.1e-3]), p, 2) <= 1e-9
+    engine.close()
+
+
+def _pair_counts(cells):
+    """Ordered pairs per squared distance, as whole numbers (autocorrelation of the cells)."""
+    cells = cells - cells.min(axis=0)
+    span = cells.max(axis=0) + 1
+    box = np.zeros(2 * span)
+    box[tuple(cells.T)] = 1.0
+    f = np.fft.rfftn(box)
+    count = np.rint(np.fft.irfftn(f * f.conj(), s=box.shape, axes=(0, 1, 2))).astype(np.int64)
+    axes = [np.minimum(np.arange(2 * n), 2 * n - np.arange(2 * n)) ** 2 for n in span]
+    n2 = axes[0][:, None, None] + axes[1][None, :, None] + axes[2][None, None, :]
+    return np.bincount(n2.ravel(), weights=count.ravel())
+
+
+@pytest.mark.parametrize("side", [30.0, 43.5, 44.5, 45.5, 46.1, 54.0])
+def test_lattices_about_the_shared_counters(engine, side):
+    """A 1 Å shell around the corners of a cube: spans on both sides of 11,264 squared cells, by the bound and by the
+    cells themselves.  Against whole numbers of pairs per distance (the oracle's running sum of 1e8 terms is itself off
+    by 1e-9)."""
+    p = cs.SolventParams(hydration_model=cs.HydrationModel.AdaptiveGrid, hydration_grid_spacing_angstrom=1.0)
+    q = np.linspace(0.0, 0.5, 9)
+
+    def row(xyz):
+        s = cs.Structure(xyz, np.full(len(xyz), 1, dtype=np.int8))
+        sites, _ = cs.hydration_grid_adaptive(s, 1.0, engine=engine)
+        cells = np.rint(sites - sites[0]).astype(np.int64)
+        count = _pair_counts(cells)
+        r = np.sqrt(np.arange(len(count)))
+        total = np.array([(count * np.sinc(k * r / np.pi)).sum() for k in q])
+        return cs.debye_solvent_basis(s, q, p, engine=engine)[2] / total, (np.ptp(cells, axis=0) ** 2).sum()
+
+    site2, _ = row(np.array([[0.37, 0.37, 0.37]]))  # a site's squared amplitude
+    got, span2 = row(np.stack(np.meshgrid(*[[0.0, side]] * 3, indexing="ij"), -1).reshape(-1, 3) + 0.37)
+    assert (span2 >= 11264) == (side >= 46.0)
+    assert np.abs(got / site2 - 1.0).max() <= 1e-9
