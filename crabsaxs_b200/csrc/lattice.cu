@@ -38,9 +38,7 @@ __global__ void __launch_bounds__(kLThreads)
                    unsigned long long* __restrict__ hist) {
   __shared__ int4 sj[kLT];
   __shared__ unsigned int sh[kSharedBins];
-  const bool shared_hist = bins <= kSharedBins;
-  if (shared_hist)
-    for (int b = threadIdx.x; b < bins; b += kLThreads) sh[b] = 0u;
+  for (int b = threadIdx.x; b < bins; b += kLThreads) sh[b] = 0u;
   auto flush = [&]() {
     __syncthreads();
     for (int b = threadIdx.x; b < bins; b += kLThreads)
@@ -58,7 +56,7 @@ __global__ void __launch_bounds__(kLThreads)
     while (tj * (tj + 1) / 2 > w) --tj;
     while ((tj + 1) * (tj + 2) / 2 <= w) ++tj;
     const int64_t ti = w - tj * (tj + 1) / 2;
-    if (shared_hist && ++since == kLFlush) {
+    if (++since == kLFlush) {
       flush();
       since = 0;
     }
@@ -76,12 +74,33 @@ __global__ void __launch_bounds__(kLThreads)
       const int4 cj = sj[j];
       if (cj.w < 0 || (ti == tj && j <= li)) continue;  // past the last site, or the pair's other order
       const int dx = ci.x - cj.x, dy = ci.y - cj.y, dz = ci.z - cj.z;
-      const int n = dx * dx + dy * dy + dz * dz;
-      if (shared_hist) atomicAdd(&sh[n], 1u);
-      else atomicAdd(&hist[n], 1ull);
+      atomicAdd(&sh[dx * dx + dy * dy + dz * dz], 1u);
     }
   }
-  if (shared_hist) flush();
+  flush();
+}
+
+// The same for spans past the shared counters: every pair into device memory,
+// a CTA per tile pair (tj, ti) and a thread per i site.  Bound by the L2's
+// atomics, which runs of tile pairs on 256 threads as above drive into each
+// other (47,663 sites with spans past the line, a call: 24.8 ms, 16.7 so).
+__global__ void __launch_bounds__(kLT)
+    k_lattice_hist_wide(const int4* __restrict__ cells, int64_t m, unsigned long long* __restrict__ hist) {
+  __shared__ int4 sj[kLT];
+  const int64_t ti = blockIdx.y, tj = blockIdx.x;
+  if (tj < ti) return;  // upper triangle of tile pairs only
+  const int64_t j = tj * kLT + threadIdx.x, i = ti * kLT + threadIdx.x;
+  sj[threadIdx.x] = j < m ? cells[j] : make_int4(0, 0, 0, -1);
+  __syncthreads();
+  if (i >= m) return;
+  const int4 ci = cells[i];
+  for (int k = 0; k < kLT; ++k) {
+    const int4 cj = sj[k];
+    if (cj.w < 0) break;  // past the last site
+    if (ti == tj && k <= (int)threadIdx.x) continue;
+    const int dx = ci.x - cj.x, dy = ci.y - cj.y, dz = ci.z - cj.z;
+    atomicAdd(&hist[dx * dx + dy * dy + dz * dz], 1ull);
+  }
 }
 
 // out[d], out[3 + d]: least and largest cell along d (set to INT_MAX and INT_MIN before).
@@ -206,8 +225,12 @@ void lattice_plan_launch(crab_ctx* ctx, PairPlan& P, cudaStream_t s) {
   CRAB_CUDA_CHECK(cudaMemsetAsync(Lp.d_hist, 0, (size_t)Lp.bins * sizeof(unsigned long long), s));
   if (Lp.m >= 2) {
     const int64_t nt = (Lp.m + kLT - 1) / kLT;
-    const unsigned grid = (unsigned)std::min<int64_t>(nt * (nt + 1) / 2, 4 * ctx->sm_count);  // four CTAs an SM
-    k_lattice_hist<<<grid, kLThreads, 0, s>>>(Lp.d_cells, Lp.m, nt, Lp.bins, Lp.d_hist);
+    if (Lp.bins <= kSharedBins) {
+      const unsigned grid = (unsigned)std::min<int64_t>(nt * (nt + 1) / 2, 4 * ctx->sm_count);  // four CTAs an SM
+      k_lattice_hist<<<grid, kLThreads, 0, s>>>(Lp.d_cells, Lp.m, nt, Lp.bins, Lp.d_hist);
+    } else {
+      k_lattice_hist_wide<<<dim3((unsigned)nt, (unsigned)nt), kLT, 0, s>>>(Lp.d_cells, Lp.m, Lp.d_hist);
+    }
     CRAB_CUDA_CHECK(cudaGetLastError());
     ctx->launches += 1;
   }
