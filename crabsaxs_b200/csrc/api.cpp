@@ -258,9 +258,9 @@ GridResult hydration_sites(crab_ctx* ctx, const crab_struct* st, const crab_solv
 }
 
 void debye_basis(crab_ctx* ctx, const crab_struct* st, const double* q, int64_t nq, const crab_solvent& s,
-                 bool implicit, double* out6, bool fp64, int shard, int n_shards) {
+                 bool implicit, double* out6, bool fp64, int shard, int n_shards, bool front) {
   TraceScope trace("debye_basis");
-  if (!fp64 && debye_terms_device(ctx, st, q, nq, &s, implicit, out6, shard, n_shards)) return;
+  if (front && !fp64 && debye_terms_device(ctx, st, q, nq, &s, implicit, out6, shard, n_shards)) return;
   GridResult g;
   const bool grid = s.hydration_model != CRAB_HYD_ANALYTIC;
   if (grid) {

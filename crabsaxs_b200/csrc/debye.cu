@@ -1268,6 +1268,24 @@ std::vector<int2> q_blocks(const std::vector<double>& q, int Qmax) {
   return out;
 }
 
+// Their number alone.
+int64_t q_block_count(const std::vector<double>& q, int Qmax) {
+  const int64_t nq = (int64_t)q.size();
+  if (nq == 0) return 0;
+  const double tol = 1e-9 * std::max(std::fabs(q[nq - 1]), 1e-12);
+  int64_t count = 0;
+  for (int64_t s0 = 0; s0 < nq; ++count) {
+    int64_t e = s0 + 1;
+    if (e < nq) {
+      const double dq = q[s0 + 1] - q[s0];
+      e = s0 + 2;
+      while (e < nq && e - s0 < Qmax && std::fabs(q[e] - (q[s0] + (double)(e - s0) * dq)) <= tol) ++e;
+    }
+    s0 = e;
+  }
+  return count;
+}
+
 std::vector<int32_t> shard_owners(const int64_t* cost, int64_t n, int n_shards) {
   require(n_shards >= 1, "shard count must be positive");
   std::vector<int64_t> load((size_t)n_shards, 0);
@@ -1340,7 +1358,7 @@ int2 default_variant(const std::vector<double>& q) {
   int bestQ = 64;
   long best_cost = -1;
   for (int Qc : kQBlocks) {
-    const long cost = (long)q_blocks(q, Qc).size() * (3 * Qc + 60);
+    const long cost = (long)q_block_count(q, Qc) * (3 * Qc + 60);
     if (best_cost < 0 || cost < best_cost) {
       best_cost = cost;
       bestQ = Qc;
@@ -1364,7 +1382,7 @@ void configure_fp32(crab_ctx* ctx, PairPlan& P, int Q, int jb) {
   P.hist.active = false;
   if (!P.d_atoms)
     P.d_atoms = upload(ctx, P, P.owned, "atoms", (const float4*)P.L.atoms.data(), (size_t)P.L.n_pad, ctx->stream);
-  if (!P.d_fill) {  // slots of each tile up to its last atom with a weight
+  if (!P.d_fill && jb != 2 && jb != 4) {  // q-packed kernels: slots of each tile up to its last atom with a weight
     std::vector<int> fill(P.L.n_tiles);
     for (int t = 0; t < P.L.n_tiles; ++t) {
       int n = kTile;
@@ -1442,28 +1460,58 @@ void configure_fp32(crab_ctx* ctx, PairPlan& P, int Q, int jb) {
   P.d_work = upload(ctx, P, P.qcfg, "work", work.data(), work.size(), ctx->stream);
 }
 
+// What the recurrence kernels take for these classes beside the launch, in us,
+// at the untuned choice of block: the packed kernels by warp steps (32 i atoms
+// against one j atom), with each tile pair's flush, the others by whole tile
+// pairs.  Fitted to the plans of hist_us: half of them within 13 %.
+double recurrence_us(const HistShape& X, int T, bool skip_last, const std::vector<double>& q) {
+  const int2 v = default_variant(q);
+  const double Q = v.x, blocks = (double)q_block_count(q, v.x);
+  double us = 0.0;
+  for (int c = 0; c < X.S; ++c) {
+    double atoms = 0.0, warps = 0.0, tiles = 0.0, types = 0.0, steps = 0.0, pairs = 0.0;
+    for (int a = 0; a < T; ++a) {
+      const double n = (double)(X.uni[(size_t)c * T + a].atoms + X.loose[(size_t)c * T + a].atoms);
+      const double w = std::ceil(n / 32.0), t = std::ceil(n / kTile);
+      atoms += n;
+      warps += w;
+      tiles += t;
+      types += n > 0.0;
+      if (skip_last && a == T - 1) {
+        steps -= 0.5 * w * n;
+        pairs -= 0.5 * t * (t + 1.0);
+      }
+    }
+    steps += 0.5 * (warps + 1.0) * atoms;
+    pairs += 0.5 * tiles * (tiles + 1.0);
+    if (v.y != 2)
+      us += 0.21 * Q * std::min(1.0, atoms / (kTile * std::max(types, 1.0))) +
+            blocks * (3.7e-6 * steps * (Q + 20.0) + 4.5e-5 * pairs * Q);
+    else
+      us += blocks * pairs * (0.037 + 0.0025 * Q);
+  }
+  return us;
+}
+
 // Kernel variant `v` (Q*16 + jb, or kHistVariant) for a plan; false where the
-// histogram does not fit.
-bool pair_plan_use(crab_ctx* ctx, PairPlan& P, int v) {
+// histogram does not fit, or with if_faster does not pay.
+bool pair_plan_use(crab_ctx* ctx, PairPlan& P, int v, bool if_faster = false) {
   if (v != kHistVariant) {
     configure_fp32(ctx, P, v / 16, v % 16);
     return true;
   }
   if (P.hist.d_pts) P.hist.active = true;
-  return P.hist.active || hist_plan_init(ctx, P);
+  return P.hist.active || hist_plan_init(ctx, P, if_faster);
 }
 
 // The FP32 form of a new plan: the context's variant if one is set, else the
-// distance histogram, else the recurrence, which has no bins to hold: where
-// q_max times the largest distance is over 168 the histogram of one class pair
-// would not fit an SM's shared memory (debye_hist.cu).  There is no size below
-// which the recurrence is the better one; kernels of one call, histogram
-// against the best recurrence variant: 20 atoms, 20 q 30 / 31 us; 300 atoms of
-// 14 classes, 101 q 33 / 60 us; 1,000 atoms, 100 q 37 / 72 us; 20,000 atoms of
-// four, 100 q 0.23 / 2.7 ms, 500 q 0.23 / 11.3 ms.
+// distance histogram where it pays (hist_plan_init), else the recurrence, which
+// has no bins to hold: where q_max times the largest distance is over 168 the
+// histogram of one class pair would not fit an SM's shared memory (debye_hist.cu).
 void configure_auto(crab_ctx* ctx, PairPlan& P) {
   const int2 v = default_variant(P.q);
-  if (!pair_plan_use(ctx, P, ctx->pair_variant ? ctx->pair_variant : kHistVariant)) configure_fp32(ctx, P, v.x, v.y);
+  const int set = ctx->pair_variant;
+  if (!pair_plan_use(ctx, P, set ? set : kHistVariant, !set)) configure_fp32(ctx, P, v.x, v.y);
 }
 
 std::unique_ptr<PairPlan> make_pair_plan(crab_ctx* ctx, Layout&& L, const double* q, int64_t nq, bool fp64,
@@ -1815,7 +1863,7 @@ void pair_plan_select(crab_ctx* ctx, PairPlan& P, int variant) {
   require(!P.fp64, "the FP64 plan has a single kernel");
   require(pair_variant_known(variant), "unknown kernel variant " + std::to_string(variant));
   if (P.nq == 0 || P.L.n_tiles == 0) return;
-  require(pair_plan_use(ctx, P, variant), "the distance histogram of this plan exceeds the shared memory");
+  require(pair_plan_use(ctx, P, variant), "the distance histogram of this plan does not fit");
   CRAB_CUDA_CHECK(cudaStreamSynchronize(ctx->stream));
 }
 

@@ -159,11 +159,31 @@ __global__ void __launch_bounds__(kTQ * kTR) k_debye_terms(TermsArg A, double* _
   }
 }
 
+// Whether a call of these classes is faster here than on the general path, whose
+// tables, layout and quadratic forms one host core makes and whose sites come
+// back to the host.  For few q, or few atoms of many classes with weights of
+// their own, it is not (vacuum calls: 36 classes, 2,790 atoms, 2 q 379 us here, 178
+// there; four classes, 737 atoms, 10 q 119 / 99 us; 1,000 atoms of 14 classes, 100 q
+// 112 / 291).  Fitted with hist_us to 664 calls of 1 to 42 classes, 2 to 4,000 atoms
+// and 2 to 300 q.
+bool front_pays(const HistShape& X, int T, bool grid, const crab_solvent* solvent, const std::vector<double>& q,
+                int64_t n) {
+  if (solvent && solvent->hydration_model == CRAB_HYD_GRID) return true;  // 1.05 to 7 times faster at any size
+  const double nq = (double)q.size();
+  double rows;
+  const double us = hist_us(X, T, false, (int64_t)q.size(), &rows);
+  const double types = T - (grid ? 1 : 0);
+  const double host = nq * (0.027 * types + 0.0016 * types * (types + 1.0) * (solvent ? 3.2 : 1.0)) +
+                      (grid ? 40.0 + 0.02 * (double)n : 0.0);
+  const double least = 5.7e-8 * (double)n * (double)n * nq;  // of the recurrence, without a look at the q grid
+  return us < host + 0.8 * least + 1.0 || us < host + 0.8 * recurrence_us(X, T, false, q) + 1.0;
+}
+
 }  // namespace
 
 // The six solvent terms (out [6][nq]), or with solvent null the vacuum curve's
-// unclamped sum (out [nq]); false where the histogram does not apply (nothing
-// done, the caller takes the general path).
+// unclamped sum (out [nq]); false where the histogram does not apply or does not
+// pay (nothing done, the caller takes the general path).
 bool debye_terms_device(crab_ctx* ctx, const crab_struct* st, const double* q, int64_t nq, const crab_solvent* solvent,
                         bool implicit, double* out, int shard, int n_shards, FrontKeep* keep) {
   const int64_t n = st->n;
@@ -171,26 +191,6 @@ bool debye_terms_device(crab_ctx* ctx, const crab_struct* st, const double* q, i
   const bool grid = solvent && solvent->hydration_model != CRAB_HYD_ANALYTIC;
   double qmax = 0.0;
   for (int64_t k = 0; k < nq; ++k) qmax = std::max(qmax, q[k]);
-  // box, centre and the largest distance from it
-  const double* x = st->xyz.data();
-  double lo[3] = {x[0], x[1], x[2]}, hi[3] = {x[0], x[1], x[2]}, c[3], r2 = 0.0;
-  for (int64_t i = 0; i < n; ++i)
-    for (int d = 0; d < 3; ++d) {
-      lo[d] = min_num(lo[d], x[3 * i + d]);
-      hi[d] = max_num(hi[d], x[3 * i + d]);
-    }
-  for (int d = 0; d < 3; ++d) c[d] = 0.5 * (lo[d] + hi[d]);
-  for (int64_t i = 0; i < n; ++i) {
-    const double dx = x[3 * i] - c[0], dy = x[3 * i + 1] - c[1], dz = x[3 * i + 2] - c[2];
-    r2 = max_num(r2, dx * dx + dy * dy + dz * dz);
-  }
-  const double rmax = std::sqrt(r2);
-  HistShape X;
-  X.bins.resize(1);
-  X.inv_h.resize(1);
-  // the sites lie within a shell of 16 Å at most around the atoms; refused here
-  // rather than after the grid is built
-  if (!hist_structure_bins(2.0 * (rmax + (grid ? 16.0 : 0.0)), qmax, &X.bins[0], &X.inv_h[0])) return false;
   // classes present, in (element, group) order
   const int8_t *el = st->elem.data(), *gr = st->group.data();
   int64_t part[4][kCodes] = {};
@@ -213,6 +213,49 @@ bool debye_terms_device(crab_ctx* ctx, const crab_struct* st, const double* q, i
   }
   const int TA = (int)cls.size(), T = TA + (grid ? 1 : 0);
   if (TA == 0 || T > kFrontClasses) return false;
+  const double* x = st->xyz.data();
+  const double* occ = st->occ.data();
+  HistShape X;
+  X.bins.assign(1, kHistMinBins);
+  X.inv_h.resize(1);
+  X.uni.resize(T);
+  X.loose.resize(T);
+  const std::vector<double> qs(q, q + nq);
+  // the share of loose atoms in a sample decides, before anything is as long as
+  // the atom list but the classes; with the fewest bins first
+  std::vector<double> w0(TA, 0.0);
+  const int64_t stride = std::max<int64_t>(1, n / 256);
+  int64_t seen = 0, odd = 0;
+  for (int64_t i = 0; i < n; i += stride) {
+    const int k = cls_of[el[i] * 16 + ((gr[i] + 1) & gmask)];
+    if (k < 0 || occ[i] == 0.0) continue;
+    if (w0[k] == 0.0) w0[k] = occ[i];
+    odd += occ[i] != w0[k];
+    ++seen;
+  }
+  const double share = seen ? (double)odd / (double)seen : 0.0;
+  for (int k = 0; k < TA; ++k) {
+    X.loose[k].atoms = (int64_t)(share * (double)count[k] + 0.5);
+    X.uni[k].atoms = count[k] - X.loose[k].atoms;
+  }
+  if (!front_pays(X, T, grid, solvent, qs, n)) return false;
+  // box, centre and the largest distance from it
+  double lo[3] = {x[0], x[1], x[2]}, hi[3] = {x[0], x[1], x[2]}, c[3], r2 = 0.0;
+  for (int64_t i = 0; i < n; ++i)
+    for (int d = 0; d < 3; ++d) {
+      lo[d] = min_num(lo[d], x[3 * i + d]);
+      hi[d] = max_num(hi[d], x[3 * i + d]);
+    }
+  for (int d = 0; d < 3; ++d) c[d] = 0.5 * (lo[d] + hi[d]);
+  for (int64_t i = 0; i < n; ++i) {
+    const double dx = x[3 * i] - c[0], dy = x[3 * i + 1] - c[1], dz = x[3 * i + 2] - c[2];
+    r2 = max_num(r2, dx * dx + dy * dy + dz * dz);
+  }
+  const double rmax = std::sqrt(r2);
+  // the sites lie within a shell of 16 Å at most around the atoms; refused here
+  // rather than after the grid is built
+  if (!hist_structure_bins(2.0 * (rmax + (grid ? 16.0 : 0.0)), qmax, &X.bins[0], &X.inv_h[0])) return false;
+  if (!front_pays(X, T, grid, solvent, qs, n)) return false;
   auto* hx = (double*)ctx->host("front.xyz", (size_t)n * 3 * sizeof(double));
   std::memcpy(hx, x, (size_t)n * 3 * sizeof(double));
   auto* d_xyz = (double*)ctx->dev("front.xyz", (size_t)n * 3 * sizeof(double));
@@ -229,8 +272,7 @@ bool debye_terms_device(crab_ctx* ctx, const crab_struct* st, const double* q, i
   // words: a class's candidate for its counted weight is the weight of its
   // first atom; should that turn out rarer than half, the majority vote's
   auto* word = (uint32_t*)ctx->host("front.word", (size_t)n * sizeof(uint32_t));
-  const double* occ = st->occ.data();
-  std::vector<double> w0(TA, 0.0);
+  std::fill(w0.begin(), w0.end(), 0.0);
   std::vector<int64_t> nu(TA), nl(TA);
   std::vector<double> sw(T, 0.0), sw2(T, 0.0);
   double s_abs = 0.0;
@@ -270,8 +312,6 @@ bool debye_terms_device(crab_ctx* ctx, const crab_struct* st, const double* q, i
     }
   }
   // tiles: a class's loose atoms, then its counted ones
-  X.uni.resize(T);
-  X.loose.resize(T);
   std::vector<int> tile0(2 * (size_t)T, 0);
   auto tiles = [&](HistRange& R, int64_t m, double w) {
     R.t0 = (int)X.tile_cnt.size();
@@ -315,7 +355,7 @@ bool debye_terms_device(crab_ctx* ctx, const crab_struct* st, const double* q, i
   P.shard = shard;
   P.n_shards = n_shards;
   P.nq = nq;
-  P.q.assign(q, q + nq);
+  P.q = qs;
   P.L.T = T;
   P.L.n = points;
   P.L.n_tiles = (int)X.tile_cnt.size();

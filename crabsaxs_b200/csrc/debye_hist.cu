@@ -65,10 +65,10 @@ constexpr int kHWarps = kHT / 32;
 constexpr int kChunkAtoms = kHistChunkAtoms;  // j atoms of a unit
 constexpr int kChunkBytes = kHistChunkBytes;  // 32 x {x0,x1,y0,y1}, then 32 x {z0,z1}
 constexpr int kHistMaxBins = 22400;           // 2 words per bin beside the warps' double buffers in 227 KB
-constexpr int kHistMinBins = 4096;
 constexpr double kHistStep = 0.005;           // q_max h aimed at
 constexpr double kHistMaxStep = 0.0075;       // beyond it (q_max x extent > 168) the recurrence kernels run
 constexpr double kHistMaxReach = 1e18;        // squares of distances below FP32's largest number
+constexpr int64_t kHistMaxBytes = (int64_t)8 << 30;  // sums of a plan in device memory
 constexpr int kHistFlush = 256;               // units between flushes: 2^21 pairs, |Σu| 2^11 < 2^31 in one bin
 constexpr int kHistStagingBytes = kHWarps * 2 * kChunkBytes;
 constexpr int kHistBarBytes = kHWarps * 2 * 8;
@@ -527,7 +527,44 @@ bool hist_structure_bins(double reach, double qmax, int* bins, float* inv_h) {
   return true;
 }
 
-bool hist_plan_init(crab_ctx* ctx, PairPlan& P) {
+// What the histogram of these classes takes beside its launches, in us: a row's
+// bins are cleared and transformed, those that its pairs hit flushed, and rows
+// with loose members do so a second time; loose pairs, whose sums are 64 bits
+// wide, cost themselves.  Fitted to 1,670 plans of 1 to 400 types and 2 to 20,000
+// atoms at 4 to 500 q: half of them within 17 %.
+double hist_us(const HistShape& X, int T, bool skip_last, int64_t nq, double* n_rows) {
+  const double blocks = std::ceil((double)nq / kHistQ);
+  double us = 0.0;
+  *n_rows = 0.0;
+  for (int c = 0; c < X.S; ++c) {
+    double types = 0.0, loose_types = 0.0, counted = 0.0, loose = 0.0;
+    for (int a = 0; a < T; ++a) {
+      const double u = (double)X.uni[(size_t)c * T + a].atoms, l = (double)X.loose[(size_t)c * T + a].atoms;
+      types += u + l > 0.0;
+      loose_types += l > 0.0;
+      counted += u;
+      loose += l;
+    }
+    const double bins = X.bins[c], rows = 0.5 * types * (types + 1.0) - (skip_last ? 1.0 : 0.0);
+    // each loose class against the loose and the counted atoms of the others
+    const double loose_rows = loose_types * (types + 1.0) * (counted > loose ? 1.0 : 0.5);
+    const double loose_pairs = loose * (counted + 0.5 * loose);
+    const double hit = std::min(bins, 0.5 * (counted + loose) * (counted + loose) / std::max(rows, 1.0));
+    us += std::min(0.03 * loose_pairs, 25.0) + 6e-6 * loose_pairs +
+          rows * (bins * (6e-6 + 1.35e-5 * blocks) + 6e-6 * hit) + loose_rows * (2e-6 * bins + 1.2e-5 * hit);
+    *n_rows += rows + loose_rows;
+  }
+  return us;
+}
+
+// if_faster: only where the recurrence kernels would take longer.  They are the
+// better ones for many types of few atoms and for few q, where the bins of every
+// class pair cost more than its pairs (kernel time, histogram against
+// recurrence: 14 types, 1,400 atoms with weights of their own, 8 q 107 / 31 us;
+// 213 types, 20,000 atoms, 12 q 5.8 / 1.7 ms; 250 types, 2,500 atoms, 100 q 4.7 /
+// 0.37 ms).  The choice depends on the problem alone, not on the shard or the
+// device, so that all parts of one sum take the same kernels.
+bool hist_plan_init(crab_ctx* ctx, PairPlan& P, bool if_faster) {
   double qmax = 0.0;
   for (double v : P.q) qmax = std::max(qmax, v);
   const Layout& L = P.L;
@@ -546,12 +583,81 @@ bool hist_plan_init(crab_ctx* ctx, PairPlan& P) {
   X.uni.resize((size_t)S * T);
   X.loose.resize((size_t)S * T);
   std::vector<HistRange>&uni = X.uni, &loose = X.loose;
+  std::vector<int>& tcnt = X.tile_cnt;
+  double& sumw = X.sum_abs_w;
+  if (if_faster) {
+    // atoms by tile, and the share of loose ones in a sample (three atoms of a
+    // tile against its first): what the choice needs without a pass over all
+    for (int c = 0; c < S; ++c) {
+      const int every = std::max(1, (seg[c + 1] - seg[c]) / 256);
+      int64_t seen = 0, odd = 0;
+      for (int t = seg[c]; t < seg[c + 1]; ++t) {
+        const float* w = L.atoms.data() + 4 * (size_t)t * kTile + 3;
+        int n = kTile;
+        while (n > 0 && w[4 * (n - 1)] == 0.0f) --n;
+        uni[(size_t)c * T + L.tile_type[t]].atoms += n;
+        if (n < 2 || t % every) continue;
+        for (const int k : {n / 3, 2 * n / 3, n - 1})
+          if (k > 0) {
+            odd += w[4 * k] != w[0];
+            ++seen;
+          }
+      }
+      for (int a = 0; a < T && odd; ++a) {
+        HistRange &U = uni[(size_t)c * T + a], &Lo = loose[(size_t)c * T + a];
+        Lo.atoms = (int64_t)((double)U.atoms * (double)odd / (double)seen + 0.5);
+        U.atoms -= Lo.atoms;
+      }
+    }
+    double rows;
+    const double us = hist_us(X, T, P.skip_last, P.nq, &rows);
+    // 15 us: its launches above the recurrence's one, of which a plan of one call
+    // gets ten back from the shorter tables; 0.05 us a row and 0.01 us an atom:
+    // its tables and points on the host
+    const double extra = (P.pooled ? 5.0 : 15.0) + 0.05 * rows + 0.01 * (double)L.n;
+    if (!(us + extra < 0.8 * recurrence_us(X, T, P.skip_last, P.q))) return false;
+    for (HistRange& r : uni) r.atoms = 0;
+    for (HistRange& r : loose) r.atoms = 0;
+  }
+  // a type's atoms: the commonest weight if it has a majority, else whichever the vote leaves
+  struct Run {
+    size_t range;
+    const float* a;
+    int64_t m;
+  };
+  std::vector<Run> runs;
+  for (int c = 0; c < S; ++c) {
+    double s1 = 0.0;
+    for (int t0 = seg[c]; t0 < seg[c + 1];) {
+      const int ty = L.tile_type[t0];
+      int t1 = t0 + 1;
+      while (t1 < seg[c + 1] && L.tile_type[t1] == ty) ++t1;
+      const Run r{(size_t)c * T + ty, L.atoms.data() + (size_t)t0 * kTile * 4, (int64_t)(t1 - t0) * kTile};
+      const float* a = r.a;
+      float major = 0.0f;
+      int64_t votes = 0;
+      for (int64_t i = 0; i < r.m; ++i) {
+        const float w = a[4 * i + 3];
+        if (!std::isfinite(a[4 * i]) || !std::isfinite(a[4 * i + 1]) || !std::isfinite(a[4 * i + 2]) ||
+            !std::isfinite(w))
+          return false;
+        if (w == 0.0f) continue;  // padding, or an atom without weight
+        if (votes == 0) major = w;
+        votes += w == major ? 1 : -1;
+        s1 += std::fabs((double)w);
+      }
+      uni[r.range].w = (double)major;
+      for (int64_t i = 0; i < r.m; ++i)
+        if (a[4 * i + 3] != 0.0f) ++(a[4 * i + 3] == major ? uni : loose)[r.range].atoms;
+      X.any_loose = X.any_loose || loose[r.range].atoms > 0;
+      runs.push_back(r);
+      t0 = t1;
+    }
+    sumw = std::max(sumw, s1);
+  }
   std::vector<unsigned char> pts;
   pts.reserve((size_t)(L.n_tiles + 2 * S) * 2 * kChunkBytes);
   std::vector<double> weight;
-  std::vector<int>& tcnt = X.tile_cnt;
-  double& sumw = X.sum_abs_w;
-  std::vector<int64_t> other;
   auto append = [&](HistRange& R, const float* a, double w, int64_t& fill) {
     if (fill % kTile == 0) {
       pts.resize(pts.size() + 2 * kChunkBytes, 0);
@@ -571,46 +677,16 @@ bool hist_plan_init(crab_ctx* ctx, PairPlan& P) {
     ++fill;
     ++R.atoms;
   };
-  for (int c = 0; c < S; ++c) {
-    double s1 = 0.0;
-    for (int t0 = seg[c]; t0 < seg[c + 1];) {
-      const int ty = L.tile_type[t0];
-      int t1 = t0 + 1;
-      while (t1 < seg[c + 1] && L.tile_type[t1] == ty) ++t1;
-      const float* a = L.atoms.data() + (size_t)t0 * kTile * 4;
-      const int64_t m = (int64_t)(t1 - t0) * kTile;
-      // the commonest weight if it has a majority, else whichever the vote leaves
-      float major = 0.0f;
-      int64_t votes = 0;
-      for (int64_t i = 0; i < m; ++i) {
-        const float w = a[4 * i + 3];
-        if (!std::isfinite(a[4 * i]) || !std::isfinite(a[4 * i + 1]) || !std::isfinite(a[4 * i + 2]) ||
-            !std::isfinite(w))
-          return false;
-        if (w == 0.0f) continue;
-        if (votes == 0) major = w;
-        votes += w == major ? 1 : -1;
-      }
-      HistRange& U = uni[(size_t)c * T + ty];
-      HistRange& Lo = loose[(size_t)c * T + ty];
-      U.w = (double)major;
+  for (const Run& r : runs) {
+    // the class's loose tiles, then right after them its counted ones
+    for (HistRange* R : {&loose[r.range], &uni[r.range]}) {
       int64_t fill = 0;
-      other.clear();
-      for (int64_t i = 0; i < m; ++i) {
-        const float w = a[4 * i + 3];
-        if (w == 0.0f) continue;  // padding, or an atom without weight
-        s1 += std::fabs((double)w);
-        if (w != major) other.push_back(i);
+      R->atoms = 0;
+      for (int64_t i = 0; i < r.m; ++i) {
+        const float w = r.a[4 * i + 3];
+        if (w != 0.0f && ((double)w == uni[r.range].w) == (R == &uni[r.range])) append(*R, r.a + 4 * i, w, fill);
       }
-      // the class's loose tiles, then right after them its counted ones
-      for (int64_t i : other) append(Lo, a + 4 * i, (double)a[4 * i + 3], fill);
-      fill = 0;
-      for (int64_t i = 0; i < m; ++i)
-        if (a[4 * i + 3] != 0.0f && a[4 * i + 3] == major) append(U, a + 4 * i, (double)major, fill);
-      X.any_loose = X.any_loose || !other.empty();
-      t0 = t1;
     }
-    sumw = std::max(sumw, s1);
   }
   return hist_build(ctx, P, X, &pts, &weight);
 }
@@ -687,7 +763,7 @@ bool hist_build(crab_ctx* ctx, PairPlan& P, HistShape& X, const std::vector<unsi
         if (o.uniform >= 0 || o.loose >= 0) outs.push_back(o);
       }
   if (any_loose && !std::isfinite(sumw * sumw)) return false;  // no fixed-point scale
-  // unit numbers are 32-bit, and rows with loose members are all resident
+  // unit numbers are 32-bit, and with loose members all rows are resident
   if (outs.empty() || !fits || loose_bins > (int64_t)1 << 27) return false;
   // loose sums: the largest power of two that keeps Σ|w w| below 2^61 steps
   int ex = 0;
@@ -763,6 +839,7 @@ bool hist_build(crab_ctx* ctx, PairPlan& P, HistShape& X, const std::vector<unsi
         hist_starts(drows, dpairs, H.loose_row0, drows.size(), H.loose_grid, P.shard, P.n_shards, kRowCost);
     starts.insert(starts.end(), st.begin(), st.end());
   }
+  if ((acc_bins + loose_bins) * 16 > kHistMaxBytes) return false;
   HistBlob blob;
   blob.bytes.reserve((pts ? pts->size() + weight->size() * 8 : 0) + drows.size() * 64 + outs.size() * 64 + 65536);
   const size_t o_cnt = blob.add(tcnt), o_rows = blob.add(drows), o_outs = blob.add(outs), o_blocks = blob.add(blocks),

@@ -379,10 +379,15 @@ struct LatticeSpec {
   int64_t m = 0;
   double spacing = 0.0;
 };
+constexpr int kHistMinBins = 4096;
 constexpr int kHistVariant = 16;  // the distance histogram's variant code
 // Builds the histogram form of a plan and makes it active; false when its
-// bins do not fit an SM's shared memory or there is no pair to sum.
-bool hist_plan_init(crab_ctx* ctx, PairPlan& P);
+// bins do not fit an SM's shared memory or its sums kHistMaxBytes, when there is
+// no pair to sum, and with if_faster where the recurrence kernels take less.
+bool hist_plan_init(crab_ctx* ctx, PairPlan& P, bool if_faster);
+// Estimates in us from the atoms per (structure, type), and the histogram's rows.
+double hist_us(const HistShape& X, int T, bool skip_last, int64_t nq, double* n_rows);
+double recurrence_us(const HistShape& X, int T, bool skip_last, const std::vector<double>& q);
 // Bins and 1/h of a structure of that largest distance (false: no fit).
 bool hist_structure_bins(double reach, double qmax, int* bins, float* inv_h);
 // Tables, work lists and buffers from the tiles; with pts null the points (and

@@ -228,7 +228,7 @@ void chi2_grad_impl(crab_ctx* ctx, const crab_struct* st, const double* q, const
   if (!placed) {
     t = type_atoms(st, implicit, TermSet::SolventAnalytic, nullptr);
     amplitude_tables(t, q, nq, &s, implicit, 0.0, V, E, H);
-    debye_basis(ctx, st, q, nq, s, implicit, b6.data(), false);
+    debye_basis(ctx, st, q, nq, s, implicit, b6.data(), false, 0, 1, false);
   }
   const int T = t.T;
   combine_basis(q, nq, b6.data(), s.c1, s.c2, I.data());

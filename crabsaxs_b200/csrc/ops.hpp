@@ -46,7 +46,7 @@ GridResult hydration_sites(crab_ctx* ctx, const crab_struct* st, const crab_solv
 // With n_shards > 1 only shard `shard`'s part of the six rows (self terms on
 // shard 0 only): the element-wise sum over all shards is the whole basis.
 void debye_basis(crab_ctx* ctx, const crab_struct* st, const double* q, int64_t nq, const crab_solvent& s,
-                 bool implicit, double* out6, bool fp64, int shard = 0, int n_shards = 1);
+                 bool implicit, double* out6, bool fp64, int shard = 0, int n_shards = 1, bool front = true);
 // What a caller of debye_terms_device goes on with: the atoms as they lie on the
 // device (valid until the context's next call) and where each one's slot is.
 struct FrontKeep {

@@ -10,6 +10,19 @@ from crabsaxs_b200 import _native as N
 
 pytestmark = pytest.mark.gpu
 
+HIST = 16  # the histogram's variant code
+
+
+@pytest.fixture(scope="module")
+def hist_engine():
+    """A context whose pair sums take the histogram wherever it fits, also where the recurrence is faster."""
+    from crabsaxs_b200.api import Engine
+
+    e = Engine(0)
+    e.check(N.lib.crab_ctx_set_pair_variant(e.handle, HIST))
+    yield e
+    e.close()
+
 
 def _mirrored(n, reach, rng):
     """n points in a ball of that diameter, symmetric about the origin (so the centroid is there), two of them one
@@ -30,7 +43,7 @@ def _tol(q, reach):
 # staging (up to 11,424), its last 448 past what the counting kernel takes, then those whose sums are in device memory.
 @pytest.mark.parametrize("bins", [5200, 10960, 10980, 11100, 11250, 11405, 11430, 12000, 16000, 22300])
 @pytest.mark.parametrize("weights", ["few", "distinct"])
-def test_loose_weights_over_the_range_of_bins(engine, bins, weights):
+def test_loose_weights_over_the_range_of_bins(hist_engine, bins, weights):
     rng = np.random.default_rng(bins)
     reach = (0.005 * bins / 0.5 - 1e-3) / 1.0001
     xyz = _mirrored(520, reach, rng)
@@ -39,7 +52,7 @@ def test_loose_weights_over_the_range_of_bins(engine, bins, weights):
         w = np.where(rng.random(520) < 0.1, 0.4, 0.75)
     t = rng.integers(0, 3, size=520)
     q = np.sort(np.concatenate([[0.0], rng.uniform(0.0, 0.5, size=60), [0.5]]))
-    got, _ = cs.debye_partials(xyz, w, t, 3, q, engine=engine)
+    got, _ = cs.debye_partials(xyz, w, t, 3, q, engine=hist_engine)
     ref, _ = O.debye_partials(xyz, w, t, 3, q)
     s = np.array([w[t == a].sum() for a in range(3)])
     scale = np.array([s[a] * s[b] for a in range(3) for b in range(a, 3)])[:, None]
@@ -70,7 +83,7 @@ def test_what_is_not_finite_takes_the_recurrence(engine, where, bad):
     q = np.array([0.0, 0.01, 0.2, 0.4])
     plan = _plan(engine, xyz, w, t, 1, q)
     try:
-        assert N.lib.crab_pair_plan_select(engine.handle, plan, 16) == N.EINVAL
+        assert N.lib.crab_pair_plan_select(engine.handle, plan, HIST) == N.EINVAL
     finally:
         N.lib.crab_pair_plan_destroy(plan)
     got, _ = cs.debye_partials(xyz, w, t, 1, q, engine=engine)
@@ -80,7 +93,7 @@ def test_what_is_not_finite_takes_the_recurrence(engine, where, bad):
 
 
 @pytest.mark.parametrize("scale", [1e15, 1e17, 1e19, 1e21, 1e30])
-def test_reach_whose_squares_leave_fp32(engine, scale):
+def test_reach_whose_squares_leave_fp32(engine, hist_engine, scale):
     """Distances of 1e15 and more, with q_max x reach small: the histogram while the squares are FP32 numbers, refused
     beyond."""
     rng = np.random.default_rng(11)
@@ -89,11 +102,11 @@ def test_reach_whose_squares_leave_fp32(engine, scale):
     q = np.linspace(0.5, 6.0, 12) / scale
     plan = _plan(engine, xyz, w, t, 1, q)
     try:
-        fits = N.lib.crab_pair_plan_select(engine.handle, plan, 16) == N.OK
+        fits = N.lib.crab_pair_plan_select(engine.handle, plan, HIST) == N.OK
     finally:
         N.lib.crab_pair_plan_destroy(plan)
     assert fits == (scale < 1e18)
-    got, _ = cs.debye_partials(xyz, w, t, 1, q, engine=engine)
+    got, _ = cs.debye_partials(xyz, w, t, 1, q, engine=hist_engine)
     if fits:
         ref, _ = O.debye_partials(xyz, w, t, 1, q)
         assert np.abs(got - ref).max() / 64.0 ** 2 <= _tol(q * scale, 2.0)
@@ -226,3 +239,103 @@ def test_lattices_about_the_shared_counters(engine, side):
     got, span2 = row(np.stack(np.meshgrid(*[[0.0, side]] * 3, indexing="ij"), -1).reshape(-1, 3) + 0.37)
     assert (span2 >= 11264) == (side >= 46.0)
     assert np.abs(got / site2 - 1.0).max() <= 1e-9
+
+
+@pytest.mark.parametrize("weights", ["ones", "few", "distinct"])
+@pytest.mark.parametrize("n,T", [(2, 1), (31, 1), (33, 2), (64, 1), (65, 1), (127, 1), (129, 1), (257, 3), (700, 14),
+                                 (300, 90)])
+def test_tile_edges_on_the_histogram(hist_engine, n, T, weights):
+    """The sizes of the histogram's tile edges, on the histogram whatever the choice for them is."""
+    rng = np.random.default_rng(n + T)
+    xyz = rng.uniform(-12.0, 12.0, size=(n, 3)) + 31.0
+    w = rng.uniform(0.2, 1.0, size=n)
+    if weights != "distinct":
+        w = np.where((rng.random(n) < 0.1) & (weights == "few"), 0.4, 0.75)
+        w[rng.random(n) < (0.05 if weights == "few" else 0.0)] = 0.0
+    t = rng.integers(0, T, size=n)
+    q = np.sort(np.concatenate([[0.0], rng.uniform(0.0, 0.6, size=40)]))
+    got, _ = cs.debye_partials(xyz, w, t, T, q, engine=hist_engine)
+    ref, _ = O.debye_partials(xyz, w, t, T, q)
+    s = np.array([w[t == a].sum() for a in range(T)])
+    scale = np.array([max(s[a] * s[b], 1e-12) for a in range(T) for b in range(a, T)])[:, None]
+    assert (np.abs(got - ref) / scale).max() <= _tol(q, 42.0)
+    parts = [cs.debye_partials(xyz, w, t, T, q, engine=hist_engine, shard=(k, 3))[0] for k in range(3)]
+    assert np.abs(sum(parts) - got).max() <= 1e-12 * max(np.abs(got).max(), 1e-300)
+
+
+def _launches(engine, call):
+    before = engine.stats()[0]
+    out = call()
+    return out, engine.stats()[0] - before
+
+
+@pytest.mark.parametrize("n,T,nq,weights,hist", [
+    (4000, 4, 100, "ones", True), (20000, 14, 8, "ones", True), (3000, 14, 300, "distinct", True),
+    (1386, 14, 8, "distinct", False), (330, 66, 17, "distinct", False), (2500, 250, 100, "ones", False),
+    (960, 60, 6, "distinct", False), (9000, 250, 5, "few", False), (310, 2, 9, "distinct", False)])
+def test_the_faster_kernels_are_taken(engine, n, T, nq, weights, hist):
+    """Where bins cost more than pairs the recurrence runs, in one launch; shards take the same kernels as the whole."""
+    rng = np.random.default_rng(n)
+    R = 0.8 * n ** (1.0 / 3.0) + 4.0
+    xyz, t = rng.uniform(-R, R, size=(n, 3)), np.arange(n) % T
+    w = np.ones(n) if weights == "ones" else rng.uniform(0.2, 1.0, size=n)
+    if weights == "few":
+        w = np.where(rng.random(n) < 0.1, 0.4, 1.0)
+    q = np.linspace(0.5 / nq, 0.5, nq)
+    (got, _), launches = _launches(engine, lambda: cs.debye_partials(xyz, w, t, T, q, engine=engine))
+    assert (launches > 1) == hist
+    parts = [cs.debye_partials(xyz, w, t, T, q, engine=engine, shard=(k, 2))[0] for k in range(2)]
+    assert np.abs(sum(parts) - got).max() <= 1e-12 * np.abs(got).max()
+
+
+@pytest.mark.parametrize("n,nq,solvent,hist", [(2790, 2, False, False), (700, 5, False, False), (300, 200, False, True),
+                                               (1500, 100, True, True), (1881, 3, True, False)])
+def test_structure_calls_take_the_faster_path(engine, n, nq, solvent, hist):
+    """Few q of many classes: the general path with the recurrence.  Both against the FP64 path, relative to the terms
+    at q = 0 of positive amplitudes."""
+    rng = np.random.default_rng(n)
+    codes = [(e, -1) for e in range(1, 15)] + [(1, g) for g in range(14)]
+    pick = rng.integers(0, len(codes), size=n)
+    el, group = (np.array([codes[k][i] for k in pick], dtype=np.int8) for i in (0, 1))
+    R = 0.9 * n ** (1.0 / 3.0) + 3.0
+    xyz = rng.uniform(-R, R, size=(n, 3))
+    s = cs.Structure(xyz, el, np.where(rng.random(n) < 0.1, 0.4, 1.0), group)
+    q = np.linspace(0.5 / nq, 0.5, nq)
+    if solvent:
+        p = cs.SolventParams(c1=1.0, c2=0.7, hydration_model=cs.HydrationModel.AdaptiveGrid)
+        got, launches = _launches(engine, lambda: cs.debye_solvent_basis(s, q, p, engine=engine))
+        ref = cs.debye_solvent_basis(s, q, p, engine=engine, fp64=True)[0]
+        top = cs.debye_solvent_basis(s, [0.0], p, engine=engine, fp64=True)[0, 0]
+        got = got[0]
+        assert (launches > 9) == hist
+    else:
+        got, launches = _launches(engine, lambda: cs.debye_intensity(s, q, engine=engine))
+        p = cs.SolventParams()
+        ref = cs.debye_solvent_basis(s, q, p, engine=engine, fp64=True)[0]
+        top = cs.debye_solvent_basis(s, [0.0], p, engine=engine, fp64=True)[0, 0]
+        assert (launches > 1) == hist
+    assert np.abs(got - ref).max() / top <= 1e-5
+
+
+def test_sums_that_would_not_fit_the_device(engine):
+    """600 types at 22,400 bins with one odd weight: 65 GB of sums, refused before anything is allocated."""
+    rng = np.random.default_rng(2)
+    n, T = 1800, 600
+    reach = 0.005 * 22300 / 0.5
+    xyz = _mirrored(n, reach, rng)
+    w, t = np.ones(n), np.arange(n) % T
+    w[7] = 0.5
+    q = np.array([0.01, 0.2, 0.5])
+    plan = _plan(engine, xyz, w, t, T, q)
+    held, after = C.c_int64(), C.c_int64()
+    try:
+        engine.check(N.lib.crab_ctx_workspace_bytes(engine.handle, C.byref(held)))
+        assert N.lib.crab_pair_plan_select(engine.handle, plan, HIST) == N.EINVAL
+        engine.check(N.lib.crab_ctx_workspace_bytes(engine.handle, C.byref(after)))
+        engine.check(N.lib.crab_pair_plan_run(engine.handle, plan, 1, 0, None))
+    finally:
+        N.lib.crab_pair_plan_destroy(plan)
+    assert after.value == held.value
+    got, _ = cs.debye_partials(xyz, w, t, T, q, engine=engine)
+    ref, _ = cs.debye_partials(xyz, w, t, T, q, engine=engine, fp64=True)
+    assert np.abs(got - ref).max() <= 9.0 * 1e-4 and np.isfinite(got).all()  # nine pairs a row, FP32 phases q r
