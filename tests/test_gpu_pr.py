@@ -270,3 +270,19 @@ def test_steps_whose_inverse_is_not_an_fp32_number(engine, scale, n):
         assert _mode(engine) == 0
         rd, rh = O.pair_distance_histogram(xyz, np.ones(n), bins)
         assert d == rd and np.array_equal(h, rh), bins
+
+
+@pytest.mark.parametrize("n,k,bins", [(3, 3, 5449), (40, 1, 6112), (150, 58, 6386), (344, 3, 7296), (500, 2, 1500),
+                                      (500, 2, 8000), (427, 41, 200), (700, 3, 100000 // 13)])
+def test_few_pairs_and_many_bins(engine, n, k, bins):
+    """Both widths of the shared counters, with class pairs of fewer pairs than bins among them: whole numbers, equal
+    to the oracle's for products that f64 sums exactly."""
+    rng = np.random.default_rng(n + bins)
+    xyz = rng.uniform(-9.0, 9.0, size=(n, 3))
+    w = 1.0 + rng.integers(0, k, size=n)
+    w[: k] = 1.0 + np.arange(k)  # classes of very different sizes
+    w[rng.random(n) < 0.5] = 1.0
+    d, h = cs.pair_distance_histogram(xyz, w, bins, engine=engine)
+    assert _mode(engine) == 0
+    rd, rh = O.pair_distance_histogram(xyz, w, bins)
+    assert d == rd and np.array_equal(h, rh)
