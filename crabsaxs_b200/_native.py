@@ -185,6 +185,7 @@ _SIGS = {
     "crab_pair_plan_pairq": (C.c_double, [P]),
     "crab_pair_plan_destroy": (C.c_int, [P]),
     "crab_measure_fp32_peak": (C.c_int, [P, C.c_double, D]),
+    "crab_probe_quotients": (C.c_int, [P, D, D, I64, D, D]),
     "crab_ctx_transfer_stats": (C.c_int, [P, C.POINTER(I64), C.POINTER(I64)]),
 }
 

@@ -700,6 +700,11 @@ int crab_measure_fp32_peak(crab_ctx* ctx, double ms, double* tflops) {
   GUARD(ctx, { *tflops = measure_fp32_peak(ctx, ms); });
 }
 
+int crab_probe_quotients(crab_ctx* ctx, const double* a, const double* b, int64_t n, double* by, double* div) {
+  if (!ctx || n < 0 || (n > 0 && (!a || !b || !by || !div))) return CRAB_EINVAL;
+  GUARD(ctx, { probe_quotients(ctx, a, b, n, by, div); });
+}
+
 int crab_ctx_transfer_stats(crab_ctx* ctx, int64_t* h2d, int64_t* d2h) {
   if (!ctx) return CRAB_EINVAL;
   std::lock_guard<std::mutex> g(ctx->mu);

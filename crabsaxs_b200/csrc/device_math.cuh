@@ -125,5 +125,19 @@ __device__ __forceinline__ bool mbar_spin(uint64_t* bar, unsigned phase, int bud
   return false;
 }
 
+// a / b with y = 1/b correctly rounded: Markstein's quotient (IBM J. Res. Dev.
+// 34, 1990), one step to bring q within an ulp and one that rounds it
+// correctly.  For a zero (whose sign may be lost) or in the range below, b within
+// 1e-100 .. 1e100 (equal to the division in 8.6e9 random quotients, half of them
+// at mantissa ends).
+__device__ __forceinline__ double div_by(double a, double b, double y) {
+  // biased exponent within 2^-480 .. 2^480, or a zero
+  const unsigned ex = ((unsigned)__double2hiint(a) >> 20 & 0x7ffu) - 543u;
+  if (ex > 960u && a != 0.0) return a / b;
+  double q = a * y;
+  q = fma(fma(-q, b, a), y, q);
+  return fma(fma(-q, b, a), y, q);
+}
+
 }  // namespace dev
 }  // namespace crab

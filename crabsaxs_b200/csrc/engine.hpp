@@ -430,6 +430,7 @@ void pair_plan_select(crab_ctx* ctx, PairPlan& P, int variant);
 // True when `variant` (Q*16 + jb) names a compiled FP32 pair kernel.
 bool pair_variant_known(int variant);
 double measure_fp32_peak(crab_ctx* ctx, double target_ms);
+void probe_quotients(crab_ctx* ctx, const double* a, const double* b, int64_t n, double* by, double* div);
 
 // Quadratic form Σ_ij X_i Y_j sinc(q r_ij) for per-type amplitude tables
 // X[t*nq+k], Y[t*nq+k] from partials.

@@ -27,6 +27,7 @@
 #include <numeric>
 #include <random>
 
+#include "device_math.cuh"
 #include "engine.hpp"
 #include "ops.hpp"
 
@@ -226,19 +227,6 @@ __device__ void project_simplex_dev(double* v, int K, double* sorted, int n2, in
   __syncthreads();
 }
 
-// a / b with y = 1/b correctly rounded: Markstein's quotient (IBM J. Res. Dev.
-// 34, 1990), one step to bring q within an ulp and one that rounds it
-// correctly.  For a zero or in the range below, b within 1e-100 .. 1e100 (equal
-// to the division in 8.6e9 random quotients, half of them at mantissa ends).
-__device__ __forceinline__ double div_by(double a, double b, double y) {
-  // biased exponent within 2^-480 .. 2^480, or a zero
-  const unsigned ex = ((unsigned)__double2hiint(a) >> 20 & 0x7ffu) - 543u;
-  if (ex > 960u && a != 0.0) return a / b;
-  double q = a * y;
-  q = fma(fma(-q, b, a), y, q);
-  return fma(fma(-q, b, a), y, q);
-}
-
 // The weight kernel's shared memory, in doubles: weights, gradients and
 // proposals, the sorted values and their running sums; per q the mixture, the
 // weighted residual, y, sigma, 1/sigma and 1/sigma²; two chunks of gradient
@@ -283,7 +271,7 @@ __device__ __forceinline__ void ew_gradient(const double* cv, int K, int nq, con
 #pragma unroll 2
     for (int k = k_first; k < K; k += k_step, c += k_step * nq, d += k_step) {
       const double a = r * *c;
-      *d = plain ? a / b : div_by(a, b, y);
+      *d = plain ? a / b : dev::div_by(a, b, y);
     }
   };
   double acc[kMaxK / kWT] = {0.0, 0.0};

@@ -1,3 +1,4 @@
+// Quotients by a reciprocal beside the division's own, for tests, and the
 // FP32 FMA throughput probe: the roofline denominator of the Debye pair
 // kernel (FP32-pipe bound).  Eight independent register-resident FFMA chains
 // per thread on every SM; FLOP counted as 2 per FMA.
@@ -5,10 +6,19 @@
 
 #include <algorithm>
 
+#include "device_math.cuh"
 #include "engine.hpp"
 
 namespace crab {
 namespace {
+__global__ void k_quotients(const double* __restrict__ a, const double* __restrict__ b, int64_t n,
+                            double* __restrict__ by, double* __restrict__ div) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  by[i] = dev::div_by(a[i], b[i], 1.0 / b[i]);
+  div[i] = a[i] / b[i];
+}
+
 constexpr int kIter = 4096;
 __global__ void k_ffma_peak(float* out, float m, float c, int outer) {
   float a[8];
@@ -53,6 +63,22 @@ double measure_fp32_peak(crab_ctx* ctx, double target_ms) {
   }
   ctx->launches += 5;
   return best;
+}
+
+// by[i] = dev::div_by(a[i], b[i], 1 / b[i]), div[i] = a[i] / b[i].
+void probe_quotients(crab_ctx* ctx, const double* a, const double* b, int64_t n, double* by, double* div) {
+  if (n == 0) return;
+  const size_t bytes = (size_t)n * sizeof(double);
+  auto* d = (double*)ctx->dev("probe.quotients", 4 * bytes);
+  cudaStream_t s = ctx->stream;
+  copy_h2d(ctx, d, a, bytes, s);
+  copy_h2d(ctx, d + n, b, bytes, s);
+  k_quotients<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(d, d + n, n, d + 2 * n, d + 3 * n);
+  CRAB_CUDA_CHECK(cudaGetLastError());
+  ctx->launches += 1;
+  copy_d2h(ctx, by, d + 2 * n, bytes, s);
+  copy_d2h(ctx, div, d + 3 * n, bytes, s);
+  CRAB_CUDA_CHECK(cudaStreamSynchronize(s));
 }
 
 }  // namespace crab

@@ -281,6 +281,9 @@ int crab_pair_plan_destroy(crab_pair_plan* plan);
 /* Measured FP32 FMA throughput of the device (TFLOP/s, FMA = 2 FLOP): a
  * register-resident FFMA loop on every SM for about `ms` milliseconds. */
 int crab_measure_fp32_peak(crab_ctx* ctx, double ms, double* tflops);
+/* Quotients as the ensemble's weight fit forms them, from the reciprocal of the
+ * divisor (by[i]), beside a[i] / b[i] (div[i]); 0 < b, host arrays. */
+int crab_probe_quotients(crab_ctx* ctx, const double* a, const double* b, int64_t n, double* by, double* div);
 /* Bytes copied host->device and device->host by this context since the last
  * crab_ctx_reset_stats. */
 int crab_ctx_transfer_stats(crab_ctx* ctx, int64_t* h2d_bytes, int64_t* d2h_bytes);
