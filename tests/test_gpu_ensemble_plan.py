@@ -95,3 +95,52 @@ def test_wait_that_runs_out_is_reported_by_every_ensemble_call(engine, variant):
     assert np.array_equal(calls[1]().weights, before[1]) and np.array_equal(calls[2](), before[2])
     plan.close()
     fresh.close()
+
+
+def _uneven(k, classes, rng, loose):
+    """Conformers of one atom to several tiles, of extents 4 to 120 Å, each with some of the classes."""
+    out = []
+    for c in range(k):
+        n = [1, 2, 127, 128, 129, 400][c % 6] + int(rng.integers(0, 3))
+        el = rng.integers(1, 15, size=n).astype(np.int8) if classes > 4 else rng.integers(1, 5, size=n).astype(np.int8)
+        group = np.where(el == 1, rng.integers(-1, 4, size=n), -1).astype(np.int8)
+        occ = np.ones(n)
+        if loose:
+            occ[rng.random(n) < 0.2] = 0.35
+            occ[rng.random(n) < 0.05] = 0.0
+        out.append(cs.Structure(rng.uniform(-1.0, 1.0, size=(n, 3)) * [2.0, 15.0, 60.0][c % 3], el, occ, group))
+    return out
+
+
+@pytest.mark.parametrize("k,classes,loose", [(1, 4, False), (6, 4, True), (7, 14, False), (48, 14, False),
+                                             (13, 14, True)])
+def test_histogram_of_many_structures(engine, k, classes, loose):
+    """The distance histogram of a whole ensemble (variant 16, chosen before the plan is made): every structure has its
+    own bins, rows are resident in groups of 96 MB (48 conformers of 17 classes: several), and a structure may lack
+    classes.  Against the FP64 path of each conformer, relative to its curve at q = 0 with positive amplitudes: bins of
+    at most 0.0075 / q_max leave 0.0075² / 36, FP32 distances 2^-24 of the reach."""
+    from crabsaxs_b200 import _native as N
+    from crabsaxs_b200.api import Engine
+
+    rng = np.random.default_rng(100 + k)
+    structures = _uneven(k, classes, rng, loose)
+    q = np.concatenate([[0.0], np.linspace(0.01, 0.5, 40)])
+    cand = np.array([[1.0, 0.0], [1.03, 0.8]])
+    hist = Engine(0)
+    hist.check(N.lib.crab_ctx_set_pair_variant(hist.handle, 16))
+    got = cs.ensemble_curves(structures, q, cs.SolventParams(), cand, engine=hist)
+    again = cs.ensemble_curves(structures, q, cs.SolventParams(), cand, engine=hist)
+    rec = cs.ensemble_curves(structures, q, cs.SolventParams(), cand, engine=engine)
+    assert np.array_equal(got, again)
+    for c, s in enumerate(structures):
+        reach = 2.0 * np.sqrt(((s.xyz - s.xyz.mean(axis=0)) ** 2).sum(axis=1).max()) + 1e-3
+        tol = 0.0075 ** 2 / 36.0 + 0.44 * 0.5 * 2.0 ** -24 * reach * (2 * np.sqrt(3.0) + 3.0) + 1e-12
+        b = cs.debye_solvent_basis(s, q, cs.SolventParams(), True, engine=engine, fp64=True)
+        top = cs.debye_solvent_basis(s, [0.0], cs.SolventParams(), True, engine=engine, fp64=True)[:, 0]
+        for i, (c1, c2) in enumerate(cand):
+            ref = cs.combine_solvent_basis(b, q, c1, c2)
+            parts = [1.0, 1.3, c2 * c2, 2.3, 2.3 * c2, 2.3 * c2]
+            scale = max(float(np.abs(top) @ parts), 1e-9)
+            assert np.abs(got[i, c] - ref).max() / scale <= tol, (c, i)
+            assert np.abs(rec[i, c] - ref).max() / scale <= 168 * 2.0 ** -23 + tol, (c, i)
+    hist.close()
