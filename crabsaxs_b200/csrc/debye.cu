@@ -1504,6 +1504,18 @@ bool pair_plan_use(crab_ctx* ctx, PairPlan& P, int v, bool if_faster = false) {
   return P.hist.active || hist_plan_init(ctx, P, if_faster);
 }
 
+// The histogram where nobody asked for it: not where the device has no room for
+// its sums either.
+bool pair_plan_try_hist(crab_ctx* ctx, PairPlan& P, bool if_faster) {
+  try {
+    return pair_plan_use(ctx, P, kHistVariant, if_faster);
+  } catch (const Error& e) {
+    if (e.code != CRAB_ENOMEM) throw;
+    cudaGetLastError();  // of the allocation: not the next launch's
+    return false;
+  }
+}
+
 // The FP32 form of a new plan: the context's variant if one is set, else the
 // distance histogram where it pays (hist_plan_init), else the recurrence, which
 // has no bins to hold: where q_max times the largest distance is over 168 the
@@ -1511,7 +1523,8 @@ bool pair_plan_use(crab_ctx* ctx, PairPlan& P, int v, bool if_faster = false) {
 void configure_auto(crab_ctx* ctx, PairPlan& P) {
   const int2 v = default_variant(P.q);
   const int set = ctx->pair_variant;
-  if (!pair_plan_use(ctx, P, set ? set : kHistVariant, !set)) configure_fp32(ctx, P, v.x, v.y);
+  const bool done = set ? pair_plan_use(ctx, P, set) : pair_plan_try_hist(ctx, P, true);
+  if (!done) configure_fp32(ctx, P, v.x, v.y);
 }
 
 std::unique_ptr<PairPlan> make_pair_plan(crab_ctx* ctx, Layout&& L, const double* q, int64_t nq, bool fp64,
@@ -1880,11 +1893,19 @@ int pair_plan_autotune(crab_ctx* ctx, PairPlan& P, int* variants, double* ms_out
                                      {84, kSplit3}, {100, kSplit3}};
   int bestQ = 0, bestJ = 0, n = 0;
   float best_ms = -1.0f;
-  cudaEvent_t a, b;
+  cudaEvent_t a = nullptr, b = nullptr;
+  struct Guard {
+    cudaEvent_t &a, &b;
+    ~Guard() {
+      if (a) cudaEventDestroy(a);
+      if (b) cudaEventDestroy(b);
+    }
+  } guard{a, b};
   CRAB_CUDA_CHECK(cudaEventCreate(&a));
   CRAB_CUDA_CHECK(cudaEventCreate(&b));
   for (const auto& v : kVariants) {
-    if (!pair_plan_use(ctx, P, v[0] * 16 + v[1])) continue;
+    const int code = v[0] * 16 + v[1];
+    if (!(code == kHistVariant ? pair_plan_try_hist(ctx, P, false) : pair_plan_use(ctx, P, code))) continue;
     pair_plan_launch(ctx, P, ctx->stream, false);  // warm-up
     CRAB_CUDA_CHECK(cudaEventRecord(a, ctx->stream));
     pair_plan_launch(ctx, P, ctx->stream, false);
@@ -1903,8 +1924,6 @@ int pair_plan_autotune(crab_ctx* ctx, PairPlan& P, int* variants, double* ms_out
       bestJ = v[1];
     }
   }
-  cudaEventDestroy(a);
-  cudaEventDestroy(b);
   pair_plan_use(ctx, P, bestQ * 16 + bestJ);
   CRAB_CUDA_CHECK(cudaStreamSynchronize(ctx->stream));
   if (n_out) *n_out = std::min(n, capacity);

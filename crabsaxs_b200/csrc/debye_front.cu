@@ -362,8 +362,13 @@ bool debye_terms_device(crab_ctx* ctx, const crab_struct* st, const double* q, i
   P.n_pairs = T * (T + 1) / 2;
   P.skip_last = grid;
   cudaStream_t s = ctx->stream;
-  const bool pairs = hist_build(ctx, P, X, nullptr, nullptr);
-  if (!pairs) return false;
+  try {
+    if (!hist_build(ctx, P, X, nullptr, nullptr)) return false;
+  } catch (const Error& e) {  // no room on the device for its sums: the general path has less to hold
+    if (e.code != CRAB_ENOMEM) throw;
+    cudaGetLastError();
+    return false;
+  }
   HistPart& H = P.hist;
   const int terms = solvent ? 6 : 1;
   P.d_out = (double*)ctx->dev("pair.out", (size_t)P.n_pairs * nq * sizeof(double));

@@ -1180,11 +1180,11 @@ int crab_ensemble_plan_create(crab_ctx* ctx, crab_struct* const* structures, int
 int crab_ensemble_plan_autotune(crab_ctx* ctx, crab_ensemble_plan* plan, int32_t* chosen) {
   if (!ctx || !plan) return CRAB_EINVAL;
   return guarded_impl(ctx, [&]() {
-    const int c = pair_plan_autotune(ctx, *plan->plan->pair, nullptr, nullptr, 0, nullptr);
-    if (plan->plan->graph) {
+    if (plan->plan->graph) {  // first: the tuner frees tables that it holds, also where it fails later
       cudaGraphExecDestroy(plan->plan->graph);
       plan->plan->graph = nullptr;
     }
+    const int c = pair_plan_autotune(ctx, *plan->plan->pair, nullptr, nullptr, 0, nullptr);
     if (chosen) *chosen = c;
   });
 }

@@ -339,3 +339,72 @@ def test_sums_that_would_not_fit_the_device(engine):
     got, _ = cs.debye_partials(xyz, w, t, T, q, engine=engine)
     ref, _ = cs.debye_partials(xyz, w, t, T, q, engine=engine, fp64=True)
     assert np.abs(got - ref).max() <= 9.0 * 1e-4 and np.isfinite(got).all()  # nine pairs a row, FP32 phases q r
+
+
+def test_no_room_for_the_histogram_falls_back(engine):
+    """The histogram was not asked for: where its buffers cannot be had the recurrence serves, with those it has."""
+    from crabsaxs_b200.api import Engine
+
+    rng = np.random.default_rng(4)
+    n, T, q = 3000, 4, np.linspace(0.005, 0.5, 200)
+    xyz, t, w = rng.uniform(-15.0, 15.0, size=(n, 3)), rng.integers(0, T, size=n), np.ones(n)
+    ref, launches = _launches(engine, lambda: cs.debye_partials(xyz, w, t, T, q, engine=engine)[0])
+    assert launches > 1  # the histogram, where there is room
+    fresh = Engine(0)
+    fresh.check(N.lib.crab_ctx_set_pair_variant(fresh.handle, 100 * 16 + 7))
+    rec = cs.debye_partials(xyz, w, t, T, q, engine=fresh)[0]
+    fresh.check(N.lib.crab_ctx_set_pair_variant(fresh.handle, 0))
+    fresh.fail_allocations(0)
+    got, launches = _launches(fresh, lambda: cs.debye_partials(xyz, w, t, T, q, engine=fresh)[0])
+    fresh.fail_allocations(None)
+    assert launches == 1 and np.array_equal(got, rec)
+    got, launches = _launches(fresh, lambda: cs.debye_partials(xyz, w, t, T, q, engine=fresh)[0])
+    assert launches > 1 and np.array_equal(got, ref)
+    fresh.close()
+
+
+def test_autotune_that_fails_leaves_a_plan_that_works():
+    from crabsaxs_b200.api import Engine, Other
+
+    rng = np.random.default_rng(6)
+    fresh = Engine(0)
+    structures = [cs.Structure(rng.uniform(-9.0, 9.0, size=(150, 3)), np.full(150, 1, dtype=np.int8)) for _ in range(4)]
+    q, cand = np.linspace(0.01, 0.5, 60), np.array([[1.0, 0.5]])
+    c = cs.ensemble_curves(structures, q, cs.SolventParams(), cand, engine=fresh)[0]
+    y, sigma = c.mean(axis=0) * 1.1 + 3.0, 0.02 * c.mean(axis=0) + 1.0
+    plan = cs.EnsemblePlan(structures, q, candidates=cand, engine=fresh)
+    want = plan.score(y, sigma)
+    for after in (0, 1, 3, 6, 9):
+        fresh.fail_allocations(after)
+        with pytest.raises(Other, match="ENOMEM"):
+            plan.autotune()
+        fresh.fail_allocations(None)
+        plan.autotune()
+        got = plan.score(y, sigma)
+        assert np.abs(got["kl_weights"] - want["kl_weights"]).max() <= 1e-3
+        assert got["kl_reduced_chi2"] == pytest.approx(want["kl_reduced_chi2"], rel=1e-3)
+    plan.close()
+    fresh.close()
+
+
+def test_no_room_for_a_structure_call_falls_back(engine):
+    """As above for a structure's own call, whose histogram comes after its other buffers."""
+    from crabsaxs_b200.api import Engine
+
+    rng = np.random.default_rng(8)
+    n, q = 900, np.linspace(0.005, 0.5, 150)
+    xyz, el = rng.uniform(-12.0, 12.0, size=(n, 3)), rng.integers(1, 6, size=n).astype(np.int8)
+    whole, odd = (cs.Structure(xyz, el, occ) for occ in (np.ones(n), np.where(rng.random(n) < 0.2, 0.4, 1.0)))
+    fresh = Engine(0)
+    fresh.check(N.lib.crab_ctx_set_pair_variant(fresh.handle, 150 * 16 + 6))
+    rec = cs.debye_intensity(odd, q, engine=fresh)
+    fresh.check(N.lib.crab_ctx_set_pair_variant(fresh.handle, 0))
+    ref = cs.debye_intensity(whole, q, engine=fresh)
+    fresh.fail_allocations(0)
+    got, launches = _launches(fresh, lambda: cs.debye_intensity(odd, q, engine=fresh))
+    assert launches == 1 and np.array_equal(got, rec)
+    assert np.array_equal(cs.debye_intensity(whole, q, engine=fresh), ref)
+    fresh.fail_allocations(None)
+    got, launches = _launches(fresh, lambda: cs.debye_intensity(odd, q, engine=fresh))
+    assert launches > 1 and np.array_equal(got, cs.debye_intensity(odd, q, engine=engine))
+    fresh.close()
