@@ -457,8 +457,11 @@ constexpr int kRwCluster = 8;
 constexpr int kRwHalvings = 14;  // step lengths of a line search
 namespace cg = cooperative_groups;
 
-// Threads of a CTA: about one per q, and a warp more for the K logarithms.
-inline int rw_threads(int nq) { return std::min(512, std::max(128, (nq + 31) / 32 * 32 + 64)); }
+// Threads of a CTA: about one per q, and a warp more for the K logarithms, or
+// one per curve.
+inline int rw_threads(int K, int nq) {
+  return std::min(512, std::max({128, (nq + 31) / 32 * 32 + 64, (K + 31) / 32 * 32}));
+}
 
 // Sums over the block of N values per thread (a fixed tree, then the warps in
 // order); the two halves of `red` alternate, as in BlockSums.
@@ -812,7 +815,7 @@ void launch_reweight(cudaStream_t s, size_t smem, const double* curves, const do
                      double* w_out, double* out) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(CL * SP);
-  cfg.blockDim = dim3(rw_threads(nq));
+  cfg.blockDim = dim3(rw_threads(K, nq));
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cudaLaunchAttribute at[1];
@@ -1024,8 +1027,16 @@ static size_t weights_smem(int K, int64_t nq) {
   return (ew_doubles(K, (int)nq) + (ew_on_chip(K, (int)nq) ? (size_t)K * nq : 0)) * sizeof(double);
 }
 
-// Cluster of the reweighting: one CTA while its shared memory holds the curves.
-static int rw_cluster(int K, int64_t nq) { return rw_on_chip(K, (int)nq, 1) ? 1 : kRwCluster; }
+// Cluster of the reweighting: one CTA (or eight that search step lengths) while
+// its shared memory holds the curves and the search's buffers, else eight that
+// split the curves (1,000 of 20 q, which alone would fit one CTA: 500 steps 14 ms,
+// 65 there), unless they are few (20 of 1,200 q: 12 ms, 10 there).
+static bool rw_search(int K, int64_t nq) {
+  return rw_smem(K, (int)nq, 1) + rw_search_doubles(K, (int)nq) * sizeof(double) <= kEnsSmem;
+}
+static int rw_cluster(int K, int64_t nq) {
+  return rw_on_chip(K, (int)nq, 1) && (K <= 32 || rw_search(K, nq)) ? 1 : kRwCluster;
+}
 
 static void ensemble_fit_buffers(EnsemblePlan& E, const double* y, const double* sg) {
   crab_ctx* ctx = E.ctx;
@@ -1068,9 +1079,8 @@ static void ensemble_launch_fit(EnsemblePlan& E, int Ksel, const EnsOpts& eo, co
     CRAB_CUDA_CHECK(cudaGetLastError());
     const int cl = rw_cluster(Ksel, E.nq);
     size_t shr = rw_smem(Ksel, (int)E.nq, cl);
-    const size_t more = rw_search_doubles(Ksel, (int)E.nq) * sizeof(double);
-    const bool search = cl == 1 && shr + more <= kEnsSmem;
-    if (search) shr += more;
+    const bool search = cl == 1 && rw_search(Ksel, E.nq);
+    if (search) shr += rw_search_doubles(Ksel, (int)E.nq) * sizeof(double);
     auto* go = cl > 1 ? launch_reweight<kRwCluster, 1> : search ? launch_reweight<1, kRwCluster> : launch_reweight<1, 1>;
     go(sm, shr, E.d_curves, E.d_fit, E.n_cand, Ksel, (int)E.nq, E.d_y, E.d_sg, E.d_weights, E.d_dcurves, *ro, E.d_wkl,
        E.d_out);

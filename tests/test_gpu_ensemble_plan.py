@@ -144,3 +144,28 @@ def test_histogram_of_many_structures(engine, k, classes, loose):
             assert np.abs(got[i, c] - ref).max() / scale <= tol, (c, i)
             assert np.abs(rec[i, c] - ref).max() / scale <= 168 * 2.0 ** -23 + tol, (c, i)
     hist.close()
+
+
+@pytest.mark.parametrize("k,nq", [(33, 800), (32, 800), (20, 1200), (50, 520), (1000, 20), (300, 40), (513, 9)])
+def test_forms_of_the_reweighting(engine, k, nq):
+    """One CTA, eight that search step lengths and eight that split the curves, about the lines between them and with
+    threads by the curves instead of the q: the outcome restated from the weights in f64 (1e-9, as the fit's test)."""
+    rng = np.random.default_rng(k + nq)
+    structures = [cs.Structure(rng.uniform(-6.0, 6.0, size=(9, 3)) * rng.uniform(0.6, 1.6),
+                               rng.choice([1, 2, 3], size=9).astype(np.int8)) for _ in range(k)]
+    q, cand = np.linspace(0.01, 0.5, nq), np.array([[1.0, 0.5]])
+    c = cs.ensemble_curves(structures, q, cs.SolventParams(), cand, engine=engine)[0]
+    y = 1.3 * (rng.dirichlet(np.full(k, 0.3)) @ c)
+    sigma = 0.02 * y + 1e-3 * y.max()
+    y = y + sigma * rng.normal(size=nq)
+    plan = cs.EnsemblePlan(structures, q, candidates=cand, engine=engine)
+    try:
+        r, again = plan.score(y, sigma), plan.score(y, sigma)
+    finally:
+        plan.close()
+    assert _equal(r, again)
+    v = r["kl_weights"]
+    assert v.min() > 0.0 and abs(v.sum() - 1.0) <= 1e-9
+    res = (r["kl_scale"] * (v @ c) + r["kl_background"] - y) / sigma
+    assert r["kl_reduced_chi2"] == pytest.approx((res ** 2).sum() / (nq - 1), rel=1e-9)
+    assert r["kl_divergence"] == pytest.approx((v * np.log(v * k)).sum(), abs=1e-9)
