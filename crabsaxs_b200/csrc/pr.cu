@@ -660,7 +660,6 @@ __global__ void __launch_bounds__(kPcT, 1)
   }
 }
 
-template <int kMode>
 struct PrAcc {
   double* w;
   __device__ __forceinline__ void add(int e, double wij) const { atomicAdd(&w[e], wij); }
@@ -692,7 +691,7 @@ __global__ void __launch_bounds__(kPrThreads, 8)
     for (int k = threadIdx.x; k <= bins; k += kPrThreads) pr_dyn[k] = edges[k];
     for (int k = threadIdx.x; k < copies * bins; k += kPrThreads) Hw[k] = 0.0;
   }
-  PrAcc<kMode> acc;
+  PrAcc acc;
   acc.w = kMode == kPrWeightedGlobal ? Hw : Hw + (size_t)(warp % copies) * bins;
   const int top = kPrMagicBits + bins - 1;  // floor(x) capped at bins - 1, in magic bits
   const int64_t n_work = (int64_t)n_tiles * (n_tiles + 1) / 2;

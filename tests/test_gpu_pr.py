@@ -286,3 +286,23 @@ def test_few_pairs_and_many_bins(engine, n, k, bins):
     assert _mode(engine) == 0
     rd, rh = O.pair_distance_histogram(xyz, w, bins)
     assert d == rd and np.array_equal(h, rh)
+
+
+@pytest.mark.parametrize("weighted", [False, True])
+@pytest.mark.parametrize("shape", ["sphere", "bent rod", "two clusters", "equal atoms"])
+def test_longest_pair_past_the_size_that_looks_at_every_pair(engine, shape, weighted):
+    """Above 4,096 atoms the longest pair is searched from one pair, a centre moved off its middle (with more than 64
+    weights the box's) and the atoms about the rim: shapes whose middle lies off the atoms, or whose atoms all lie on
+    the rim."""
+    rng = np.random.default_rng(18)
+    v = rng.normal(size=(5000, 3))
+    t = rng.uniform(0.0, 2.2, size=9000)
+    two = np.concatenate([rng.normal(size=(1600, 3)), rng.normal(size=(2800, 3)) + [90.0, 3.0, -8.0]])
+    xyz = {"sphere": 40.0 * v / np.sqrt((v ** 2).sum(axis=1))[:, None],
+           "bent rod": np.stack([60 * np.cos(t), 60 * np.sin(t), 0.0 * t], axis=1) + rng.normal(size=(9000, 3)),
+           "two clusters": two, "equal atoms": np.repeat(two[:5], 1000, axis=0)}[shape]
+    w = 1.0 + (np.arange(len(xyz)) % 100 if weighted else np.zeros(len(xyz)))
+    d, h = cs.pair_distance_histogram(xyz, w, 50, engine=engine)
+    assert _mode(engine) == (1 if weighted else 0)
+    rd, rh = O.pair_distance_histogram(xyz, w, 50)
+    assert d == rd and np.array_equal(h, rh)
