@@ -255,7 +255,7 @@ bool debye_terms_device(crab_ctx* ctx, const crab_struct* st, const double* q, i
   // the sites lie within a shell of 16 Å at most around the atoms; refused here
   // rather than after the grid is built
   if (!hist_structure_bins(2.0 * (rmax + (grid ? 16.0 : 0.0)), qmax, &X.bins[0], &X.inv_h[0])) return false;
-  if (!front_pays(X, T, grid, solvent, qs, n)) return false;
+  if (X.bins[0] > kHistMinBins && !front_pays(X, T, grid, solvent, qs, n)) return false;
   auto* hx = (double*)ctx->host("front.xyz", (size_t)n * 3 * sizeof(double));
   std::memcpy(hx, x, (size_t)n * 3 * sizeof(double));
   auto* d_xyz = (double*)ctx->dev("front.xyz", (size_t)n * 3 * sizeof(double));

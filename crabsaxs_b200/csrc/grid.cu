@@ -596,8 +596,8 @@ T* pool(crab_ctx* ctx, const char* name, size_t count) {
 }
 
 void trim_slots(crab_ctx* ctx, bool keep_sites) {
-  for (auto it = ctx->bufs.begin(); it != ctx->bufs.end();) {
-    if (it->first.compare(0, 5, "grid.") == 0 && it->second.bytes > kGridKeepBytes &&
+  for (auto it = ctx->bufs.lower_bound("grid."); it != ctx->bufs.end() && it->first.compare(0, 5, "grid.") == 0;) {
+    if (it->second.bytes > kGridKeepBytes &&
         !(keep_sites && (it->first == "grid.sites" || it->first == "grid.cells"))) {
       cudaFree(it->second.ptr);
       it = ctx->bufs.erase(it);
