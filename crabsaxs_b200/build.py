@@ -44,8 +44,8 @@ def _compile(src: Path, verbose: bool) -> Path:
     else:
         # aligned, so that a change elsewhere in a file does not move the fit's inner loops off their
         # fetch blocks (1,481 atoms, 612 q: 2 to 3 % of a call)
-        cmd = ["g++", "-O3", "-falign-functions=64", "-falign-loops=32", "-std=c++17", "-fPIC", "-ffp-contract=off", "-I/usr/local/cuda/include", f"-I{INCLUDE}",
-               f"-I{CSRC}", "-c", str(src), "-o", str(obj)]
+        cmd = ["g++", "-O3", "-falign-functions=64", "-falign-loops=32", "-std=c++17", "-fPIC", "-ffp-contract=off",
+               "-I/usr/local/cuda/include", f"-I{INCLUDE}", f"-I{CSRC}", "-c", str(src), "-o", str(obj)]
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:
         raise RuntimeError(f"nvcc failed for {src.name}:\n{res.stdout}\n{res.stderr}")

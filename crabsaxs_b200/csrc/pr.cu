@@ -800,7 +800,9 @@ __global__ void k_pr_reduce(const double* __restrict__ rows, int n_rows, int bin
 
 template <int kMode>
 int pr_blocks_per_sm(size_t dyn) {
-  if (dyn) CRAB_CUDA_CHECK(cudaFuncSetAttribute(k_pr_hist<kMode>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
+  // of the function, whatever context sets it: always the same value
+  if (dyn)
+    CRAB_CUDA_CHECK(cudaFuncSetAttribute(k_pr_hist<kMode>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPrDynSmem));
   int per_sm = 0;
   CRAB_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pr_hist<kMode>, kPrThreads, dyn));
   return std::max(per_sm, 1);
