@@ -1,7 +1,8 @@
 // Debye pair sums per atom-type pair on B200 (sm_100a): plans, and the kernels
 // that sum every pair at every q.  One-structure plans use the distance
-// histogram of debye_hist.cu where its bins fit; the recurrence kernels here
-// serve ensemble plans, wider ranges and the variants a caller selects.
+// histogram of debye_hist.cu where it fits and takes less; the recurrence
+// kernels here serve ensemble plans, few q, many small types, wider ranges and
+// the variants a caller selects.
 //
 // Replaces the O(N²·Nq) pair loops of crabSAXS src/scattering.rs:99-106 and
 // src/solvent.rs:533-577.  Instead of summing amplitude products per q, the

@@ -39,8 +39,8 @@
 // lie; the counters of a bin are 32 words, one a lane (4 with over 1,500 bins),
 // so that neighbouring atoms, whose distances to one j atom fall into the same
 // bins, never meet in a word.
-// 100,000 atoms, 160 bins: 5.0e9 pairs in 3.3 ms (1.5e12 a second, issue slots
-// 82 % busy, 17 instructions a pair), where one i atom a thread, a copy of the
+// 100,000 atoms, 160 bins: 5.0e9 pairs in 2.94 ms (1.70e12 a second, issue slots
+// 79 % busy, 17 instructions a pair), where one i atom a thread, a copy of the
 // counters per warp and a branch around each near-edge pair took 5.4 ms (23
 // instructions a pair).  The call went from 10.3 to 3.6 ms: dmax takes 0.1 ms
 // (0.9 ms over spatially ordered tiles), the order itself and the packing of the

@@ -201,10 +201,12 @@ int crab_combine_solvent_basis(const double* q, int64_t nq, const double* basis6
  *   out[ab*nq+k] = Σ_{i<j,{t_i,t_j}={a,b}} w_i w_j sinc(q_k r_ij), a<=b,
  *   ab = a*T - a*(a-1)/2 + (b-a);  self_out[a] = Σ_{t_i=a} w_i².
  * xyz n*3 f64, w n f64, type n in [0,T). Distances are FP32 on the device;
- * the sums are integer counts per distance bin met by f64 sines (the default),
- * or FP32 with FP64 cross-block reduction exact on a power-of-two fixed-point
- * grid (step about 2^-52 of q_max (Σ|w|)²), so the result is bit-identical from
- * call to call on the same inputs and kernel variant. */
+ * the sums are integer counts per distance bin met by f64 sines where the library
+ * estimates that to be the faster form (many q, or many atoms a type) and the
+ * device has room, else FP32 with FP64 cross-block reduction exact on a
+ * power-of-two fixed-point grid (step about 2^-52 of q_max (Σ|w|)²), so the
+ * result is bit-identical from call to call on the same inputs and kernel
+ * variant. */
 int crab_debye_partials(crab_ctx* ctx, const double* xyz, const double* w, const int32_t* type, int64_t n,
                         int32_t n_types, const double* q, int64_t nq, double* out, double* self_out);
 /* Same partials computed in FP64 on the device with direct sin (no
@@ -247,7 +249,7 @@ int crab_pair_plan_create_lattice_shard(crab_ctx* ctx, const double* xyz, const 
 int crab_pair_plan_run(crab_ctx* ctx, crab_pair_plan* plan, int32_t repeats, int64_t flush_bytes, double* step_ms);
 /* Autotune: time every compiled kernel variant on this plan: 16, the distance
  * histogram (every pair deposited once, the bins met by the q grid; skipped
- * where its bins exceed an SM's shared memory), and Q*16 + JB (q-block length Q
+ * where its bins exceed an SM's shared memory or its sums the device's), and Q*16 + JB (q-block length Q
  * = q values one thread advances per pair between exact re-seeds, and JB = j
  * atoms per thread iteration; JB >= 8 selects the q-packed kernel, whose f32x2
  * registers hold two consecutive q points, with (JB-8) % 4 independent chains,
@@ -270,7 +272,9 @@ int crab_pair_plan_autotune(crab_ctx* ctx, crab_pair_plan* plan, int32_t* chosen
  * crab_pair_plan_autotune reports it, or 0 for the automatic choice. */
 int crab_ctx_set_pair_variant(crab_ctx* ctx, int32_t variant);
 /* Fix the kernel variant of an FP32 plan (a code as crab_pair_plan_autotune
- * reports it); CRAB_EINVAL for a variant that is not compiled. */
+ * reports it); CRAB_EINVAL for a variant that is not compiled, or for the
+ * histogram (16) where it does not fit: bins beyond an SM's shared memory, sums
+ * beyond 8 GB, values without an FP32 distance. */
 int crab_pair_plan_select(crab_ctx* ctx, crab_pair_plan* plan, int32_t variant);
 /* Copy the partials of the last run to the host (layout of crab_debye_partials). */
 int crab_pair_plan_read(crab_ctx* ctx, crab_pair_plan* plan, double* out, double* self_out);
