@@ -69,11 +69,12 @@ constexpr double kHistStep = 0.005;           // q_max h aimed at
 constexpr double kHistMaxStep = 0.0075;       // beyond it (q_max x extent > 168) the recurrence kernels run
 constexpr double kHistMaxReach = 1e18;        // squares of distances below FP32's largest number
 constexpr int64_t kHistMaxBytes = (int64_t)8 << 30;  // sums of a plan in device memory
-constexpr int kHistFlush = 256;               // units between flushes: 2^21 pairs, |Σu| 2^11 < 2^31 in one bin
+constexpr int kHistFlush = 224;               // units between flushes: less than 2^21 pairs, |Σu| 2^11 < 2^31 in one bin
 constexpr int kHistStagingBytes = kHWarps * 2 * kChunkBytes;
 constexpr int kHistBarBytes = kHWarps * 2 * 8;
 constexpr int kHistSumOffset = kHistMaxBins * 4;  // Σu words after the counts
-static_assert((long long)kHistFlush * 128 * kChunkAtoms <= (1ll << 21), "Σu of one bin must stay below 2^31");
+static_assert((long long)kHistFlush * 128 * kChunkAtoms < (1ll << 21), "Σu of one bin must stay below 2^31");
+static_assert(kHistFlush % kHWarps == 0, "the warps of a CTA take equal shares");
 constexpr float kMagicBin = 12582912.0f;      // 1.5 x 2^23: adding it rounds to an integer in the low bits
 constexpr unsigned kMagicBinBits = 0x4B400000u;
 constexpr float kMagicU = 6144.0f;            // 1.5 x 2^12: low bits in units of 2^-11

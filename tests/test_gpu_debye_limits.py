@@ -408,3 +408,19 @@ def test_no_room_for_a_structure_call_falls_back(engine):
     got, launches = _launches(fresh, lambda: cs.debye_intensity(odd, q, engine=fresh))
     assert launches > 1 and np.array_equal(got, cs.debye_intensity(odd, q, engine=engine))
     fresh.close()
+
+
+def test_offsets_of_one_bin_at_their_largest(hist_engine):
+    """Two clusters of 18,000 coincident atoms 4,088.4999 bins apart: every pair between them adds the largest positive
+    offset to one bin, and every CTA counts whole runs of such pairs between two flushes.  Against sinc itself; the
+    tolerance is that of the histogram's tile edges (4,096 bins over the reach)."""
+    n, d = 18000, 1.32246
+    xyz = np.zeros((2 * n, 3))
+    xyz[0::2, 0], xyz[1::2, 0] = -d / 2, d / 2
+    t = np.arange(2 * n) % 2
+    q = np.linspace(0.5, 12.0, 24)
+    got, _ = cs.debye_partials(xyz, np.ones(2 * n), t, 2, q, engine=hist_engine)
+    sinc = np.sinc(q * d / np.pi)
+    tol = (12.0 * d / 4000.0) ** 2 / 36.0 + 0.44 * 12.0 * 2.0 ** -24 * d * (2 * np.sqrt(3.0) + 3.0) + 1e-12
+    assert np.abs(got[1] / n ** 2 - sinc).max() <= tol
+    assert np.abs(got[0] / (0.5 * n * (n - 1)) - 1.0).max() <= tol
