@@ -1783,6 +1783,7 @@ void compute_partials(crab_ctx* ctx, Layout&& L, const double* q, int64_t nq, bo
   out.nq = nq;
   out.self = L.self_w2;
   if (shard != 0) std::fill(out.self.begin(), out.self.end(), 0.0);
+  HistPoolRelease release{ctx};
   std::unique_ptr<PairPlan> P;
   {
     TraceScope tp("make_pair_plan");

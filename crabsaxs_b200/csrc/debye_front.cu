@@ -350,6 +350,7 @@ bool debye_terms_device(crab_ctx* ctx, const crab_struct* st, const double* q, i
   std::memcpy(X.more.data() + o_sums + (size_t)T * sizeof(double), sw.data(), (size_t)T * sizeof(double));
   std::memcpy(X.more.data() + o_tile, tile0.data(), tile0.size() * sizeof(int));
 
+  HistPoolRelease hist_release{ctx};
   PairPlan P;
   P.pooled = true;
   P.shard = shard;

@@ -69,6 +69,7 @@ constexpr double kHistStep = 0.005;           // q_max h aimed at
 constexpr double kHistMaxStep = 0.0075;       // beyond it (q_max x extent > 168) the recurrence kernels run
 constexpr double kHistMaxReach = 1e18;        // squares of distances below FP32's largest number
 constexpr int64_t kHistMaxBytes = (int64_t)8 << 30;  // sums of a plan in device memory
+constexpr size_t kHistKeepBytes = (size_t)256 << 20;     // of a slot of one-shot calls, kept between them
 constexpr int kHistFlush = 224;               // units between flushes: less than 2^21 pairs, |Σu| 2^11 < 2^31 in one bin
 constexpr int kHistStagingBytes = kHWarps * 2 * kChunkBytes;
 constexpr int kHistBarBytes = kHWarps * 2 * 8;
@@ -872,6 +873,20 @@ bool hist_build(crab_ctx* ctx, PairPlan& P, HistShape& X, const std::vector<unsi
   if (!P.d_q) P.d_q = (double*)(d + o_q);
   undo.on = false;
   return true;
+}
+
+// The sums of a one-shot call reach 8 GB (hundreds of types with odd weights),
+// which its context would keep for good; such a call takes 10 ms and more, a new
+// allocation about one.
+HistPoolRelease::~HistPoolRelease() {
+  for (auto it = ctx->bufs.lower_bound("pair.hist"); it != ctx->bufs.end() && it->first.compare(0, 9, "pair.hist") == 0;) {
+    if (it->second.bytes > kHistKeepBytes) {
+      cudaFree(it->second.ptr);
+      it = ctx->bufs.erase(it);
+    } else {
+      ++it;
+    }
+  }
 }
 
 void hist_plan_launch(crab_ctx* ctx, PairPlan& P, cudaStream_t s) {

@@ -395,6 +395,11 @@ bool hist_structure_bins(double reach, double qmax, int* bins, float* inv_h);
 bool hist_build(crab_ctx* ctx, PairPlan& P, HistShape& X, const std::vector<unsigned char>* pts,
                 const std::vector<double>* weight);
 void hist_plan_launch(crab_ctx* ctx, PairPlan& P, cudaStream_t s);
+// Releases the "pair.hist" slots of one-shot calls above kHistKeepBytes, at the end of a scope.
+struct HistPoolRelease {
+  crab_ctx* ctx;
+  ~HistPoolRelease();
+};
 void lattice_plan_init(crab_ctx* ctx, PairPlan& P, const int32_t* cells, int64_t m, double spacing);
 // The same with the cells (3 int32 each) on the device, every coordinate's span at most `span` cells.
 void lattice_plan_init_device(crab_ctx* ctx, PairPlan& P, const int32_t* d_cells, int64_t m, double spacing,

@@ -424,3 +424,25 @@ def test_offsets_of_one_bin_at_their_largest(hist_engine):
     tol = (12.0 * d / 4000.0) ** 2 / 36.0 + 0.44 * 12.0 * 2.0 ** -24 * d * (2 * np.sqrt(3.0) + 3.0) + 1e-12
     assert np.abs(got[1] / n ** 2 - sinc).max() <= tol
     assert np.abs(got[0] / (0.5 * n * (n - 1)) - 1.0).max() <= tol
+
+
+def test_large_sums_are_given_back():
+    """140 types with weights of their own at 12,000 bins: 3.8 GB of sums, which a one-shot call does not leave behind;
+    the next calls are the same to the bit."""
+    from crabsaxs_b200.api import Engine
+
+    rng = np.random.default_rng(12)
+    n, T = 3000, 140
+    xyz, t = _mirrored(n, 119.0, rng), np.arange(n) % T
+    w, q = rng.uniform(0.2, 1.0, size=n), np.linspace(0.1, 0.5, 8)
+    fresh = Engine(0)
+    fresh.check(N.lib.crab_ctx_set_pair_variant(fresh.handle, HIST))
+    (got, _), launches = _launches(fresh, lambda: cs.debye_partials(xyz, w, t, T, q, engine=fresh))
+    assert launches > 1
+    held = C.c_int64()
+    fresh.check(N.lib.crab_ctx_workspace_bytes(fresh.handle, C.byref(held)))
+    assert held.value < 1 << 29
+    assert np.array_equal(cs.debye_partials(xyz, w, t, T, q, engine=fresh)[0], got)
+    ref, _ = cs.debye_partials(xyz, w, t, T, q, engine=fresh, fp64=True)
+    assert np.abs(got - ref).max() <= 22.0 ** 2 * _tol(q, 119.0)
+    fresh.close()
