@@ -261,7 +261,7 @@ bool debye_terms_device(crab_ctx* ctx, const crab_struct* st, const double* q, i
   auto* d_xyz = (double*)ctx->dev("front.xyz", (size_t)n * 3 * sizeof(double));
   copy_h2d(ctx, d_xyz, hx, (size_t)n * 3 * sizeof(double), ctx->stream);
   GridResult g;
-  GridPoolRelease grid_release{ctx};
+  GridPoolRelease grid_release{ctx, grid};
   if (grid) {
     TraceScope tg("hydration_sites");
     g = solvent->hydration_model == CRAB_HYD_ADAPTIVE

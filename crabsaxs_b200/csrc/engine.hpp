@@ -491,9 +491,14 @@ GridResult exterior_grid_device(crab_ctx* ctx, const double* xyz, const int8_t* 
 // Releases "grid." device slots above the keep size (after a caller has read
 // the sites and cells of a build made without to_host).
 void trim_grid_pool(crab_ctx* ctx);
-struct GridPoolRelease {  // the same at the end of a scope, also on an error
+// The same at the end of a scope, also on an error, of a call that builds a grid
+// (one that does not leaves alone the sites that a size query may have left).
+struct GridPoolRelease {
   crab_ctx* ctx;
-  ~GridPoolRelease() { trim_grid_pool(ctx); }
+  bool builds;
+  ~GridPoolRelease() {
+    if (builds) trim_grid_pool(ctx);
+  }
 };
 
 }  // namespace crab

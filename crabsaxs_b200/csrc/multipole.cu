@@ -2408,7 +2408,7 @@ void multipole_solvent_basis_impl(crab_ctx* ctx, const crab_struct* st, const do
     return;
   }
   MpSolventSetup u;
-  GridPoolRelease grid_release{ctx};
+  GridPoolRelease grid_release{ctx, s.hydration_model != CRAB_HYD_ANALYTIC};
   solvent_setup(ctx, st, q, nq, s, implicit, shard.n_shards == 1, u);
   MpInput in;
   u.into(in);
@@ -2435,7 +2435,7 @@ void multipole_solvent_intensity_impl(crab_ctx* ctx, const crab_struct* st, cons
     return;
   }
   MpSolventSetup u;
-  GridPoolRelease grid_release{ctx};
+  GridPoolRelease grid_release{ctx, s.hydration_model != CRAB_HYD_ANALYTIC};
   solvent_setup(ctx, st, q, nq, s, implicit, true, u);
   MpInput in;
   u.into(in);

@@ -446,3 +446,28 @@ def test_large_sums_are_given_back():
     ref, _ = cs.debye_partials(xyz, w, t, T, q, engine=fresh, fp64=True)
     assert np.abs(got - ref).max() <= 22.0 ** 2 * _tol(q, 119.0)
     fresh.close()
+
+
+def test_sites_of_a_size_query_outlive_calls_without_a_grid(engine):
+    """A size query leaves its sites on the device (12 million, above the kept slots) for the fill call that follows;
+    calls in between that build no grid leave them alone, one that builds a grid makes the fill call build again."""
+    one = cs.Structure(np.array([[1.0, 2.0, 3.0]]), np.array([1], dtype=np.int8))
+    other = cs.Structure(np.random.default_rng(0).uniform(-9.0, 9.0, size=(300, 3)), np.full(300, 2, dtype=np.int8))
+    args = (1.0, 1.4, 142.0)
+    want, _ = cs.hydration_grid_exterior(one, *args, engine=engine)
+    assert len(want) * 24 > 1 << 28
+    q = np.linspace(0.01, 0.4, 40)
+    plain, grid = cs.SolventParams(), cs.SolventParams(hydration_model=cs.HydrationModel.AdaptiveGrid)
+    between = [lambda: None, lambda: cs.debye_solvent_basis(other, q, plain, engine=engine),
+               lambda: cs.debye_intensity(other, q, engine=engine),
+               lambda: cs.multipole_solvent_basis(other, q, 12, plain, engine=engine),
+               lambda: cs.debye_solvent_basis(other, q, grid, engine=engine)]
+    h = one.handle(engine)
+    for call in between:
+        m, vol = C.c_int64(), C.c_double()
+        engine.check(N.lib.crab_hydration_grid_exterior(engine.handle, h, *args, None, 0, C.byref(m), C.byref(vol)))
+        call()
+        got = np.empty((m.value, 3))
+        engine.check(N.lib.crab_hydration_grid_exterior(engine.handle, h, *args, got.ctypes.data_as(N.D), m.value,
+                                                        C.byref(m), C.byref(vol)))
+        assert np.array_equal(got, want)
