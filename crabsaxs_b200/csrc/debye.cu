@@ -1506,12 +1506,13 @@ bool pair_plan_use(crab_ctx* ctx, PairPlan& P, int v, bool if_faster = false) {
 }
 
 // The histogram where nobody asked for it: not where the device has no room for
-// its sums either.
+// its sums either, unless other devices hold the other shards, which split the
+// pairs another way by recurrence.
 bool pair_plan_try_hist(crab_ctx* ctx, PairPlan& P, bool if_faster) {
   try {
     return pair_plan_use(ctx, P, kHistVariant, if_faster);
   } catch (const Error& e) {
-    if (e.code != CRAB_ENOMEM) throw;
+    if (e.code != CRAB_ENOMEM || P.n_shards > 1) throw;
     cudaGetLastError();  // of the allocation: not the next launch's
     return false;
   }

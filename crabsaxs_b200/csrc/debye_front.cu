@@ -366,7 +366,7 @@ bool debye_terms_device(crab_ctx* ctx, const crab_struct* st, const double* q, i
   try {
     if (!hist_build(ctx, P, X, nullptr, nullptr)) return false;
   } catch (const Error& e) {  // no room on the device for its sums: the general path has less to hold
-    if (e.code != CRAB_ENOMEM) throw;
+    if (e.code != CRAB_ENOMEM || n_shards > 1) throw;  // every shard takes the same path
     cudaGetLastError();
     return false;
   }

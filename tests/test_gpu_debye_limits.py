@@ -471,3 +471,28 @@ def test_sites_of_a_size_query_outlive_calls_without_a_grid(engine):
         engine.check(N.lib.crab_hydration_grid_exterior(engine.handle, h, *args, got.ctypes.data_as(N.D), m.value,
                                                         C.byref(m), C.byref(vol)))
         assert np.array_equal(got, want)
+
+
+def test_a_shard_without_room_does_not_fall_back():
+    """Shards split the pairs of the two kernels differently: one that falls back alone would leave the sum wrong."""
+    from crabsaxs_b200.api import Engine, Other
+
+    rng = np.random.default_rng(14)
+    n, T, q = 3000, 4, np.linspace(0.005, 0.5, 200)
+    xyz, t, w = rng.uniform(-15.0, 15.0, size=(n, 3)), rng.integers(0, T, size=n), np.ones(n)
+    el = rng.integers(1, 6, size=n).astype(np.int8)
+    whole, odd = (cs.Structure(xyz, el, occ) for occ in (w, np.where(rng.random(n) < 0.2, 0.4, 1.0)))
+    fresh = Engine(0)
+    fresh.check(N.lib.crab_ctx_set_pair_variant(fresh.handle, 100 * 16 + 7))
+    cs.debye_partials(xyz, w, t, T, q, engine=fresh, shard=(0, 2))  # the recurrence's buffers
+    cs.debye_solvent_basis(odd, q, cs.SolventParams(), engine=fresh, shard=(0, 2))
+    fresh.check(N.lib.crab_ctx_set_pair_variant(fresh.handle, 0))
+    fresh.fail_allocations(0)
+    with pytest.raises(Other, match="ENOMEM"):
+        cs.debye_partials(xyz, w, t, T, q, engine=fresh, shard=(0, 2))
+    fresh.fail_allocations(None)
+    cs.debye_solvent_basis(whole, q, cs.SolventParams(), engine=fresh, shard=(0, 2))
+    fresh.fail_allocations(0)
+    with pytest.raises(Other, match="ENOMEM"):
+        cs.debye_solvent_basis(odd, q, cs.SolventParams(), engine=fresh, shard=(0, 2))
+    fresh.close()
